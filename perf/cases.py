@@ -46,7 +46,7 @@ def listed():
         # a plain dense product with alpha and beta, the reference's benchmark size
         _gemm("gemm 1024", 1024, 1024, 1024, alpha=1.5, beta=0.5),
         # A^T B on odd sizes with odd leading dimensions: sub-blocks of larger matrices
-        _gemm("gemm ragged transa", 1999, 1501, 2743, la="col", pad=1),
+        _gemm("gemm ragged transa", 1999, 1501, 2743, la="col", pad=2),
         # a medium product on the automatic route, column-major B
         _gemm("gemm auto 3000", 3000, 2304, 2600, lb="col", precision="auto"),
         # the headline product on the automatic route
