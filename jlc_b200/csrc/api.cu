@@ -1358,14 +1358,15 @@ int jlc_bidiag_device(jlc_ctx* ctx, int64_t m, int64_t n, double* a, int64_t lda
         // workspace: tau of the column and row reflectors, the kernel's
         // partials, and the row reflectors rearranged as a QR factor
         const long long ldw = n > 1 ? round_up(n - 1, 8) : 8;
+        const long long ldt = round_up(n, 8);
         const size_t kdoubles = bidiag_work_doubles((int)m, (int)n, ctx->sm_count);
         const size_t wdoubles = v ? (size_t)ldw * (size_t)(n > 1 ? n - 1 : 1) : 0;
-        if ((rc = reserve(ctx, ctx->bufH, (2 * (size_t)n + kdoubles + wdoubles) * sizeof(double),
+        if ((rc = reserve(ctx, ctx->bufH, (2 * (size_t)ldt + kdoubles + wdoubles) * sizeof(double),
                           "bidiagonalisation workspace")))
             return rc;
         double* tauq = static_cast<double*>(ctx->bufH.ptr);
-        double* taup = tauq + n;
-        double* kwork = taup + n;
+        double* taup = tauq + ldt;
+        double* kwork = taup + ldt;
         double* wr = kwork + kdoubles;
         {
             Phase ph(ctx, JLC_PHASE_BIDIAG);

@@ -11,22 +11,36 @@
 //   * row k (k < n - 1): the same recipe on x = B(k, k+1:n), applied to the
 //     rows k.. of B from the right (and to V).
 // That is a BLAS-2 algorithm: every reflector touches the whole trailing
-// matrix.  Here all n steps run in one cooperative launch.  The m rows are
-// dealt to the CTAs (at most one per SM) in chunks of 8, round robin, so that
-// every CTA keeps rows in play as the trailing matrix shrinks; a CTA holds at
-// most 256 rows.  Four bounded grid barriers join the reductions of each step:
-//   1. each CTA's scale/ssq of its rows of column k, merged by every CTA in
-//      the same fixed order (so all derive the same beta, tau, 1/(x0 - beta));
-//   2. each CTA's v on its rows (stored below the diagonal, as QR stores its
-//      reflectors), and its partial dots v^T A(:, j) for every trailing j;
-//   3. the dots summed over the CTAs in a fixed order, a share of the columns
-//      per CTA: w_j = tau * v^T A(:, j);
-//   4. A -= v w^T on each CTA's rows; the CTA holding row k forms the row
-//      reflector u (stored in row k beyond the superdiagonal, and copied to a
-//      dense vector), tau_p and e_k;
-//   then each CTA applies the row reflector to its own rows below k: x_r =
-//   tau_p * A(r, k+1:n) u, A(r, k+1:n) -= x_r u^T (row-local, no reduction
-//   across CTAs).
+// matrix.  Here all n steps run in one cooperative launch.  Row g lives on CTA
+// g % P (at most one CTA per SM), so that every CTA keeps rows in play as the
+// trailing matrix shrinks, and a CTA's rows -- its slab -- sit in shared
+// memory for the whole reduction (row-major, a thread per column) while they
+// fit, else in a global work array laid out the same way.
+//
+// A step needs two sums over all CTAs and no more, because everything else is
+// formed redundantly from their results:
+//   * the dots of column k with every trailing column, and its norm.  As the
+//     raw column is all they need, the pass that finishes step k - 1 takes
+//     them: w_j = tau (a_kj + sum_{i>k} x_i a_ij / (x0 - beta)) =
+//     tau v^T A(:, j) follows from the sums.  A warp of some CTA sums 2
+//     columns and publishes w_j;
+//   * row k after the column reflector is a_kj - w_j: every CTA has both, forms
+//     the row reflector u from them, then x = tau_p (A - v w^T) u on its own
+//     rows (row-local), A - v w^T - x u^T, and the dots of column k + 1.
+// The values cross the CTAs in tagged 16-byte slots (jlc_device.cuh): a reader
+// waits for the datum itself, and there is no barrier.
+//
+// What bounds a step is latency: two exchanges through L2 (about 1.2 us each
+// with the waits), two norms (a cross-warp sum, a square root, a division) and
+// two short passes; and the length of the code, since a step runs straight
+// through the kernel once: at 104 KB of instructions (waits inlined with
+// per-slot branches, norms with two-level rescaling, integer divisions for the
+// row numbers) a step took 11 us, at 43 KB 7.0 us.  Measured on B200, reflectors
+// only, ms:                                       512^2  1152x1024  4096^2
+//   rows in place, four grid barriers per step       -      54.4     693.6
+//   slabs, two grid barriers per step               5.3     11.8     172
+//   slots instead of barriers                       5.4     11.4     227
+//   the same in 43 KB of code (this kernel)         3.0      7.1     191
 // U and V are formed afterwards from the stored reflectors by the blocked
 // compact-WY Q builder of the QR route (GEMM kernels).
 //
@@ -40,318 +54,478 @@
 namespace jlc {
 namespace bidiag {
 
-constexpr int BT = 256;  // threads per CTA
+constexpr int BT = 512;  // threads per CTA
 constexpr int WARPS = BT / 32;
-constexpr int CH = 16;  // loads a thread keeps in flight in the row passes and the cross-CTA sums
-constexpr int RC = 8;   // rows per chunk: CTA p holds row chunks p, p + P, p + 2P, ...
+constexpr int RC = 8;     // rows per register block: a CTA holds a multiple of RC rows
+constexpr int QL = 16;    // lanes over the CTAs in the cross-CTA sums (a warp sums 2 columns)
+constexpr int QMAX = 10;  // partials per lane: QL * QMAX >= 148 CTAs
+constexpr int PAIRS = 5;  // (exponent, sum) pairs per lane: 32 * PAIRS >= 148 CTAs
+static_assert(32 * PAIRS == QL * QMAX, "one scale factor per CTA");
+constexpr int kMaxCtas = 148;
+constexpr int kMaxRows = 256;  // rows per CTA
 constexpr double kSafeMin = 2.2250738585072014e-308;  // Double.MIN_NORMAL
+constexpr int kEmptyExp = -4096;                      // exponent of an empty sum
+constexpr int kSmemLimit = 224 * 1024;
 
 struct Args {
     double* a;  // column-major m x n, m >= n
     long long lda;
     int m, n;
-    int nloc;      // rows per CTA (a multiple of RC, at most BT): its chunks, the last ones possibly past m
-    double* d;     // n: the diagonal of B
-    double* e;     // n - 1: the superdiagonal of B
-    double* tauq;  // n: the column reflectors' tau
-    double* taup;  // n: the row reflectors' tau (n - 1 used)
-    double* part;  // 2 per CTA: scale/ssq of its rows of the current column
-    double* wpart;  // n per CTA: its dots of v with the trailing columns
-    double* w;      // n: tau * v^T A(:, j)
-    double* u;      // n: the current row reflector, u[k+1] = 1
-    double* rec;    // the current row reflector's tau (written by the CTA holding row k)
-    unsigned* counter;
+    int rows;     // rows per CTA (a multiple of RC): CTA c holds rows c, c + P, c + 2P, ...
+    int ld;       // leading dimension of the slots and slab rows (n rounded up to 4)
+    double* d;    // n: the diagonal of B
+    double* e;    // n - 1: the superdiagonal of B
+    double* tauq; // n: the column reflectors' tau
+    double* taup; // n: the row reflectors' tau (n - 1 used)
+    Slot* part;   // [CTA][ld]: dots of the pivot column with the trailing columns
+    Slot* cpair;  // [2][CTA]: exponent and sum of squares of its rows of the pivot column
+    Slot* pivot;  // [2][ld]: the pivot row before the column reflector
+    Slot* w;      // ld: w_j = tau (row k's entry + the dots, rescaled)
+    double* slab; // global slabs (null: the slab sits in shared memory)
     int* status;
 };
 
-// sum of squares as s^2 * q with s a maximum of |x| (s == 0: nothing added)
-struct Ssq {
-    double s, q;
-};
-
-__device__ __forceinline__ Ssq ssq_add(Ssq a, double x) {
-    const double ax = fabs(x);
-    if (ax == 0.0) return a;
-    if (a.s == 0.0) return Ssq{ax, 1.0};
-    if (ax > a.s) {
-        const double t = a.s / ax;
-        return Ssq{ax, 1.0 + a.q * t * t};
-    }
-    const double t = ax / a.s;
-    return Ssq{a.s, a.q + t * t};
+// Sums of squares and dots are formed from values scaled by 2^-e, e the
+// exponent of a maximum, and carried with e: nothing overflows or underflows
+// whatever the range of the input, and every rescaling is exact.
+__device__ __forceinline__ int exp_of(double x) {  // 2^e <= x < 2^(e+1) for a positive normal x, in [-1000, 1022]
+    const int ex = (int)((__double_as_longlong(x) >> 52) & 0x7ff);
+    return x > 0.0 && ex != 0x7ff ? min(1022, max(-1000, ex - 1023)) : 0;
 }
-
-__device__ __forceinline__ Ssq ssq_merge(Ssq a, Ssq b) {
-    if (a.s == 0.0) return b;
-    if (b.s == 0.0) return a;
-    if (a.s >= b.s) {
-        const double t = b.s / a.s;
-        return Ssq{a.s, a.q + b.q * t * t};
-    }
-    const double t = a.s / b.s;
-    return Ssq{b.s, b.q + a.q * t * t};
-}
-
-__device__ __forceinline__ Ssq warp_merge(Ssq a) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        Ssq b{__shfl_xor_sync(0xffffffffu, a.s, o), __shfl_xor_sync(0xffffffffu, a.q, o)};
-        a = ssq_merge(a, b);
-    }
-    return a;
-}
-
+__device__ __forceinline__ double pow2(int e) { return __longlong_as_double((long long)(e + 1023) << 52); }
+// 2^d for d <= 0, 0 where a term scaled by it is negligible
+__device__ __forceinline__ double down(int d) { return d >= -1022 ? pow2(d) : 0.0; }
+__device__ __forceinline__ double shfl_xor(double v, int o) { return __shfl_xor_sync(0xffffffffu, v, o); }
+__device__ __forceinline__ int warp_max(int v) { return __reduce_max_sync(0xffffffffu, v); }
 __device__ __forceinline__ double warp_sum(double v) {
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    for (int o = 16; o > 0; o >>= 1) v += shfl_xor(v, o);
     return v;
 }
 
-// The CTA's scale/ssq (every thread's `acc`) merged warp by warp in a fixed
-// order; the result is valid in thread 0.
-__device__ __forceinline__ Ssq cta_merge(Ssq acc, double* s_red) {
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    acc = warp_merge(acc);
-    if (lane == 0) {
-        s_red[2 * warp] = acc.s;
-        s_red[2 * warp + 1] = acc.q;
-    }
-    __syncthreads();
-    Ssq t{0.0, 0.0};
-    if (threadIdx.x == 0)
-        for (int w = 0; w < WARPS; ++w) t = ssq_merge(t, Ssq{s_red[2 * w], s_red[2 * w + 1]});
-    return t;
-}
-
-// The reference's reflector recipe for a vector with norm xnorm (x0
-// included) and first entry x0: tau, beta and 1 / (x0 - beta); tau = 0 and
+// The reference's reflector recipe for a vector with norm 2^E sqrt(S) (x0
+// included) and first entry x0: tau, beta and 2^E / (x0 - beta); tau = 0 and
 // beta = x0 when there is no reflector.
-__device__ __forceinline__ void reflector(double xnorm, double x0, double& tau, double& beta, double& inv) {
-    tau = 0.0;
-    beta = x0;
-    inv = 0.0;
+struct Reflector {
+    double tau, beta, inv;
+};
+__device__ __noinline__ Reflector reflector(int E, double S, double x0) {
+    Reflector h{0.0, x0, 0.0};
+    if (!(S > 0.0)) return h;
+    const double p2 = pow2(E);
+    const double xnorm = p2 * sqrt(S);
     if (xnorm > kSafeMin) {
         const double b = x0 >= 0.0 ? -xnorm : xnorm;
         const double t = (b - x0) / b;
         if (fabs(t) > kSafeMin) {
-            tau = t;
-            beta = b;
-            inv = 1.0 / (x0 - b);
+            h.tau = t;
+            h.beta = b;
+            h.inv = p2 / (x0 - b);
         }
     }
+    return h;
 }
 
-__global__ void __launch_bounds__(BT, 1) bidiag_kernel(const Args p) {
-    __shared__ double s_red[2 * WARPS];
-    __shared__ double s_sc[4];
-    __shared__ double s_x[BT];
-    __shared__ double s_v[BT];  // the column reflector on this CTA's rows (by local row)
-    __shared__ int s_ok;
-    // the matrix and the vectors never alias, and each is reached through its
-    // own pointer only: loads may pass earlier stores
-    double* __restrict__ A = p.a;
-    double* __restrict__ U = p.u;
-    double* __restrict__ W = p.w;
-    const int P = gridDim.x, cta = blockIdx.x;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int m = p.m, n = p.n, nloc = p.nloc, nchunk = nloc / RC;
-    // local row l of this CTA: row chunks cta, cta + P, cta + 2P, ... of RC rows
-    auto grow = [&](int l) { return ((l / RC) * P + cta) * RC + (l % RC); };
-    unsigned nbar = 0;
-    auto barrier = [&]() -> bool {
-        ++nbar;
-        return grid_barrier(p.counter, nbar * (unsigned)P, p.status, &s_ok);
-    };
-    // the row-reflector phase: thread -> (local row, part of the columns)
-    const int nparts = BT / nloc > 0 ? BT / nloc : 1;
-    const int rloc = threadIdx.x % nloc, rpart = threadIdx.x / nloc;
+// Eight per-lane values summed over the warp: on return lane 4 i holds the
+// sum of value i (a halving exchange, then two butterfly steps).
+__device__ __forceinline__ double warp_sum8(double (&v)[RC]) {
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const double keep = (lane & 16) ? v[i + 4] : v[i], give = (lane & 16) ? v[i] : v[i + 4];
+        v[i] = keep + shfl_xor(give, 16);
+    }
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+        const double keep = (lane & 8) ? v[i + 2] : v[i], give = (lane & 8) ? v[i] : v[i + 2];
+        v[i] = keep + shfl_xor(give, 8);
+    }
+    const double keep = (lane & 4) ? v[1] : v[0], give = (lane & 4) ? v[0] : v[1];
+    double s = keep + shfl_xor(give, 4);
+    s += shfl_xor(s, 2);
+    s += shfl_xor(s, 1);
+    return s;
+}
 
-    for (int k = 0; k < n; ++k) {
-        double* col = A + (long long)k * p.lda;
-        __syncthreads();  // the previous step's row updates of this CTA are done
-        // 1. scale/ssq of this CTA's rows k.. of column k
-        {
-            Ssq acc{0.0, 0.0};
-            for (int l = threadIdx.x; l < nloc; l += BT) {
-                const int g = grow(l);
-                if (g >= k && g < m) acc = ssq_add(acc, col[g]);
+template <bool SMEM, int CB>
+__global__ void __launch_bounds__(BT, 1) bidiag_kernel(const Args p) {
+    extern __shared__ double dyn[];
+    __shared__ double s_v[kMaxRows];   // the column reflector on this CTA's rows
+    __shared__ double s_x[kMaxRows];   // tau_p (A u) on this CTA's rows
+    __shared__ double s_c[kMaxRows];   // the pivot column on this CTA's rows (0 above the pivot)
+    __shared__ double s_mx[kMaxRows / RC];
+    __shared__ double s_sum[WARPS];
+    __shared__ int s_exp[WARPS];
+    __shared__ double s_f[QL * QMAX];  // 2^(e_q - E) per CTA q
+    __shared__ int s_E;
+    __shared__ double s_x0;
+    __shared__ Reflector s_h;
+    const int P = gridDim.x, cta = blockIdx.x;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int m = p.m, n = p.n, rows = p.rows, ld = p.ld;
+    double* slab = SMEM ? dyn : p.slab + (size_t)cta * rows * ld;  // [local row][column]
+    double* red = SMEM ? dyn + (size_t)rows * ld : dyn;            // [warp][local row]
+    Slot* part = p.part + (size_t)cta * ld;
+    // this CTA's rows into its slab (rows past m are zero)
+    for (int l = 0; l < rows; ++l) {
+        const int g = l * P + cta;
+#pragma unroll 1
+        for (int j = tid; j < ld; j += BT) slab[(size_t)l * ld + j] = g < m && j < n ? p.a[g + (long long)j * p.lda] : 0.0;
+    }
+    for (int l = tid; l < rows; l += BT) {
+        s_v[l] = 0.0;
+        s_x[l] = 0.0;
+    }
+    __syncthreads();
+
+    // The pivot column kn after both reflectors of the step before it (s_v,
+    // s_x; w and u at column kn), 0 above the pivot, and its maximum per row
+    // block: each warp forms the row blocks whose s_x it has formed.
+    auto pivot_column = [&](int kn, int b0, double wk, double uk) {
+#pragma unroll 1
+        for (int b = b0 + warp; b < rows / RC; b += WARPS) {
+            double c = 0.0;
+            if (lane < RC) {
+                const int l = b * RC + lane, g = l * P + cta;
+                if (g >= kn && g < m) c = fma(-s_x[l], uk, fma(-s_v[l], wk, slab[(size_t)l * ld + kn]));
+                s_c[l] = c;
             }
-            const Ssq t = cta_merge(acc, s_red);
-            if (threadIdx.x == 0) {
-                p.part[2 * cta] = t.s;
-                p.part[2 * cta + 1] = t.q;
-            }
+            double mx = fabs(c);
+#pragma unroll
+            for (int o = 4; o > 0; o >>= 1) mx = fmax(mx, shfl_xor(mx, o));
+            if (lane == 0) s_mx[b] = mx;
         }
-        if (!barrier()) return;
-        if (threadIdx.x == 0) {
-            Ssq t{0.0, 0.0};
-            for (int q = 0; q < P; ++q) t = ssq_merge(t, Ssq{p.part[2 * q], p.part[2 * q + 1]});
-            const double xnorm = t.s == 0.0 ? 0.0 : t.s * sqrt(t.q);
-            double tau, beta, inv;
-            reflector(xnorm, col[k], tau, beta, inv);
-            s_sc[0] = tau;
-            s_sc[1] = beta;
-            s_sc[2] = inv;
-            if (cta == 0) {
-                p.tauq[k] = tau;
-                p.d[k] = beta;
+    };
+    pivot_column(0, 0, 0.0, 0.0);
+    __syncthreads();
+
+    double w[CB], u[CB];  // w and u of this thread's columns
+    int l0 = 0, gl = cta;  // the first of this CTA's rows at or past the pivot: local, global
+    bool fail = false;    // a wait of this thread ran out
+    for (int k = -1; k < n - 1; ++k) {
+        const int kn = k + 1;    // the pivot whose dots are published below
+        const int c0 = kn;       // first column of this step's update
+        // pivot rows and pairs alternate between two buffers: a CTA may still wait for step
+        // k's while a faster one, which needs w only, publishes those of step k + 1
+        const Slot* prow = p.pivot + (size_t)(k & 1) * ld;
+        Slot* pnext = p.pivot + (size_t)(kn & 1) * ld;
+        Slot* cnext = p.cpair + (size_t)(kn & 1) * P;
+        double taur = 0.0, ir = 0.0;
+        // u_j for an entry r_j of the pivot row
+        auto u_of = [&](int j, double rj) { return taur != 0.0 ? (j == kn ? 1.0 : rj * ir) : 0.0; };
+        // not SMEM: w and u of a column block, from the slots this thread has waited for
+        auto reload = [&](int j0) {
+#pragma unroll
+            for (int i = 0; i < CB; ++i) {
+                const int j = j0 + tid + i * BT;
+                w[i] = j < n ? slot_value(p.w + j) : 0.0;
+                u[i] = j < n ? u_of(j, slot_value(prow + j) - w[i]) : 0.0;
             }
-        }
-        __syncthreads();
-        const double tau = s_sc[0], inv = s_sc[2];
-        const bool lact = tau != 0.0;
-        // this CTA's first chunk with rows at or past k
-        const int kc = k / RC;
-        const int i0 = kc > cta ? (kc - cta + P - 1) / P : 0;
-        // 2. v on this CTA's rows (v_k = 1, 0 above k), the tails stored in
-        //    column k; partial dots of v with the trailing columns, one column
-        //    per lane (each lane walks down its column, a chunk of RC loads in
-        //    flight, and no cross-lane sum is needed)
-        if (lact) {
-            for (int l = threadIdx.x; l < nloc; l += BT) {
-                const int g = grow(l);
-                const bool tail = g > k && g < m;
-                const double x = tail ? col[g] * inv : (g == k ? 1.0 : 0.0);
-                s_v[l] = x;
-                if (tail) col[g] = x;
+        };
+        if (k >= 0) {
+            // ---- the row reflector of row k: w of this thread's columns as it arrives, r = the
+            // pivot row - w, the norm of r over the CTA (every warp the same bits)
+            double rmax = 0.0;
+            if constexpr (SMEM) {
+                // (threads past the last column wait for it too, and drop what they get)
+                const Slot* at[CB];
+#pragma unroll
+                for (int i = 0; i < CB; ++i) at[i] = p.w + min(c0 + tid + i * BT, n - 1);
+                fail |= !slot_wait(at, kn, w, p.status);
+#pragma unroll
+                for (int i = 0; i < CB; ++i) {
+                    if (c0 + tid + i * BT >= n) w[i] = u[i] = 0.0;
+                    u[i] -= w[i];  // r
+                    rmax = fmax(rmax, fabs(u[i]));
+                }
+                if (tid == 0) s_x0 = u[0];
+            } else {
+#pragma unroll 1
+                for (int j = c0 + tid; j < n; j += BT) {
+                    const Slot* at[1] = {p.w + j};
+                    double wj[1];
+                    fail |= !slot_wait(at, kn, wj, p.status);
+                    const double r = slot_value(prow + j) - wj[0];
+                    rmax = fmax(rmax, fabs(r));
+                    if (j == c0) s_x0 = r;
+                }
             }
+            int E = rmax > 0.0 ? exp_of(rmax) : kEmptyExp;
+            E = warp_max(E);
+            double S = 0.0;
+            if (E > kEmptyExp) {
+                const double sc = pow2(-E);
+                if constexpr (SMEM) {
+#pragma unroll
+                    for (int i = 0; i < CB; ++i) S = fma(u[i] * sc, u[i] * sc, S);
+                } else {
+                    for (int j = c0 + tid; j < n; j += BT) {
+                        const double y = (slot_value(prow + j) - slot_value(p.w + j)) * sc;
+                        S = fma(y, y, S);
+                    }
+                }
+            }
+            S = warp_sum(S);
+            if (lane == 0) {
+                s_sum[warp] = S;
+                s_exp[warp] = E;
+            }
+            if (__syncthreads_or(fail)) return;
+            {
+                const int e = lane < WARPS ? s_exp[lane] : kEmptyExp;
+                E = warp_max(e);
+                S = warp_sum(lane < WARPS ? s_sum[lane] * down(2 * (e - E)) : 0.0);
+                const Reflector h = reflector(E, S, s_x0);
+                taur = h.tau;
+                ir = taur != 0.0 ? h.inv * pow2(-E) : 0.0;
+                if (cta == 0 && tid == 0) {
+                    p.taup[k] = h.tau;
+                    p.e[k] = h.beta;
+                }
+            }
+            const bool owner = gl == k;
+            double* krow = slab + (size_t)l0 * ld;
+            if (owner) {
+                ++l0;
+                gl += P;
+            }
+            const int b0 = l0 / RC;
+            if constexpr (SMEM) {
+#pragma unroll
+                for (int i = 0; i < CB; ++i) {
+                    const int j = c0 + tid + i * BT;
+                    const double rj = u[i];
+                    u[i] = u_of(j, rj);
+                    // row k is finished: x0 beside the diagonal, the reflector's tail beyond it
+                    if (owner && j < n) krow[j] = taur != 0.0 && j > kn ? u[i] : rj;
+                }
+            } else if (owner) {
+                for (int j = c0 + tid; j < n; j += BT) {
+                    const double rj = slot_value(prow + j) - slot_value(p.w + j);
+                    krow[j] = taur != 0.0 && j > kn ? rj * ir : rj;
+                }
+            }
+            const double wk = slot_value(p.w + kn);
+            // ---- pass 1: x = tau_p (A - v w^T) u on this CTA's rows below k
+            if (taur != 0.0) {
+#pragma unroll 1
+    #pragma unroll 1
+            for (int b = b0; b < rows / RC; ++b) {
+                    double acc[RC], vr[RC];
+#pragma unroll
+                    for (int r = 0; r < RC; ++r) {
+                        acc[r] = 0.0;
+                        vr[r] = s_v[b * RC + r];
+                    }
+                    for (int j0 = c0; j0 < n; j0 += CB * BT) {
+                        if constexpr (!SMEM) reload(j0);
+#pragma unroll
+                        for (int i = 0; i < CB; ++i) {
+                            const int j = j0 + tid + i * BT;
+                            if (j < n) {
+                                const double* q = slab + (size_t)b * RC * ld + j;
+#pragma unroll
+                                for (int r = 0; r < RC; ++r) acc[r] = fma(fma(-vr[r], w[i], q[(size_t)r * ld]), u[i], acc[r]);
+                            }
+                        }
+                        if constexpr (SMEM) break;
+                    }
+                    const double s = warp_sum8(acc);
+                    if ((lane & 3) == 0) red[warp * rows + b * RC + (lane >> 2)] = s;
+                }
+                __syncthreads();
+                // the warps' sums, 4 lanes per row
+#pragma unroll 1
+        #pragma unroll 1
+        for (int b = b0 + warp; b < rows / RC; b += WARPS) {
+                    const int l = b * RC + (lane >> 2);
+                    double s = 0.0;
+#pragma unroll
+                    for (int i = 0; i < WARPS / 4; ++i) s += red[((lane & 3) * (WARPS / 4) + i) * rows + l];
+                    s += shfl_xor(s, 1);
+                    s += shfl_xor(s, 2);
+                    const int g = l * P + cta;
+                    if ((lane & 3) == 0) s_x[l] = g > k && g < m ? taur * s : 0.0;
+                }
+                __syncwarp();
+            } else {
+#pragma unroll 1
+                for (int l = tid; l < rows; l += BT) s_x[l] = 0.0;
+                __syncthreads();
+            }
+            pivot_column(kn, b0, wk, taur != 0.0 ? 1.0 : 0.0);
+            __syncthreads();
         }
-        __syncthreads();
-        if (lact) {
-            for (int j = k + 1 + threadIdx.x; j < n; j += BT) {
-                const double* aj = A + (long long)j * p.lda;
-                double s = 0.0;
-                for (int i = i0; i < nchunk; ++i) {
-                    const int g0 = (i * P + cta) * RC;
-                    if (g0 + RC <= m) {
+        // ---- the pivot column scaled by 2^-e, e the exponent of this CTA's maximum
+        const int b0 = l0 / RC;
+        double mx = 0.0;
+#pragma unroll 1
+        for (int b = b0; b < rows / RC; ++b) mx = fmax(mx, s_mx[b]);
+        const int ex = exp_of(mx);
+        const double sc = pow2(-ex);
+        if (warp == WARPS - 1) {
+            double q = 0.0;
+#pragma unroll 1
+            for (int l = b0 * RC + lane; l < rows; l += 32) {
+                const double c = s_c[l] * sc;
+                q = fma(c, c, q);
+            }
+            q = warp_sum(q);
+            if (lane == 0) slot_put(cnext + cta, q, kn + 1, mx > 0.0 ? ex : kEmptyExp);
+        }
+        // ---- pass 2: A - v w^T - x u^T stored, and its dots with the pivot column
+        const bool powner = gl == kn;
+        for (int j0 = c0; j0 < n; j0 += CB * BT) {
+            double s[CB];
+#pragma unroll
+            for (int i = 0; i < CB; ++i) s[i] = 0.0;
+            if (k < 0) {
+#pragma unroll
+                for (int i = 0; i < CB; ++i) w[i] = u[i] = 0.0;
+            } else if constexpr (!SMEM) {
+                reload(j0);
+            }
+#pragma unroll 1
+            for (int b = b0; b < rows / RC; ++b) {
+                double vr[RC], xr[RC], cr[RC];
+#pragma unroll
+                for (int r = 0; r < RC; ++r) {
+                    const int l = b * RC + r;
+                    vr[r] = s_v[l];
+                    xr[r] = s_x[l];
+                    cr[r] = l * P + cta > kn ? s_c[l] * sc : 0.0;
+                }
+#pragma unroll
+                for (int i = 0; i < CB; ++i) {
+                    const int j = j0 + tid + i * BT;
+                    if (j < n) {
+                        double* q = slab + (size_t)b * RC * ld + j;
                         double x[RC];
 #pragma unroll
-                        for (int t = 0; t < RC; ++t) x[t] = aj[g0 + t];
+                        for (int r = 0; r < RC; ++r) x[r] = q[(size_t)r * ld];
 #pragma unroll
-                        for (int t = 0; t < RC; ++t) s = fma(s_v[i * RC + t], x[t], s);
-                    } else {
-                        for (int g = g0; g < m; ++g) s = fma(s_v[i * RC + g - g0], aj[g], s);
-                    }
-                }
-                p.wpart[(long long)cta * n + j] = s;
-            }
-        }
-        if (!barrier()) return;
-        // 3. w_j = tau * sum over the CTAs' dots, in CTA order; a share of the columns per thread
-        if (lact) {
-            for (int j = k + 1 + cta * BT + threadIdx.x; j < n; j += P * BT) {
-                double s = 0.0;
-                int q = 0;
-                for (; q + CH <= P; q += CH) {  // CH loads in flight, added in CTA order
-                    double x[CH];
+                        for (int r = 0; r < RC; ++r) {
+                            x[r] = fma(-xr[r], u[i], fma(-vr[r], w[i], x[r]));
+                            s[i] = fma(cr[r], x[r], s[i]);
+                        }
 #pragma unroll
-                    for (int t = 0; t < CH; ++t) x[t] = p.wpart[(long long)(q + t) * n + j];
-#pragma unroll
-                    for (int t = 0; t < CH; ++t) s += x[t];
-                }
-                for (; q < P; ++q) s += p.wpart[(long long)q * n + j];
-                W[j] = tau * s;
-            }
-        }
-        if (!barrier()) return;
-        // 4. A -= v w^T on this CTA's rows k.., one column per lane
-        if (lact) {
-            for (int j = k + 1 + threadIdx.x; j < n; j += BT) {
-                double* aj = A + (long long)j * p.lda;
-                const double wj = W[j];
-                for (int i = i0; i < nchunk; ++i) {
-                    const int g0 = (i * P + cta) * RC;
-                    if (g0 + RC <= m) {
-                        double x[RC];
-#pragma unroll
-                        for (int t = 0; t < RC; ++t) x[t] = aj[g0 + t];
-#pragma unroll
-                        for (int t = 0; t < RC; ++t) aj[g0 + t] = fma(-s_v[i * RC + t], wj, x[t]);
-                    } else {
-                        for (int g = g0; g < m; ++g) aj[g] = fma(-s_v[i * RC + g - g0], wj, aj[g]);
+                        for (int r = 0; r < RC; ++r)
+                            if (b * RC + r >= l0) q[(size_t)r * ld] = x[r];
                     }
                 }
             }
-        }
-        if (k + 1 >= n) break;
-        // the row reflector of row k, by the CTA that holds the row
-        if (kc % P == cta) {
-            __syncthreads();  // row k's updated entries
-            Ssq acc{0.0, 0.0};
-            for (int j = k + 1 + threadIdx.x; j < n; j += BT) acc = ssq_add(acc, A[k + (long long)j * p.lda]);
-            const Ssq t = cta_merge(acc, s_red);
-            if (threadIdx.x == 0) {
-                const double xnorm = t.s == 0.0 ? 0.0 : t.s * sqrt(t.q);
-                double tr, br, ir;
-                reflector(xnorm, A[k + (long long)(k + 1) * p.lda], tr, br, ir);
-                s_sc[0] = tr;
-                s_sc[2] = ir;
-                p.taup[k] = tr;
-                p.e[k] = br;
-                p.rec[0] = tr;
-                U[k + 1] = 1.0;
-            }
-            __syncthreads();
-            if (s_sc[0] != 0.0) {
-                const double ir = s_sc[2];
-                for (int j = k + 2 + threadIdx.x; j < n; j += BT) {
-                    double* q = A + k + (long long)j * p.lda;
-                    const double uj = *q * ir;
-                    *q = uj;
-                    U[j] = uj;
+#pragma unroll
+            for (int i = 0; i < CB; ++i) {
+                const int j = j0 + tid + i * BT;
+                if (j < n) {
+                    slot_put(part + j, s[i], kn + 1, 0);
+                    if (powner) slot_put(pnext + j, slab[(size_t)l0 * ld + j], kn + 1, 0);
                 }
             }
         }
-        if (!barrier()) return;
-        // the row reflector on this CTA's rows below k: x_r = tau_p * A(r, k+1:) u
-        const double taur = p.rec[0];
-        if (taur != 0.0) {
-            const int r = grow(rloc);
-            const bool live = rpart < nparts && r > k && r < m;
-            double x = 0.0;
-            if (live) {
-                const double* ar = A + r;
-                int j = k + 1 + rpart;
-                for (; j + (CH - 1) * nparts < n; j += CH * nparts) {
-                    double y[CH], uu[CH];
+        // ---- the column reflector of column kn (the last warp), while the
+        // others wait for the dots: a warp sums those of 2 columns, 16 lanes over the CTAs
+        const int qi = lane >> 1, jj = lane & 1;
+        int gr = (kn + 1) / 2 + cta + warp * P;  // group of 2 columns, absolute
+        const int glast = (n + 1) / 2;
+        if (warp == WARPS - 1) {
+            double q[PAIRS + 1];  // the CTAs' sums of squares, and the pivot
+            int eq[PAIRS + 1];
+            const Slot* at[PAIRS + 1];
 #pragma unroll
-                    for (int t = 0; t < CH; ++t) {
-                        y[t] = ar[(long long)(j + t * nparts) * p.lda];
-                        uu[t] = U[j + t * nparts];
+            for (int i = 0; i < PAIRS; ++i) at[i] = cnext + min(lane + 32 * i, P - 1);
+            at[PAIRS] = pnext + kn;
+            fail |= !slot_wait(at, kn + 1, q, p.status, eq);
+            __syncwarp();
+#pragma unroll
+            for (int i = 0; i < PAIRS; ++i)
+                if (lane + 32 * i >= P) eq[i] = kEmptyExp;
+            int E = kEmptyExp;
+#pragma unroll
+            for (int i = 0; i < PAIRS; ++i) E = max(E, eq[i]);
+            E = warp_max(E);
+            double S = 0.0;
+#pragma unroll
+            for (int i = 0; i < PAIRS; ++i) {
+                const double f = lane + 32 * i < P ? down(eq[i] - E) : 0.0;
+                S = fma(q[i] * f, f, S);
+                s_f[lane + 32 * i] = f;
+            }
+            S = warp_sum(S);
+            const Reflector h = reflector(E, S, q[PAIRS]);
+            if (lane == 0) {
+                s_h = h;
+                s_E = E;
+                if (cta == 0) {
+                    p.tauq[kn] = h.tau;
+                    p.d[kn] = h.beta;
+                }
+            }
+        }
+        double tau = 0.0, vinv = 0.0;
+#pragma unroll 1
+        for (int trip = 0, left = glast - (kn + 1) / 2; trip == 0 || left > 0; ++trip, left -= P * WARPS, gr += P * WARPS) {
+            const int j = gr * 2 + jj;
+            double x[QMAX + 1];  // the dots, and the pivot row's entry
+            if (gr < glast) {
+                // (lanes past the last CTA or column wait for a live one and drop what they get)
+                const int jl = min(max(j, kn + 1), n - 1);
+                const Slot* at[QMAX + 1];
+#pragma unroll
+                for (int i = 0; i < QMAX; ++i) at[i] = p.part + (size_t)min(qi + QL * i, P - 1) * ld + jl;
+                at[QMAX] = pnext + jl;
+                fail |= !slot_wait(at, kn + 1, x, p.status);
+            }
+            if (trip == 0) {
+                // the pivot row at this thread's columns of the next step
+                if constexpr (SMEM) {
+                    const Slot* at[CB];
+#pragma unroll
+                    for (int i = 0; i < CB; ++i) at[i] = pnext + min(kn + 1 + tid + i * BT, n - 1);
+                    fail |= !slot_wait(at, kn + 1, u, p.status);
+                } else {
+#pragma unroll 1
+                    for (int c = kn + 1 + tid; c < n; c += BT) {
+                        const Slot* at[1] = {pnext + c};
+                        double y[1];
+                        fail |= !slot_wait(at, kn + 1, y, p.status);
                     }
-#pragma unroll
-                    for (int t = 0; t < CH; ++t) x = fma(y[t], uu[t], x);
                 }
-                for (; j < n; j += nparts) x = fma(ar[(long long)j * p.lda], U[j], x);
+                if (__syncthreads_or(fail)) return;
+                tau = s_h.tau;
+                vinv = s_h.inv;
             }
-            s_x[threadIdx.x] = x;
-            __syncthreads();
-            if (live && rpart == 0) {
-                double s = 0.0;
-                for (int q = 0; q < nparts; ++q) s += s_x[rloc + q * nloc];
-                s_x[rloc] = taur * s;
-            }
-            __syncthreads();
-            if (live) {
-                const double xr = s_x[rloc];
-                double* ar = A + r;
-                int j = k + 1 + rpart;
-                for (; j + (CH - 1) * nparts < n; j += CH * nparts) {
-                    double y[CH], uu[CH];
+            if (gr < glast) {
+                __syncwarp();
+                double s0 = 0.0, s1 = 0.0;
 #pragma unroll
-                    for (int t = 0; t < CH; ++t) {
-                        y[t] = ar[(long long)(j + t * nparts) * p.lda];
-                        uu[t] = U[j + t * nparts];
-                    }
+                for (int i = 0; i < QMAX; i += 2) {
+                    s0 = fma(x[i], s_f[qi + QL * i], s0);
+                    s1 = fma(x[i + 1], s_f[qi + QL * (i + 1)], s1);
+                }
+                double s = s0 + s1;
 #pragma unroll
-                    for (int t = 0; t < CH; ++t) ar[(long long)(j + t * nparts) * p.lda] = fma(-xr, uu[t], y[t]);
-                }
-                for (; j < n; j += nparts) {
-                    double* q = ar + (long long)j * p.lda;
-                    *q = fma(-xr, U[j], *q);
-                }
+                for (int o = 2; o < 32; o <<= 1) s += shfl_xor(s, o);
+                if (qi == 0 && j > kn && j < n) slot_put(p.w + j, tau != 0.0 ? tau * fma(s, vinv, x[QMAX]) : 0.0, kn + 1, 0);
             }
         }
+        // v on this CTA's rows, its tail stored below the diagonal
+        if (tid >= BT - kMaxRows && tid - (BT - kMaxRows) < rows) {
+            const int l = tid - (BT - kMaxRows), g = l * P + cta;
+            double v = 0.0;
+            if (tau != 0.0 && g >= kn && g < m) {
+                v = g == kn ? 1.0 : (s_c[l] * pow2(-s_E)) * vinv;
+                if (g > kn) slab[(size_t)l * ld + kn] = v;
+            }
+            s_v[l] = v;
+        }
+    }
+    __syncthreads();
+    for (int l = 0; l < rows; ++l) {
+        const int g = l * P + cta;
+        if (g < m)
+#pragma unroll 1
+            for (int j = tid; j < n; j += BT) p.a[g + (long long)j * p.lda] = slab[(size_t)l * ld + j];
     }
 }
 
@@ -365,50 +539,72 @@ __global__ void bidiag_right_factor_kernel(const double* a, long long lda, int n
 
 }  // namespace bidiag
 
-// The number of CTAs for an m-row reduction and the rows each holds (row
-// chunks of RC dealt round robin, so that every CTA keeps rows in play to the
-// last steps); 0 when a CTA would hold more than 256 rows.
-int bidiag_grid(int m, int sm_count, int* nloc) {
+// The number of CTAs for an m-row reduction and the rows each holds (row g on
+// CTA g % P, so that every CTA keeps rows in play to the last steps); 0 when
+// a CTA would hold more than 256 rows.
+int bidiag_grid(int m, int sm_count, int* rows) {
     using namespace bidiag;
-    const int chunks = (m + RC - 1) / RC;
-    const int P = chunks < sm_count ? chunks : sm_count;
-    const int per = (chunks + P - 1) / P;
-    if (per * RC > BT) return 0;
-    *nloc = per * RC;
-    return P;
+    const int most = sm_count < kMaxCtas ? sm_count : kMaxCtas;
+    const int per = ((m + most - 1) / most + RC - 1) / RC * RC;
+    if (per > kMaxRows) return 0;
+    *rows = per;
+    return (m + per - 1) / per;
 }
 
+namespace bidiag {
+static size_t smem_bytes(int rows, int ld, bool slab) {
+    return ((slab ? (size_t)rows * ld : 0) + (size_t)WARPS * rows) * sizeof(double);
+}
+static bool slab_in_smem(int rows, int n, int ld) {
+    return n <= 4 * BT && smem_bytes(rows, ld, true) + 16 * 1024 <= (size_t)kSmemLimit;
+}
+}  // namespace bidiag
+
+// Slots of the exchange: part, cpair, pivot and w.
+static size_t bidiag_slots(int P, int ld) { return (size_t)P * ld + 2 * (size_t)P + 3 * (size_t)ld; }
+
 size_t bidiag_work_doubles(int m, int n, int sm_count) {
-    (void)m;
-    return (size_t)2 * sm_count + (size_t)sm_count * n + 4 * (size_t)n + 16;
+    using namespace bidiag;
+    int rows = 0;
+    const int P = bidiag_grid(m, sm_count, &rows), ld = (n + 3) / 4 * 4;
+    return 2 * bidiag_slots(P, ld) + (slab_in_smem(rows, n, ld) ? 0 : (size_t)P * rows * ld);
 }
 
 int launch_bidiag(double* a, long long lda, int m, int n, double* d, double* e, double* tauq, double* taup,
                   double* work, int sm_count, int* status, cudaStream_t st) {
     using namespace bidiag;
     Args p;
-    int nloc = 0;
-    const int P = bidiag_grid(m, sm_count, &nloc);
+    int rows = 0;
+    const int P = bidiag_grid(m, sm_count, &rows);
     if (P == 0) return JLC_E_UNSUPPORTED;
     p.a = a;
     p.lda = lda;
     p.m = m;
     p.n = n;
-    p.nloc = nloc;
+    p.rows = rows;
+    p.ld = (n + 3) / 4 * 4;
     p.d = d;
     p.e = e;
     p.tauq = tauq;
     p.taup = taup;
-    p.part = work;
-    p.wpart = p.part + 2 * sm_count;
-    p.w = p.wpart + (size_t)sm_count * n;
-    p.u = p.w + n;
-    p.rec = p.u + n;
-    p.counter = reinterpret_cast<unsigned*>(p.rec + 8);
+    const size_t slots = bidiag_slots(P, p.ld);
+    p.part = reinterpret_cast<Slot*>(work);
+    p.cpair = p.part + (size_t)P * p.ld;
+    p.pivot = p.cpair + 2 * P;
+    p.w = p.pivot + 2 * (size_t)p.ld;
+    const bool smem = slab_in_smem(rows, n, p.ld);
+    p.slab = smem ? nullptr : work + 2 * slots;
     p.status = status;
-    if (cudaMemsetAsync(p.counter, 0, sizeof(unsigned), st) != cudaSuccess) return JLC_E_CUDA;
+    const void* kern = !smem        ? (const void*)bidiag_kernel<false, 4>
+                       : n > 2 * BT ? (const void*)bidiag_kernel<true, 4>
+                                    : (const void*)bidiag_kernel<true, 2>;
+    const size_t bytes = smem_bytes(rows, p.ld, smem);
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) != cudaSuccess)
+        return JLC_E_LAUNCH;
+    // no slot may hold a tag of an earlier call
+    if (cudaMemsetAsync(work, 0, slots * sizeof(Slot), st) != cudaSuccess) return JLC_E_CUDA;
     void* args[] = {&p};
-    cudaError_t err = cudaLaunchCooperativeKernel((const void*)bidiag_kernel, dim3(P), dim3(BT), args, 0, st);
+    cudaError_t err = cudaLaunchCooperativeKernel(kern, dim3(P), dim3(BT), args, bytes, st);
     return err == cudaSuccess ? JLC_OK : JLC_E_LAUNCH;
 }
 

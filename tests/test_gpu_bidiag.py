@@ -98,3 +98,53 @@ def test_rejects_bad_arguments(ctx):
         ctx.bidiag_device(3, 5, 8, 3, 8, 8, None, 3, None, 5)   # m < n
     with pytest.raises(IllegalArgumentException):
         ctx.bidiag_device(5, 3, 8, 4, 8, 8, None, 5, None, 3)   # lda < m
+
+
+@pytest.mark.parametrize("m,n", [
+    (1025, 1025),   # rows per CTA 8, more than two columns per thread
+    (1191, 520),    # 16 rows per CTA, the last CTA's slab partly past m
+    (513, 513), (9, 2), (8, 8),   # one column past a thread each; two CTAs; one CTA
+    (6000, 700),    # the slab does not fit in shared memory
+    (2300, 2100),   # nor here; several column blocks per thread
+])
+def test_slab_and_column_block_edges(ctx, m, n):
+    """A = U B V^T with U and V orthogonal, at the sizes where the kernel's slab
+    placement and column blocks change, checked with torch in FP64.  A
+    backward stable reduction leaves residuals of a small multiple of
+    max(m, n) u."""
+    import torch
+    g = torch.Generator(device="cuda").manual_seed(2400 + m + n)
+    a = torch.rand(n, m, dtype=torch.float64, device="cuda", generator=g) * 2 - 1   # column-major m x n
+    f, u, v = a.clone(), torch.empty(m, m, dtype=torch.float64, device="cuda"), \
+        torch.empty(n, n, dtype=torch.float64, device="cuda")
+    d = torch.empty(n, dtype=torch.float64, device="cuda")
+    e = torch.empty(n, dtype=torch.float64, device="cuda")
+    torch.cuda.synchronize()
+    ctx.bidiag_device(m, n, f.data_ptr(), m, d.data_ptr(), e.data_ptr(), u.data_ptr(), m, v.data_ptr(), n)
+    b = torch.zeros(m, n, dtype=torch.float64, device="cuda")
+    i = torch.arange(n, device="cuda")
+    b[i, i] = d
+    b[i[:-1], i[1:]] = e[:n - 1]
+    u, v = u.T, v.T
+    tol = 1e-14 * max(m, n)
+    assert float((a.T - u @ b @ v.T).norm() / a.norm()) < tol
+    assert float((u.T @ u - torch.eye(m, dtype=torch.float64, device="cuda")).norm()) < tol * m ** 0.5
+    assert float((v.T @ v - torch.eye(n, dtype=torch.float64, device="cuda")).norm()) < tol * n ** 0.5
+
+
+@pytest.mark.parametrize("s", [900, -900])
+def test_range_of_the_input(ctx, s):
+    """Scaling A by 2^s scales d and e by 2^s exactly and leaves the reflectors
+    as they are: every sum is formed from values scaled by a power of two."""
+    import torch
+    m, n = 150, 130
+    a = O.uniform((n, m), 2501)
+    outs = []
+    for scale in (1.0, 2.0 ** s):
+        at = torch.from_numpy(a * scale).cuda()
+        u, v = torch.empty(m, m, dtype=torch.float64).cuda(), torch.empty(n, n, dtype=torch.float64).cuda()
+        d, e = torch.empty(n, dtype=torch.float64).cuda(), torch.empty(n - 1, dtype=torch.float64).cuda()
+        ctx.bidiag_device(m, n, at.data_ptr(), m, d.data_ptr(), e.data_ptr(), u.data_ptr(), m, v.data_ptr(), n)
+        outs.append((d.cpu().numpy() / scale, e.cpu().numpy() / scale, u.cpu().numpy(), v.cpu().numpy()))
+    for x, y in zip(*outs):
+        np.testing.assert_array_equal(x, y)
