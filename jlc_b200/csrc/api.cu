@@ -1262,7 +1262,25 @@ int jlc_hessenberg_device(jlc_ctx* ctx, int64_t n, double* a, int64_t lda, doubl
     cudaEventRecord(ctx->ev0, st);
     int rc = JLC_OK;
     if (q && (rc = launch_set_identity(q, ldq, n, n, st))) return set_err(ctx, rc, "Hessenberg: identity launch failed");
-    if (n > 2) {
+    if (n > 2 && hess_slab_fits((int)n, ctx->sm_count)) {
+        // the whole reduction in one launch, then Q = diag(1, H_0 ... H_{n-3}) from the reflectors
+        // below the subdiagonal, which sit there as in the QR factor of rows 1..
+        const long long ldt = round_up(n, 8);
+        if ((rc = reserve(ctx, ctx->bufH, (ldt + hess_slab_work_doubles((int)n, ctx->sm_count)) * sizeof(double),
+                          "Hessenberg workspace")))
+            return rc;
+        double* tau = static_cast<double*>(ctx->bufH.ptr);
+        {
+            Phase ph(ctx, JLC_PHASE_HESS_PANEL);
+            rc = launch_hess_slab(a, lda, (int)n, tau, tau + ldt, ctx->sm_count, ctx->d_status, st);
+            if (rc) return set_err(ctx, rc, "Hessenberg: launch failed");
+            ctx->launches += 1;
+        }
+        if (q && (rc = qr_build_q_enqueue(ctx, n - 1, n - 2, n - 1, a + 1, lda, tau, q + 1 + ldq, ldq, precision)))
+            return rc;
+        if ((rc = launch_hess_clear(a, lda, (int)n, st))) return set_err(ctx, rc, "Hessenberg: clear launch failed");
+        ctx->launches += 1;
+    } else if (n > 2) {
         const long long ldv = round_up(n, 8), ldw = ldv;
         const size_t work_bytes = hess_work_doubles(n) * sizeof(double);
         if ((rc = reserve(ctx, ctx->bufH, work_bytes + hess_panel_scratch_bytes(ctx->sm_count),
@@ -1350,7 +1368,7 @@ int jlc_bidiag_device(jlc_ctx* ctx, int64_t m, int64_t n, double* a, int64_t lda
     ctx->err[0] = 0;
     cudaStream_t st = ctx->stream;
     int rows_per_cta = 0;
-    if (m > 0 && n > 0 && bidiag_grid((int)m, ctx->sm_count, &rows_per_cta) == 0)
+    if (m > 0 && n > 0 && bidiag_grid((int)m, (int)n, ctx->sm_count, &rows_per_cta) == 0)
         return set_err(ctx, JLC_E_UNSUPPORTED, "bidiagonalisation: more than 256 rows per SM");
     cudaEventRecord(ctx->ev0, st);
     int rc = JLC_OK;

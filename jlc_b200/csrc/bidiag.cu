@@ -50,6 +50,7 @@
 
 #include "jlc_device.cuh"
 #include "jlc_internal.h"
+#include "jlc_slab.cuh"
 
 namespace jlc {
 namespace bidiag {
@@ -95,13 +96,6 @@ __device__ __forceinline__ int exp_of(double x) {  // 2^e <= x < 2^(e+1) for a p
 __device__ __forceinline__ double pow2(int e) { return __longlong_as_double((long long)(e + 1023) << 52); }
 // 2^d for d <= 0, 0 where a term scaled by it is negligible
 __device__ __forceinline__ double down(int d) { return d >= -1022 ? pow2(d) : 0.0; }
-__device__ __forceinline__ double shfl_xor(double v, int o) { return __shfl_xor_sync(0xffffffffu, v, o); }
-__device__ __forceinline__ int warp_max(int v) { return __reduce_max_sync(0xffffffffu, v); }
-__device__ __forceinline__ double warp_sum(double v) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += shfl_xor(v, o);
-    return v;
-}
 
 // The reference's reflector recipe for a vector with norm 2^E sqrt(S) (x0
 // included) and first entry x0: tau, beta and 2^E / (x0 - beta); tau = 0 and
@@ -124,27 +118,6 @@ __device__ __noinline__ Reflector reflector(int E, double S, double x0) {
         }
     }
     return h;
-}
-
-// Eight per-lane values summed over the warp: on return lane 4 i holds the
-// sum of value i (a halving exchange, then two butterfly steps).
-__device__ __forceinline__ double warp_sum8(double (&v)[RC]) {
-    const int lane = threadIdx.x & 31;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const double keep = (lane & 16) ? v[i + 4] : v[i], give = (lane & 16) ? v[i] : v[i + 4];
-        v[i] = keep + shfl_xor(give, 16);
-    }
-#pragma unroll
-    for (int i = 0; i < 2; ++i) {
-        const double keep = (lane & 8) ? v[i + 2] : v[i], give = (lane & 8) ? v[i] : v[i + 2];
-        v[i] = keep + shfl_xor(give, 8);
-    }
-    const double keep = (lane & 4) ? v[1] : v[0], give = (lane & 4) ? v[0] : v[1];
-    double s = keep + shfl_xor(give, 4);
-    s += shfl_xor(s, 2);
-    s += shfl_xor(s, 1);
-    return s;
 }
 
 template <bool SMEM, int CB>
@@ -542,10 +515,13 @@ __global__ void bidiag_right_factor_kernel(const double* a, long long lda, int n
 // The number of CTAs for an m-row reduction and the rows each holds (row g on
 // CTA g % P, so that every CTA keeps rows in play to the last steps); 0 when
 // a CTA would hold more than 256 rows.
-int bidiag_grid(int m, int sm_count, int* rows) {
+int bidiag_grid(int m, int n, int sm_count, int* rows) {
     using namespace bidiag;
     const int most = sm_count < kMaxCtas ? sm_count : kMaxCtas;
-    const int per = ((m + most - 1) / most + RC - 1) / RC * RC;
+    int per = ((m + most - 1) / most + RC - 1) / RC * RC;
+    // past two columns per thread 16 rows per CTA (1168 x 1100: 9.3 ms, against 10.4 with 8: half as
+    // many partials cross), below it 8 (1152 x 1024: 7.2 against 7.6; 512^2: 3.1 against 3.2)
+    if (n > 2 * BT && per < 2 * RC) per = 2 * RC;
     if (per > kMaxRows) return 0;
     *rows = per;
     return (m + per - 1) / per;
@@ -566,7 +542,7 @@ static size_t bidiag_slots(int P, int ld) { return (size_t)P * ld + 2 * (size_t)
 size_t bidiag_work_doubles(int m, int n, int sm_count) {
     using namespace bidiag;
     int rows = 0;
-    const int P = bidiag_grid(m, sm_count, &rows), ld = (n + 3) / 4 * 4;
+    const int P = bidiag_grid(m, n, sm_count, &rows), ld = (n + 3) / 4 * 4;
     return 2 * bidiag_slots(P, ld) + (slab_in_smem(rows, n, ld) ? 0 : (size_t)P * rows * ld);
 }
 
@@ -575,7 +551,7 @@ int launch_bidiag(double* a, long long lda, int m, int n, double* d, double* e, 
     using namespace bidiag;
     Args p;
     int rows = 0;
-    const int P = bidiag_grid(m, sm_count, &rows);
+    const int P = bidiag_grid(m, n, sm_count, &rows);
     if (P == 0) return JLC_E_UNSUPPORTED;
     p.a = a;
     p.lda = lda;

@@ -1,4 +1,6 @@
-// Blocked Hessenberg reduction on the device: the kernels of one panel.
+// Hessenberg reduction on the device: one launch for matrices that fit in the
+// shared memory of the chip (hess_slab_kernel), and the kernels of one panel
+// of the blocked reduction for larger ones.
 //
 // The reference (BlockedHessenbergQR.decompose, eigen/qr/BlockedHessenbergQR.java:99-146)
 // factors each 32-column panel on a working copy of the whole matrix --
@@ -29,17 +31,12 @@
 
 #include "jlc_device.cuh"
 #include "jlc_internal.h"
+#include "jlc_slab.cuh"
 
 namespace jlc {
 namespace hess {
 
 constexpr int PW = 32;  // panel width of the reference
-
-__device__ __forceinline__ double warp_sum(double v) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    return v;
-}
 
 // Entries below the first subdiagonal set to zero (the reference clears the
 // fill-in its block updates leave there, BlockedHessenbergQR.java:137-141).
@@ -318,7 +315,359 @@ __global__ void __launch_bounds__(PT, 1) hess_panel_kernel(const PanelArgs p) {
     }
 }
 
+// ---------------------------------------------------------------------------
+// The whole reduction in one cooperative launch, for matrices whose rows fit on
+// the chip.  Row g lives on CTA g % P, its slab of rows in shared memory
+// (row-major, a thread per column).  Step k, with the reflector v (v_{k+1} = 1,
+// zero above) and tau that take column k below row k to beta e:
+//   w_j = tau v^T H(:, j),  x = tau (H - v w^T) v = tau (H v - v (w . v)),
+//   H <- H - v w^T - x v^T    (columns k+1..; column k is finished).
+// Two sums over the CTAs, as in bidiag.cu: the dots of the raw column with
+// the trailing columns, taken in the pass that finishes the step before, and
+// published w_j (a warp sums 2 columns).  The column itself is gathered by
+// every CTA, so H v runs while the dots are on their way.  Values cross in
+// tagged slots; there is no barrier.  The reflectors stay below the
+// subdiagonal, from which the blocked Q builder of the QR route forms Q.
+//
+// A step is bound by latency: two exchanges through L2 (about 1500 cycles each
+// from store to load), then the sums and the scalar recipe between them; it
+// takes 5.1 us at n = 1024 and 4.2 us at n = 128.  The panel route pays two
+// grid barriers and a GEMV from L2 per reflector (15 us at n = 1024), six GEMMs
+// per panel, and 107 KB of straight-line code per reflector against 32 KB
+// here.  Measured on B200, H and Q, ms: n = 1024 20.8 -> 6.9.
+constexpr int SLT = 512;  // threads per CTA
+constexpr int SLW = SLT / 32;
+constexpr int RC = 8;     // rows per register block: a CTA holds a multiple of RC rows
+constexpr int QL = 16;    // lanes over the CTAs in the cross-CTA sums (a warp sums 2 columns)
+constexpr int QMAX = 10;  // partials per lane: QL * QMAX >= 148 CTAs
+constexpr int PAIRS = 5;  // sums per lane of one warp: 32 * PAIRS >= 148 CTAs
+constexpr int kSlabMaxCtas = 148;
+constexpr int kSlabMaxRows = 32;
+constexpr int kSlabSmemLimit = 224 * 1024;
+
+struct SlabArgs {
+    double* h;
+    long long ldh;
+    int n, rows, ld;  // rows per CTA (a multiple of RC), row length of slab and slots
+    double* tau;      // n - 2
+    Slot* part;       // [CTA][ld]: dots of the column's tail with the trailing columns
+    Slot* sig;        // [2][CTA]: sums of squares of the tail
+    Slot* colv;       // [2][ld]: the column
+    Slot* prow;       // [2][ld]: row k + 1
+    Slot* w;          // [ld]
+    int* status;
+    double eps;
+};
+
+struct SlabReflector {
+    double tau, beta, inv;
+};
+// the reference's recipe from x0 and sigma = |tail|^2 (tau = 0: no reflector)
+__device__ __noinline__ SlabReflector slab_reflector(double x0, double sigma, double eps) {
+    SlabReflector r{0.0, x0, 0.0};
+    if (sigma > eps) {
+        const double beta = -copysign(sqrt(x0 * x0 + sigma), x0);
+        const double v0 = x0 - beta, v0sq = v0 * v0;
+        if (v0sq > eps) {
+            r.tau = 2.0 * v0sq / (sigma + v0sq);
+            r.beta = beta;
+            r.inv = 1.0 / v0;
+        }
+    }
+    return r;
+}
+
+template <int CB>
+__global__ void __launch_bounds__(SLT, 1) hess_slab_kernel(const SlabArgs p) {
+    extern __shared__ double slab[];  // [local row][column], then [warp][local row] sums
+    __shared__ double s_v[kSlabMaxRows], s_x[kSlabMaxRows], s_c[kSlabMaxRows];
+    __shared__ double s_wv[SLW];  // the warps' parts of w . v
+    __shared__ double s_wk;
+    __shared__ SlabReflector s_h;
+    const int P = gridDim.x, cta = blockIdx.x;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int n = p.n, rows = p.rows, ld = p.ld;
+    double* red = slab + (size_t)rows * ld;
+    Slot* part = p.part + (size_t)cta * ld;
+    for (int l = 0; l < rows; ++l) {
+        const int g = l * P + cta;
+#pragma unroll 1
+        for (int j = tid; j < ld; j += SLT) slab[(size_t)l * ld + j] = g < n && j < n ? p.h[g + (long long)j * p.ldh] : 0.0;
+    }
+    if (tid < rows) {
+        s_v[tid] = 0.0;
+        s_x[tid] = 0.0;
+    }
+    __syncthreads();
+    if (tid < rows) s_c[tid] = slab[(size_t)tid * ld];
+    __syncthreads();
+    double w[CB], u[CB];  // w and v of this thread's columns
+#pragma unroll
+    for (int i = 0; i < CB; ++i) w[i] = u[i] = 0.0;
+    bool fail = false;
+    int gl = cta, lf = 0;  // the first of this CTA's rows past row k: global, local
+    if (gl == 0) {
+        gl += P;
+        ++lf;
+    }
+    // step k: the update of step k - 1 on columns k.., and the reflector of column k
+    for (int k = 0;; ++k) {
+        const int kn = k + 1;
+        const bool more = k < n - 2, owner = gl == kn;  // owner: of row k + 1
+        Slot* sig = p.sig + (size_t)(k & 1) * P;
+        Slot* colv = p.colv + (size_t)(k & 1) * ld;
+        Slot* prow = p.prow + (size_t)(k & 1) * ld;
+        if (more) {
+            // the column (its rows past k) and its tail's sum of squares, ahead of the pass
+            if (tid < rows && tid >= lf && tid * P + cta < n) slot_put(colv + tid * P + cta, s_c[tid], kn, 0);
+            if (warp == SLW - 1) {
+                const double c = lane < rows && lane >= lf + owner ? s_c[lane] : 0.0;
+                const double q = warp_sum(c * c);
+                if (lane == 0) slot_put(sig + cta, q, kn, 0);
+            }
+        }
+        // ---- H - v w^T - x v^T stored, and its dots with the column's tail
+        {
+            double s[CB];
+#pragma unroll
+            for (int i = 0; i < CB; ++i) s[i] = 0.0;
+#pragma unroll 1
+            for (int b = 0; b < rows / RC; ++b) {
+                double vr[RC], xr[RC], cr[RC];
+#pragma unroll
+                for (int r = 0; r < RC; ++r) {
+                    const int l = b * RC + r;
+                    vr[r] = s_v[l];
+                    xr[r] = s_x[l];
+                    cr[r] = l >= lf + owner ? s_c[l] : 0.0;
+                }
+#pragma unroll
+                for (int i = 0; i < CB; ++i) {
+                    const int j = k + tid + i * SLT;
+                    if (j < n) {
+                        double* q = slab + (size_t)b * RC * ld + j;
+                        double y[RC];
+#pragma unroll
+                        for (int r = 0; r < RC; ++r) y[r] = q[(size_t)r * ld];
+#pragma unroll
+                        for (int r = 0; r < RC; ++r) {
+                            y[r] = fma(-xr[r], u[i], fma(-vr[r], w[i], y[r]));
+                            s[i] = fma(cr[r], y[r], s[i]);
+                        }
+#pragma unroll
+                        for (int r = 0; r < RC; ++r) q[(size_t)r * ld] = y[r];
+                    }
+                }
+            }
+            if (!more) break;
+#pragma unroll
+            for (int i = 0; i < CB; ++i) {
+                const int j = k + tid + i * SLT;
+                if (j < n) {
+                    slot_put(part + j, s[i], kn, 0);
+                    if (owner) slot_put(prow + j, slab[(size_t)lf * ld + j], kn, 0);
+                }
+            }
+        }
+        // ---- the reflector (the last warp, every CTA the same bits) and v at this thread's columns
+        if (warp == SLW - 1) {
+            double q[PAIRS + 1];
+            const Slot* at[PAIRS + 1];
+#pragma unroll
+            for (int i = 0; i < PAIRS; ++i) at[i] = sig + min(lane + 32 * i, P - 1);
+            at[PAIRS] = colv + kn;
+            fail |= !slot_wait(at, kn, q, p.status);
+            __syncwarp();
+            double sigma = 0.0;
+#pragma unroll
+            for (int i = 0; i < PAIRS; ++i) sigma += lane + 32 * i < P ? q[i] : 0.0;
+            sigma = warp_sum(sigma);
+            const SlabReflector r = slab_reflector(q[PAIRS], sigma, p.eps);
+            if (lane == 0) {
+                s_h = r;
+                if (cta == 0) p.tau[k] = r.tau;
+            }
+        }
+        {
+            const Slot* at[CB];
+#pragma unroll
+            for (int i = 0; i < CB; ++i) at[i] = colv + min(kn + tid + i * SLT, n - 1);
+            fail |= !slot_wait(at, kn, u, p.status);
+        }
+        if (__syncthreads_or(fail)) return;
+        const double tau = s_h.tau, inv = s_h.inv;
+#pragma unroll
+        for (int i = 0; i < CB; ++i) {
+            const int j = kn + tid + i * SLT;
+            u[i] = j < n ? (j == kn ? (tau != 0.0 ? 1.0 : 0.0) : u[i] * inv) : 0.0;
+        }
+        // ---- w of 2 columns per warp, 16 lanes over the CTAs
+        const int qi = lane >> 1, jj = lane & 1;
+#pragma unroll 1
+        for (int gr = kn / 2 + cta + warp * P; gr < (n + 1) / 2; gr += P * SLW) {
+            // (lanes past the last CTA or column wait for a live one and drop what they get)
+            const int j = gr * 2 + jj, jl = min(max(j, kn), n - 1);
+            double x[QMAX + 1];
+            const Slot* at[QMAX + 1];
+#pragma unroll
+            for (int i = 0; i < QMAX; ++i) at[i] = p.part + (size_t)min(qi + QL * i, P - 1) * ld + jl;
+            at[QMAX] = prow + jl;
+            fail |= !slot_wait(at, kn, x, p.status);
+            __syncwarp();
+            double s0 = 0.0, s1 = 0.0;
+#pragma unroll
+            for (int i = 0; i < QMAX; i += 2) {
+                s0 += qi + QL * i < P ? x[i] : 0.0;
+                s1 += qi + QL * (i + 1) < P ? x[i + 1] : 0.0;
+            }
+            double sum = s0 + s1;
+#pragma unroll
+            for (int o = 2; o < 32; o <<= 1) sum += shfl_xor(sum, o);
+            if (qi == 0 && j >= kn && j < n) slot_put(p.w + j, tau != 0.0 ? tau * fma(sum, inv, x[QMAX]) : 0.0, kn, 0);
+        }
+        // v on this CTA's rows; column k is finished: beta, and v's tail below it
+        if (tid < rows) {
+            double v = 0.0;
+            if (tid >= lf && tid * P + cta < n && tau != 0.0) {
+                const bool first = owner && tid == lf;
+                v = first ? 1.0 : s_c[tid] * inv;
+                slab[(size_t)tid * ld + k] = first ? s_h.beta : v;
+            }
+            s_v[tid] = v;
+        }
+        // ---- H v on this CTA's rows, while w is on its way
+#pragma unroll 1
+        for (int b = 0; b < rows / RC; ++b) {
+            double acc[RC];
+#pragma unroll
+            for (int r = 0; r < RC; ++r) acc[r] = 0.0;
+#pragma unroll
+            for (int i = 0; i < CB; ++i) {
+                const int j = kn + tid + i * SLT;
+                if (j < n) {
+                    const double* q = slab + (size_t)b * RC * ld + j;
+#pragma unroll
+                    for (int r = 0; r < RC; ++r) acc[r] = fma(q[(size_t)r * ld], u[i], acc[r]);
+                }
+            }
+            const double s = warp_sum8(acc);
+            if ((lane & 3) == 0) red[warp * rows + b * RC + (lane >> 2)] = s;
+        }
+        {
+            const Slot* at[CB];
+#pragma unroll
+            for (int i = 0; i < CB; ++i) at[i] = p.w + min(kn + tid + i * SLT, n - 1);
+            fail |= !slot_wait(at, kn, w, p.status);
+            __syncwarp();
+            double s = 0.0;
+#pragma unroll
+            for (int i = 0; i < CB; ++i) {
+                if (kn + tid + i * SLT >= n) w[i] = 0.0;
+                s = fma(w[i], u[i], s);
+            }
+            s = warp_sum(s);
+            if (lane == 0) s_wv[warp] = s;
+            if (tid == 0) s_wk = w[0];
+        }
+        if (__syncthreads_or(fail)) return;
+        if (owner) {
+            gl += P;
+            ++lf;
+        }
+        // ---- x on this CTA's rows, and the next column on its rows past k + 1: 4 lanes per row
+#pragma unroll 1
+        for (int b = warp; b < rows / RC; b += SLW) {
+            const int l = b * RC + (lane >> 2), part4 = lane & 3;
+            double y = 0.0, wv = 0.0;
+#pragma unroll
+            for (int i = 0; i < SLW / 4; ++i) {
+                y += red[(part4 * (SLW / 4) + i) * rows + l];
+                wv += s_wv[part4 * (SLW / 4) + i];
+            }
+            y += shfl_xor(y, 1);
+            wv += shfl_xor(wv, 1);
+            y += shfl_xor(y, 2);
+            wv += shfl_xor(wv, 2);
+            if (part4 == 0) {
+                const double v = s_v[l], x = tau * fma(-v, wv, y);
+                s_x[l] = x;
+                s_c[l] = fma(-x, tau != 0.0 ? 1.0 : 0.0, fma(-v, s_wk, slab[(size_t)l * ld + kn]));
+            }
+        }
+        __syncthreads();
+    }
+    __syncthreads();
+    for (int l = 0; l < rows; ++l) {
+        const int g = l * P + cta;
+        if (g < n)
+#pragma unroll 1
+            for (int j = tid; j < n; j += SLT) p.h[g + (long long)j * p.ldh] = slab[(size_t)l * ld + j];
+    }
+}
+
 }  // namespace hess
+
+namespace hess {
+static int slab_rows(int n, int sm_count) {
+    const int most = sm_count < kSlabMaxCtas ? sm_count : kSlabMaxCtas;
+    const int rows = ((n + most - 1) / most + RC - 1) / RC * RC;
+    // past two columns per thread at least 16 rows per CTA (n = 1056: 5.9 ms, against 7.3 with 8: half
+    // as many partials cross), below it 8 (n = 1024: 5.3 against 5.5; n = 256: 1.1 against 1.2)
+    return n > 2 * SLT && rows < 2 * RC ? 2 * RC : rows;
+}
+static size_t slab_smem(int n, int rows) { return ((size_t)rows * ((n + 3) / 4 * 4) + (size_t)SLW * rows) * sizeof(double); }
+static size_t slab_slots(int n, int P) {
+    const size_t ld = (n + 3) / 4 * 4;
+    return (size_t)P * ld + 2 * (size_t)P + 5 * ld;
+}
+}  // namespace hess
+
+// Whether an n x n reduction runs in the one-launch kernel: its rows fit in the
+// shared memory of the chip (n up to 1 744 on 148 SMs).  It is the faster route
+// wherever it fits (n = 1744: 14.9 ms with Q against 38.9 ms on the panel route; n = 64: 0.33 against 1.02).
+bool hess_slab_fits(int n, int sm_count) {
+    using namespace hess;
+    const int rows = slab_rows(n, sm_count);
+    return n > 2 && n <= 4 * SLT && rows <= kSlabMaxRows && slab_smem(n, rows) + 4 * 1024 <= (size_t)kSlabSmemLimit;
+}
+
+size_t hess_slab_work_doubles(int n, int sm_count) {
+    using namespace hess;
+    const int rows = slab_rows(n, sm_count);
+    return 2 * slab_slots(n, (n + rows - 1) / rows);
+}
+
+// All reflectors of the reduction: on return H's upper part is the Hessenberg
+// form, with the reflectors' tails below its subdiagonal and their scales in
+// tau (n - 2); a skipped reflector has tau 0 and leaves its column's tail.
+int launch_hess_slab(double* h, long long ldh, int n, double* tau, double* work, int sm_count, int* status,
+                     cudaStream_t st) {
+    using namespace hess;
+    SlabArgs a;
+    a.h = h;
+    a.ldh = ldh;
+    a.n = n;
+    a.rows = slab_rows(n, sm_count);
+    a.ld = (n + 3) / 4 * 4;
+    a.tau = tau;
+    const int P = (n + a.rows - 1) / a.rows;
+    a.part = reinterpret_cast<Slot*>(work);
+    a.sig = a.part + (size_t)P * a.ld;
+    a.colv = a.sig + 2 * P;
+    a.prow = a.colv + 2 * (size_t)a.ld;
+    a.w = a.prow + 2 * (size_t)a.ld;
+    a.status = status;
+    a.eps = 1e-12;
+    const void* kern = n > 2 * SLT ? (const void*)hess_slab_kernel<4> : (const void*)hess_slab_kernel<2>;
+    const size_t bytes = slab_smem(n, a.rows);
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) != cudaSuccess)
+        return JLC_E_LAUNCH;
+    // no slot may hold a tag of an earlier call
+    if (cudaMemsetAsync(work, 0, slab_slots(n, P) * sizeof(Slot), st) != cudaSuccess) return JLC_E_CUDA;
+    void* args[] = {&a};
+    return cudaLaunchCooperativeKernel(kern, dim3(P), dim3(SLT), args, bytes, st) == cudaSuccess ? JLC_OK
+                                                                                                  : JLC_E_LAUNCH;
+}
 
 int hess_panel_grid(int m, int sm_count, int* slab) {
     int P = (m + 31) / 32;

@@ -170,82 +170,6 @@ __device__ __forceinline__ bool grid_barrier(unsigned* counter, unsigned target,
     return *s_ok != 0;
 }
 
-// Values exchanged between CTAs of one cooperative launch without a barrier:
-// a slot is 16 bytes, the value and a word that carries the tag of its use
-// and a small integer.  It is written and read by single 128-bit accesses at
-// gpu scope, so a reader that finds the tag has the value: the data is its
-// own flag, and an exchange costs one store and one load through L2 instead of
-// store, fence, counter, poll and load.  Tags grow from use to use; slots are
-// zeroed before the launch and tag 0 is never waited for.
-struct __align__(16) Slot {
-    double v;
-    unsigned lo, tag;
-};
-
-__device__ __forceinline__ void slot_put(Slot* s, double v, unsigned tag, int aux) {
-    const unsigned long long hi = ((unsigned long long)tag << 32) | (unsigned)aux;
-    asm volatile("{\n\t.reg .b128 t;\n\tmov.b128 t, {%1, %2};\n\tst.relaxed.gpu.global.b128 [%0], t;\n\t}" ::"l"(s),
-                 "l"(__double_as_longlong(v)), "l"(hi)
-                 : "memory");
-}
-
-__device__ __forceinline__ void slot_load(const Slot* s, double& v, unsigned& tag, int& aux) {
-    long long lo;
-    unsigned long long hi;
-    asm volatile("{\n\t.reg .b128 t;\n\tld.relaxed.gpu.global.b128 t, [%2];\n\tmov.b128 {%0, %1}, t;\n\t}"
-                 : "=l"(lo), "=l"(hi)
-                 : "l"(s)
-                 : "memory");
-    v = __longlong_as_double(lo);
-    tag = (unsigned)(hi >> 32);
-    aux = (int)(unsigned)hi;
-}
-
-// the value of a slot this thread has already waited for
-__device__ __forceinline__ double slot_value(const Slot* s) {
-    double v;
-    unsigned tag;
-    int aux;
-    slot_load(s, v, tag, aux);
-    return v;
-}
-
-// A wait's occasional check, out of line so that the waits stay small: given
-// the time the wait began (0 at the first check), returns it, or 0 once the
-// limit has passed (which it records) or an error is recorded.
-static __device__ __noinline__ uint64_t slot_check(uint64_t t0, int* status) {
-    const uint64_t now = globaltimer_ns();
-    if (*(volatile int*)status != 0) return 0;
-    if (t0 == 0) return now;
-    if (now - t0 <= wait_limit_ns(status)) return t0;
-    atomicOr(status, JLC_DEV_TIMEOUT);
-    return 0;
-}
-
-// Waits until every one of the N slots carries `tag` and takes their values
-// (and integers): all loads of a round are in flight together.  Bounded like
-// mbar_wait: false once the wait limit has passed or an error is recorded.
-template <int N>
-__device__ __forceinline__ bool slot_wait(const Slot* const (&s)[N], unsigned tag, double (&v)[N], int* status,
-                                          int* aux = nullptr) {
-    uint64_t t0 = 0;
-    unsigned it = 0;
-#pragma unroll 1
-    for (;;) {
-        unsigned bad = 0;
-#pragma unroll
-        for (int i = 0; i < N; ++i) {
-            unsigned tg;
-            int ax;
-            slot_load(s[i], v[i], tg, ax);
-            if (aux) aux[i] = ax;
-            bad |= tg ^ tag;
-        }
-        if (bad == 0) return true;
-        if ((++it & 255u) == 0u && (t0 = slot_check(t0, status)) == 0) return false;
-    }
-}
-
 // --- TMA (cp.async.bulk.tensor), no multicast anywhere in this library ---
 __device__ __forceinline__ void tma_prefetch_desc(const CUtensorMap* map) {
     asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(map)) : "memory");

@@ -96,12 +96,17 @@ size_t hess_work_doubles(long long n);
 // Golub-Kahan bidiagonalisation (bidiag.cu): rows per CTA and CTA count (0:
 // too many rows), the kernel's workspace in doubles, the cooperative launch,
 // and the row reflectors rearranged as the columns of a QR factor.
-int bidiag_grid(int m, int sm_count, int* rows_per_cta);
+int bidiag_grid(int m, int n, int sm_count, int* rows_per_cta);
 size_t bidiag_work_doubles(int m, int n, int sm_count);
 int launch_bidiag(double* a, long long lda, int m, int n, double* d, double* e, double* tauq, double* taup,
                   double* work, int sm_count, int* status, cudaStream_t st);
 int launch_bidiag_right_factor(const double* a, long long lda, int n, double* w, long long ldw, cudaStream_t st);
 int launch_hess_clear(double* h, long long ldh, int n, cudaStream_t st);
+// the whole reduction in one launch, for matrices that fit in the chip's shared memory
+bool hess_slab_fits(int n, int sm_count);
+size_t hess_slab_work_doubles(int n, int sm_count);
+int launch_hess_slab(double* h, long long ldh, int n, double* tau, double* work, int sm_count, int* status,
+                     cudaStream_t st);
 // all reflectors of one panel in one cooperative launch (rows in slabs over
 // up to sm_count CTAs); scratch of hess_panel_scratch_bytes
 size_t hess_panel_scratch_bytes(int sm_count);

@@ -128,3 +128,34 @@ def test_device_entry_arguments(ctx):
     ctx.hessenberg_device(4, a.data_ptr(), 4, None, 4)
     h = a.cpu().numpy().T  # the buffer is column-major
     assert np.all(np.tril(h, -2) == 0.0)
+
+
+@pytest.mark.parametrize("n,with_q", [
+    (3, True), (9, True),            # one CTA, two CTAs
+    (513, True), (1024, False),      # one column past a thread's first; 8 rows per CTA
+    (1025, True), (1200, True),      # 16 rows per CTA, three columns per thread
+    (1744, True), (1745, True),      # the largest order in shared memory, the smallest of the panel route
+])
+def test_route_edges(ctx, n, with_q):
+    """A = Q H Q^T (or the eigenvalue-preserving norms without Q) at the sizes
+    where the one-launch kernel's layout or the route changes, checked with
+    torch in FP64 against a backward stable reduction's residual (a small
+    multiple of n u)."""
+    import torch
+    g = torch.Generator(device="cuda").manual_seed(2300 + n)
+    a = torch.rand(n, n, dtype=torch.float64, device="cuda", generator=g) * 2 - 1   # column-major
+    f = torch.zeros(n, n + 3, dtype=torch.float64, device="cuda")                   # padded leading dimension
+    f[:, :n] = a
+    q = torch.empty(n, n, dtype=torch.float64, device="cuda") if with_q else None
+    torch.cuda.synchronize()
+    ctx.hessenberg_device(n, f.data_ptr(), n + 3, q.data_ptr() if with_q else None, n)
+    assert float(f[:, n:].abs().max()) == 0.0
+    h = f[:, :n].T
+    assert float(torch.tril(h, -2).abs().max()) == 0.0
+    tol = 1e-14 * n
+    assert abs(float(h.norm() / a.norm()) - 1.0) < tol
+    assert abs(float(h.trace() - a.trace())) < tol * float(a.norm())
+    if with_q:
+        q = q.T
+        assert float((a.T - q @ h @ q.T).norm() / a.norm()) < tol
+        assert float((q.T @ q - torch.eye(n, dtype=torch.float64, device="cuda")).norm()) < tol * n ** 0.5
