@@ -5,9 +5,10 @@
 // to the panel's later columns), then the trailing columns are updated with
 // the compact-WY form Q^T C = C - V T^T V^T C as three GEMMs (api.cu).
 //
-//   qr_panel_cl_kernel: the panel on one thread-block cluster (1..16 CTAs,
-//                      each holding a slab of rows in shared memory), one
-//                      cluster barrier per column;
+//   qr_panel_rg_kernel: the panel on one thread-block cluster (1..16 CTAs),
+//                      the rows held in registers; panels of up to 4096 rows;
+//   qr_panel_cl_kernel: the same with the rows in shared memory and one
+//                      cluster barrier per column; panels of up to 6400 rows;
 //   qr_panel_sm_kernel / qr_panel_mp_kernel: taller panels on a cooperative
 //                      grid of up to one CTA per SM, slabs in shared memory
 //                      or (taller still) in place, one grid barrier per column;
@@ -27,15 +28,11 @@
 
 #include "jlc_device.cuh"
 #include "jlc_internal.h"
+#include "jlc_slab.cuh"
 
 namespace jlc {
 namespace qr {
 
-__device__ __forceinline__ double warp_sum(double v) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    return v;
-}
 __device__ __forceinline__ double warp_max(double v) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
@@ -633,6 +630,273 @@ __global__ void __launch_bounds__(CL_THREADS, 1) qr_panel_cl_kernel(double* A, l
     }
 }
 
+// The panel on one cluster with the rows held in registers: lane l of warp w
+// holds rows l, l + 32, ... (NR of them) of columns w, w + 16, w + 32, w + 48
+// for the whole panel.  Per column:
+//   * the warp that holds the pivot column scales its entries below the pivot
+//     by 2^-e (e the exponent of the CTA's maximum) into shared memory; one CTA
+//     barrier, the only one of the step;
+//   * every warp forms the dots of its columns with it and sends them to all
+//     CTAs of the cluster (16 destinations x 4 values, one 16-byte st.async per
+//     lane); the last warp also sends the sum of squares and e, and the CTA
+//     that holds row k its entries of the row;
+//   * the stores signal the destination's mbarrier, which expects a fixed
+//     number of bytes per column; every warp waits for it, merges the CTAs'
+//     values for its own columns and forms the reflector (the same bits in
+//     every warp and CTA), and updates its registers.
+// Two buffers alternate by column parity: a CTA sends column k + 2 only after
+// it has every CTA's column k + 1, which each sends after merging column k.
+//
+// A column is a chain of latencies: the exchange (about 900 cycles from the
+// first send to the last arrival at 16 CTAs), the merge and the reflector
+// (FP64 sums over lanes, a square root, a division: 1 100), the update and the
+// next pivot column (800), the dots (300); no pass touches shared memory but
+// for the pivot column.  The shared-memory cluster kernel walks its slab three
+// times per column between five CTA barriers and a cluster barrier, in 53 KB of
+// code.  us per column on B200: 2304 rows 5.7 -> 2.5, 1024 rows 5.1 -> 2.1.
+constexpr int RG_THREADS = 512, RG_WARPS = RG_THREADS / 32;
+constexpr int RG_MAX = 16;              // CTAs of the cluster
+constexpr int RG_COLS = 64 / RG_WARPS;  // columns per warp
+constexpr int RG_PART = 66;             // doubles from one CTA: 64 dots (4 w + j: column w + 16 j), sum of squares, exponent
+constexpr int RG_MAX_NR = 8;
+constexpr int kRgEmpty = -4096;
+
+__device__ __forceinline__ uint32_t cluster_addr(const void* p, int rank) {
+    uint32_t a;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_u32(p)), "r"(rank));
+    return a;
+}
+// 16 bytes to a CTA of the cluster, counted by the mbarrier `bar` there
+__device__ __forceinline__ void send2(uint32_t dst, double x, double y, uint32_t bar) {
+    asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v2.f64 [%0], {%1, %2}, [%3];" ::"r"(dst),
+                 "d"(x), "d"(y), "r"(bar)
+                 : "memory");
+}
+// Bounded wait for what the CTAs of the cluster send (false: the wait limit has passed or an error is recorded)
+__device__ __forceinline__ bool wait_sent(uint64_t* bar, uint32_t parity, int* status) {
+    const uint32_t b = smem_u32(bar);
+    uint64_t t0 = 0;
+    unsigned it = 0;
+#pragma unroll 1
+    for (;;) {
+        uint32_t ok;
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+            "selp.u32 %0, 1, 0, p;\n\t}"
+            : "=r"(ok)
+            : "r"(b), "r"(parity)
+            : "memory");
+        if (ok) return true;
+        if ((++it & 255u) == 0u && (t0 = slot_check(t0, status)) == 0) return false;
+    }
+}
+
+struct RgReflector {
+    double tau, beta, v0s;  // v0s = 2^E / (x0 - beta)
+    int mode;               // 0: no reflector, 1: reflector, 2: sign flip (tau = 2)
+};
+// computeHouseholder's recipe from x0, the tail's sum of squares S 4^E and E,
+// by a whole warp: the half-warps take one of the two quotients each
+__device__ __forceinline__ RgReflector rg_reflector(double x0, double S, int E) {
+    RgReflector h{0.0, x0, 0.0, 0};
+    if (S > 0.0) {
+        const double xn = x0 * sp_pow2(-E);
+        const double nb = -copysign(sqrt(fma(xn, xn, S)), xn);
+        const bool lower = (threadIdx.x & 16) == 0;
+        const double q = (lower ? nb - xn : 1.0) / (lower ? nb : xn - nb);
+        h.mode = 1;
+        h.beta = nb * sp_pow2(E);
+        h.tau = __shfl_sync(0xffffffffu, q, 0);
+        h.v0s = __shfl_sync(0xffffffffu, q, 16);
+    } else if (x0 < 0.0) {
+        h.mode = 2;
+        h.beta = -x0;
+        h.tau = 2.0;
+    }
+    return h;
+}
+// how many of the 32 column pairs (columns w + 32 i, w + 32 i + 16) still hold a column >= kk
+__device__ __forceinline__ int rg_live_pairs(int kk) { return 32 - min(16, max(0, kk - 16)) - min(16, max(0, kk - 48)); }
+
+template <int NR>
+__global__ void __launch_bounds__(RG_THREADS, 1) qr_panel_rg_kernel(double* A, long long lda, int m, int k0, int kb,
+                                                                    double* tau, int* status) {
+    __shared__ __align__(16) double part[2][RG_MAX][RG_PART];
+    __shared__ __align__(16) double rrec[2][64];  // row k, by the dots' index
+    __shared__ double s_x[NR * 32];               // the pivot column below the pivot, times 2^-e
+    __shared__ int s_e;
+    __shared__ __align__(16) double s_row[64];
+    __shared__ __align__(8) uint64_t bar[2];
+    cg::cluster_group cluster = cg::this_cluster();
+    const int P = (int)cluster.num_blocks(), cta = (int)cluster.block_rank();
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int R = (m - k0 + P - 1) / P;
+    const int r0 = k0 + cta * R, rows = max(0, min(m - r0, R));
+    // what column kk's mbarrier phase expects: the live pairs' dots and one pair of scalars from
+    // every CTA, and the row's live pairs
+    auto bytes = [&](int kk) { return (uint32_t)((P + 1) * rg_live_pairs(kk) + P) * 16u; };
+    if (tid == 0) {
+        mbar_init(&bar[0], 1);
+        mbar_init(&bar[1], 1);
+        fence_barrier_init();
+        mbar_arrive_expect_tx(&bar[0], bytes(0));
+        mbar_arrive_expect_tx(&bar[1], bytes(1));
+    }
+    double a[RG_COLS][NR], x[NR];
+#pragma unroll
+    for (int j = 0; j < RG_COLS; ++j)
+#pragma unroll
+        for (int r = 0; r < NR; ++r) {
+            const int c = warp + RG_WARPS * j, i = lane + 32 * r;
+            a[j][r] = c < kb && i < rows ? A[(long long)(k0 + c) * lda + r0 + i] : 0.0;
+        }
+    cluster.sync();  // every CTA's mbarriers are ready
+    bool fail = false;
+    // sends: lane 2 d + h the warp's column pair h to CTA d
+    const int dest = lane >> 1, half = lane & 1;
+    const uint32_t to_part = cluster_addr(&part[0][cta][warp * 4 + 2 * half], dest < P ? dest : 0);
+    const uint32_t to_rrec = cluster_addr(&rrec[0][warp * 4 + 2 * half], dest < P ? dest : 0);
+    const uint32_t to_bar = cluster_addr(&bar[0], dest < P ? dest : 0);
+    // Column c of this warp (y), below the pivot and scaled by 2^-e, into shared memory
+    auto put_pivot = [&](double (&y)[NR], int k) {
+        unsigned hi = 0;
+#pragma unroll
+        for (int r = 0; r < NR; ++r) {
+            if (r0 + lane + 32 * r < k) y[r] = 0.0;
+            hi = max(hi, (unsigned)__double2hiint(y[r]) & 0x7fffffffu);
+        }
+        hi = __reduce_max_sync(0xffffffffu, hi) >> 20;  // the maximum's biased exponent
+        const int e = hi == 0x7ff ? 0 : min(1000, max(-1000, (int)hi - 1023));
+        const double sc = sp_pow2(-e);
+#pragma unroll
+        for (int r = 0; r < NR; ++r) s_x[lane + 32 * r] = r0 + lane + 32 * r > k ? y[r] * sc : 0.0;
+        if (lane == 0) s_e = hi == 0 ? kRgEmpty : e;  // (zeros and denormals: no reflector)
+    };
+    if (warp == 0) {
+        double y[NR];
+#pragma unroll
+        for (int r = 0; r < NR; ++r) y[r] = a[0][r];
+        put_pivot(y, k0);
+    }
+#pragma unroll 1
+    for (int kk = 0; kk < kb; ++kk) {
+        const int k = k0 + kk, par = kk & 1;
+        const bool live = dest < P && warp + RG_WARPS * (2 * half + 1) >= kk;
+        // ---- row k's entries of this warp's columns, from the lane that holds them
+        if (k >= r0 && k < r0 + rows) {
+#pragma unroll
+            for (int r = 0; r < NR; ++r)
+                if (r0 + lane + 32 * r == k) {
+#pragma unroll
+                    for (int j = 0; j < RG_COLS; ++j) s_row[warp * 4 + j] = a[j][r];
+                }
+            __syncwarp();
+            const double2 v = *reinterpret_cast<const double2*>(&s_row[warp * 4 + 2 * half]);
+            if (live) send2(to_rrec + par * 512u, v.x, v.y, to_bar + par * 8u);
+        }
+        if (__syncthreads_or(fail)) break;  // the pivot column is in shared memory
+        // ---- this CTA's dots with it
+        const int e_own = s_e;
+        double d[RG_COLS];
+#pragma unroll
+        for (int j = 0; j < RG_COLS; ++j) d[j] = 0.0;
+#pragma unroll
+        for (int r = 0; r < NR; ++r) {
+            x[r] = s_x[lane + 32 * r];
+#pragma unroll
+            for (int j = 0; j < RG_COLS; ++j) d[j] = fma(x[r], a[j][r], d[j]);
+        }
+        {
+            // the four sums over the lanes: lanes with bit 0 = half keep columns 2 half, 2 half + 1
+            double k0v = half ? d[2] : d[0], k1v = half ? d[3] : d[1];
+            k0v += shfl_xor(half ? d[0] : d[2], 1);
+            k1v += shfl_xor(half ? d[1] : d[3], 1);
+            const bool second = lane & 2;
+            double v = (second ? k1v : k0v) + shfl_xor(second ? k0v : k1v, 2);
+            v += shfl_xor(v, 4);
+            v += shfl_xor(v, 8);
+            v += shfl_xor(v, 16);
+            const double o = shfl_xor(v, 2);
+            if (live)
+                send2(to_part + par * (uint32_t)sizeof(part[0]), second ? o : v, second ? v : o, to_bar + par * 8u);
+        }
+        if (warp == RG_WARPS - 1) {
+            double q = 0.0;
+#pragma unroll
+            for (int r = 0; r < NR; ++r) q = fma(x[r], x[r], q);
+            q = warp_sum(q);
+            if (lane < P) send2(cluster_addr(&part[par][cta][64], lane), q, (double)e_own, cluster_addr(&bar[par], lane));
+        }
+        // ---- merge: lane q (and q + 16) takes CTA q's dots of columns 0, 1 (2, 3) of this warp
+        fail |= !wait_sent(&bar[par], (kk >> 1) & 1, status);
+        __syncwarp();
+        const int q = lane & 15, h = lane >> 4;
+        const double* pq = part[par][q < P ? q : 0];
+        const double2 se = *reinterpret_cast<const double2*>(pq + 64);
+        const double2 dd = *reinterpret_cast<const double2*>(pq + warp * 4 + 2 * h);
+        const double2 rr = *reinterpret_cast<const double2*>(&rrec[par][warp * 4 + 2 * h]);
+        const double x0 = rrec[par][(kk & (RG_WARPS - 1)) * 4 + kk / RG_WARPS];
+        const int eq = q < P ? (int)se.y : kRgEmpty;
+        const int E = __reduce_max_sync(0xffffffffu, eq);
+        const double f = eq - E >= -1022 && q < P ? sp_pow2(eq - E) : 0.0;
+        double S = (se.x * f) * f;
+        const bool second = lane & 8;
+        double dot = (second ? dd.y : dd.x) * f + shfl_xor((second ? dd.x : dd.y) * f, 8);
+        S += shfl_xor(S, 8);
+#pragma unroll
+        for (int o = 4; o > 0; o >>= 1) {
+            S += shfl_xor(S, o);
+            dot += shfl_xor(dot, o);
+        }
+        const RgReflector hh = m - k > 1 && E > kRgEmpty ? rg_reflector(x0, S, E) : RgReflector{0.0, x0, 0.0, 0};
+        if (cta == 0 && tid == 0) tau[k] = hh.tau;
+        if (tid == 0) mbar_arrive_expect_tx(&bar[par], bytes(kk + 2));  // armed for column kk + 2
+        // ---- update: f_t = tau (a_kt + dot v0s), columns right of the pivot
+        const double ft = hh.tau * fma(dot, hh.v0s, second ? rr.y : rr.x);
+        const double sv = hh.mode == 1 && e_own - E >= -1022 ? sp_pow2(e_own - E) * hh.v0s : 0.0;
+        double fj[RG_COLS];
+#pragma unroll
+        for (int j = 0; j < RG_COLS; ++j) {
+            const double v = __shfl_sync(0xffffffffu, ft, (j >> 1) * 16 + (j & 1) * 8);
+            fj[j] = warp + RG_WARPS * j > kk && hh.mode != 0 ? v : 0.0;
+        }
+#pragma unroll
+        for (int r = 0; r < NR; ++r) x[r] = r0 + lane + 32 * r == k ? 1.0 : x[r] * sv;  // v (0 above row k)
+        if (kk + 1 < kb && warp == ((kk + 1) & (RG_WARPS - 1))) {
+            // the next pivot column ahead of the rest: the other warps wait for it
+            const int jn = (kk + 1) / RG_WARPS;
+            const double f = jn == 0 ? fj[0] : jn == 1 ? fj[1] : jn == 2 ? fj[2] : fj[3];
+            double y[NR];
+#pragma unroll
+            for (int r = 0; r < NR; ++r)
+                y[r] = fma(-f, x[r], jn == 0 ? a[0][r] : jn == 1 ? a[1][r] : jn == 2 ? a[2][r] : a[3][r]);
+            put_pivot(y, k + 1);
+        }
+#pragma unroll
+        for (int j = 0; j < RG_COLS; ++j) {
+#pragma unroll
+            for (int r = 0; r < NR; ++r) a[j][r] = fma(-fj[j], x[r], a[j][r]);
+            if (warp + RG_WARPS * j == kk) {  // the pivot column itself: its tail, and beta on row k
+#pragma unroll
+                for (int r = 0; r < NR; ++r) {
+                    const int g = r0 + lane + 32 * r;
+                    if (g == k) a[j][r] = hh.beta;
+                    else if (g > k && hh.mode == 1) a[j][r] = x[r];
+                }
+            }
+        }
+    }
+    cluster.sync();  // no CTA leaves while another may still send to it
+#pragma unroll
+    for (int j = 0; j < RG_COLS; ++j)
+#pragma unroll
+        for (int r = 0; r < NR; ++r) {
+            const int c = warp + RG_WARPS * j, i = lane + 32 * r;
+            if (c < kb && i < rows) A[(long long)(k0 + c) * lda + r0 + i] = a[j][r];
+        }
+}
+
 // V (ldv x 64, column-major): column i < kb holds reflector k0+i (zeros above
 // row k0+i, one on it, A's tail below); columns kb .. 63 are zero.
 __global__ void qr_pack_v_kernel(const double* A, long long lda, int m, int k0, int kb, double* V, long long ldv) {
@@ -825,6 +1089,31 @@ int launch_qr_panel(double* a, long long lda, int m, int k0, int kb, double* tau
     // one CTA per 64 rows, up to the largest cluster (measured against 128
     // rows per CTA: 13.8 vs 14.2 ms at 2048^2, 32.6 vs 33.0 at 4096^2)
     const int cl = max(1, min((m - k0) / 64, min(cluster_max, qr::CL_MAX)));
+    const int rows = (m - k0 + cl - 1) / cl;
+    // rows in registers while every CTA has at most 256 (3.2 us per column at 4000 rows, against 6.8
+    // with the slab in shared memory and 9.4 on the grid)
+    if (rows <= 32 * qr::RG_MAX_NR) {
+        using namespace qr;
+        static void (*const kerns[RG_MAX_NR + 1])(double*, long long, int, int, int, double*, int*) = {
+            nullptr,
+            qr_panel_rg_kernel<1>, qr_panel_rg_kernel<2>, qr_panel_rg_kernel<3>, qr_panel_rg_kernel<4>,
+            qr_panel_rg_kernel<5>, qr_panel_rg_kernel<6>, qr_panel_rg_kernel<7>, qr_panel_rg_kernel<8>};
+        auto kern = kerns[(rows + 31) / 32];
+        if (cudaFuncSetAttribute((const void*)kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess)
+            return JLC_E_LAUNCH;
+        cudaLaunchConfig_t cfg = {};
+        cudaLaunchAttribute at[1];
+        cfg.gridDim = dim3(cl);
+        cfg.blockDim = dim3(qr::RG_THREADS);
+        cfg.stream = st;
+        at[0].id = cudaLaunchAttributeClusterDimension;
+        at[0].val.clusterDim.x = cl;
+        at[0].val.clusterDim.y = 1;
+        at[0].val.clusterDim.z = 1;
+        cfg.attrs = at;
+        cfg.numAttrs = 1;
+        return cudaLaunchKernelEx(&cfg, kern, a, lda, m, k0, kb, tau, status) == cudaSuccess ? JLC_OK : JLC_E_LAUNCH;
+    }
     if ((size_t)((m - k0 + cl - 1) / cl) * kb * sizeof(double) <= (size_t)qr::CL_MAX_SLAB_BYTES) {
         const void* kern = (const void*)qr::qr_panel_cl_kernel;
         if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, qr::CL_MAX_SLAB_BYTES) !=

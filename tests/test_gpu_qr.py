@@ -179,3 +179,35 @@ def test_qr_extreme_column_scales(ctx, oracle, m, n):
     tol = 1e-11 * max(1.0, np.abs(f_ref).max())
     np.testing.assert_allclose(np.where(up, f / s, 0.0), np.where(up, f_ref, 0.0), rtol=0, atol=tol)
     np.testing.assert_allclose(np.where(up, 0.0, f), np.where(up, 0.0, f_ref), rtol=0, atol=tol)
+
+
+@pytest.mark.parametrize("m,n", [
+    (64, 64), (127, 70), (128, 64), (129, 30),      # one CTA of up to four row slots, two CTAs
+    (1024, 70), (1025, 70), (2049, 64), (2561, 70),  # 16 CTAs of 64, 65, 129 and 161 rows
+    (4096, 37), (4097, 70), (4500, 130),            # the last size in registers; past it; both in one factorisation
+])
+def test_panel_kernel_edges(ctx, oracle, m, n):
+    """The panel at the row counts where its cluster size, its rows per lane
+    and its kernel change, and panels narrower than 64 columns, against the
+    restatement (tolerances as for the other sizes)."""
+    a = oracle.uniform((m, n), 7 * m + n)
+    if n > 40:
+        a[3:, 2] = 0.0      # a reflector whose tail vanishes after two steps, or nearly
+        a[:, 20] = 0.0      # a zero column
+    at, tau = _factor(ctx, a)
+    f = at[:, :m].cpu().numpy().T
+    f_ref, tau_ref = oracle.householder_qr_blocked(a)
+    np.testing.assert_allclose(tau.cpu().numpy()[:n], tau_ref, rtol=0, atol=1e-12)
+    np.testing.assert_allclose(f, f_ref, rtol=0, atol=1e-11 * max(1.0, np.abs(f_ref).max()))
+
+
+def test_panel_sign_flip_and_last_row(ctx, oracle):
+    """A column that is zero below a negative diagonal entry (tau = 2, a sign
+    flip) and a square panel, whose last column has no reflector."""
+    a = np.triu(oracle.uniform((64, 64), 71))
+    a[5, 5] = -0.75
+    a[6, 6] = 0.5
+    at, tau = _factor(ctx, a)
+    f_ref, tau_ref = oracle.householder_qr_blocked(a)
+    np.testing.assert_allclose(tau.cpu().numpy(), tau_ref, rtol=0, atol=1e-12)
+    np.testing.assert_allclose(at[:, :64].cpu().numpy().T, f_ref, rtol=0, atol=1e-11)
