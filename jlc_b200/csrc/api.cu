@@ -217,7 +217,7 @@ int run_device(jlc_ctx* ctx, const GemmDesc& g0, int precision, int slices, jlc_
     // the Ozaki split data when the FP64 kernel is the gated fallback, so
     // that its split choice, and with it its sums, match the native route).
     const int ksplit = g.dot_mat ? 1 : dmma_splitk(whole_m, g.n, g.k, ctx->sm_count);
-    const size_t splitk_bytes = dmma_splitk_bytes(g.m, g.n, ksplit);
+    const size_t splitk_bytes = dmma_splitk_bytes(g.m, g.n, g.k, ksplit, ctx->sm_count);
     size_t splitk_off = 0;
     int rc = JLC_OK;
     if (ozaki) {
@@ -314,7 +314,8 @@ int run_device(jlc_ctx* ctx, const GemmDesc& g0, int precision, int slices, jlc_
     ctx->launches += 1;
     return launch_dgemm_dmma(g, ctx->stream, ctx->sm_count, ctx->d_status, ozaki ? ctx->d_flags : nullptr,
                              ctx->dmma_k, ctx->err, sizeof(ctx->err), ksplit,
-                             splitk_bytes ? static_cast<char*>(ctx->ws.ptr) + splitk_off : nullptr, splitk_bytes);
+                             splitk_bytes ? static_cast<char*>(ctx->ws.ptr) + splitk_off : nullptr, splitk_bytes,
+                             ctx->d_counters);
 }
 
 int finish_sync(jlc_ctx* ctx) {
@@ -325,6 +326,8 @@ int finish_sync(jlc_ctx* ctx) {
     if (e != cudaSuccess) return cuda_err(ctx, e, "status read");
     if (st != 0) {
         cudaMemset(ctx->d_status, 0, sizeof(int));
+        // a kernel that gave up may have left split-K arrivals behind
+        cudaMemset(ctx->d_counters, 0, kSplitTiles * sizeof(int));
         if (st & JLC_DEV_TIMEOUT) return set_err(ctx, JLC_E_TIMEOUT, "a device wait timed out (status 0x%x)", st);
         return set_err(ctx, JLC_E_CUDA, "device status 0x%x", st);
     }
@@ -795,9 +798,11 @@ int jlc_init(int device, jlc_ctx** out) {
     bool ok = cudaStreamCreateWithFlags(&ctx->own_stream, cudaStreamNonBlocking) == cudaSuccess &&
               cudaMalloc(&ctx->d_status, 4 * sizeof(int)) == cudaSuccess &&
               cudaMalloc(&ctx->d_flags, 4 * sizeof(int)) == cudaSuccess &&
+              cudaMalloc(&ctx->d_counters, kSplitTiles * sizeof(int)) == cudaSuccess &&
               cudaEventCreate(&ctx->ev0) == cudaSuccess && cudaEventCreate(&ctx->ev1) == cudaSuccess;
     if (ok) ok = cudaMemset(ctx->d_status, 0, 4 * sizeof(int)) == cudaSuccess &&
-                 cudaMemset(ctx->d_flags, 0, 4 * sizeof(int)) == cudaSuccess;
+                 cudaMemset(ctx->d_flags, 0, 4 * sizeof(int)) == cudaSuccess &&
+                 cudaMemset(ctx->d_counters, 0, kSplitTiles * sizeof(int)) == cudaSuccess;
     if (!ok) {
         cudaGetLastError();
         jlc_destroy(ctx);
@@ -856,13 +861,13 @@ int jlc_autotune_splitk(jlc_ctx* ctx, int64_t m, int64_t n, int64_t k, int* spli
     float best_ms = 0.f;
     for (int s = 1; s <= 8; ++s) {
         if (!dmma_splitk_legal(tiles, kbl, s, ctx->sm_count)) continue;
-        const size_t wsb = dmma_splitk_bytes(m, n, s);
+        const size_t wsb = dmma_splitk_bytes(m, n, k, s, ctx->sm_count);
         if (wsb && (rc = ws_reserve(ctx, wsb))) return rc;
         float ms_min = 0.f;
         for (int rep = 0; rep < 4; ++rep) {  // one warm-up, three timed
             cudaEventRecord(ctx->ev0, ctx->stream);
             rc = launch_dgemm_dmma(g, ctx->stream, ctx->sm_count, ctx->d_status, nullptr, ctx->dmma_k, ctx->err,
-                                   sizeof(ctx->err), s, wsb ? ctx->ws.ptr : nullptr, wsb);
+                                   sizeof(ctx->err), s, wsb ? ctx->ws.ptr : nullptr, wsb, ctx->d_counters);
             if (rc) return rc;
             cudaEventRecord(ctx->ev1, ctx->stream);
             cudaError_t e = cudaEventSynchronize(ctx->ev1);
@@ -907,6 +912,7 @@ void jlc_destroy(jlc_ctx* ctx) {
     if (ctx->ws.ptr) cudaFree(ctx->ws.ptr);
     if (ctx->d_status) cudaFree(ctx->d_status);
     if (ctx->d_flags) cudaFree(ctx->d_flags);
+    if (ctx->d_counters) cudaFree(ctx->d_counters);
     stager_destroy(ctx->stager);
     for (int i = 0; i < 2 * jlc_ctx::kMaxRec; ++i)
         if (ctx->rec_ev[i]) cudaEventDestroy(ctx->rec_ev[i]);

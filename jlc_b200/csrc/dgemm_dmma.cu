@@ -16,17 +16,19 @@
 // Structure: persistent CTAs (one per SM), warp-specialised, 3 warpgroups.
 // Warpgroup 0 is the producer (one lane issues TMA into a STAGES-deep ring
 // guarded by full/empty mbarriers) and gives registers back with
-// setmaxnreg.dec; warpgroups 1-2 are the 8 consumer warps, arranged 2 (M) x
-// 4 (N), each owning a 64 x 32 slab of the 128 x 128 C tile as 4 x 4 m16n8
-// accumulators, and take the registers with setmaxnreg.inc.
+// setmaxnreg.dec; warpgroups 1-2 are the 8 consumer warps (for a 128 x 128 C
+// tile 2 (M) x 4 (N), each owning a 64 x 32 slab as 4 x 4 m16n8 accumulators),
+// and take the registers with setmaxnreg.inc.
 // Register budget: the launch gives 384 threads x 168 = 64512 registers;
 // after the split 128 x 40 + 256 x 224 = 62464 are in use.
 //
-// Split-K (small products, fewer tiles than half the SMs): the k-blocks of a
-// tile are cut into ksplit contiguous parts, one work unit each.  A unit's
-// partial tile goes to workspace; the CTA whose unit arrives last at the
-// tile's counter sums the parts in index order (deterministic whatever the
-// arrival order) and runs the normal epilogue.  No CTA waits for another.
+// Split-K (products whose tiles would leave SMs idle): the k-blocks of a tile
+// are cut into ksplit contiguous parts, one work unit each.  A unit's partial
+// tile goes to workspace; the CTA whose unit arrives last at the tile's counter
+// sums the parts in index order (deterministic whatever the arrival order),
+// clears the counter and runs the normal epilogue.  No CTA waits for another.
+// The tile shape does not enter the sums: an element is the same chain of MMAs
+// over k in every shape, so only the split decides a result's bits.
 //
 // K permutation: inside each k-step the logical k index of the mma fragment
 // layout is remapped to a physical column of the shared tile so that the four
@@ -46,38 +48,31 @@
 namespace jlc {
 namespace dmma {
 
-constexpr int BM = 128, BN = 128, BK = 16;  // BK in doubles: one 128-byte swizzle row
-constexpr int STAGES = 5;
-constexpr int WARPS_M = 2, WARPS_N = 4, MMA_WARPS = WARPS_M * WARPS_N;
-constexpr int WM = BM / WARPS_M, WN = BN / WARPS_N;  // 64 x 32 per warp
-constexpr int MT = WM / 16, NT = WN / 8;              // 4 x 4 m16n8 tiles
+constexpr int BK = 16;  // in doubles: one 128-byte swizzle row
+constexpr int MMA_WARPS = 8;
 constexpr int PRODUCER_WARPS = 4;  // one full warpgroup, required by setmaxnreg
 constexpr int THREADS = (MMA_WARPS + PRODUCER_WARPS) * 32;
 constexpr int PRODUCER_REGS = 40, CONSUMER_REGS = 224;
 static_assert(PRODUCER_WARPS * 32 * PRODUCER_REGS + MMA_WARPS * 32 * CONSUMER_REGS <= THREADS * 168,
               "setmaxnreg split exceeds the registers the CTA is launched with");
-constexpr int A_STAGE = BM * BK * 8;  // 16 KB
-constexpr int B_STAGE = BN * BK * 8;  // 16 KB
-constexpr int STAGE_BYTES = A_STAGE + B_STAGE;
-constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 + 2 * STAGES * 8 + MMA_WARPS * 8;
 
-// Tile shapes of the kernel: 128 x 128 (2 x 4 warps of 64 x 32), and for
-// products with few rows -- the panel GEMMs of blocked factorisations, 32 or
-// 64 rows -- 64 x 128 or 32 x 128 (1 x 8 warps of 64 x 16 or 32 x 16), so
-// that a thin product does not run 128-row tiles that are mostly empty.
-// Smaller tiles take more ring stages in the same shared memory.
-template <int TBM>
+// Tile shapes of the kernel, WARPS_M x WARPS_N warps each: 128 x 128 (2 x 4
+// warps of 64 x 32) and smaller ones, down to 32 x 32, for products that would
+// leave SMs idle or run tiles that are mostly empty (dmma_plan).  Smaller tiles
+// take more ring stages in the same shared memory.
+template <int TBM, int TBN>
 struct Cfg {
-    static constexpr int BM = TBM;
-    static constexpr int WARPS_M = TBM >= 128 ? 2 : 1, WARPS_N = MMA_WARPS / WARPS_M;
+    static constexpr int BM = TBM, BN = TBN;
+    static constexpr int WARPS_M = TBN == 128 ? (TBM >= 128 ? 2 : 1) : (TBM >= 128 || TBN == 32) && TBM > 32 ? 4 : 2;
+    static constexpr int WARPS_N = MMA_WARPS / WARPS_M;
     static constexpr int WM = BM / WARPS_M, WN = BN / WARPS_N;
-    static constexpr int MT = WM / 16, NT = WN / 8;
-    static constexpr int A_STAGE = BM * BK * 8;
+    static constexpr int MT = WM / 16, NT = WN / 8;  // m16n8 tiles per warp
+    static constexpr int A_STAGE = BM * BK * 8, B_STAGE = BN * BK * 8;
     static constexpr int STAGE_BYTES = A_STAGE + B_STAGE;
-    static constexpr int STAGES = (160 * 1024) / STAGE_BYTES;
+    static constexpr int STAGES = (160 * 1024) / STAGE_BYTES > 10 ? 10 : (160 * 1024) / STAGE_BYTES;
     static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 + 2 * STAGES * 8 + MMA_WARPS * 8;
+    static_assert(MT * 16 == WM && NT * 8 == WN && MT > 0 && NT > 0, "warp tile");
 };
-static_assert(Cfg<128>::STAGES == STAGES && Cfg<128>::SMEM_BYTES == SMEM_BYTES, "128-row tile");
 constexpr int RASTER_GROUP = 8;
 
 struct Params {
@@ -92,7 +87,7 @@ struct Params {
     int tiles_m, tiles_n, num_tiles, k_blocks;
     int ksplit;         // k parts per tile (1: no split)
     double* part;       // ksplit > 1: BM*BN partial sums per (tile, part)
-    int* counters;      // ksplit > 1: arrivals per tile, zero at launch
+    int* counters;      // ksplit > 1: arrivals per tile, zero between launches
     int* status;
     const int* gate;  // when non-null the kernel runs only if an Ozaki call's flags ask for FP64
     int withhold;     // test hook: CTA 0 leaves its first stage unloaded, so a bounded wait runs out
@@ -112,13 +107,12 @@ __device__ __forceinline__ void drain_wait(uint64_t* bar, uint32_t parity, int* 
     }
 }
 
-template <bool A_KMAJOR, bool B_KMAJOR, int MMA_K, int TBM>
+template <bool A_KMAJOR, bool B_KMAJOR, int MMA_K, int TBM, int TBN>
 __global__ void __launch_bounds__(THREADS, 1)
     dgemm_dmma_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB,
                       const Params p) {
-    // this instance's tile shape (shadows the 128-row defaults)
-    using C = Cfg<TBM>;
-    constexpr int BM = C::BM, WARPS_N = C::WARPS_N, WM = C::WM, WN = C::WN, MT = C::MT, NT = C::NT;
+    using C = Cfg<TBM, TBN>;
+    constexpr int BM = C::BM, BN = C::BN, WARPS_N = C::WARPS_N, WM = C::WM, WN = C::WN, MT = C::MT, NT = C::NT;
     constexpr int A_STAGE = C::A_STAGE, STAGE_BYTES = C::STAGE_BYTES, STAGES = C::STAGES;
     if (p.gate != nullptr && (p.gate[kFlagNonfiniteA] | p.gate[kFlagFallback] | p.gate[kFlagNonfiniteB]) == 0) return;
     extern __shared__ __align__(1024) unsigned char smem_raw[];
@@ -319,7 +313,11 @@ __global__ void __launch_bounds__(THREADS, 1)
             __threadfence();
             int* last_flag = reinterpret_cast<int*>(empty + STAGES);
             asm volatile("bar.sync 2, %0;" ::"n"(MMA_WARPS * 32) : "memory");
-            if (ct == 0) *last_flag = atomicAdd(&p.counters[tile], 1) == p.ksplit - 1;
+            if (ct == 0) {
+                const bool last = atomicAdd(&p.counters[tile], 1) == p.ksplit - 1;
+                if (last) p.counters[tile] = 0;  // as the next launch expects it
+                *last_flag = last;
+            }
             asm volatile("bar.sync 2, %0;" ::"n"(MMA_WARPS * 32) : "memory");
             // (the next unit's write of the flag comes after its first barrier,
             // which every consumer reaches only after reading this one)
@@ -411,11 +409,11 @@ __global__ void __launch_bounds__(THREADS, 1)
     }
 }
 
-template <bool AK, bool BK_, int MK, int TBM>
+template <bool AK, bool BK_, int MK, int TBM, int TBN>
 static int launch_variant(const CUtensorMap& ma, const CUtensorMap& mb, const Params& p, int grid,
                           cudaStream_t st) {
-    auto kern = dgemm_dmma_kernel<AK, BK_, MK, TBM>;
-    constexpr int smem = Cfg<TBM>::SMEM_BYTES;
+    auto kern = dgemm_dmma_kernel<AK, BK_, MK, TBM, TBN>;
+    constexpr int smem = Cfg<TBM, TBN>::SMEM_BYTES;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return JLC_E_LAUNCH;
     kern<<<grid, THREADS, smem, st>>>(ma, mb, p);
@@ -424,14 +422,51 @@ static int launch_variant(const CUtensorMap& ma, const CUtensorMap& mb, const Pa
 
 }  // namespace dmma
 
-// tile height for an m-row product: 32 or 64 rows for thin products, else 128
+// tile height of the split-K classes: 32 or 64 rows for thin products, else 128
 int dmma_bm(long long m) { return m <= 32 ? 32 : (m <= 64 ? 64 : 128); }
 
-int dmma_grid(long long m, long long n, int sm_count) {
-    const long long bm = dmma_bm(m);
-    const long long tiles = ((m + bm - 1) / bm) * ((n + dmma::BN - 1) / dmma::BN);
-    return (int)(tiles < sm_count ? tiles : sm_count);
+namespace {
+struct Tile {
+    int bm, bn;
+};
+// the shapes the kernel is built for, largest first
+constexpr Tile kTiles[] = {{128, 128}, {128, 64}, {64, 128}, {64, 64}, {32, 128}, {64, 32}, {32, 64}, {32, 32}};
+
+// Estimated cycles of an m x n x k product on (bm x bn) tiles with k in s
+// parts: waves of the persistent grid, each of a unit's k-blocks (an area's
+// worth of MMAs at 0.88 of the DMMA rate and the ring's hand-over), its
+// epilogue, and with a split the partial tile's trip through L2.  Fitted to a
+// sweep of all tiles and splits over products from 32 x 32 x 4096 to 4096 x
+// 4096 x 256 on B200; the shape it picks is within 3 % of the best of the sweep,
+// in us (128 x 128 tiles with their best split -> this rule): 96 x 80 x 112
+// 23.6 -> 8.9, 256^3 47 -> 10, 512^3 54 -> 17, 700^3 70 -> 33, 1024^3 93 -> 84,
+// 2048^3 597 -> 569, 32 x 32 x 4096 93 -> 15, 64 x 2048 x 2304 63 -> 33.
+double tile_cost(const Tile& t, long long m, long long n, long long k, int s, int sm_count) {
+    const long long tiles = ((m + t.bm - 1) / t.bm) * ((n + t.bn - 1) / t.bn);
+    const long long kbl = (k + dmma::BK - 1) / dmma::BK, part = (kbl + s - 1) / s;
+    const long long waves = (tiles * s + sm_count - 1) / sm_count;
+    const double area = t.bm * t.bn;
+    double unit = part * (0.28 * area + 100.0) + 0.7 * area + 1000.0;
+    if (s > 1) unit += 0.8 * area;
+    return waves * unit + (s > 1 ? 4000.0 : 0.0);
 }
+
+// the tile for an m x n x k product whose k is cut into s parts
+Tile dmma_tile(long long m, long long n, long long k, int s, int sm_count) {
+    Tile best = kTiles[0];
+    double cost = tile_cost(best, m, n, k, s, sm_count);
+    for (const Tile& t : kTiles) {
+        const long long tiles = ((m + t.bm - 1) / t.bm) * ((n + t.bn - 1) / t.bn);
+        if (s > 1 && tiles > kSplitTiles) continue;
+        const double c = tile_cost(t, m, n, k, s, sm_count);
+        if (c < cost) {
+            best = t;
+            cost = c;
+        }
+    }
+    return best;
+}
+}  // namespace
 
 bool dmma_operand_ok(const void* ptr, long long ld) {
     return (reinterpret_cast<uintptr_t>(ptr) % 16 == 0) && ((ld * 8) % 16 == 0) && ld > 0;
@@ -478,40 +513,32 @@ int dmma_splitk_tuned(int sm_count, long long tiles, long long kbl) {
 int dmma_splitk(long long m, long long n, long long k, int sm_count) {
     using namespace dmma;
     const long long bm = dmma_bm(m);
-    const long long tiles = ((m + bm - 1) / bm) * ((n + BN - 1) / BN);
+    const long long tiles = ((m + bm - 1) / bm) * ((n + 127) / 128);
     const long long kbl = (k + BK - 1) / BK;
     const int tuned = dmma_splitk_tuned(sm_count, tiles, kbl);
     if (tuned > 0 && dmma_splitk_legal(tiles, kbl, tuned, sm_count)) return tuned;
-    // wave balance of the persistent grid: units / (waves * SMs); a split must
-    // gain 5 % of it
-    auto balance = [&](long long units) {
-        const long long waves = (units + sm_count - 1) / sm_count;
-        return (double)units / (double)(waves * sm_count);
-    };
     int best = 1;
-    double best_b = balance(tiles);
-    for (int s = 2; s <= 8; ++s) {
+    double cost = 0.0;
+    for (int s = 1; s <= 8; ++s) {
         if (!dmma_splitk_legal(tiles, kbl, s, sm_count)) break;
-        const double b = balance(tiles * s);
-        if (b > best_b * 1.05) {
+        const double c = tile_cost(dmma_tile(m, n, k, s, sm_count), m, n, k, s, sm_count);
+        if (s == 1 || c < cost) {
             best = s;
-            best_b = b;
+            cost = c;
         }
     }
     return best;
 }
 
-size_t dmma_splitk_bytes(long long m, long long n, int ksplit) {
-    using namespace dmma;
+size_t dmma_splitk_bytes(long long m, long long n, long long k, int ksplit, int sm_count) {
     if (ksplit < 2) return 0;
-    const long long bm = dmma_bm(m);
-    const long long tiles = ((m + bm - 1) / bm) * ((n + BN - 1) / BN);
-    const int s = ksplit;
-    return (size_t)(tiles * s) * bm * BN * sizeof(double) + (size_t)tiles * sizeof(int);
+    const Tile t = dmma_tile(m, n, k, ksplit, sm_count);
+    const long long tiles = ((m + t.bm - 1) / t.bm) * ((n + t.bn - 1) / t.bn);
+    return (size_t)(tiles * ksplit) * t.bm * t.bn * sizeof(double);
 }
 
 int launch_dgemm_dmma(const GemmDesc& g, cudaStream_t st, int sm_count, int* status, const int* gate,
-                      int mma_k, char* err, size_t errlen, int ksplit, void* splitk_ws, size_t splitk_ws_bytes) {
+                      int mma_k, char* err, size_t errlen, int ksplit, void* splitk_ws, size_t splitk_ws_bytes, int* splitk_counters) {
     using namespace dmma;
     if (!dmma_operand_ok(g.a, g.lda) || !dmma_operand_ok(g.b, g.ldb)) {
         snprintf(err, errlen, "DMMA kernel needs 16-byte aligned A/B and even leading dimensions");
@@ -519,7 +546,13 @@ int launch_dgemm_dmma(const GemmDesc& g, cudaStream_t st, int sm_count, int* sta
     }
     const bool a_k = g.layout_a == 0;  // row-major A: k contiguous
     const bool b_k = g.layout_b == 1;  // column-major B: k contiguous
-    const int bm = dmma_bm(g.m);
+    // split-K needs the caller's workspace; the adjoint's fused dot keeps one
+    // unit per tile (its per-CTA partial dots must not depend on arrival order)
+    const int kbl = (int)((g.k + BK - 1) / BK);
+    int split = ksplit > 1 && splitk_ws && splitk_counters && !g.dot_mat ? (ksplit < kbl ? ksplit : kbl) : 1;
+    if (split > 1 && dmma_splitk_bytes(g.m, g.n, g.k, split, sm_count) > splitk_ws_bytes) split = 1;
+    const Tile tile = dmma_tile(g.m, g.n, g.k, split, sm_count);
+    const int bm = tile.bm, bn = tile.bn;
     CUtensorMap ma, mb;
     int rc;
     if (a_k)
@@ -530,7 +563,7 @@ int launch_dgemm_dmma(const GemmDesc& g, cudaStream_t st, int sm_count, int* sta
                           CU_TENSOR_MAP_SWIZZLE_128B, err, errlen);
     if (rc) return rc;
     if (b_k)
-        rc = make_tmap_2d(&mb, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 8, (void*)g.b, g.k, g.n, g.ldb, BK, BN,
+        rc = make_tmap_2d(&mb, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 8, (void*)g.b, g.k, g.n, g.ldb, BK, bn,
                           CU_TENSOR_MAP_SWIZZLE_128B, err, errlen);
     else
         rc = make_tmap_2d(&mb, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 8, (void*)g.b, g.n, g.k, g.ldb, 16, BK,
@@ -550,49 +583,45 @@ int launch_dgemm_dmma(const GemmDesc& g, cudaStream_t st, int sm_count, int* sta
     p.dot_ld = g.dot_ld;
     p.dot_partials = g.dot_partials;
     p.tiles_m = (int)((g.m + bm - 1) / bm);
-    p.tiles_n = (int)((g.n + BN - 1) / BN);
+    p.tiles_n = (int)((g.n + bn - 1) / bn);
     p.num_tiles = p.tiles_m * p.tiles_n;
-    p.k_blocks = (int)((g.k + BK - 1) / BK);
+    p.k_blocks = kbl;
     p.status = status;
     p.gate = gate;
     p.withhold = g.withhold_stage ? 1 : 0;
     p.ksplit = 1;
     p.part = nullptr;
     p.counters = nullptr;
-    // split-K needs the caller's workspace; the adjoint's fused dot keeps one
-    // unit per tile (its per-CTA partial dots must not depend on arrival order)
-    if (ksplit > 1 && splitk_ws && !g.dot_mat) {
-        const int s = ksplit < p.k_blocks ? ksplit : p.k_blocks;
-        const size_t need = dmma_splitk_bytes(g.m, g.n, s);
-        if (s > 1 && need <= splitk_ws_bytes) {
-            p.ksplit = s;
-            p.part = static_cast<double*>(splitk_ws);
-            p.counters = reinterpret_cast<int*>(static_cast<char*>(splitk_ws) +
-                                                (size_t)p.num_tiles * s * bm * BN * sizeof(double));
-            if (cudaMemsetAsync(p.counters, 0, (size_t)p.num_tiles * sizeof(int), st) != cudaSuccess) {
-                snprintf(err, errlen, "split-K counters: %s", cudaGetErrorString(cudaGetLastError()));
-                return JLC_E_LAUNCH;
-            }
-        }
+    if (split > 1) {
+        p.ksplit = split;
+        p.part = static_cast<double*>(splitk_ws);
+        p.counters = splitk_counters;
     }
     const int units = p.num_tiles * p.ksplit;
     const int grid = units < sm_count ? units : sm_count;
 
-#define JLC_DMMA_DISPATCH(MK, TB)                                                     \
-    if (a_k && b_k) rc = launch_variant<true, true, MK, TB>(ma, mb, p, grid, st);      \
-    else if (a_k) rc = launch_variant<true, false, MK, TB>(ma, mb, p, grid, st);       \
-    else if (b_k) rc = launch_variant<false, true, MK, TB>(ma, mb, p, grid, st);       \
-    else rc = launch_variant<false, false, MK, TB>(ma, mb, p, grid, st);
-    if (bm == 32) {
-        JLC_DMMA_DISPATCH(8, 32)  // thin tiles: the default k step only
-    } else if (bm == 64) {
-        JLC_DMMA_DISPATCH(8, 64)
-    } else if (mma_k == 4) {
-        JLC_DMMA_DISPATCH(4, 128)
-    } else if (mma_k == 16) {
-        JLC_DMMA_DISPATCH(16, 128)
-    } else {
-        JLC_DMMA_DISPATCH(8, 128)
+#define JLC_DMMA_DISPATCH(MK, TM, TN)                                                     \
+    if (a_k && b_k) rc = launch_variant<true, true, MK, TM, TN>(ma, mb, p, grid, st);      \
+    else if (a_k) rc = launch_variant<true, false, MK, TM, TN>(ma, mb, p, grid, st);       \
+    else if (b_k) rc = launch_variant<false, true, MK, TM, TN>(ma, mb, p, grid, st);       \
+    else rc = launch_variant<false, false, MK, TM, TN>(ma, mb, p, grid, st);
+    // (the k steps other than the default 8 are built for the largest tile)
+    switch (bm * 1000 + bn) {
+        case 32032: JLC_DMMA_DISPATCH(8, 32, 32) break;
+        case 32064: JLC_DMMA_DISPATCH(8, 32, 64) break;
+        case 32128: JLC_DMMA_DISPATCH(8, 32, 128) break;
+        case 64032: JLC_DMMA_DISPATCH(8, 64, 32) break;
+        case 64064: JLC_DMMA_DISPATCH(8, 64, 64) break;
+        case 64128: JLC_DMMA_DISPATCH(8, 64, 128) break;
+        case 128064: JLC_DMMA_DISPATCH(8, 128, 64) break;
+        default:
+            if (mma_k == 4) {
+                JLC_DMMA_DISPATCH(4, 128, 128)
+            } else if (mma_k == 16) {
+                JLC_DMMA_DISPATCH(16, 128, 128)
+            } else {
+                JLC_DMMA_DISPATCH(8, 128, 128)
+            }
     }
 #undef JLC_DMMA_DISPATCH
     if (rc) snprintf(err, errlen, "DMMA kernel launch failed: %s", cudaGetErrorString(cudaGetLastError()));

@@ -47,11 +47,9 @@ struct GemmDesc {
     bool withhold_stage = false;
 };
 
-// number of CTAs the DMMA / Ozaki GEMM kernels launch for this shape (the
-// length of dot_partials they fill)
-int dmma_grid(long long m, long long n, int sm_count);
-// tile height the DMMA kernel uses for an m-row product (32, 64 or 128)
+// tile height of an m-row product's split-K class (32, 64 or 128)
 int dmma_bm(long long m);
+// number of CTAs the Ozaki GEMM kernel launches for this shape
 int ozaki_grid(long long m, long long n, int sm_count);
 
 // Grow-only device scratch owned by a context.
@@ -75,7 +73,7 @@ bool dmma_operand_ok(const void* ptr, long long ld);
 // dimensions.  gate != nullptr: the kernel only runs if one of the Ozaki
 // call's flags gate[kFlagNonfiniteA], gate[kFlagFallback],
 // gate[kFlagNonfiniteB] is set.
-// ksplit > 1 with splitk_ws of at least dmma_splitk_bytes(m, n, ksplit):
+// ksplit > 1 with splitk_counters and splitk_ws of at least dmma_splitk_bytes(m, n, k, ksplit, sm_count):
 // split-K over ksplit parts; otherwise every tile is one work unit.
 // blocked Householder QR kernels (qr.cu)
 size_t qr_panel_mp_scratch_bytes(int P);
@@ -115,7 +113,10 @@ int launch_hess_panel(const double* h, long long ldh, int n, int k, int pw, doub
                       cudaStream_t st);
 int launch_dgemm_dmma(const GemmDesc& g, cudaStream_t st, int sm_count, int* status, const int* gate, int mma_k,
                       char* err, size_t errlen, int ksplit = 1, void* splitk_ws = nullptr,
-                      size_t splitk_ws_bytes = 0);
+                      size_t splitk_ws_bytes = 0, int* splitk_counters = nullptr);
+// tiles a split product may have (the length of splitk_counters, all zero
+// between launches: the unit that finishes a tile clears its counter)
+constexpr int kSplitTiles = 4096;
 int dmma_splitk(long long m, long long n, long long k, int sm_count);
 // split-K tuning (dgemm_dmma.cu): legal factors, the shape class, and the
 // tuned factor of a class (0: none cached); remember() records a new choice
@@ -128,7 +129,7 @@ namespace grp {
 int tune_lookup(const std::string& key);
 void tune_store(const std::string& key, int value);
 }  // namespace grp
-size_t dmma_splitk_bytes(long long m, long long n, int ksplit);
+size_t dmma_splitk_bytes(long long m, long long n, long long k, int ksplit, int sm_count);
 
 // y[i*incy] = alpha * sum_p M(i,p) x[p*incx] + beta * y[i*incy], M(i,p) = mat[i*rs + p*cs]
 // with rs == 1 or cs == 1.  scratch: ceil-split partial sums for the rs == 1 form.
@@ -265,6 +266,7 @@ struct jlc_ctx {
     cudaStream_t stream = nullptr;
     int* d_status = nullptr;  // status block: JLC_DEV_* bits written by kernels, wait limit at byte 8
     int* d_flags = nullptr;   // control words of an Ozaki call (kFlag*)
+    int* d_counters = nullptr;  // split-K arrivals per tile (kSplitTiles, zero between launches)
     DevBuf bufA, bufB, bufC;
     DevBuf bufR;  // reduction partials (adjoint)
     DevBuf bufQ;  // blocked QR: V, G, T and the two W panels

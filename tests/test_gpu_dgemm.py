@@ -413,3 +413,39 @@ def test_thin_tiles(ctx, oracle, m, la, lb):
         runs.append(dC.cpu().numpy())
     np.testing.assert_array_equal(runs[1], runs[0])
     assert_fp64_bound(f"thin {m} {la}{lb}", runs[0], A, B, C, -0.5, 1.25)
+
+
+@pytest.mark.parametrize("la,lb", [(0, 0), (1, 0), (0, 1), (1, 1)])
+@pytest.mark.parametrize("m,n,k", [
+    (31, 33, 17), (97, 79, 113),                  # 32 x 32 tiles, one k-block and a k tail
+    (32, 9001, 20), (41, 2500, 100),              # 32 x 64, 64 x 32
+    (700, 651, 200), (32, 4737, 33),              # 64 x 64, 32 x 128
+    (999, 1100, 520), (64, 9473, 33),             # 128 x 64, 64 x 128
+    (1501, 1500, 33),                             # 128 x 128
+    (33, 65, 4100), (130, 257, 1537),             # split k on the smallest tiles
+])
+def test_tile_shapes(ctx, oracle, la, lb, m, n, k):
+    """Products whose tile shapes differ, ragged at every edge, in all four
+    layouts with padded leading dimensions, alpha and beta: inside the FP64
+    bound, and the padding of C untouched."""
+    import torch
+    rng = np.random.default_rng(m * 7 + n)
+    a, b, c = rng.uniform(-1, 1, (m, k)), rng.uniform(-1, 1, (k, n)), rng.uniform(-1, 1, (m, n))
+
+    def stored(x, layout, pad):
+        x = x if layout == 0 else x.T
+        out = np.full((x.shape[0], (x.shape[1] + pad + 1) // 2 * 2), 7.5)
+        out[:, :x.shape[1]] = x
+        return torch.from_numpy(out).cuda()
+
+    at, bt, ct = stored(a, la, 3), stored(b, lb, 5), stored(c, 0, 1)
+    torch.cuda.synchronize()
+    ctx.dgemm_device(la, lb, m, n, k, 1.5, at.data_ptr(), at.shape[1], bt.data_ptr(), bt.shape[1], -0.5,
+                     ct.data_ptr(), ct.shape[1])
+    ctx.synchronize()
+    out = ct.cpu().numpy()
+    assert (out[:, n:] == 7.5).all()
+    rows = rng.integers(0, m, 400)
+    cols = rng.integers(0, n, 400)
+    rows[:4], cols[:4] = (0, 0, m - 1, m - 1), (0, n - 1, 0, n - 1)
+    assert_fp64_bound(f"{m}x{n}x{k}", out[:, :n], a, b, c, 1.5, -0.5, rows=rows, cols=cols)
