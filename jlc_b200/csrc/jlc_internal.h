@@ -47,6 +47,14 @@ struct GemmDesc {
     bool withhold_stage = false;
 };
 
+// a row-major window copied to rows of ld_dst (a multiple of 2 doubles, 16-byte aligned)
+struct RepackDesc {
+    const double* src = nullptr;
+    long long ld_src = 0;
+    double* dst = nullptr;
+    long long ld_dst = 0, rows = 0, cols = 0;
+};
+int launch_repack(const RepackDesc& d0, const RepackDesc& d1, const int* gate, cudaStream_t st);
 // tile height of an m-row product's split-K class (32, 64 or 128)
 int dmma_bm(long long m);
 // number of CTAs the Ozaki GEMM kernel launches for this shape

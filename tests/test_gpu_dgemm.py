@@ -449,3 +449,29 @@ def test_tile_shapes(ctx, oracle, la, lb, m, n, k):
     cols = rng.integers(0, n, 400)
     rows[:4], cols[:4] = (0, 0, m - 1, m - 1), (0, n - 1, 0, n - 1)
     assert_fp64_bound(f"{m}x{n}x{k}", out[:, :n], a, b, c, 1.5, -0.5, rows=rows, cols=cols)
+
+
+@pytest.mark.parametrize("m,n,k", [(3, 5, 2), (9, 513, 511), (600, 7, 8)])
+def test_operands_copied_for_tma(ctx, oracle, m, n, k):
+    """Odd leading dimensions and 8-byte aligned bases of either operand, at
+    the edges of the copy's row and column blocks: bit for bit the product of
+    aligned operands."""
+    import torch
+    rng = np.random.default_rng(m + n + k)
+    a, b = rng.uniform(-1, 1, (m, k)), rng.uniform(-1, 1, (k, n))
+    outs = []
+    for lda, ldb, off in ((k + k % 2, n + n % 2, 0), (k + 1 + k % 2, n + 1 + n % 2, 0), (k + k % 2, n + n % 2, 1)):
+        bufs = []
+        for x, ld in ((a, lda), (b, ldb)):
+            flat = torch.full((off + x.shape[0] * ld,), 3.5, dtype=torch.float64)
+            flat[off:].view(x.shape[0], ld)[:, :x.shape[1]] = torch.from_numpy(x)
+            bufs.append(flat.cuda())
+        c = torch.zeros(m, n, dtype=torch.float64, device="cuda")
+        torch.cuda.synchronize()
+        ctx.dgemm_device(0, 0, m, n, k, 1.0, bufs[0].data_ptr() + 8 * off, lda, bufs[1].data_ptr() + 8 * off, ldb, 0.0,
+                         c.data_ptr(), n)
+        ctx.synchronize()
+        outs.append(c.cpu().numpy())
+    assert_fp64_bound("aligned", outs[0], a, b, None, 1.0, 0.0)
+    np.testing.assert_array_equal(outs[1], outs[0])
+    np.testing.assert_array_equal(outs[2], outs[0])
