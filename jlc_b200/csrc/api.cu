@@ -684,68 +684,61 @@ namespace {
 constexpr int kQrPanel = 64;  // panel width (HouseholderQR.java BLOCK_SIZE)
 
 struct QrWork {
-    double *v, *g, *t, *w, *w2;
+    double *v, *vt, *t, *w;
     long long ldv, ldw;
+    int batch;            // panels whose V, T and V op(T) fit
     void* panel_scratch;  // multi-CTA panel: partials, row records, barrier counter
-    double* gram;         // row-slab partials of G = V^T V
+    double* gram;         // row-slab partials of V^T V (tall panels)
 };
 
-int qr_work(jlc_ctx* ctx, long long m, long long cols, QrWork& q) {
+// Workspace for an m-row factor applied to `cols` columns, with V, T and V op(T)
+// of up to `panels` panels at a time, within 256 MB (one panel at least).
+int qr_work(jlc_ctx* ctx, long long m, long long cols, long long panels, QrWork& q) {
     q.ldv = round_up(m > 0 ? m : 1, 8);
     q.ldw = round_up(cols > 0 ? cols : 1, 8);
-    const size_t doubles = (size_t)(q.ldv * kQrPanel + 2 * kQrPanel * kQrPanel + 2 * kQrPanel * q.ldw);
+    const long long per = 2 * q.ldv * kQrPanel + kQrPanel * kQrPanel;  // doubles per panel
+    const long long most = (256LL << 20) / (per * (long long)sizeof(double));
+    q.batch = (int)(panels < 1 ? 1 : (most < 1 ? 1 : (panels < most ? panels : most)));
+    const size_t doubles = (size_t)(per * q.batch + kQrPanel * q.ldw);
     const size_t scratch = round_up(qr_panel_mp_scratch_bytes(ctx->sm_count > 0 ? ctx->sm_count : 1), 256);
     const size_t gram = qr_gram_scratch_bytes(ctx->sm_count);
     int rc = reserve(ctx, ctx->bufQ, doubles * sizeof(double) + scratch + gram, "QR workspace");
     if (rc) return rc;
+    if (ctx->qr_cluster_max == 0) ctx->qr_cluster_max = qr_panel_cluster_max();
     q.v = static_cast<double*>(ctx->bufQ.ptr);
-    q.g = q.v + q.ldv * kQrPanel;
-    q.t = q.g + kQrPanel * kQrPanel;
-    q.w = q.t + kQrPanel * kQrPanel;
-    q.w2 = q.w + kQrPanel * q.ldw;
-    q.panel_scratch = q.w2 + kQrPanel * q.ldw;
+    q.vt = q.v + q.ldv * kQrPanel * q.batch;
+    q.t = q.vt + q.ldv * kQrPanel * q.batch;
+    q.w = q.t + kQrPanel * kQrPanel * q.batch;
+    q.panel_scratch = q.w + kQrPanel * q.ldw;
     q.gram = reinterpret_cast<double*>(static_cast<char*>(q.panel_scratch) + scratch);
     return JLC_OK;
 }
 
-// V and T of panel [k0, k0+kb) of the factored column-major matrix f (rows
-// from k0 down): V packed, G = V^T V over those rows, then T.
-int qr_panel_vt(jlc_ctx* ctx, const double* f, long long ldf, long long m, long long k0, int kb, const double* tau,
-                const QrWork& q, int precision) {
-    cudaStream_t st = ctx->stream;
-    int rc;
-    {
-        Phase ph(ctx, JLC_PHASE_QR_VT);
-        rc = launch_qr_pack_v(f, ldf, (int)m, (int)k0, kb, q.v, q.ldv, st);
-    }
-    if (rc) return set_err(ctx, rc, "QR: V packing launch failed");
-    // G (64 x 64, row-major) = V(k0:, :)^T V(k0:, :) over row slabs (a 64 x 64
-    // output is one tile of a GEMM, too few CTAs for k = m - k0), then T
+// V, T and V op(T) of panels p0 .. p0 + panels - 1 of the factor f (m rows, kmax
+// reflectors, reflector k's unit entry in row k + shift).
+int qr_panels_vt(jlc_ctx* ctx, const double* f, long long ldf, long long m, long long kmax, long long p0, int panels,
+                 int shift, const double* tau, bool trans, const QrWork& q) {
     Phase ph(ctx, JLC_PHASE_QR_VT);
-    rc = launch_qr_gram(q.v, q.ldv, (int)k0, (int)m, q.g, q.gram, ctx->sm_count, st);
-    if (!rc) rc = launch_qr_build_t(q.g, tau + k0, kb, q.t, st);
-    return rc ? set_err(ctx, rc, "QR: V^T V / T launch failed") : JLC_OK;
+    ctx->launches += 2;
+    const int rc = launch_qr_vt(f, ldf, (int)m, (int)kmax, (int)p0, panels, shift, tau, q.v, q.ldv, q.t, q.vt, trans,
+                                q.gram, ctx->qr_cluster_max, ctx->sm_count, ctx->stream);
+    return rc ? set_err(ctx, rc, "QR: V / T launch failed") : JLC_OK;
 }
 
-// C (rows k0.. of a column-major m x cols block, ld ldc) <- H C with
-// H = I - V T V^T (trans_t = false) or H^T = I - V T^T V^T (trans_t = true):
-// W = V^T C, W2 = op(T) W, C -= V W2, the last as C^T -= W2^T V^T so that the
+// C (rows k0.. of a column-major m x cols block, ld ldc) <- H C with H = I - V T
+// V^T, or H^T C, by the i-th panel of the workspace, whose vt is V T or V T^T:
+// W = V^T C, C -= (V op(T)) W, the latter as C^T -= W^T (V op(T))^T so that the
 // column-major C is the GEMM's row-major output.
-int qr_apply_wy(jlc_ctx* ctx, long long m, long long k0, long long cols, double* c, long long ldc, bool trans_t,
-                const QrWork& q, int precision) {
+int qr_apply_wy(jlc_ctx* ctx, long long m, long long k0, long long cols, double* c, long long ldc, const QrWork& q,
+                int i, int precision) {
     if (cols <= 0) return JLC_OK;
     const long long rows = m - k0;
-    GemmDesc w{JLC_ROW_MAJOR, JLC_COL_MAJOR, kQrPanel, cols, rows, 1.0, 0.0, q.v + k0, q.ldv, c + k0, ldc, q.w,
-               q.ldw};
+    const double* v = q.v + i * q.ldv * kQrPanel + k0;
+    const double* vt = q.vt + i * q.ldv * kQrPanel + k0;
+    GemmDesc w{JLC_ROW_MAJOR, JLC_COL_MAJOR, kQrPanel, cols, rows, 1.0, 0.0, v, q.ldv, c + k0, ldc, q.w, q.ldw};
     int rc = run_device(ctx, w, precision, 0, nullptr);
     if (rc) return rc;
-    // op(T): T is row-major, so T^T is the same array read column-major
-    GemmDesc t{trans_t ? JLC_COL_MAJOR : JLC_ROW_MAJOR, JLC_ROW_MAJOR, kQrPanel, cols, kQrPanel, 1.0, 0.0, q.t,
-               kQrPanel, q.w, q.ldw, q.w2, q.ldw};
-    rc = run_device(ctx, t, JLC_PREC_NATIVE, 0, nullptr);
-    if (rc) return rc;
-    GemmDesc u{JLC_COL_MAJOR, JLC_ROW_MAJOR, cols, rows, kQrPanel, -1.0, 1.0, q.w2, q.ldw, q.v + k0, q.ldv,
-               c + k0, ldc};
+    GemmDesc u{JLC_COL_MAJOR, JLC_ROW_MAJOR, cols, rows, kQrPanel, -1.0, 1.0, q.w, q.ldw, vt, q.ldv, c + k0, ldc};
     return run_device(ctx, u, precision, 0, nullptr);
 }
 
@@ -908,6 +901,7 @@ void jlc_destroy(jlc_ctx* ctx) {
     if (ctx->bufB.ptr) cudaFree(ctx->bufB.ptr);
     if (ctx->bufC.ptr) cudaFree(ctx->bufC.ptr);
     if (ctx->bufR.ptr) cudaFree(ctx->bufR.ptr);
+    if (ctx->bufQ.ptr) cudaFree(ctx->bufQ.ptr);
     if (ctx->ws.ptr) cudaFree(ctx->ws.ptr);
     if (ctx->d_status) cudaFree(ctx->d_status);
     if (ctx->d_flags) cudaFree(ctx->d_flags);
@@ -1147,7 +1141,7 @@ int jlc_qr_factor_device(jlc_ctx* ctx, int64_t m, int64_t n, double* a, int64_t 
     cudaSetDevice(ctx->device);
     ctx->err[0] = 0;
     QrWork q;
-    int rc = qr_work(ctx, m, n, q);
+    int rc = qr_work(ctx, m, n, 1, q);
     if (rc) return rc;
     cudaEventRecord(ctx->ev0, ctx->stream);
     const long long kmax = m < n ? m : n;
@@ -1162,15 +1156,14 @@ int jlc_qr_factor_device(jlc_ctx* ctx, int64_t m, int64_t n, double* a, int64_t 
             long long ctas = (m - k0) / 128;
             if (ctas > ctx->sm_count) ctas = ctx->sm_count;
             if (ctas < 1) ctas = 1;
-            if (ctx->qr_cluster_max == 0) ctx->qr_cluster_max = qr_panel_cluster_max();
             rc = launch_qr_panel(a, lda, (int)m, (int)k0, kb, tau, (int)ctas, ctx->qr_cluster_max, q.panel_scratch,
                                  ctx->d_status, ctx->stream);
             if (rc) return set_err(ctx, rc, "QR: panel launch failed");
         }
         const long long trail = n - (k0 + kb);
         if (trail <= 0) continue;
-        rc = qr_panel_vt(ctx, a, lda, m, k0, kb, tau, q, precision);
-        if (!rc) rc = qr_apply_wy(ctx, m, k0, trail, a + (k0 + kb) * lda, lda, true, q, precision);
+        rc = qr_panels_vt(ctx, a, lda, m, kmax, k0 / kQrPanel, 1, 0, tau, true, q);
+        if (!rc) rc = qr_apply_wy(ctx, m, k0, trail, a + (k0 + kb) * lda, lda, q, 0, precision);
         if (rc) return rc;
     }
     cudaEventRecord(ctx->ev1, ctx->stream);
@@ -1228,23 +1221,30 @@ int hess_apply_right(jlc_ctx* ctx, double* mat, long long ldm, long long n, long
 }  // extern "C"
 
 namespace {
-// Q (first qcols columns) of the reflectors stored in f (below its diagonal,
-// QR style) with scales tau, enqueued on the context stream without a sync:
-// the identity, then the panels' block reflectors in reverse order.
-int qr_build_q_enqueue(jlc_ctx* ctx, long long m, long long n, long long qcols, const double* f, long long ldf,
-                       const double* tau, double* q_out, long long ldq, int precision) {
-    const long long kmax = m < n ? m : n;
+// Q (first qcols columns) of kmax reflectors stored in f (QR style; reflector
+// k's unit entry, implied, in row k + shift and its tail below) with scales tau,
+// enqueued on the context stream without a sync: the identity, then the panels'
+// block reflectors in reverse order.  The panels' V and T do not depend on one
+// another: a batch of panels forms them in two launches.
+int qr_build_q_enqueue(jlc_ctx* ctx, long long m, long long kmax, long long qcols, const double* f, long long ldf,
+                       int shift, const double* tau, double* q_out, long long ldq, int precision) {
+    const long long live = kmax < qcols ? kmax : qcols;  // a panel past the last column has nothing to change
+    const long long panels = (live + kQrPanel - 1) / kQrPanel;
     QrWork q;
-    int rc = qr_work(ctx, m, qcols, q);
+    int rc = qr_work(ctx, m, qcols, panels, q);
     if (rc) return rc;
     rc = launch_set_identity(q_out, ldq, m, qcols, ctx->stream);
     if (rc) return set_err(ctx, rc, "QR: identity launch failed");
-    for (long long k0 = (kmax - 1) / kQrPanel * kQrPanel; k0 >= 0 && kmax > 0; k0 -= kQrPanel) {
-        const int kb = (int)(kmax - k0 < kQrPanel ? kmax - k0 : kQrPanel);
-        if (k0 >= qcols) continue;
-        rc = qr_panel_vt(ctx, f, ldf, m, k0, kb, tau, q, precision);
-        if (!rc) rc = qr_apply_wy(ctx, m, k0, qcols - k0, q_out + k0 * ldq, ldq, false, q, precision);
+    for (long long last = panels; last > 0;) {
+        const int nb = (int)(last < q.batch ? last : q.batch);
+        const long long first = last - nb;
+        rc = qr_panels_vt(ctx, f, ldf, m, kmax, first, nb, shift, tau, false, q);
+        for (int i = nb - 1; i >= 0 && !rc; --i) {
+            const long long k0 = (first + i) * kQrPanel;
+            rc = qr_apply_wy(ctx, m, k0, qcols - k0, q_out + k0 * ldq, ldq, q, i, precision);
+        }
         if (rc) return rc;
+        last = first;
     }
     return JLC_OK;
 }
@@ -1268,8 +1268,7 @@ int jlc_hessenberg_device(jlc_ctx* ctx, int64_t n, double* a, int64_t lda, doubl
     int rc = JLC_OK;
     if (q && (rc = launch_set_identity(q, ldq, n, n, st))) return set_err(ctx, rc, "Hessenberg: identity launch failed");
     if (n > 2 && hess_slab_fits((int)n, ctx->sm_count)) {
-        // the whole reduction in one launch, then Q = diag(1, H_0 ... H_{n-3}) from the reflectors
-        // below the subdiagonal, which sit there as in the QR factor of rows 1..
+        // the whole reduction in one launch, then Q from the reflectors below the subdiagonal
         const long long ldt = round_up(n, 8);
         if ((rc = reserve(ctx, ctx->bufH, (ldt + hess_slab_work_doubles((int)n, ctx->sm_count)) * sizeof(double),
                           "Hessenberg workspace")))
@@ -1281,8 +1280,7 @@ int jlc_hessenberg_device(jlc_ctx* ctx, int64_t n, double* a, int64_t lda, doubl
             if (rc) return set_err(ctx, rc, "Hessenberg: launch failed");
             ctx->launches += 1;
         }
-        if (q && (rc = qr_build_q_enqueue(ctx, n - 1, n - 2, n - 1, a + 1, lda, tau, q + 1 + ldq, ldq, precision)))
-            return rc;
+        if (q && (rc = qr_build_q_enqueue(ctx, n, n - 2, n, a, lda, 1, tau, q, ldq, precision))) return rc;
         if ((rc = launch_hess_clear(a, lda, (int)n, st))) return set_err(ctx, rc, "Hessenberg: clear launch failed");
         ctx->launches += 1;
     } else if (n > 2) {
@@ -1344,7 +1342,7 @@ int jlc_qr_build_q_device(jlc_ctx* ctx, int64_t m, int64_t n, int64_t qcols, con
     cudaSetDevice(ctx->device);
     ctx->err[0] = 0;
     cudaEventRecord(ctx->ev0, ctx->stream);
-    int rc = qr_build_q_enqueue(ctx, m, n, qcols, f, ldf, tau, q_out, ldq, precision);
+    int rc = qr_build_q_enqueue(ctx, m, kmax, qcols, f, ldf, 0, tau, q_out, ldq, precision);
     if (rc) return rc;
     cudaEventRecord(ctx->ev1, ctx->stream);
     rc = finish_sync(ctx);
@@ -1380,10 +1378,10 @@ int jlc_bidiag_device(jlc_ctx* ctx, int64_t m, int64_t n, double* a, int64_t lda
     if (m > 0 && n > 0) {
         // workspace: tau of the column and row reflectors, the kernel's
         // partials, and the row reflectors rearranged as a QR factor
-        const long long ldw = n > 1 ? round_up(n - 1, 8) : 8;
+        const long long ldw = round_up(n, 8);
         const long long ldt = round_up(n, 8);
         const size_t kdoubles = bidiag_work_doubles((int)m, (int)n, ctx->sm_count);
-        const size_t wdoubles = v ? (size_t)ldw * (size_t)(n > 1 ? n - 1 : 1) : 0;
+        const size_t wdoubles = v ? (size_t)ldw * (size_t)n : 0;
         if ((rc = reserve(ctx, ctx->bufH, (2 * (size_t)ldt + kdoubles + wdoubles) * sizeof(double),
                           "bidiagonalisation workspace")))
             return rc;
@@ -1398,15 +1396,15 @@ int jlc_bidiag_device(jlc_ctx* ctx, int64_t m, int64_t n, double* a, int64_t lda
             ctx->launches += 1;
         }
         // U = H_0 H_1 ... H_{n-1}: the column reflectors sit below the diagonal as in a QR factor
-        if (u && (rc = qr_build_q_enqueue(ctx, m, n, m, a, lda, tauq, u, ldu, precision))) return rc;
+        if (u && (rc = qr_build_q_enqueue(ctx, m, n, m, a, lda, 0, tauq, u, ldu, precision))) return rc;
         if (v) {
-            // V = diag(1, G_0 ... G_{n-2}): row k's reflector acts on columns k+1..
-            if ((rc = launch_set_identity(v, ldv, n, n, st))) return set_err(ctx, rc, "identity launch failed");
+            // V = G_0 ... G_{n-2}: row k's reflector acts on columns k+1..
             if (n > 1) {
                 if ((rc = launch_bidiag_right_factor(a, lda, (int)n, wr, ldw, st)))
                     return set_err(ctx, rc, "bidiagonalisation: right factor launch failed");
-                if ((rc = qr_build_q_enqueue(ctx, n - 1, n - 1, n - 1, wr, ldw, taup, v + 1 + ldv, ldv, precision)))
-                    return rc;
+                if ((rc = qr_build_q_enqueue(ctx, n, n - 1, n, wr, ldw, 1, taup, v, ldv, precision))) return rc;
+            } else if ((rc = launch_set_identity(v, ldv, n, n, st))) {
+                return set_err(ctx, rc, "identity launch failed");
             }
         }
     } else {

@@ -503,11 +503,11 @@ __global__ void __launch_bounds__(BT, 1) bidiag_kernel(const Args p) {
 }
 
 // Right reflectors, stored in the rows of A beyond the superdiagonal, as the
-// columns of a QR factor: W(r, k) = A(k, r + 1) for r > k (r, k < n - 1).
+// columns of a factor: W(r, k) = A(k, r) for r > k + 1 (k < n - 1).
 __global__ void bidiag_right_factor_kernel(const double* a, long long lda, int n, double* w, long long ldw) {
     const int k = blockIdx.y;
-    for (int r = k + 1 + blockIdx.x * blockDim.x + threadIdx.x; r < n - 1; r += gridDim.x * blockDim.x)
-        w[r + (long long)k * ldw] = a[k + (long long)(r + 1) * lda];
+    for (int r = k + 2 + blockIdx.x * blockDim.x + threadIdx.x; r < n; r += gridDim.x * blockDim.x)
+        w[r + (long long)k * ldw] = a[k + (long long)r * lda];
 }
 
 }  // namespace bidiag

@@ -88,14 +88,11 @@ size_t qr_panel_mp_scratch_bytes(int P);
 int qr_panel_cluster_max();
 int launch_qr_panel(double* a, long long lda, int m, int k0, int kb, double* tau, int P, int cluster_max,
                     void* scratch, int* status, cudaStream_t st);
-int launch_qr_pack_v(const double* a, long long lda, int m, int k0, int kb, double* v, long long ldv,
-                     cudaStream_t st);
-int launch_qr_build_t(const double* g, const double* tau, int kb, double* t, cudaStream_t st);
-// G = V^T V (64 x 64, row-major) over rows [r0, r1) of the packed V; scratch
-// holds qr_gram_scratch_bytes(sm_count)
+// V, T and V op(T) of consecutive panels; gram holds qr_gram_scratch_bytes(sm_count)
 size_t qr_gram_scratch_bytes(int sm_count);
-int launch_qr_gram(const double* v, long long ldv, int r0, int r1, double* g, double* scratch, int sm_count,
-                   cudaStream_t st);
+int launch_qr_vt(const double* a, long long lda, int m, int kmax, int p0, int panels, int shift, const double* tau,
+                 double* v, long long ldv, double* t, double* vt, bool trans, double* gram, int cluster_max,
+                 int sm_count, cudaStream_t st);
 int launch_set_identity(double* q, long long ldq, long long m, long long cols, cudaStream_t st);
 // blocked Hessenberg reduction kernels (hess.cu)
 size_t hess_work_doubles(long long n);

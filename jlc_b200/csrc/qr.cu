@@ -14,19 +14,22 @@
 //                      or (taller still) in place, one grid barrier per column;
 //                      all merge partials in a fixed order, so the
 //                      factorisation is deterministic;
-//   qr_pack_v_kernel:  V = the panel's reflectors with unit diagonal and zeros
-//                      above it (packV, HouseholderQR.java:445-471);
-//   qr_gram_partial_kernel / qr_gram_sum_kernel: G = V^T V over row slabs,
-//                      one CTA per slab, partials added in slab order;
-//   qr_build_t_kernel: T from the Gram matrix G = V^T V and tau: the
-//                      reference's recurrence (buildT, :300-325) inside
-//                      16 x 16 diagonal blocks, joined blockwise.
+//   qr_vt_kernel:      V = the panel's reflectors with unit diagonal and zeros
+//                      above it (packV, HouseholderQR.java:445-471) and the T
+//                      of their compact-WY form (buildT, :300-325), one cluster
+//                      per panel, any number of panels per launch;
+//   qr_vt_product_kernel: V T or V T^T, so that a block reflector is applied in
+//                      two GEMMs;
+//   qr_pack_v_kernel, qr_gram_partial_kernel / qr_gram_sum_kernel,
+//   qr_build_t_kernel: V and T of panels above 4096 rows, V^T V over row slabs
+//                      on the whole grid.
 #include <cfloat>
 #include <cmath>
 
 #include <cooperative_groups.h>
 
 #include "jlc_device.cuh"
+#include "jlc_dmma.cuh"
 #include "jlc_internal.h"
 #include "jlc_slab.cuh"
 
@@ -898,16 +901,17 @@ __global__ void __launch_bounds__(RG_THREADS, 1) qr_panel_rg_kernel(double* A, l
 }
 
 // V (ldv x 64, column-major): column i < kb holds reflector k0+i (zeros above
-// row k0+i, one on it, A's tail below); columns kb .. 63 are zero.
-__global__ void qr_pack_v_kernel(const double* A, long long lda, int m, int k0, int kb, double* V, long long ldv) {
+// row k0+i+shift, one on it, A's tail below); columns kb .. 63 are zero.
+__global__ void qr_pack_v_kernel(const double* A, long long lda, int m, int k0, int kb, int shift, double* V,
+                                 long long ldv) {
     const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= ldv * 64) return;
     const int i = (int)(e / ldv);
     const int row = (int)(e % ldv);
     double v = 0.0;
     if (i < kb && row < m) {
-        const int k = k0 + i;
-        v = row < k ? 0.0 : (row == k ? 1.0 : A[(long long)k * lda + row]);
+        const int k = k0 + i + shift;
+        v = row < k ? 0.0 : (row == k ? 1.0 : A[(long long)(k0 + i) * lda + row]);
     }
     V[e] = v;
 }
@@ -967,70 +971,240 @@ __global__ void qr_gram_sum_kernel(const double* part, int parts, double* G) {
     G[e] = s;
 }
 
-// T (64 x 64, row-major, upper triangular) from G = V^T V (row-major) and tau,
-// the factor of H_0 H_1 ... H_63 = I - V T V^T.  The reference builds it
-// column by column: T[i][i] = tau_i, T[r][i] = sum_{c=r}^{i-1} T[r][c] t0[c][i]
-// with t0[c][i] = -tau_i G[c][i] (buildT).  Here that recurrence runs inside
-// the four 16 x 16 diagonal blocks at once, and the blocks are joined by the
-// same identity applied to blocks of reflectors, T_ab = -T_aa G_ab T_bb (two
-// 16-wide joins, then one 32-wide).  Equal to the column recurrence up to
-// rounding; columns from kb on are zero.
-constexpr int BT_THREADS = 256;
+// T (64 x 64, row-major, upper triangular) of H_0 H_1 ... H_63 = I - V T V^T from
+// G = V^T V and tau, in one CTA of 256 threads.  The reference builds it column
+// by column (buildT); that recurrence solves T (D^-1 + U) = I with D = diag(tau)
+// and U the part of G above its diagonal, so T = (I + D U)^-1 D, which also
+// holds where tau is 0.  The unit triangular inverse comes from the four 16 x 16
+// diagonal blocks at once, a thread per column with the column in registers (no
+// barrier in the substitution), and two joins X_ab = -X_aa (N_ab X_bb), 16 and
+// then 32 wide.  On entry t holds G above its diagonal; x is scratch.
+constexpr int BT_THREADS = 256, BT_LD = 65;
 
-__global__ void __launch_bounds__(BT_THREADS) qr_build_t_kernel(const double* G, const double* tau, int kb,
-                                                                double* T) {
-    __shared__ double t[64][65];
-    __shared__ double x[32][33];
+__device__ void build_t(double (*t)[BT_LD], double (*x)[33], const double* tau, int kb, double* T) {
     const int tid = threadIdx.x;
-#pragma unroll 4
+    __shared__ double s_tau[64];
+    if (tid < 64) s_tau[tid] = tid < kb ? tau[tid] : 0.0;
+    __syncthreads();
     for (int e = tid; e < 64 * 64; e += BT_THREADS) {
-        const int row = e >> 6, c = e & 63;
-        double v = 0.0;
-        if (c < kb) v = row < c ? -tau[c] * G[e] : (row == c ? tau[c] : 0.0);
-        t[row][c] = v;
+        const int r = e >> 6, c = e & 63;
+        t[r][c] = r < c ? s_tau[r] * t[r][c] : (r == c ? 1.0 : 0.0);
+    }
+    __syncthreads();
+    double y[16];
+    const int o = (tid >> 4) * 16, j = tid & 15;
+    if (tid < 64) {
+#pragma unroll
+        for (int i = 0; i < 16; ++i) y[i] = i == j ? 1.0 : 0.0;
+#pragma unroll
+        for (int c = 15; c > 0; --c)
+#pragma unroll
+            for (int i = 0; i < c; ++i) y[i] = fma(-t[o + i][o + c], y[c], y[i]);
+    }
+    __syncthreads();
+    if (tid < 64) {
+#pragma unroll
+        for (int i = 0; i < 16; ++i) t[o + i][o + j] = y[i];
     }
     __syncthreads();
     {
-        // diagonal blocks: 64 threads per block, rows r < 16
-        const int o = (tid >> 6) * 16, r = tid & 63;
-        for (int i = 1; i < 16; ++i) {
-            double s0 = 0.0, s1 = 0.0;
-            if (r < i) {
-                int c = r;
-                for (; c + 1 < i; c += 2) {
-                    s0 = fma(t[o + r][o + c], t[o + c][o + i], s0);
-                    s1 = fma(t[o + r][o + c + 1], t[o + c + 1][o + i], s1);
-                }
-                if (c < i) s0 = fma(t[o + r][o + c], t[o + c][o + i], s0);
+        // blocks (0, 1) and (2, 3): two entries per thread of each 16 x 16 product
+        const int p = tid >> 7, a0 = 32 * p, b0 = a0 + 16, r = (tid >> 3) & 15, c = tid & 7;
+        double s0 = 0.0, s1 = 0.0;
+#pragma unroll
+        for (int q = 0; q < 16; ++q) {
+            s0 = fma(t[a0 + r][b0 + q], t[b0 + q][b0 + c], s0);
+            s1 = fma(t[a0 + r][b0 + q], t[b0 + q][b0 + c + 8], s1);
+        }
+        x[16 * p + r][c] = s0;
+        x[16 * p + r][c + 8] = s1;
+        __syncthreads();
+        s0 = s1 = 0.0;
+#pragma unroll
+        for (int q = 0; q < 16; ++q) {
+            s0 = fma(t[a0 + r][a0 + q], x[16 * p + q][c], s0);
+            s1 = fma(t[a0 + r][a0 + q], x[16 * p + q][c + 8], s1);
+        }
+        t[a0 + r][b0 + c] = -s0;
+        t[a0 + r][b0 + c + 8] = -s1;
+        __syncthreads();
+    }
+    {
+        const int r = tid >> 3, c = tid & 7;
+        double s4[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll 8
+        for (int q = 0; q < 32; ++q) {
+            const double v = t[r][32 + q];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) s4[i] = fma(v, t[32 + q][32 + c + 8 * i], s4[i]);
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            x[r][c + 8 * i] = s4[i];
+            s4[i] = 0.0;
+        }
+        __syncthreads();
+#pragma unroll 8
+        for (int q = 0; q < 32; ++q) {
+            const double v = t[r][q];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) s4[i] = fma(v, x[q][c + 8 * i], s4[i]);
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) t[r][32 + c + 8 * i] = -s4[i];
+        __syncthreads();
+    }
+    for (int e = tid; e < 64 * 64; e += BT_THREADS) T[e] = t[e >> 6][e & 63] * s_tau[e & 63];
+}
+
+__global__ void __launch_bounds__(BT_THREADS) qr_build_t_kernel(const double* G, const double* tau, int kb,
+                                                                double* T) {
+    extern __shared__ double dyn[];
+    double(*t)[BT_LD] = reinterpret_cast<double(*)[BT_LD]>(dyn);
+    double(*x)[33] = reinterpret_cast<double(*)[33]>(dyn + 64 * BT_LD);
+    for (int e = threadIdx.x; e < 64 * 64; e += BT_THREADS) t[e >> 6][e & 63] = G[e];
+    __syncthreads();
+    build_t(t, x, tau, kb, T);
+}
+constexpr int BT_SMEM = (64 * BT_LD + 32 * 33) * 8;
+
+// V and T of one panel per cluster, panels p0, p0 + 1, ... in one launch: the
+// cluster's CTAs pack their rows of V, 32 at a time, and sum V^T V over them on
+// the DMMA path (the 20 of its 16 x 8 blocks that reach above the diagonal);
+// each CTA then adds its share of the CTAs' partial sums in rank order, through
+// distributed shared memory, and rank 0 forms T.  Latency-bound: 14 us for one
+// panel of 2304 rows (four launches before, 30 us: packing 2, partial sums 7,
+// their total 4, T 17.5), 24 us for the 16 panels of n = 1024 together (480 us
+// one by one).
+constexpr int VT_THREADS = 256, VT_CHUNK = 32, VT_LD = 68;  // VT_LD: fragment loads hit distinct banks
+constexpr int VT_SMEM = (64 * 64 + 64 * BT_LD + VT_CHUNK * VT_LD) * 8;
+constexpr int VT_MAX_ROWS = 4096;
+
+__global__ void __launch_bounds__(VT_THREADS) qr_vt_kernel(const double* A, long long lda, int m, int kmax, int p0,
+                                                           int shift, const double* tau, double* V, long long ldv,
+                                                           double* T) {
+    extern __shared__ double dyn[];
+    double* part = dyn;                                                           // 64 x 64
+    double(*t)[BT_LD] = reinterpret_cast<double(*)[BT_LD]>(dyn + 64 * 64);
+    double(*sv)[VT_LD] = reinterpret_cast<double(*)[VT_LD]>(dyn + 64 * 64 + 64 * BT_LD);  // [row][column]
+    cg::cluster_group cluster = cg::this_cluster();
+    const int P = (int)cluster.num_blocks(), cta = (int)cluster.block_rank();
+    const int pi = blockIdx.x / P, k0 = (p0 + pi) * 64, kb = min(64, kmax - k0);
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, tq = lane & 3;
+    const int R = ((m - k0 + P - 1) / P + VT_CHUNK - 1) / VT_CHUNK * VT_CHUNK;
+    const int r0 = k0 + cta * R, r1 = min(m, r0 + R);
+    double* Vp = V + (size_t)pi * ldv * 64;
+    constexpr int CW = 64 / (VT_THREADS / 32);  // columns per warp
+    double v[CW];
+    auto fetch = [&](int c0) {
+        const int row = c0 + lane;
+#pragma unroll
+        for (int i = 0; i < CW; ++i) {
+            const int c = warp * CW + i, k = k0 + c + shift;
+            v[i] = c < kb && row > k && row < r1 ? A[(long long)(k0 + c) * lda + row] : (c < kb && row == k ? 1.0 : 0.0);
+        }
+    };
+    // this warp's 16 x 8 blocks: 0 .. 19 in rows of 8, 6, 4, 2
+    int bi[3], bj[3];
+#pragma unroll
+    for (int q = 0; q < 3; ++q) {
+        const int b = warp + 8 * q;
+        bi[q] = b < 8 ? 0 : b < 14 ? 1 : b < 18 ? 2 : 3;
+        bj[q] = b < 8 ? b : b < 14 ? b - 6 : b < 18 ? b - 10 : b - 12;
+    }
+    double acc[3][4] = {};
+    if (r0 < r1) fetch(r0);
+    for (int c0 = r0; c0 < r1; c0 += VT_CHUNK) {
+#pragma unroll
+        for (int i = 0; i < CW; ++i) {
+            sv[lane][warp * CW + i] = v[i];
+            if (c0 + lane < r1) Vp[(size_t)(warp * CW + i) * ldv + c0 + lane] = v[i];
+        }
+        __syncthreads();
+        if (c0 + VT_CHUNK < r1) fetch(c0 + VT_CHUNK);
+#pragma unroll
+        for (int ks = 0; ks < VT_CHUNK; ks += 8)
+#pragma unroll
+            for (int q = 0; q < 3; ++q) {
+                if (q == 2 && warp >= 4) continue;
+                double fa[4], fb[2];
+#pragma unroll
+                for (int i = 0; i < 4; ++i) fa[i] = sv[ks + tq + 4 * (i >> 1)][16 * bi[q] + g + 8 * (i & 1)];
+#pragma unroll
+                for (int i = 0; i < 2; ++i) fb[i] = sv[ks + tq + 4 * i][8 * bj[q] + g];
+                dmma::mma_f64<8>(acc[q], fa, fb);
             }
-            __syncthreads();  // column i of the block is read in full before it is overwritten
-            if (r < i) t[o + r][o + i] = s0 + s1;
-            __syncthreads();
-        }
-    }
-    // joins: x = G_ab T_bb, then T_ab = -T_aa x (T_aa, T_bb upper triangular)
-    for (int level = 0; level < 2; ++level) {
-        const int w = level == 0 ? 16 : 32;
-        for (int e = tid; e < 2 * 16 * 16 * (1 - level) + 32 * 32 * level; e += BT_THREADS) {
-            const int p = level == 0 ? e >> 8 : 0, q = level == 0 ? e & 255 : e;
-            const int rr = q / w, j = q % w;
-            const int a0 = level == 0 ? 32 * p : 0, b0 = a0 + w;
-            double s = 0.0;
-            for (int c = 0; c <= j; ++c) s = fma(G[(a0 + rr) * 64 + b0 + c], t[b0 + c][b0 + j], s);
-            x[p * 16 + rr][j] = s;
-        }
-        __syncthreads();
-        for (int e = tid; e < 2 * 16 * 16 * (1 - level) + 32 * 32 * level; e += BT_THREADS) {
-            const int p = level == 0 ? e >> 8 : 0, q = level == 0 ? e & 255 : e;
-            const int rr = q / w, j = q % w;
-            const int a0 = level == 0 ? 32 * p : 0, b0 = a0 + w;
-            double s = 0.0;
-            for (int c = rr; c < w; ++c) s = fma(t[a0 + rr][a0 + c], x[p * 16 + c][j], s);
-            t[a0 + rr][b0 + j] = -s;
-        }
         __syncthreads();
     }
-    for (int e = tid; e < 64 * 64; e += BT_THREADS) T[e] = t[e >> 6][e & 63];
+#pragma unroll
+    for (int q = 0; q < 3; ++q) {
+        if (q == 2 && warp >= 4) continue;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) part[(16 * bi[q] + g + 8 * (i >> 1)) * 64 + 8 * bj[q] + 2 * tq + (i & 1)] = acc[q][i];
+    }
+    cluster.sync();
+    // entries above the diagonal only: the blocks below it were not formed
+    for (int e = cta * VT_THREADS + tid; e < 64 * 64; e += P * VT_THREADS) {
+        if ((e >> 6) >= (e & 63)) continue;
+        double s[RG_MAX];
+#pragma unroll
+        for (int q = 0; q < RG_MAX; ++q) s[q] = q < P ? *cluster.map_shared_rank(&part[e], q) : 0.0;
+        double sum = s[0];
+#pragma unroll
+        for (int q = 1; q < RG_MAX; ++q) sum += s[q];
+        *cluster.map_shared_rank(&t[e >> 6][e & 63], 0) = sum;
+    }
+    cluster.sync();
+    if (cta == 0) build_t(t, reinterpret_cast<double(*)[33]>(&sv[0][0]), tau + k0, kb, T + (size_t)pi * 64 * 64);
+}
+
+// VT = V op(T) (op: T, or T^T), panels p0, p0 + 1, ...: 64 rows of one panel per CTA
+constexpr int VP_SMEM = 2 * 64 * VT_LD * 8;
+__global__ void __launch_bounds__(VT_THREADS) qr_vt_product_kernel(const double* V, long long ldv, int m, int p0,
+                                                                   const double* T, int trans, double* VT) {
+    extern __shared__ double dyn[];
+    double(*sv)[VT_LD] = reinterpret_cast<double(*)[VT_LD]>(dyn);                // [column][row]
+    double(*st)[VT_LD] = reinterpret_cast<double(*)[VT_LD]>(dyn + 64 * VT_LD);   // T: [row][column]
+    const int pi = blockIdx.y, k0 = (p0 + pi) * 64, r0 = k0 + 64 * blockIdx.x;
+    if (r0 >= m) return;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, tq = lane & 3;
+    const double* Vp = V + (size_t)pi * ldv * 64;
+    const double* Tp = T + (size_t)pi * 64 * 64;
+    for (int e = tid; e < 64 * 64; e += VT_THREADS) {
+        const int r = e & 63, c = e >> 6;
+        sv[c][r] = r0 + r < m ? Vp[(size_t)c * ldv + r0 + r] : 0.0;
+        st[e >> 6][e & 63] = Tp[e];
+    }
+    __syncthreads();
+    const int wr = (warp >> 2) * 32, wc = (warp & 3) * 16;
+    double acc[2][2][4] = {};
+#pragma unroll
+    for (int ks = 0; ks < 64; ks += 8) {
+        double fa[2][4], fb[2][2];
+#pragma unroll
+        for (int a = 0; a < 2; ++a)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) fa[a][i] = sv[ks + tq + 4 * (i >> 1)][wr + 16 * a + g + 8 * (i & 1)];
+#pragma unroll
+        for (int b = 0; b < 2; ++b)
+#pragma unroll
+            for (int i = 0; i < 2; ++i)
+                fb[b][i] = trans ? st[wc + 8 * b + g][ks + tq + 4 * i] : st[ks + tq + 4 * i][wc + 8 * b + g];
+#pragma unroll
+        for (int a = 0; a < 2; ++a)
+#pragma unroll
+            for (int b = 0; b < 2; ++b) dmma::mma_f64<8>(acc[a][b], fa[a], fb[b]);
+    }
+    double* out = VT + (size_t)pi * ldv * 64;
+#pragma unroll
+    for (int a = 0; a < 2; ++a)
+#pragma unroll
+        for (int b = 0; b < 2; ++b)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const int row = r0 + wr + 16 * a + g + 8 * (i >> 1), col = wc + 8 * b + 2 * tq + (i & 1);
+                if (row < m) out[(size_t)col * ldv + row] = acc[a][b][i];
+            }
 }
 
 // ones on the diagonal of a column-major matrix
@@ -1158,13 +1332,6 @@ int launch_qr_panel(double* a, long long lda, int m, int k0, int kb, double* tau
     return e == cudaSuccess ? JLC_OK : JLC_E_LAUNCH;
 }
 
-int launch_qr_pack_v(const double* a, long long lda, int m, int k0, int kb, double* v, long long ldv,
-                     cudaStream_t st) {
-    const long long total = ldv * 64;
-    qr::qr_pack_v_kernel<<<(unsigned)((total + 255) / 256), 256, 0, st>>>(a, lda, m, k0, kb, v, ldv);
-    return cudaGetLastError() == cudaSuccess ? JLC_OK : JLC_E_LAUNCH;
-}
-
 int launch_set_identity(double* q, long long ldq, long long m, long long cols, cudaStream_t st) {
     if (cudaMemset2DAsync(q, (size_t)ldq * sizeof(double), 0, (size_t)m * sizeof(double), (size_t)cols, st) !=
         cudaSuccess)
@@ -1174,23 +1341,60 @@ int launch_set_identity(double* q, long long ldq, long long m, long long cols, c
     return cudaGetLastError() == cudaSuccess ? JLC_OK : JLC_E_LAUNCH;
 }
 
-size_t qr_gram_scratch_bytes(int sm_count) { return (size_t)(sm_count > 0 ? sm_count : 1) * 64 * 64 * sizeof(double); }
-
-int launch_qr_gram(const double* v, long long ldv, int r0, int r1, double* g, double* scratch, int sm_count,
-                   cudaStream_t st) {
-    const int rows = r1 - r0;
-    int parts = (rows + qr::GR_CHUNK - 1) / qr::GR_CHUNK;
-    if (parts > sm_count) parts = sm_count;
-    if (parts < 1) parts = 1;
-    const int slab = (rows + parts - 1) / parts;
-    parts = rows > 0 ? (rows + slab - 1) / slab : 1;
-    qr::qr_gram_partial_kernel<<<parts, qr::GR_THREADS, 0, st>>>(v, ldv, r0, r1, rows > 0 ? slab : 0, scratch);
-    qr::qr_gram_sum_kernel<<<(64 * 64 + 255) / 256, 256, 0, st>>>(scratch, parts, g);
-    return cudaGetLastError() == cudaSuccess ? JLC_OK : JLC_E_LAUNCH;
+size_t qr_gram_scratch_bytes(int sm_count) {
+    return ((size_t)(sm_count > 0 ? sm_count : 1) + 1) * 64 * 64 * sizeof(double);
 }
 
-int launch_qr_build_t(const double* g, const double* tau, int kb, double* t, cudaStream_t st) {
-    qr::qr_build_t_kernel<<<1, qr::BT_THREADS, 0, st>>>(g, tau, kb, t);
+// V, T and V op(T) of the panels p0 .. p0 + panels - 1 (64 columns each) of the
+// reflectors stored in a (below the diagonal shifted down by `shift` rows):
+// panel p0 + i's at v + i 64 ldv, t + i 64^2 and vt + i 64 ldv.
+int launch_qr_vt(const double* a, long long lda, int m, int kmax, int p0, int panels, int shift, const double* tau,
+                 double* v, long long ldv, double* t, double* vt, bool trans, double* gram, int cluster_max,
+                 int sm_count, cudaStream_t st) {
+    using namespace qr;
+    const int rows = m - 64 * p0;  // of the tallest panel
+    if (rows <= VT_MAX_ROWS) {
+        cudaLaunchConfig_t cfg = {};
+        cudaLaunchAttribute at[1];
+        const int cl = max(1, min((rows + 63) / 64, min(cluster_max, RG_MAX)));
+        cfg.gridDim = dim3(cl * panels);
+        cfg.blockDim = dim3(VT_THREADS);
+        cfg.dynamicSmemBytes = VT_SMEM;
+        cfg.stream = st;
+        at[0].id = cudaLaunchAttributeClusterDimension;
+        at[0].val.clusterDim.x = cl;
+        at[0].val.clusterDim.y = 1;
+        at[0].val.clusterDim.z = 1;
+        cfg.attrs = at;
+        cfg.numAttrs = 1;
+        const void* kern = (const void*)qr_vt_kernel;
+        if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, VT_SMEM) != cudaSuccess ||
+            cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
+            cudaLaunchKernelEx(&cfg, qr_vt_kernel, a, lda, m, kmax, p0, shift, tau, v, ldv, t) != cudaSuccess)
+            return JLC_E_LAUNCH;
+    } else {
+        if (cudaFuncSetAttribute((const void*)qr_build_t_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 BT_SMEM) != cudaSuccess)
+            return JLC_E_LAUNCH;
+        for (int i = 0; i < panels; ++i) {
+            const int k0 = 64 * (p0 + i), kb = min(64, kmax - k0);
+            double* vi = v + (size_t)i * ldv * 64;
+            qr_pack_v_kernel<<<(unsigned)((ldv * 64 + 255) / 256), 256, 0, st>>>(a, lda, m, k0, kb, shift, vi, ldv);
+            int parts = (m - k0 + GR_CHUNK - 1) / GR_CHUNK;
+            if (parts > sm_count) parts = sm_count;
+            const int slab = (m - k0 + parts - 1) / parts;
+            parts = (m - k0 + slab - 1) / slab;
+            double* g = gram + (size_t)sm_count * 64 * 64;
+            qr_gram_partial_kernel<<<parts, GR_THREADS, 0, st>>>(vi, ldv, k0, m, slab, gram);
+            qr_gram_sum_kernel<<<(64 * 64 + 255) / 256, 256, 0, st>>>(gram, parts, g);
+            qr_build_t_kernel<<<1, BT_THREADS, BT_SMEM, st>>>(g, tau + k0, kb, t + (size_t)i * 64 * 64);
+        }
+    }
+    if (cudaFuncSetAttribute((const void*)qr_vt_product_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, VP_SMEM) !=
+        cudaSuccess)
+        return JLC_E_LAUNCH;
+    qr_vt_product_kernel<<<dim3((unsigned)((rows + 63) / 64), (unsigned)panels), VT_THREADS, VP_SMEM, st>>>(
+        v, ldv, m, p0, t, trans ? 1 : 0, vt);
     return cudaGetLastError() == cudaSuccess ? JLC_OK : JLC_E_LAUNCH;
 }
 

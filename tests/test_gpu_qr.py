@@ -211,3 +211,26 @@ def test_panel_sign_flip_and_last_row(ctx, oracle):
     f_ref, tau_ref = oracle.householder_qr_blocked(a)
     np.testing.assert_allclose(tau.cpu().numpy(), tau_ref, rtol=0, atol=1e-12)
     np.testing.assert_allclose(at[:, :64].cpu().numpy().T, f_ref, rtol=0, atol=1e-11)
+
+
+@pytest.mark.parametrize("m,n,qcols", [
+    (300, 200, 100), (300, 130, 300), (65, 64, 65), (200, 300, 150),   # fewer, more columns than reflectors
+    (20000, 1000, 1000),   # more panels than one batch's workspace; panels above 4096 rows
+])
+def test_q_in_batches(ctx, m, n, qcols):
+    """The first columns of Q, formed from panels whose V and T come in
+    batches: orthonormal, and Q^T A is R.  Checked with torch in FP64; a
+    backward stable Q leaves a small multiple of m u."""
+    import torch
+    g = torch.Generator(device="cuda").manual_seed(m + n)
+    a = torch.rand(n, m, dtype=torch.float64, device="cuda", generator=g) * 2 - 1   # column-major m x n
+    f, tau = a.clone(), torch.zeros(min(m, n), dtype=torch.float64, device="cuda")
+    q = torch.zeros(qcols, m, dtype=torch.float64, device="cuda")
+    torch.cuda.synchronize()
+    ctx.qr_factor_device(m, n, f.data_ptr(), m, tau.data_ptr())
+    ctx.qr_build_q_device(m, n, qcols, f.data_ptr(), m, tau.data_ptr(), q.data_ptr(), m)
+    tol = 1e-14 * max(m, n)
+    assert float((q @ q.T - torch.eye(qcols, dtype=torch.float64, device="cuda")).norm()) < tol
+    r = torch.triu(f.T[:min(m, n)])
+    rows = min(qcols, min(m, n))
+    assert float((q[:rows] @ a.T - r[:rows]).norm() / a.norm()) < tol
