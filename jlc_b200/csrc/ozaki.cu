@@ -79,15 +79,12 @@ constexpr int STAGES = 6;
 constexpr int A_STAGE = BM * BKB;   // 16 KB
 constexpr int B_STAGE = BNH * BKB;  // 16 KB
 constexpr int STAGE_BYTES = A_STAGE + B_STAGE;  // per CTA; a stage of the pair completes 2x this
-constexpr int THREADS = 320;  // warp 0 TMA, warp 1 MMA, warps 2..9 epilogue
-constexpr int EPI_WARPS = 8;
 constexpr int TMEM_COLS = 512;
 constexpr int GROUP_CAP = 1040;      // k-blocks per INT32 run: 1040*128*127*127 < 2^31
 constexpr int GROUP_CAP_CRT = 128;  // residues up to 128 in magnitude: 128*128*128*128 = 2^28 (crt::kAccBound)
-constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 + 256;
+constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 + 512;
 constexpr int SCRATCH_DOUBLES = BM * BN;  // per CTA, slice scheme (FP64 running sums)
 constexpr int MAX_MODULI = 15;            // product of 15 moduli < 2^123 = three 41-bit digits
-constexpr int RECON_GROUPS = BN / 2 / 4;  // groups of 4 columns per epilogue thread and tile
 constexpr int CRT_SLOT_WORDS = (BN / 4) * BM;  // one residue byte per element, 4 per word
 
 // the moduli, scaling helpers and digit encoder live in jlc_residue.cuh
@@ -106,6 +103,26 @@ using CrtConsts = crt::Consts;
 constexpr int kModeSlices = 0;  // slice pairs, FP64 recombination
 constexpr int kModeCrt = 1;     // residues, exact CRT reconstruction
 constexpr int kModeCert = 2;    // accuracy certificate: one product of the magnitude planes
+
+// Warps: 0 TMA, 1 MMA, the rest epilogue.  The residue and certificate epilogues
+// are chains of integer and FP32 operations that two warps per scheduler leave
+// mostly waiting, so they take 16 warps (64 of the 256 columns each), as many as
+// the registers allow.  us at (m, n, k), 8 -> 16 warps: residue GEMM 2048 x 2048 x
+// 2600 (one tile per pair) 232 -> 201, 3000 x 2304 x 2600 400 -> 350, 4096 x 4096 x
+// 2048 664 -> 565, 4096^3 852 -> 823; certificate 3000 x 2304 x 2600 64 -> 45, 8192^3
+// 379 -> 338.  Where the MMAs of many long tiles hide the epilogue the GEMM runs at
+// the power cap and 8 warps are as fast or faster (6144 x 6144 x 8192 2887 against
+// 2893, 8192^3 5053 against 5095).  The slice epilogue holds FP64 sums in 166
+// registers and keeps 8.
+template <int EW>
+struct Epi {
+    static constexpr int PARTS = EW / 4;    // warps that share a lane quarter split the columns
+    static constexpr int COLS = BN / PARTS;  // columns per warp
+    static constexpr int THREADS = 64 + 32 * EW;
+    static constexpr int RECON_GROUPS = COLS / 4;  // groups of 4 columns per thread and tile
+};
+// epilogue warps of the residue GEMM
+static int crt_epi_warps(long long tiles, int pairs, long long k) { return k > 6144 && tiles > 4LL * pairs ? 8 : 16; }
 
 // Route decision of the certificate (kModeCert), made by the CTA that
 // finishes last.  For a level (slice or modulus count) the certified ratio is
@@ -204,12 +221,13 @@ __device__ __forceinline__ void cert_decide(const Params& p) {
     __threadfence();
 }
 
-template <int MODE>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
+template <int MODE, int EPI_WARPS>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(Epi<EPI_WARPS>::THREADS, 1)
     ozaki_gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB,
                       const Params p) {
     constexpr bool CRT = MODE == kModeCrt;
     constexpr bool CERT = MODE == kModeCert;
+    constexpr int COLS = Epi<EPI_WARPS>::COLS, RECON_GROUPS = Epi<EPI_WARPS>::RECON_GROUPS;
     // both CTAs of a pair read the same flags, so both leave here or neither
     if ((p.flags[kFlagNonfiniteA] | p.flags[kFlagNonfiniteB]) != 0) return;
     if (p.route_want >= 0 && p.flags[kFlagRoute] != p.route_want) return;
@@ -352,11 +370,11 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
             drain_wait(mma_done, 0, p.status);
         }
     } else {
-        // ---------------- epilogue (warps 2..9) ----------------
+        // ---------------- epilogue (warps 2..) ----------------
         // Warp w reads TMEM lanes 32*(w%4)..+31 (one C row per thread); the
-        // two warps sharing a lane quarter split the 256 columns in halves.
+        // warps sharing a lane quarter split the 256 columns.
         const int quarter = warp & 3;
-        const int half = (warp - 2) >> 2;
+        const int part0 = ((warp - 2) >> 2) * COLS;  // this warp's first column
         const int row = quarter * 32 + lane;
         const bool c_vec = ((reinterpret_cast<uintptr_t>(p.C) & 15) == 0) && ((p.ldc & 1) == 0);
         const double out_scale = p.epi_scale == 1.0 ? p.alpha : p.alpha * p.epi_scale;
@@ -431,7 +449,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
         // Residue scheme: a finished tile's Chinese remainder reconstruction is
         // spread over the next tile's runs (a share after each accumulator is
         // released), so the MMAs never wait for it.  Each thread owns one row
-        // and 128 columns of the tile: RECON_GROUPS groups of 4 columns.
+        // and COLS columns of the tile: RECON_GROUPS groups of 4 columns.
         int pend_left = 0, pend_n0 = 0, pend_grow = 0, pend_ei = 0;
         bool pend_row_ok = false;
         const uint32_t* pend_slots = crt_base;
@@ -443,7 +461,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
         // in flight while the current group is reconstructed.
         auto recon_load = [&](int g, uint32_t(&w)[MAX_MODULI], int(&sc)[4]) {
             const CrtConsts& cc = p.crt;
-            const int c = half * (BN / 2) + 4 * g;
+            const int c = part0 + 4 * g;
             const uint32_t* gbase = pend_slots + (size_t)(c >> 2) * BM + row;
 #pragma unroll
             for (int l = 0; l < MAX_MODULI; ++l) w[l] = l < cc.nmod ? gbase[(size_t)l * CRT_SLOT_WORDS] : 0u;
@@ -468,7 +486,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
                 if (g + 1 < g1) recon_load(g + 1, w, sc);
                 double out[4];
                 crt::reconstruct4(p.crt, cur, scur, out);
-                const int c = half * (BN / 2) + 4 * g;
+                const int c = part0 + 4 * g;
 #pragma unroll
                 for (int e = 0; e < 4; ++e)
                     if (pend_n0 + c + e >= p.N) out[e] = 0.0;
@@ -505,10 +523,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
                     }
                     tc_fence_after();
                     const bool last = (di == runs.ndiag - 1 && gi == ngroups - 1);
-                    const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + buf * BN + half * (BN / 2);
+                    const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + buf * BN + part0;
 #pragma unroll 1
-                    for (int ch = 0; ch < BN / 64; ++ch) {
-                        const int c0 = half * (BN / 2) + ch * 32;  // first column of this chunk in the tile
+                    for (int ch = 0; ch < COLS / 32; ++ch) {
+                        const int c0 = part0 + ch * 32;  // first column of this chunk in the tile
                         uint32_t r[32];
                         tmem_ld32(taddr + ch * 32, r);
                         tmem_wait_ld();
@@ -1227,14 +1245,18 @@ static int launch_mode(int mode, const GemmDesc& g, const OzakiBufs& b, int coun
         p.dot_partials = g.dot_partials;
     }
     if (mode == kModeCrt) crt_constants(count, g.k, p.crt);
-    auto kern = mode == kModeCrt ? ozaki_gemm_kernel<kModeCrt>
-                                 : (mode == kModeSlices ? ozaki_gemm_kernel<kModeSlices> : ozaki_gemm_kernel<kModeCert>);
+    const int ew = mode == kModeSlices ? 8 : mode == kModeCert ? 16 : crt_epi_warps(b.tiles_m * b.tiles_n, b.grid / 2, g.k);
+    auto kern = mode == kModeSlices ? ozaki_gemm_kernel<kModeSlices, 8>
+                : mode == kModeCert ? ozaki_gemm_kernel<kModeCert, 16>
+                : ew == 16          ? ozaki_gemm_kernel<kModeCrt, 16>
+                                    : ozaki_gemm_kernel<kModeCrt, 8>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
     if (e != cudaSuccess) {
         snprintf(err, errlen, "Ozaki smem attribute: %s", cudaGetErrorString(e));
         return JLC_E_LAUNCH;
     }
-    kern<<<b.grid, THREADS, SMEM_BYTES, st>>>(ma, mb, p);
+    const int threads = ew == 16 ? Epi<16>::THREADS : Epi<8>::THREADS;
+    kern<<<b.grid, threads, SMEM_BYTES, st>>>(ma, mb, p);
     e = cudaGetLastError();
     if (e != cudaSuccess) {
         snprintf(err, errlen, "Ozaki GEMM launch failed: %s", cudaGetErrorString(e));
