@@ -203,7 +203,7 @@ int run_device(jlc_ctx* ctx, const GemmDesc& g0, int precision, int slices, jlc_
         }
         if (rep) rep->kernel = JLC_KERNEL_GEMV;
         Phase ph(ctx, JLC_PHASE_GEMV);
-        ctx->launches += v.cs == 1 ? 1 : 2;
+        ctx->launches += need == 0 ? 1 : 2;
         return launch_gemv(v, ctx->ws.ptr, ctx->stream, ctx->sm_count, ctx->err, sizeof(ctx->err));
     }
     // a row block of a pipelined product follows the whole product's choice

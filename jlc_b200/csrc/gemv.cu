@@ -10,84 +10,154 @@
 namespace jlc {
 namespace {
 
-constexpr int GEMV_ROWS = 4;      // rows per warp in the dot form: x is loaded once for 4 rows
-constexpr int GEMV_UNROLL = 4;    // 32-wide column chunks per loop trip
-constexpr int GEMV_THREADS = 256;
+constexpr int GEMV_THREADS = 256, GEMV_WARPS = GEMV_THREADS / 32;
+constexpr int GEMV_LOADS = 16;     // matrix loads a lane keeps in flight (dot form)
+constexpr int GEMV_AXPY_CTAS = 8;  // resident CTAs per SM (axpy form)
 
-// Dot form: M(i,p) = mat[i*rs + p]; one warp per GEMV_ROWS rows, lanes stride the row.
-__global__ void __launch_bounds__(GEMV_THREADS) gemv_dot_kernel(GemvDesc g) {
-    const int lane = threadIdx.x & 31;
-    const long long warp_global = (long long)blockIdx.x * (GEMV_THREADS / 32) + (threadIdx.x >> 5);
-    const long long row0 = warp_global * GEMV_ROWS;
-    if (row0 >= g.rows) return;
-    double acc[GEMV_ROWS];
-    const double* rowp[GEMV_ROWS];
+// How a product's rows and columns are dealt to CTAs.  The kernels are bound by
+// HBM, so every SM needs enough loads in flight and an equal share of the work: a
+// wave of CTAs, or many short waves.  A dot-form CTA that owned 32 rows left 512
+// CTAs for 16384 rows, 3.46 per SM, so that the SMs with three idled while the
+// others ran a fourth, and 16 CTAs for 512 rows.  The warps of a CTA therefore
+// split the columns wk ways as the rows run out, each warp takes fewer rows, and
+// at last the columns are split over CTAs.  us before -> after, A row-major:
+// 16384^2 371 -> 335 (6.4 TB/s), 4096 x 8192 145 -> 44, 512 x 16384 293 -> 16;
+// column-major: 16384^2 457 -> 316, 2000 x 16000 67 -> 49, 512 x 16384 60 -> 26.
+struct GemvShape {
+    int rows_per_warp;  // dot form: 4, 2 or 1
+    int wk;             // warps that share a row group and split its columns (1, 2, 4, 8)
+    int chunks;         // column chunks over CTAs (partial sums in scratch when > 1)
+    long long chunk;    // columns per chunk
+};
+
+__device__ __forceinline__ void gemv_store(const GemvDesc& g, long long row, double s) {
+    double* y = g.y + row * g.incy;
+    *y = (g.beta == 0.0) ? g.alpha * s : fma(g.alpha, s, g.beta * *y);
+}
+
+// Dot form: M(i,p) = mat[i*rs + p]; a warp takes R rows (x is loaded once for
+// them) of its share of the columns, lanes along the row.
+template <int R>
+__global__ void __launch_bounds__(GEMV_THREADS) gemv_dot_kernel(GemvDesc g, int wk, long long chunk, double* partial) {
+    __shared__ double red[GEMV_WARPS * R];
+    constexpr int U = GEMV_LOADS / R;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const long long row0 = ((long long)blockIdx.x * (GEMV_WARPS / wk) + warp / wk) * R;
+    const long long c0 = (long long)blockIdx.y * chunk, c1 = c0 + chunk < g.cols ? c0 + chunk : g.cols;
+    // this warp's columns: its share of the chunk in whole trips
+    const long long trips = (c1 - c0 + 32 * U - 1) / (32 * U), per = (trips + wk - 1) / wk * (32 * U);
+    const long long p0 = c0 + (warp % wk) * per, p1 = p0 + per < c1 ? p0 + per : c1;
+    double acc[R];
+    const double* rowp[R];
 #pragma unroll
-    for (int r = 0; r < GEMV_ROWS; ++r) {
+    for (int r = 0; r < R; ++r) {
         acc[r] = 0.0;
         const long long row = row0 + r < g.rows ? row0 + r : g.rows - 1;
         rowp[r] = g.mat + row * g.rs;
     }
-    const long long K = g.cols;
-    const long long step = 32 * GEMV_UNROLL;
-    long long p = lane;
-    for (; p + 32 * (GEMV_UNROLL - 1) < K; p += step) {
-        double xv[GEMV_UNROLL];
+    long long p = p0 + lane;
+    for (; p + 32 * (U - 1) < p1; p += 32 * U) {
+        double xv[U], m[R][U];
 #pragma unroll
-        for (int u = 0; u < GEMV_UNROLL; ++u) xv[u] = __ldg(g.x + (p + 32 * u) * g.incx);
+        for (int r = 0; r < R; ++r)
 #pragma unroll
-        for (int r = 0; r < GEMV_ROWS; ++r)
+            for (int u = 0; u < U; ++u) m[r][u] = __ldcs(rowp[r] + p + 32 * u);
 #pragma unroll
-            for (int u = 0; u < GEMV_UNROLL; ++u) acc[r] = fma(__ldcs(rowp[r] + p + 32 * u), xv[u], acc[r]);
+        for (int u = 0; u < U; ++u) xv[u] = __ldg(g.x + (p + 32 * u) * g.incx);
+#pragma unroll
+        for (int r = 0; r < R; ++r)
+#pragma unroll
+            for (int u = 0; u < U; ++u) acc[r] = fma(m[r][u], xv[u], acc[r]);
     }
-    for (; p < K; p += 32) {
-        const double xv = __ldg(g.x + p * g.incx);
+    if (p < p1) {
+        double xv[U], m[R][U];
 #pragma unroll
-        for (int r = 0; r < GEMV_ROWS; ++r) acc[r] = fma(__ldcs(rowp[r] + p), xv, acc[r]);
+        for (int r = 0; r < R; ++r)
+#pragma unroll
+            for (int u = 0; u < U; ++u) m[r][u] = p + 32 * u < p1 ? __ldcs(rowp[r] + p + 32 * u) : 0.0;
+#pragma unroll
+        for (int u = 0; u < U; ++u) xv[u] = p + 32 * u < p1 ? __ldg(g.x + (p + 32 * u) * g.incx) : 0.0;
+#pragma unroll
+        for (int r = 0; r < R; ++r)
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+                if (p + 32 * u < p1) acc[r] = fma(m[r][u], xv[u], acc[r]);
     }
 #pragma unroll
-    for (int r = 0; r < GEMV_ROWS; ++r)
+    for (int r = 0; r < R; ++r)
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) acc[r] += __shfl_xor_sync(0xffffffffu, acc[r], o);
-    if (lane == 0) {
+    double mine = acc[0];
 #pragma unroll
-        for (int r = 0; r < GEMV_ROWS; ++r) {
-            const long long row = row0 + r;
-            if (row < g.rows) {
-                double* y = g.y + row * g.incy;
-                *y = (g.beta == 0.0) ? g.alpha * acc[r] : fma(g.alpha, acc[r], g.beta * *y);
-            }
+    for (int r = 1; r < R; ++r)
+        if (lane == r) mine = acc[r];
+    if (wk > 1) {
+        if (lane < R) red[warp * R + lane] = mine;
+        __syncthreads();
+        if (warp % wk != 0) return;
+        if (lane < R) {
+            mine = 0.0;
+            for (int w = 0; w < wk; ++w) mine += red[(warp + w) * R + lane];
         }
     }
-}
-
-// Axpy form: M(i,p) = mat[i + p*cs]; threads own rows, blockIdx.y owns a
-// chunk of columns, partial sums go to scratch[chunk][row].
-__global__ void __launch_bounds__(GEMV_THREADS) gemv_axpy_partial_kernel(GemvDesc g, double* partial,
-                                                                         long long chunk) {
-    const long long row = (long long)blockIdx.x * GEMV_THREADS + threadIdx.x;
-    if (row >= g.rows) return;
-    const long long p0 = (long long)blockIdx.y * chunk;
-    const long long p1 = p0 + chunk < g.cols ? p0 + chunk : g.cols;
-    double a0 = 0.0, a1 = 0.0, a2 = 0.0, a3 = 0.0;
-    long long p = p0;
-    for (; p + 3 < p1; p += 4) {
-        a0 = fma(__ldcs(g.mat + row + (p + 0) * g.cs), __ldg(g.x + (p + 0) * g.incx), a0);
-        a1 = fma(__ldcs(g.mat + row + (p + 1) * g.cs), __ldg(g.x + (p + 1) * g.incx), a1);
-        a2 = fma(__ldcs(g.mat + row + (p + 2) * g.cs), __ldg(g.x + (p + 2) * g.incx), a2);
-        a3 = fma(__ldcs(g.mat + row + (p + 3) * g.cs), __ldg(g.x + (p + 3) * g.incx), a3);
+    const long long row = row0 + lane;
+    if (lane < R && row < g.rows) {
+        if (partial) partial[(long long)blockIdx.y * g.rows + row] = mine;
+        else gemv_store(g, row, mine);
     }
-    for (; p < p1; ++p) a0 = fma(__ldcs(g.mat + row + p * g.cs), __ldg(g.x + p * g.incx), a0);
-    partial[(long long)blockIdx.y * g.rows + row] = (a0 + a1) + (a2 + a3);
 }
 
-__global__ void gemv_axpy_reduce_kernel(GemvDesc g, const double* partial, int nchunks) {
-    const long long row = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (row >= g.rows) return;
+// Axpy form: M(i,p) = mat[i + p*cs]; lanes own rows, the WK warps of a row group
+// split the chunk's columns, partial sums go to scratch[chunk][row].
+template <int WK>
+__global__ void __launch_bounds__(GEMV_THREADS) gemv_axpy_partial_kernel(GemvDesc g, double* partial, long long chunk) {
+    __shared__ double red[WK > 1 ? GEMV_THREADS : 1];
+    const int lane = threadIdx.x & 31, part = (threadIdx.x >> 5) % WK;
+    const long long row = (long long)blockIdx.x * (GEMV_THREADS / WK) + (threadIdx.x >> 5) / WK * 32 + lane;
+    if (WK == 1 && row >= g.rows) return;
+    const long long c0 = (long long)blockIdx.y * chunk;
+    const long long c1 = c0 + chunk < g.cols ? c0 + chunk : g.cols;
+    const long long per = WK == 1 ? c1 - c0 : (c1 - c0 + WK - 1) / WK;
+    const long long p0 = c0 + part * per;
+    const long long p1 = WK == 1 || p0 + per > c1 ? c1 : p0 + per;
+    double a0 = 0.0, a1 = 0.0, a2 = 0.0, a3 = 0.0;
+    if (WK == 1 || row < g.rows) {
+        long long p = p0;
+        for (; p + 3 < p1; p += 4) {
+            a0 = fma(__ldcs(g.mat + row + (p + 0) * g.cs), __ldg(g.x + (p + 0) * g.incx), a0);
+            a1 = fma(__ldcs(g.mat + row + (p + 1) * g.cs), __ldg(g.x + (p + 1) * g.incx), a1);
+            a2 = fma(__ldcs(g.mat + row + (p + 2) * g.cs), __ldg(g.x + (p + 2) * g.incx), a2);
+            a3 = fma(__ldcs(g.mat + row + (p + 3) * g.cs), __ldg(g.x + (p + 3) * g.incx), a3);
+        }
+        for (; p < p1; ++p) a0 = fma(__ldcs(g.mat + row + p * g.cs), __ldg(g.x + p * g.incx), a0);
+    }
+    double s = (a0 + a1) + (a2 + a3);
+    if (WK > 1) {
+        red[threadIdx.x] = s;
+        __syncthreads();
+        if (part != 0) return;
+#pragma unroll
+        for (int w = 1; w < WK; ++w) s += red[threadIdx.x + 32 * w];
+    }
+    if (WK == 1 || row < g.rows) partial[(long long)blockIdx.y * g.rows + row] = s;
+}
+
+// y from the chunks' partial sums: 32 rows per CTA, its warps split the chunks
+__global__ void __launch_bounds__(GEMV_THREADS) gemv_reduce_kernel(GemvDesc g, const double* partial, int nchunks) {
+    __shared__ double red[GEMV_THREADS];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const long long row = (long long)blockIdx.x * 32 + lane;
     double s = 0.0;
-    for (int c = 0; c < nchunks; ++c) s += partial[(long long)c * g.rows + row];
-    double* y = g.y + row * g.incy;
-    *y = (g.beta == 0.0) ? g.alpha * s : fma(g.alpha, s, g.beta * *y);
+    if (row < g.rows) {
+#pragma unroll 8
+        for (int c = warp; c < nchunks; c += GEMV_WARPS) s += partial[(long long)c * g.rows + row];
+    }
+    red[threadIdx.x] = s;
+    __syncthreads();
+    if (warp != 0 || row >= g.rows) return;
+    s = 0.0;
+    for (int w = 0; w < GEMV_WARPS; ++w) s += red[lane + 32 * w];
+    gemv_store(g, row, s);
 }
 
 __global__ void scale_c_kernel(double* c, long long ldc, long long m, long long n, double beta) {
@@ -100,45 +170,73 @@ __global__ void scale_c_kernel(double* c, long long ldc, long long m, long long 
     }
 }
 
-void axpy_split(const GemvDesc& g, int sm_count, long long& chunk, int& nchunks) {
-    const long long row_blocks = (g.rows + GEMV_THREADS - 1) / GEMV_THREADS;
-    long long want = (8LL * sm_count + row_blocks - 1) / row_blocks;  // ~8 blocks of 256 per SM
-    if (want < 1) want = 1;
-    if (want > 64) want = 64;
-    chunk = (g.cols + want - 1) / want;
-    if (chunk < 64) chunk = 64;
-    nchunks = (int)((g.cols + chunk - 1) / chunk);
-    if (nchunks < 1) nchunks = 1;
+GemvShape gemv_shape(const GemvDesc& g, int sm_count) {
+    const long long target = 6LL * sm_count;
+    GemvShape s{4, 1, 1, g.cols};
+    if (g.cs == 1) {
+        auto ctas = [&] { return (g.rows * s.wk + (long long)GEMV_WARPS * s.rows_per_warp - 1) / (GEMV_WARPS * s.rows_per_warp); };
+        // a warp keeps at least one trip (512 / rows_per_warp columns) of its rows
+        while (ctas() < target && s.wk < GEMV_WARPS && g.cols >= 2 * s.wk * 128) s.wk *= 2;
+        while (ctas() < target && s.rows_per_warp > 1) s.rows_per_warp /= 2;
+        const long long most = g.cols / (512 * s.wk);  // chunks of at least 512 columns per warp
+        if (ctas() < target / 2 && most > 1) {
+            long long want = (target + ctas() - 1) / ctas();
+            if (want > most) want = most;
+            if (want > 64) want = 64;
+            s.chunk = (g.cols + want - 1) / want;
+        }
+    } else {
+        // CTAs of 256 rows (2 KB runs of each column) over column chunks, as many as are resident at
+        // once and no more (a second wave of a few CTAs took 457 us at 16384^2, one wave 330); where
+        // that is too few CTAs, the warps of a CTA split the columns.  At least 32 columns per warp.
+        const long long groups = (g.rows + 31) / 32, resident = (long long)GEMV_AXPY_CTAS * sm_count;
+        long long want = 1;
+        for (s.wk = 1;; s.wk *= 2) {
+            const long long ctas = (groups * s.wk + GEMV_WARPS - 1) / GEMV_WARPS;
+            const long long most = g.cols / (32 * s.wk);
+            want = resident / ctas;
+            if (want > most) want = most;
+            if (want > 256) want = 256;
+            if (want < 1) want = 1;
+            if (s.wk == GEMV_WARPS || 2 * ctas * want >= resident || g.cols < 64 * s.wk) break;
+        }
+        s.chunk = (g.cols + want - 1) / want;
+    }
+    s.chunks = (int)((g.cols + s.chunk - 1) / s.chunk);
+    return s;
 }
 
 }  // namespace
 
+// partial sums: the axpy form's always, the dot form's when its columns are split over CTAs
 size_t gemv_scratch_bytes(const GemvDesc& g, int sm_count) {
-    if (g.cs == 1) return 0;
-    long long chunk;
-    int nchunks;
-    axpy_split(g, sm_count, chunk, nchunks);
-    return (size_t)nchunks * (size_t)g.rows * sizeof(double);
+    if (g.rows <= 0 || g.cols <= 0) return 0;
+    const GemvShape s = gemv_shape(g, sm_count);
+    return g.cs == 1 && s.chunks == 1 ? 0 : (size_t)s.chunks * (size_t)g.rows * sizeof(double);
 }
 
 int launch_gemv(const GemvDesc& g, void* scratch, cudaStream_t st, int sm_count, char* err, size_t errlen) {
     if (g.rows <= 0) return JLC_OK;
-    if (g.cs == 1) {
-        const long long warps = (g.rows + GEMV_ROWS - 1) / GEMV_ROWS;
-        const long long blocks = (warps + GEMV_THREADS / 32 - 1) / (GEMV_THREADS / 32);
-        gemv_dot_kernel<<<(unsigned)blocks, GEMV_THREADS, 0, st>>>(g);
-    } else if (g.rs == 1) {
-        long long chunk;
-        int nchunks;
-        axpy_split(g, sm_count, chunk, nchunks);
-        dim3 grid((unsigned)((g.rows + GEMV_THREADS - 1) / GEMV_THREADS), (unsigned)nchunks);
-        gemv_axpy_partial_kernel<<<grid, GEMV_THREADS, 0, st>>>(g, (double*)scratch, chunk);
-        gemv_axpy_reduce_kernel<<<(unsigned)((g.rows + 255) / 256), 256, 0, st>>>(g, (const double*)scratch,
-                                                                                  nchunks);
-    } else {
+    if (g.cs != 1 && g.rs != 1) {
         snprintf(err, errlen, "gemv needs a unit row or column stride");
         return JLC_E_UNSUPPORTED;
     }
+    const GemvShape s = gemv_shape(g, sm_count);
+    double* partial = g.cs == 1 && s.chunks == 1 ? nullptr : static_cast<double*>(scratch);
+    const long long groups = g.cs == 1 ? (g.rows + s.rows_per_warp - 1) / s.rows_per_warp : (g.rows + 31) / 32;
+    const dim3 grid((unsigned)((groups * s.wk + GEMV_WARPS - 1) / GEMV_WARPS), (unsigned)s.chunks);
+    if (g.cs == 1) {
+        auto kern = s.rows_per_warp == 4 ? gemv_dot_kernel<4> : s.rows_per_warp == 2 ? gemv_dot_kernel<2> : gemv_dot_kernel<1>;
+        kern<<<grid, GEMV_THREADS, 0, st>>>(g, s.wk, s.chunk, partial);
+    } else {
+        auto kern = s.wk == 1   ? gemv_axpy_partial_kernel<1>
+                    : s.wk == 2 ? gemv_axpy_partial_kernel<2>
+                    : s.wk == 4 ? gemv_axpy_partial_kernel<4>
+                                : gemv_axpy_partial_kernel<8>;
+        kern<<<grid, GEMV_THREADS, 0, st>>>(g, partial, s.chunk);
+    }
+    if (partial)
+        gemv_reduce_kernel<<<(unsigned)((g.rows + 31) / 32), GEMV_THREADS, 0, st>>>(g, partial, s.chunks);
     if (cudaGetLastError() != cudaSuccess) {
         snprintf(err, errlen, "gemv launch failed");
         return JLC_E_LAUNCH;

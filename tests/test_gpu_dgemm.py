@@ -475,3 +475,34 @@ def test_operands_copied_for_tma(ctx, oracle, m, n, k):
     assert_fp64_bound("aligned", outs[0], a, b, None, 1.0, 0.0)
     np.testing.assert_array_equal(outs[1], outs[0])
     np.testing.assert_array_equal(outs[2], outs[0])
+
+
+@pytest.mark.parametrize("la", [0, 1])
+@pytest.mark.parametrize("m,k", [
+    (2, 1), (31, 33), (33, 1000), (257, 70),    # fewer rows or columns than a warp's share
+    (512, 4100), (1100, 513), (5000, 300),      # warps, then CTAs, that split the columns; whole rows
+    (65, 40001), (3, 70000),                    # column chunks over CTAs in both forms
+])
+def test_matvec_shapes(ctx, oracle, la, m, k):
+    """Matrix-vector products over the row and column splits of both forms,
+    with a strided x and y, and the row-vector product with the transpose."""
+    import torch
+    rng = np.random.default_rng(m + k)
+    a, x, c = rng.uniform(-1, 1, (m, k)), rng.uniform(-1, 1, (k, 1)), rng.uniform(-1, 1, (m, 1))
+    stored = a if la == 0 else a.T
+    at = torch.from_numpy(np.ascontiguousarray(stored)).cuda()
+    xt = torch.full((k, 3), 9.0, dtype=torch.float64)
+    xt[:, 0] = torch.from_numpy(x[:, 0])
+    yt = torch.full((m, 2), 7.0, dtype=torch.float64)
+    yt[:, 0] = torch.from_numpy(c[:, 0])
+    xt, yt = xt.cuda(), yt.cuda()
+    row = torch.from_numpy(c.T.copy()).cuda()
+    torch.cuda.synchronize()
+    ctx.dgemm_device(la, 0, m, 1, k, 1.5, at.data_ptr(), at.shape[1], xt.data_ptr(), 3, -0.5, yt.data_ptr(), 2)
+    # y^T = x^T A^T: B = A^T is stored as A is, in the other layout
+    ctx.dgemm_device(1, 1 - la, 1, m, k, 1.5, xt.data_ptr(), 3, at.data_ptr(), at.shape[1], -0.5, row.data_ptr(), m)
+    ctx.synchronize()
+    y = yt.cpu().numpy()
+    assert (y[:, 1] == 7.0).all()
+    assert_fp64_bound(f"matvec {m}x{k}", y[:, :1], a, x, c, 1.5, -0.5)
+    assert_fp64_bound(f"vecmat {m}x{k}", row.cpu().numpy(), x.T, a.T, c.T, 1.5, -0.5)
