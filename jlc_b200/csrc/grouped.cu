@@ -731,11 +731,14 @@ __global__ void __launch_bounds__(WT_THREADS, STAGES == 2 ? 3 : 2)
 //     the slot's full barrier (cp.async.mbarrier.arrive.noinc), and the ring
 //     runs on across items.  One copy warp alone was measured busy issuing
 //     copies two thirds of the time while the DMMA warps waited for data.
-//   * DMMA warp q owns the 32 x 32 quadrant (q >> 1, q & 1) of the tile: it
-//     waits for a slot, runs the slot's m16n8k8 MMAs on its quadrant (trimmed
-//     to 16-row x 8-column blocks as the warp tiles are) and passes the slot
-//     back on its empty barrier.  A quadrant without valid rows or columns
-//     issues no MMAs but still passes every slot back.
+//   * DMMA warp q owns the quadrant (q >> 1, q & 1) of the tile, whose 16-row and
+//     8-column blocks are halved: an item takes as long as its slowest warp, and a
+//     ragged tile cut at row and column 32 left one warp all of it (9 % of the
+//     slowest warps' blocks over a batch of sizes log-uniform on [8, 512]; 2.57 ->
+//     2.53 ms).  It waits for a slot, runs the slot's m16n8k8 MMAs on its quadrant
+//     (trimmed to those blocks) and passes the slot back on its empty barrier.  A
+//     quadrant without valid rows or columns issues no MMAs but still passes every
+//     slot back.
 //   * Every wait is bounded by the status block's limit; a warp that gives up
 //     records JLC_DEV_TIMEOUT and leaves, and the copy warp first waits for
 //     its own copies in flight.
@@ -958,19 +961,34 @@ __device__ bool ct_consume(const TileItem& w, int wm, int wn, uint32_t ring, uin
                            uint32_t& cidx, int* status, int lane) {
     const int g = lane >> 2, t = lane & 3;
     const int kblocks = (w.k + GBK - 1) / GBK;
-    const int qrows = min(32, w.rows - 32 * wm), qcols = min(32, w.cols - 32 * wn);  // the quadrant's
+    // the quadrant: the tile's 16-row and 8-column blocks are halved, the larger halves first
+    const int rh = (w.rows + 31) >> 5, ch = (w.cols + 15) >> 4;
+    const int r0 = 16 * rh * wm, b0 = ch * wn;  // first row, first 8-column block
+    const int qrows = min(16 * rh, w.rows - r0), qcols = min(8 * ch, w.cols - 8 * b0);
     const int mtv = qrows > 16 ? 2 : (qrows > 0 ? 1 : 0);
     const int ntv = qcols > 0 ? (qcols + 7) >> 3 : 0;
     const bool active = mtv > 0 && ntv > 0;
+    double* const qc = w.c + (long long)r0 * w.ldc + 8 * b0;
     if (active && w.beta != 0.0 && lane < qrows) {
         // C rows of the quadrant into L2 ahead of the epilogue
-        const double* r = w.c + (long long)(32 * wm + lane) * w.ldc + 32 * wn;
+        const double* r = qc + (long long)lane * w.ldc;
         asm volatile("prefetch.global.L2 [%0];" ::"l"(r));
         if (qcols > 16) asm volatile("prefetch.global.L2 [%0];" ::"l"(r + 16));
     }
     uint32_t fa[4], fb[4];
     frag_bases<AK>(fa, g, t, true);
     frag_bases<BK>(fb, g, t, false);
+    const uint32_t qa = ring + 128 * r0;  // the quadrant in slot 0
+    const uint32_t qb = ring + 64 * 128 + (BK ? 1024 * b0 : 2048 * (b0 >> 1));
+    if (!BK && (b0 & 1)) {
+        // the first block is the second half of a 16-column chunk, the next one the first half of
+        // the chunk after it
+        const uint32_t f0 = fb[0], f1 = fb[1];
+        fb[0] = fb[2];
+        fb[1] = fb[3];
+        fb[2] = f0 + 2048;
+        fb[3] = f1 + 2048;
+    }
     double acc[2][4][4];
 #pragma unroll
     for (int i = 0; i < 2; ++i)
@@ -978,8 +996,6 @@ __device__ bool ct_consume(const TileItem& w, int wm, int wn, uint32_t ring, uin
         for (int j = 0; j < 4; ++j)
 #pragma unroll
             for (int e = 0; e < 4; ++e) acc[i][j][e] = 0.0;
-    double* const qc = w.c + (long long)(32 * wm) * w.ldc + 32 * wn;
-    const uint32_t qa = ring + 4096 * wm, qb = ring + 64 * 128 + 4096 * wn;  // the quadrant in slot 0
     for (int kb = 0; kb < kblocks; ++kb)
         if (!ct_slot<AK, BK>(acc, qa, qb, fa, fb, mtv, ntv, full, empty, cidx, status, lane)) return false;
     if (active)

@@ -410,3 +410,30 @@ def test_grouped_ozaki_default_runs_fp64_tiles(ctx, oracle):
     arena.copy_(before)
     rep = ctx.dgemm_grouped_device(probs, precision=JLC_PREC_OZAKI_CRT)
     assert rep["precision"] == JLC_PREC_NATIVE  # the precision actually used
+
+
+@pytest.mark.parametrize("la,lb", [(0, 0), (1, 0), (0, 1), (1, 1)])
+def test_ragged_tiles_of_every_cut(ctx, oracle, la, lb):
+    """64 x 64 tile items of every row and column count at which the cut into
+    the four DMMA warps' quadrants changes (1 .. 4 blocks of 16 rows, 1 .. 8 of
+    8 columns), as a problem's only tile and as its edge tile."""
+    import torch
+    rng = np.random.default_rng(2600 + 2 * la + lb)
+    shapes = [(m, n) for m in (33, 47, 64, 65, 81, 97, 113) for n in (33, 41, 49, 57, 64, 65, 73, 81, 89, 97, 105, 113, 121)]
+    k = 37
+    hosts, keep, probs = [], [], []
+    for m, n in shapes:
+        a, b, c = rng.uniform(-1, 1, (m, k)), rng.uniform(-1, 1, (k, n)), rng.uniform(-1, 1, (m, n))
+        dev = [torch.from_numpy(np.ascontiguousarray(x)).cuda()
+               for x in (a if la == 0 else a.T, b if lb == 0 else b.T, c)]
+        hosts.append((a, b, c))
+        keep.append(dev)
+        probs.append(dict(m=m, n=n, k=k, layout_a=la, layout_b=lb, lda=dev[0].shape[1], ldb=dev[1].shape[1], ldc=n,
+                          alpha=1.5, beta=-0.5, a=dev[0].data_ptr(), b=dev[1].data_ptr(), c=dev[2].data_ptr()))
+    torch.cuda.synchronize()
+    plan = ctx.grouped_plan(probs)
+    plan.run()
+    ctx.synchronize()
+    plan.close()
+    for (m, n), (a, b, c), dev in zip(shapes, hosts, keep):
+        assert_fp64_bound(f"{m}x{n}", dev[2].cpu().numpy(), a, b, c, 1.5, -0.5)
