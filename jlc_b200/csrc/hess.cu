@@ -325,16 +325,18 @@ __global__ void __launch_bounds__(PT, 1) hess_panel_kernel(const PanelArgs p) {
 // Two sums over the CTAs, as in bidiag.cu: the dots of the raw column with
 // the trailing columns, taken in the pass that finishes the step before, and
 // published w_j (a warp sums 2 columns).  The column itself is gathered by
-// every CTA, so H v runs while the dots are on their way.  Values cross in
+// every CTA, so H v runs while w is on its way, and the dots are fetched while
+// the last warp forms the reflector (4.4 us a step at n = 1024 against 5.1 with
+// the fetch after it).  Values cross in
 // tagged slots; there is no barrier.  The reflectors stay below the
 // subdiagonal, from which the blocked Q builder of the QR route forms Q.
 //
 // A step is bound by latency: two exchanges through L2 (about 1500 cycles each
 // from store to load), then the sums and the scalar recipe between them; it
-// takes 5.1 us at n = 1024 and 4.2 us at n = 128.  The panel route pays two
+// takes 4.2 us at n = 1024 and 3.2 us at n = 128.  The panel route pays two
 // grid barriers and a GEMV from L2 per reflector (15 us at n = 1024), six GEMMs
-// per panel, and 107 KB of straight-line code per reflector against 32 KB
-// here.  Measured on B200, H and Q, ms: n = 1024 20.8 -> 6.9.
+// per panel, and 107 KB of straight-line code per reflector against 34 KB
+// here.  Measured on B200, H and Q, ms: n = 1024 20.9 -> 4.7.
 constexpr int SLT = 512;  // threads per CTA
 constexpr int SLW = SLT / 32;
 constexpr int RC = 8;     // rows per register block: a CTA holds a multiple of RC rows
@@ -494,36 +496,49 @@ __global__ void __launch_bounds__(SLT, 1) hess_slab_kernel(const SlabArgs p) {
             for (int i = 0; i < CB; ++i) at[i] = colv + min(kn + tid + i * SLT, n - 1);
             fail |= !slot_wait(at, kn, u, p.status);
         }
-        if (__syncthreads_or(fail)) return;
-        const double tau = s_h.tau, inv = s_h.inv;
+        // ---- w of 2 columns per warp, 16 lanes over the CTAs (the dots are fetched while the last
+        // warp forms the reflector)
+        const int qi = lane >> 1, jj = lane & 1;
+        int gr = kn / 2 + cta + warp * P;  // group of 2 columns, absolute
+        const int glast = (n + 1) / 2;
+        double tau = 0.0, inv = 0.0;
+#pragma unroll 1
+        for (int trip = 0, left = glast - kn / 2; trip == 0 || left > 0; ++trip, left -= P * SLW, gr += P * SLW) {
+            const int j = gr * 2 + jj;
+            double x[QMAX + 1];
+            if (gr < glast) {
+                // (lanes past the last CTA or column wait for a live one and drop what they get)
+                const int jl = min(max(j, kn), n - 1);
+                const Slot* at[QMAX + 1];
+#pragma unroll
+                for (int i = 0; i < QMAX; ++i) at[i] = p.part + (size_t)min(qi + QL * i, P - 1) * ld + jl;
+                at[QMAX] = prow + jl;
+                fail |= !slot_wait(at, kn, x, p.status);
+            }
+            if (trip == 0) {
+                if (__syncthreads_or(fail)) return;
+                tau = s_h.tau;
+                inv = s_h.inv;
+            }
+            if (gr < glast) {
+                __syncwarp();
+                double s0 = 0.0, s1 = 0.0;
+#pragma unroll
+                for (int i = 0; i < QMAX; i += 2) {
+                    s0 += qi + QL * i < P ? x[i] : 0.0;
+                    s1 += qi + QL * (i + 1) < P ? x[i + 1] : 0.0;
+                }
+                double sum = s0 + s1;
+#pragma unroll
+                for (int o = 2; o < 32; o <<= 1) sum += shfl_xor(sum, o);
+                if (qi == 0 && j >= kn && j < n)
+                    slot_put(p.w + j, tau != 0.0 ? tau * fma(sum, inv, x[QMAX]) : 0.0, kn, 0);
+            }
+        }
 #pragma unroll
         for (int i = 0; i < CB; ++i) {
             const int j = kn + tid + i * SLT;
             u[i] = j < n ? (j == kn ? (tau != 0.0 ? 1.0 : 0.0) : u[i] * inv) : 0.0;
-        }
-        // ---- w of 2 columns per warp, 16 lanes over the CTAs
-        const int qi = lane >> 1, jj = lane & 1;
-#pragma unroll 1
-        for (int gr = kn / 2 + cta + warp * P; gr < (n + 1) / 2; gr += P * SLW) {
-            // (lanes past the last CTA or column wait for a live one and drop what they get)
-            const int j = gr * 2 + jj, jl = min(max(j, kn), n - 1);
-            double x[QMAX + 1];
-            const Slot* at[QMAX + 1];
-#pragma unroll
-            for (int i = 0; i < QMAX; ++i) at[i] = p.part + (size_t)min(qi + QL * i, P - 1) * ld + jl;
-            at[QMAX] = prow + jl;
-            fail |= !slot_wait(at, kn, x, p.status);
-            __syncwarp();
-            double s0 = 0.0, s1 = 0.0;
-#pragma unroll
-            for (int i = 0; i < QMAX; i += 2) {
-                s0 += qi + QL * i < P ? x[i] : 0.0;
-                s1 += qi + QL * (i + 1) < P ? x[i + 1] : 0.0;
-            }
-            double sum = s0 + s1;
-#pragma unroll
-            for (int o = 2; o < 32; o <<= 1) sum += shfl_xor(sum, o);
-            if (qi == 0 && j >= kn && j < n) slot_put(p.w + j, tau != 0.0 ? tau * fma(sum, inv, x[QMAX]) : 0.0, kn, 0);
         }
         // v on this CTA's rows; column k is finished: beta, and v's tail below it
         if (tid < rows) {
@@ -611,8 +626,8 @@ namespace hess {
 static int slab_rows(int n, int sm_count) {
     const int most = sm_count < kSlabMaxCtas ? sm_count : kSlabMaxCtas;
     const int rows = ((n + most - 1) / most + RC - 1) / RC * RC;
-    // past two columns per thread at least 16 rows per CTA (n = 1056: 5.9 ms, against 7.3 with 8: half
-    // as many partials cross), below it 8 (n = 1024: 5.3 against 5.5; n = 256: 1.1 against 1.2)
+    // past two columns per thread at least 16 rows per CTA (n = 1056: 5.6 ms, against 6.5 with 8: half
+    // as many partials cross), below it 8 (n = 1024: 4.3 against 5.0; n = 256: 0.84 against 0.99)
     return n > 2 * SLT && rows < 2 * RC ? 2 * RC : rows;
 }
 static size_t slab_smem(int n, int rows) { return ((size_t)rows * ((n + 3) / 4 * 4) + (size_t)SLW * rows) * sizeof(double); }
@@ -658,7 +673,11 @@ int launch_hess_slab(double* h, long long ldh, int n, double* tau, double* work,
     a.w = a.prow + 2 * (size_t)a.ld;
     a.status = status;
     a.eps = 1e-12;
-    const void* kern = n > 2 * SLT ? (const void*)hess_slab_kernel<4> : (const void*)hess_slab_kernel<2>;
+    // columns per thread: the fewest of 1, 2, 4 (n = 512: 3.9 us a step with 1 against 4.1 with 2;
+    // n = 128: 3.6 against 3.9)
+    const void* kern = n > 2 * SLT ? (const void*)hess_slab_kernel<4>
+                       : n > SLT   ? (const void*)hess_slab_kernel<2>
+                                   : (const void*)hess_slab_kernel<1>;
     const size_t bytes = slab_smem(n, a.rows);
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) != cudaSuccess)
         return JLC_E_LAUNCH;

@@ -132,6 +132,7 @@ def test_device_entry_arguments(ctx):
 
 @pytest.mark.parametrize("n,with_q", [
     (3, True), (9, True),            # one CTA, two CTAs
+    (512, True),                     # one column per thread
     (513, True), (1024, False),      # one column past a thread's first; 8 rows per CTA
     (1025, True), (1200, True),      # 16 rows per CTA, three columns per thread
     (1744, True), (1745, True),      # the largest order in shared memory, the smallest of the panel route
