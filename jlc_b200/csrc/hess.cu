@@ -333,10 +333,10 @@ __global__ void __launch_bounds__(PT, 1) hess_panel_kernel(const PanelArgs p) {
 //
 // A step is bound by latency: two exchanges through L2 (about 1500 cycles each
 // from store to load), then the sums and the scalar recipe between them; it
-// takes 4.2 us at n = 1024 and 3.2 us at n = 128.  The panel route pays two
+// takes 4.0 us at n = 1024 and 3.2 us at n = 128.  The panel route pays two
 // grid barriers and a GEMV from L2 per reflector (15 us at n = 1024), six GEMMs
 // per panel, and 107 KB of straight-line code per reflector against 34 KB
-// here.  Measured on B200, H and Q, ms: n = 1024 20.9 -> 4.7.
+// here.  Measured on B200, H and Q, ms: n = 1024 20.9 -> 4.6.
 constexpr int SLT = 512;  // threads per CTA
 constexpr int SLW = SLT / 32;
 constexpr int RC = 8;     // rows per register block: a CTA holds a multiple of RC rows
@@ -490,12 +490,7 @@ __global__ void __launch_bounds__(SLT, 1) hess_slab_kernel(const SlabArgs p) {
                 if (cta == 0) p.tau[k] = r.tau;
             }
         }
-        {
-            const Slot* at[CB];
-#pragma unroll
-            for (int i = 0; i < CB; ++i) at[i] = colv + min(kn + tid + i * SLT, n - 1);
-            fail |= !slot_wait(at, kn, u, p.status);
-        }
+        fail |= !slot_wait_columns<SLT>(colv, kn, n, kn, u, p.status);
         // ---- w of 2 columns per warp, 16 lanes over the CTAs (the dots are fetched while the last
         // warp forms the reflector)
         const int qi = lane >> 1, jj = lane & 1;
@@ -569,10 +564,7 @@ __global__ void __launch_bounds__(SLT, 1) hess_slab_kernel(const SlabArgs p) {
             if ((lane & 3) == 0) red[warp * rows + b * RC + (lane >> 2)] = s;
         }
         {
-            const Slot* at[CB];
-#pragma unroll
-            for (int i = 0; i < CB; ++i) at[i] = p.w + min(kn + tid + i * SLT, n - 1);
-            fail |= !slot_wait(at, kn, w, p.status);
+            fail |= !slot_wait_columns<SLT>(p.w, kn, n, kn, w, p.status);
             __syncwarp();
             double s = 0.0;
 #pragma unroll
@@ -625,10 +617,7 @@ __global__ void __launch_bounds__(SLT, 1) hess_slab_kernel(const SlabArgs p) {
 namespace hess {
 static int slab_rows(int n, int sm_count) {
     const int most = sm_count < kSlabMaxCtas ? sm_count : kSlabMaxCtas;
-    const int rows = ((n + most - 1) / most + RC - 1) / RC * RC;
-    // past two columns per thread at least 16 rows per CTA (n = 1056: 5.6 ms, against 6.5 with 8: half
-    // as many partials cross), below it 8 (n = 1024: 4.3 against 5.0; n = 256: 0.84 against 0.99)
-    return n > 2 * SLT && rows < 2 * RC ? 2 * RC : rows;
+    return ((n + most - 1) / most + RC - 1) / RC * RC;
 }
 static size_t slab_smem(int n, int rows) { return ((size_t)rows * ((n + 3) / 4 * 4) + (size_t)SLW * rows) * sizeof(double); }
 static size_t slab_slots(int n, int P) {
@@ -673,11 +662,12 @@ int launch_hess_slab(double* h, long long ldh, int n, double* tau, double* work,
     a.w = a.prow + 2 * (size_t)a.ld;
     a.status = status;
     a.eps = 1e-12;
-    // columns per thread: the fewest of 1, 2, 4 (n = 512: 3.9 us a step with 1 against 4.1 with 2;
-    // n = 128: 3.6 against 3.9)
-    const void* kern = n > 2 * SLT ? (const void*)hess_slab_kernel<4>
-                       : n > SLT   ? (const void*)hess_slab_kernel<2>
-                                   : (const void*)hess_slab_kernel<1>;
+    // the fewest columns per thread, as empty ones cost a step their issue slots (n = 512: 3.9 us with 1
+    // against 4.1 with 2; n = 1400: 5.5 with 3 against 6.0 with 4)
+    const void* kern = n > 3 * SLT   ? (const void*)hess_slab_kernel<4>
+                       : n > 2 * SLT ? (const void*)hess_slab_kernel<3>
+                       : n > SLT     ? (const void*)hess_slab_kernel<2>
+                                     : (const void*)hess_slab_kernel<1>;
     const size_t bytes = slab_smem(n, a.rows);
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) != cudaSuccess)
         return JLC_E_LAUNCH;

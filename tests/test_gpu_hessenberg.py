@@ -134,7 +134,8 @@ def test_device_entry_arguments(ctx):
     (3, True), (9, True),            # one CTA, two CTAs
     (512, True),                     # one column per thread
     (513, True), (1024, False),      # one column past a thread's first; 8 rows per CTA
-    (1025, True), (1200, True),      # 16 rows per CTA, three columns per thread
+    (1025, True), (1184, False),     # three columns per thread, 8 rows per CTA
+    (1200, True), (1537, True),      # 16 rows per CTA, three columns per thread; four
     (1744, True), (1745, True),      # the largest order in shared memory, the smallest of the panel route
 ])
 def test_route_edges(ctx, n, with_q):
