@@ -27,20 +27,30 @@
 //   * row k after the column reflector is a_kj - w_j: every CTA has both, forms
 //     the row reflector u from them, then x = tau_p (A - v w^T) u on its own
 //     rows (row-local), A - v w^T - x u^T, and the dots of column k + 1.
-// The values cross the CTAs in tagged 16-byte slots (jlc_device.cuh): a reader
+// The values cross the CTAs in tagged 16-byte slots (jlc_slab.cuh): a reader
 // waits for the datum itself, and there is no barrier.
 //
-// What bounds a step is latency: two exchanges through L2 (about 1.2 us each
-// with the waits), two norms (a cross-warp sum, a square root, a division) and
-// two short passes; and the length of the code, since a step runs straight
-// through the kernel once: at 104 KB of instructions (waits inlined with
-// per-slot branches, norms with two-level rescaling, integer divisions for the
-// row numbers) a step took 11 us, at 43 KB 7.0 us.  Measured on B200, reflectors
-// only, ms:                                       512^2  1152x1024  4096^2
-//   rows in place, four grid barriers per step       -      54.4     693.6
-//   slabs, two grid barriers per step               5.3     11.8     172
-//   slots instead of barriers                       5.4     11.4     227
-//   the same in 43 KB of code (this kernel)         3.0      7.1     191
+// What bounds a step is latency: two exchanges through L2 (about 1500 cycles
+// each from store to load), two norms (a cross-warp sum, a square root, a
+// division) and two short passes.  Hence
+//   * A r (r the row before its reflector is known) and the norm of r are summed
+//     in one pass between the same barriers: x = tau_p (t + (A r - v (w . r)) /
+//     (x0 - beta)), t the pivot column, by the warps that have rows to finish
+//     (before: norm, barrier, reflector, pass, barrier);
+//   * few polls: what every CTA polls early delays the stores that it waits
+//     for.  Only the dots are polled for in the first exchange, the pivot row is
+//     fetched once the dots have come, and no warp polls for columns that it
+//     does not have;
+//   * short code, since a step runs straight through the kernel once: at 104 KB
+//     (waits inlined with per-slot branches, two-level rescaling, integer
+//     divisions for the row numbers) a step took 11 us, at 43 KB 7.0.
+// Measured on B200, reflectors only, ms:        512^2  1152x1024  1400^2  4096^2
+//   rows in place, four grid barriers per step    -      54.4       -     693.6
+//   slabs, two grid barriers per step            5.3     11.8       -     172
+//   slots instead of barriers                    5.4     11.4       -     227
+//   the same in 43 KB of code                    3.1      7.1      13.4   191
+//   one pass for A r and its norm, few polls,
+//   3 columns per thread (this kernel)           2.5      5.4       9.0   183
 // U and V are formed afterwards from the stored reflectors by the blocked
 // compact-WY Q builder of the QR route (GEMM kernels).
 //
@@ -99,7 +109,8 @@ __device__ __forceinline__ double down(int d) { return d >= -1022 ? pow2(d) : 0.
 
 // The reference's reflector recipe for a vector with norm 2^E sqrt(S) (x0
 // included) and first entry x0: tau, beta and 2^E / (x0 - beta); tau = 0 and
-// beta = x0 when there is no reflector.
+// beta = x0 when there is no reflector.  By a whole warp: its halves take one of
+// the two quotients each (a quotient is 135 cycles).
 struct Reflector {
     double tau, beta, inv;
 };
@@ -110,11 +121,13 @@ __device__ __noinline__ Reflector reflector(int E, double S, double x0) {
     const double xnorm = p2 * sqrt(S);
     if (xnorm > kSafeMin) {
         const double b = x0 >= 0.0 ? -xnorm : xnorm;
-        const double t = (b - x0) / b;
+        const bool lower = (threadIdx.x & 16) == 0;
+        const double q = (lower ? b - x0 : p2) / (lower ? b : x0 - b);
+        const double t = __shfl_sync(0xffffffffu, q, 0), inv = __shfl_sync(0xffffffffu, q, 16);
         if (fabs(t) > kSafeMin) {
             h.tau = t;
             h.beta = b;
-            h.inv = p2 / (x0 - b);
+            h.inv = inv;
         }
     }
     return h;
@@ -127,12 +140,12 @@ __global__ void __launch_bounds__(BT, 1) bidiag_kernel(const Args p) {
     __shared__ double s_x[kMaxRows];   // tau_p (A u) on this CTA's rows
     __shared__ double s_c[kMaxRows];   // the pivot column on this CTA's rows (0 above the pivot)
     __shared__ double s_mx[kMaxRows / RC];
-    __shared__ double s_sum[WARPS];
+    __shared__ double s_sum[WARPS], s_wy[WARPS];
     __shared__ int s_exp[WARPS];
     __shared__ double s_f[QL * QMAX];  // 2^(e_q - E) per CTA q
     __shared__ int s_E;
-    __shared__ double s_x0;
-    __shared__ Reflector s_h;
+    __shared__ double s_x0, s_wk;      // the row reflector's first entry before it, w there
+    __shared__ Reflector s_h, s_hr;    // the column reflector, the row reflector (inv: 1 / (x0 - beta))
     const int P = gridDim.x, cta = blockIdx.x;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int m = p.m, n = p.n, rows = p.rows, ld = p.ld;
@@ -151,25 +164,37 @@ __global__ void __launch_bounds__(BT, 1) bidiag_kernel(const Args p) {
     }
     __syncthreads();
 
-    // The pivot column kn after both reflectors of the step before it (s_v,
-    // s_x; w and u at column kn), 0 above the pivot, and its maximum per row
-    // block: each warp forms the row blocks whose s_x it has formed.
-    auto pivot_column = [&](int kn, int b0, double wk, double uk) {
+    // From the warps' sums (red, scaled by 2^-e of each warp's exponent; f lane i: 2^(e_i - E) of
+    // warp i; wy: w . r, 2^-E): x = tau_p (A - v w^T) u = tau_p (t + hinv (sum - v wy)), t the pivot
+    // column kn after the column reflector; then the column after both, 0 above the pivot, and its
+    // maximum per row block.  Four lanes per row, a warp per row block.
+    auto finish_rows = [&](int kn, int b0, double wk, double wy, double tau, double hinv, double f) {
+        double fw[WARPS / 4];
+#pragma unroll
+        for (int i = 0; i < WARPS / 4; ++i) fw[i] = __shfl_sync(0xffffffffu, f, (lane & 3) * (WARPS / 4) + i);
 #pragma unroll 1
         for (int b = b0 + warp; b < rows / RC; b += WARPS) {
-            double c = 0.0;
-            if (lane < RC) {
-                const int l = b * RC + lane, g = l * P + cta;
-                if (g >= kn && g < m) c = fma(-s_x[l], uk, fma(-s_v[l], wk, slab[(size_t)l * ld + kn]));
+            const int l = b * RC + (lane >> 2), g = l * P + cta;
+            const double v = s_v[l], t = fma(-v, wk, slab[(size_t)l * ld + kn]);
+            double s = 0.0;
+#pragma unroll
+            for (int i = 0; i < WARPS / 4; ++i) s = fma(red[((lane & 3) * (WARPS / 4) + i) * rows + l], fw[i], s);
+            s += shfl_xor(s, 1);
+            s += shfl_xor(s, 2);
+            const bool in = g >= kn && g < m;
+            const double x = in && tau != 0.0 ? tau * fma(hinv, fma(-v, wy, s), t) : 0.0;
+            const double c = in ? t - x : 0.0;
+            if ((lane & 3) == 0) {
+                s_x[l] = x;
                 s_c[l] = c;
             }
             double mx = fabs(c);
 #pragma unroll
-            for (int o = 4; o > 0; o >>= 1) mx = fmax(mx, shfl_xor(mx, o));
+            for (int o = 4; o < 32; o <<= 1) mx = fmax(mx, shfl_xor(mx, o));
             if (lane == 0) s_mx[b] = mx;
         }
     };
-    pivot_column(0, 0, 0.0, 0.0);
+    finish_rows(0, 0, 0.0, 0.0, 0.0, 0.0, 0.0);
     __syncthreads();
 
     double w[CB], u[CB];  // w and u of this thread's columns
@@ -183,16 +208,15 @@ __global__ void __launch_bounds__(BT, 1) bidiag_kernel(const Args p) {
         const Slot* prow = p.pivot + (size_t)(k & 1) * ld;
         Slot* pnext = p.pivot + (size_t)(kn & 1) * ld;
         Slot* cnext = p.cpair + (size_t)(kn & 1) * P;
-        double taur = 0.0, ir = 0.0;
-        // u_j for an entry r_j of the pivot row
-        auto u_of = [&](int j, double rj) { return taur != 0.0 ? (j == kn ? 1.0 : rj * ir) : 0.0; };
-        // not SMEM: w and u of a column block, from the slots this thread has waited for
-        auto reload = [&](int j0) {
+        double u0 = 0.0, ir = 0.0;  // u at column kn (1, or 0 without a row reflector), 1 / (x0 - beta)
+        // not SMEM: w of a column block and the scaled pivot row - w (u0 at column kn), from the
+        // slots this thread has waited for
+        auto reload = [&](int j0, double first, double scale) {
 #pragma unroll
             for (int i = 0; i < CB; ++i) {
                 const int j = j0 + tid + i * BT;
                 w[i] = j < n ? slot_value(p.w + j) : 0.0;
-                u[i] = j < n ? u_of(j, slot_value(prow + j) - w[i]) : 0.0;
+                u[i] = j >= n ? 0.0 : j == kn ? first : (slot_value(prow + j) - w[i]) * scale;
             }
         };
         if (k >= 0) {
@@ -200,18 +224,17 @@ __global__ void __launch_bounds__(BT, 1) bidiag_kernel(const Args p) {
             // pivot row - w, the norm of r over the CTA (every warp the same bits)
             double rmax = 0.0;
             if constexpr (SMEM) {
-                // (threads past the last column wait for it too, and drop what they get)
-                const Slot* at[CB];
-#pragma unroll
-                for (int i = 0; i < CB; ++i) at[i] = p.w + min(c0 + tid + i * BT, n - 1);
-                fail |= !slot_wait(at, kn, w, p.status);
+                fail |= !slot_wait_columns<BT>(p.w, c0, n, kn, w, p.status);
 #pragma unroll
                 for (int i = 0; i < CB; ++i) {
                     if (c0 + tid + i * BT >= n) w[i] = u[i] = 0.0;
                     u[i] -= w[i];  // r
                     rmax = fmax(rmax, fabs(u[i]));
                 }
-                if (tid == 0) s_x0 = u[0];
+                if (tid == 0) {
+                    s_x0 = u[0];
+                    s_wk = w[0];
+                }
             } else {
 #pragma unroll 1
                 for (int j = c0 + tid; j < n; j += BT) {
@@ -220,40 +243,10 @@ __global__ void __launch_bounds__(BT, 1) bidiag_kernel(const Args p) {
                     fail |= !slot_wait(at, kn, wj, p.status);
                     const double r = slot_value(prow + j) - wj[0];
                     rmax = fmax(rmax, fabs(r));
-                    if (j == c0) s_x0 = r;
-                }
-            }
-            int E = rmax > 0.0 ? exp_of(rmax) : kEmptyExp;
-            E = warp_max(E);
-            double S = 0.0;
-            if (E > kEmptyExp) {
-                const double sc = pow2(-E);
-                if constexpr (SMEM) {
-#pragma unroll
-                    for (int i = 0; i < CB; ++i) S = fma(u[i] * sc, u[i] * sc, S);
-                } else {
-                    for (int j = c0 + tid; j < n; j += BT) {
-                        const double y = (slot_value(prow + j) - slot_value(p.w + j)) * sc;
-                        S = fma(y, y, S);
+                    if (j == c0) {
+                        s_x0 = r;
+                        s_wk = wj[0];
                     }
-                }
-            }
-            S = warp_sum(S);
-            if (lane == 0) {
-                s_sum[warp] = S;
-                s_exp[warp] = E;
-            }
-            if (__syncthreads_or(fail)) return;
-            {
-                const int e = lane < WARPS ? s_exp[lane] : kEmptyExp;
-                E = warp_max(e);
-                S = warp_sum(lane < WARPS ? s_sum[lane] * down(2 * (e - E)) : 0.0);
-                const Reflector h = reflector(E, S, s_x0);
-                taur = h.tau;
-                ir = taur != 0.0 ? h.inv * pow2(-E) : 0.0;
-                if (cta == 0 && tid == 0) {
-                    p.taup[k] = h.tau;
-                    p.e[k] = h.beta;
                 }
             }
             const bool owner = gl == k;
@@ -263,71 +256,94 @@ __global__ void __launch_bounds__(BT, 1) bidiag_kernel(const Args p) {
                 gl += P;
             }
             const int b0 = l0 / RC;
+            // ---- pass 1, ahead of the norm: A r beyond column kn on this CTA's rows below k, r scaled
+            // by 2^-e of the warp's maximum; the sums of the norm and of w . r go with it
+            const int ew = warp_max(rmax > 0.0 ? exp_of(rmax) : kEmptyExp);
+            const double sc = ew > kEmptyExp ? pow2(-ew) : 0.0;
+            double S = 0.0, wy = 0.0, y[CB];
+            if constexpr (SMEM) {
+#pragma unroll
+                for (int i = 0; i < CB; ++i) {
+                    y[i] = ew > kEmptyExp ? u[i] * sc : 0.0;
+                    S = fma(y[i], y[i], S);
+                }
+                if (tid == 0) y[0] = 0.0;  // column kn: finish_rows adds it
+#pragma unroll
+                for (int i = 0; i < CB; ++i) wy = fma(w[i], y[i], wy);
+            } else if (ew > kEmptyExp) {
+                for (int j = c0 + tid; j < n; j += BT) {
+                    const double wj = slot_value(p.w + j), t = (slot_value(prow + j) - wj) * sc;
+                    S = fma(t, t, S);
+                    wy = fma(wj, j == kn ? 0.0 : t, wy);
+                }
+            }
+#pragma unroll 1
+            for (int b = b0; b < rows / RC; ++b) {
+                double acc[RC];
+#pragma unroll
+                for (int r = 0; r < RC; ++r) acc[r] = 0.0;
+                for (int j0 = c0; j0 < n; j0 += CB * BT) {
+                    if constexpr (!SMEM) reload(j0, 0.0, sc);
+#pragma unroll
+                    for (int i = 0; i < CB; ++i) {
+                        const int j = j0 + tid + i * BT;
+                        const double yi = SMEM ? y[i] : u[i];
+                        if (j < n) {
+                            const double* q = slab + (size_t)b * RC * ld + j;
+#pragma unroll
+                            for (int r = 0; r < RC; ++r) acc[r] = fma(q[(size_t)r * ld], yi, acc[r]);
+                        }
+                    }
+                    if constexpr (SMEM) break;
+                }
+                const double s = warp_sum8(acc);
+                if ((lane & 3) == 0) red[warp * rows + b * RC + (lane >> 2)] = s;
+            }
+            S = warp_sum(S);
+            wy = warp_sum(wy);
+            if (lane == 0) {
+                s_sum[warp] = S;
+                s_wy[warp] = wy;
+                s_exp[warp] = ew;
+            }
+            if (__syncthreads_or(fail)) return;
+            // ---- the row reflector of row k, x and the pivot column, by the warps that have row
+            // blocks (each the same bits)
+            if (warp == 0 || b0 + warp < rows / RC) {
+                const int e = lane < WARPS ? s_exp[lane] : kEmptyExp;
+                const int E = warp_max(e);
+                const double f = down(e - E);
+                S = warp_sum(lane < WARPS ? (s_sum[lane] * f) * f : 0.0);
+                wy = warp_sum(lane < WARPS ? s_wy[lane] * f : 0.0);
+                const Reflector h = reflector(E, S, s_x0);
+                finish_rows(kn, b0, s_wk, wy, h.tau, h.inv, f);
+                if (tid == 0) {
+                    s_hr.tau = h.tau;
+                    s_hr.inv = h.tau != 0.0 ? h.inv * pow2(-E) : 0.0;
+                    if (cta == 0) {
+                        p.taup[k] = h.tau;
+                        p.e[k] = h.beta;
+                    }
+                }
+            }
+            __syncthreads();
+            u0 = s_hr.tau != 0.0 ? 1.0 : 0.0;
+            ir = s_hr.inv;
+            // row k is finished: x0 beside the diagonal, the reflector's tail beyond it
             if constexpr (SMEM) {
 #pragma unroll
                 for (int i = 0; i < CB; ++i) {
                     const int j = c0 + tid + i * BT;
                     const double rj = u[i];
-                    u[i] = u_of(j, rj);
-                    // row k is finished: x0 beside the diagonal, the reflector's tail beyond it
-                    if (owner && j < n) krow[j] = taur != 0.0 && j > kn ? u[i] : rj;
+                    u[i] = j == kn ? u0 : u0 != 0.0 ? rj * ir : 0.0;
+                    if (owner && j < n) krow[j] = u0 != 0.0 && j > kn ? u[i] : rj;
                 }
             } else if (owner) {
                 for (int j = c0 + tid; j < n; j += BT) {
                     const double rj = slot_value(prow + j) - slot_value(p.w + j);
-                    krow[j] = taur != 0.0 && j > kn ? rj * ir : rj;
+                    krow[j] = u0 != 0.0 && j > kn ? rj * ir : rj;
                 }
             }
-            const double wk = slot_value(p.w + kn);
-            // ---- pass 1: x = tau_p (A - v w^T) u on this CTA's rows below k
-            if (taur != 0.0) {
-#pragma unroll 1
-    #pragma unroll 1
-            for (int b = b0; b < rows / RC; ++b) {
-                    double acc[RC], vr[RC];
-#pragma unroll
-                    for (int r = 0; r < RC; ++r) {
-                        acc[r] = 0.0;
-                        vr[r] = s_v[b * RC + r];
-                    }
-                    for (int j0 = c0; j0 < n; j0 += CB * BT) {
-                        if constexpr (!SMEM) reload(j0);
-#pragma unroll
-                        for (int i = 0; i < CB; ++i) {
-                            const int j = j0 + tid + i * BT;
-                            if (j < n) {
-                                const double* q = slab + (size_t)b * RC * ld + j;
-#pragma unroll
-                                for (int r = 0; r < RC; ++r) acc[r] = fma(fma(-vr[r], w[i], q[(size_t)r * ld]), u[i], acc[r]);
-                            }
-                        }
-                        if constexpr (SMEM) break;
-                    }
-                    const double s = warp_sum8(acc);
-                    if ((lane & 3) == 0) red[warp * rows + b * RC + (lane >> 2)] = s;
-                }
-                __syncthreads();
-                // the warps' sums, 4 lanes per row
-#pragma unroll 1
-        #pragma unroll 1
-        for (int b = b0 + warp; b < rows / RC; b += WARPS) {
-                    const int l = b * RC + (lane >> 2);
-                    double s = 0.0;
-#pragma unroll
-                    for (int i = 0; i < WARPS / 4; ++i) s += red[((lane & 3) * (WARPS / 4) + i) * rows + l];
-                    s += shfl_xor(s, 1);
-                    s += shfl_xor(s, 2);
-                    const int g = l * P + cta;
-                    if ((lane & 3) == 0) s_x[l] = g > k && g < m ? taur * s : 0.0;
-                }
-                __syncwarp();
-            } else {
-#pragma unroll 1
-                for (int l = tid; l < rows; l += BT) s_x[l] = 0.0;
-                __syncthreads();
-            }
-            pivot_column(kn, b0, wk, taur != 0.0 ? 1.0 : 0.0);
-            __syncthreads();
         }
         // ---- the pivot column scaled by 2^-e, e the exponent of this CTA's maximum
         const int b0 = l0 / RC;
@@ -356,7 +372,7 @@ __global__ void __launch_bounds__(BT, 1) bidiag_kernel(const Args p) {
 #pragma unroll
                 for (int i = 0; i < CB; ++i) w[i] = u[i] = 0.0;
             } else if constexpr (!SMEM) {
-                reload(j0);
+                reload(j0, u0, ir);
             }
 #pragma unroll 1
             for (int b = b0; b < rows / RC; ++b) {
@@ -450,20 +466,6 @@ __global__ void __launch_bounds__(BT, 1) bidiag_kernel(const Args p) {
                 fail |= !slot_wait(at, kn + 1, x, p.status);
             }
             if (trip == 0) {
-                // the pivot row at this thread's columns of the next step
-                if constexpr (SMEM) {
-                    const Slot* at[CB];
-#pragma unroll
-                    for (int i = 0; i < CB; ++i) at[i] = pnext + min(kn + 1 + tid + i * BT, n - 1);
-                    fail |= !slot_wait(at, kn + 1, u, p.status);
-                } else {
-#pragma unroll 1
-                    for (int c = kn + 1 + tid; c < n; c += BT) {
-                        const Slot* at[1] = {pnext + c};
-                        double y[1];
-                        fail |= !slot_wait(at, kn + 1, y, p.status);
-                    }
-                }
                 if (__syncthreads_or(fail)) return;
                 tau = s_h.tau;
                 vinv = s_h.inv;
@@ -492,6 +494,18 @@ __global__ void __launch_bounds__(BT, 1) bidiag_kernel(const Args p) {
             }
             s_v[l] = v;
         }
+        // the pivot row at this thread's columns of the next step, which has long arrived (waiting
+        // for it ahead of the dots, every thread polls and delays them: 7.0 us a step against 6.3)
+        if constexpr (SMEM) {
+            fail |= !slot_wait_columns<BT>(pnext, kn + 1, n, kn + 1, u, p.status);
+        } else {
+#pragma unroll 1
+            for (int c = kn + 1 + tid; c < n; c += BT) {
+                const Slot* at[1] = {pnext + c};
+                double y[1];
+                fail |= !slot_wait(at, kn + 1, y, p.status);
+            }
+        }
     }
     __syncthreads();
     for (int l = 0; l < rows; ++l) {
@@ -519,8 +533,8 @@ int bidiag_grid(int m, int n, int sm_count, int* rows) {
     using namespace bidiag;
     const int most = sm_count < kMaxCtas ? sm_count : kMaxCtas;
     int per = ((m + most - 1) / most + RC - 1) / RC * RC;
-    // past two columns per thread 16 rows per CTA (1168 x 1100: 9.3 ms, against 10.4 with 8: half as
-    // many partials cross), below it 8 (1152 x 1024: 7.2 against 7.6; 512^2: 3.1 against 3.2)
+    // past two columns per thread 16 rows per CTA (1168 x 1100: 6.7 ms, against 7.0 with 8: half as
+    // many partials cross), below it 8 (1152 x 1024: 5.4 against 6.0; 512^2: 2.45 against 2.7)
     if (n > 2 * BT && per < 2 * RC) per = 2 * RC;
     if (per > kMaxRows) return 0;
     *rows = per;
@@ -571,8 +585,10 @@ int launch_bidiag(double* a, long long lda, int m, int n, double* d, double* e, 
     const bool smem = slab_in_smem(rows, n, p.ld);
     p.slab = smem ? nullptr : work + 2 * slots;
     p.status = status;
+    // (1400^2: 9.0 ms with 3 columns per thread, 11.4 with 4; up to 512 columns 1 gains nothing on 2)
     const void* kern = !smem        ? (const void*)bidiag_kernel<false, 4>
-                       : n > 2 * BT ? (const void*)bidiag_kernel<true, 4>
+                       : n > 3 * BT ? (const void*)bidiag_kernel<true, 4>
+                       : n > 2 * BT ? (const void*)bidiag_kernel<true, 3>
                                     : (const void*)bidiag_kernel<true, 2>;
     const size_t bytes = smem_bytes(rows, p.ld, smem);
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) != cudaSuccess)

@@ -103,6 +103,7 @@ def test_rejects_bad_arguments(ctx):
 @pytest.mark.parametrize("m,n", [
     (1025, 1025),   # 16 rows per CTA, more than two columns per thread
     (1191, 520),    # 16 rows per CTA, the last CTA's slab partly past m
+    (1600, 1537),   # more than three columns per thread
     (513, 513), (9, 2), (8, 8),   # one column past a thread each; two CTAs; one CTA
     (6000, 700),    # the slab does not fit in shared memory
     (2300, 2100),   # nor here; several column blocks per thread
