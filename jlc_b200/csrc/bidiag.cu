@@ -136,10 +136,12 @@ __device__ __noinline__ Reflector reflector(int E, double S, double x0) {
 template <bool SMEM, int CB>
 __global__ void __launch_bounds__(BT, 1) bidiag_kernel(const Args p) {
     extern __shared__ double dyn[];
-    __shared__ double s_v[kMaxRows];   // the column reflector on this CTA's rows
-    __shared__ double s_x[kMaxRows];   // tau_p (A u) on this CTA's rows
-    __shared__ double s_c[kMaxRows];   // the pivot column on this CTA's rows (0 above the pivot)
-    __shared__ double s_mx[kMaxRows / RC];
+    // (aligned for vector loads: the passes read 8 rows of each)
+    __shared__ __align__(16) double s_v[kMaxRows];  // the column reflector on this CTA's rows
+    __shared__ __align__(16) double s_x[kMaxRows];  // tau_p (A u) on this CTA's rows
+    __shared__ __align__(16) double s_c[kMaxRows];  // the pivot column on this CTA's rows (0 above the pivot)
+    __shared__ __align__(16) double s_t[kMaxRows];  // its tail (0 at the pivot too)
+    __shared__ unsigned s_mx[kMaxRows / RC];        // high word of the column's maximum per row block
     __shared__ double s_sum[WARPS], s_wy[WARPS];
     __shared__ int s_exp[WARPS];
     __shared__ double s_f[QL * QMAX];  // 2^(e_q - E) per CTA q
@@ -164,37 +166,42 @@ __global__ void __launch_bounds__(BT, 1) bidiag_kernel(const Args p) {
     }
     __syncthreads();
 
-    // From the warps' sums (red, scaled by 2^-e of each warp's exponent; f lane i: 2^(e_i - E) of
-    // warp i; wy: w . r, 2^-E): x = tau_p (A - v w^T) u = tau_p (t + hinv (sum - v wy)), t the pivot
-    // column kn after the column reflector; then the column after both, 0 above the pivot, and its
-    // maximum per row block.  Four lanes per row, a warp per row block.
-    auto finish_rows = [&](int kn, int b0, double wk, double wy, double tau, double hinv, double f) {
-        double fw[WARPS / 4];
+    // The warps' sums of a row block (red, scaled by 2^-e of each warp's exponent; f lane i: 2^(e_i - E)
+    // of warp i): four lanes per row, all with its sum
+    auto row_sum = [&](int b, double f) {
+        const int l = b * RC + (lane >> 2);
+        double s = 0.0;
 #pragma unroll
-        for (int i = 0; i < WARPS / 4; ++i) fw[i] = __shfl_sync(0xffffffffu, f, (lane & 3) * (WARPS / 4) + i);
+        for (int i = 0; i < WARPS / 4; ++i) {
+            const int q = (lane & 3) * (WARPS / 4) + i;
+            s = fma(red[q * rows + l], __shfl_sync(0xffffffffu, f, q), s);
+        }
+        s += shfl_xor(s, 1);
+        s += shfl_xor(s, 2);
+        return s;
+    };
+    // x = tau_p (A - v w^T) u = tau_p (t + hinv (sum - v wy)), t the pivot column kn after the column
+    // reflector, wy = 2^-E w . r; then the column after both, 0 above the pivot, and its maximum per
+    // row block.  A warp per row block; s: the sums of the warp's first one.
+    auto finish_rows = [&](int kn, int b0, double s, double f, double wk, double wy, double tau, double hinv) {
 #pragma unroll 1
         for (int b = b0 + warp; b < rows / RC; b += WARPS) {
+            if (b >= b0 + WARPS) s = row_sum(b, f);
             const int l = b * RC + (lane >> 2), g = l * P + cta;
             const double v = s_v[l], t = fma(-v, wk, slab[(size_t)l * ld + kn]);
-            double s = 0.0;
-#pragma unroll
-            for (int i = 0; i < WARPS / 4; ++i) s = fma(red[((lane & 3) * (WARPS / 4) + i) * rows + l], fw[i], s);
-            s += shfl_xor(s, 1);
-            s += shfl_xor(s, 2);
             const bool in = g >= kn && g < m;
             const double x = in && tau != 0.0 ? tau * fma(hinv, fma(-v, wy, s), t) : 0.0;
             const double c = in ? t - x : 0.0;
             if ((lane & 3) == 0) {
                 s_x[l] = x;
                 s_c[l] = c;
+                s_t[l] = g > kn ? c : 0.0;
             }
-            double mx = fabs(c);
-#pragma unroll
-            for (int o = 4; o < 32; o <<= 1) mx = fmax(mx, shfl_xor(mx, o));
+            const unsigned mx = __reduce_max_sync(0xffffffffu, max((unsigned)__double2hiint(c) & 0x7fffffffu, c != 0.0 ? 1u : 0u));
             if (lane == 0) s_mx[b] = mx;
         }
     };
-    finish_rows(0, 0, 0.0, 0.0, 0.0, 0.0, 0.0);
+    finish_rows(0, 0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0);
     __syncthreads();
 
     double w[CB], u[CB];  // w and u of this thread's columns
@@ -315,8 +322,9 @@ __global__ void __launch_bounds__(BT, 1) bidiag_kernel(const Args p) {
                 const double f = down(e - E);
                 S = warp_sum(lane < WARPS ? (s_sum[lane] * f) * f : 0.0);
                 wy = warp_sum(lane < WARPS ? s_wy[lane] * f : 0.0);
+                const double s = row_sum(min(b0 + warp, rows / RC - 1), f);
                 const Reflector h = reflector(E, S, s_x0);
-                finish_rows(kn, b0, s_wk, wy, h.tau, h.inv, f);
+                finish_rows(kn, b0, s, f, s_wk, wy, h.tau, h.inv);
                 if (tid == 0) {
                     s_hr.tau = h.tau;
                     s_hr.inv = h.tau != 0.0 ? h.inv * pow2(-E) : 0.0;
@@ -347,10 +355,10 @@ __global__ void __launch_bounds__(BT, 1) bidiag_kernel(const Args p) {
         }
         // ---- the pivot column scaled by 2^-e, e the exponent of this CTA's maximum
         const int b0 = l0 / RC;
-        double mx = 0.0;
+        unsigned mx = 0;
 #pragma unroll 1
-        for (int b = b0; b < rows / RC; ++b) mx = fmax(mx, s_mx[b]);
-        const int ex = exp_of(mx);
+        for (int b = b0; b < rows / RC; ++b) mx = max(mx, s_mx[b]);
+        const int ex = mx >> 20 >= 0x7ff ? 0 : min(1022, max(-1000, (int)(mx >> 20) - 1023));
         const double sc = pow2(-ex);
         if (warp == WARPS - 1) {
             double q = 0.0;
@@ -360,7 +368,7 @@ __global__ void __launch_bounds__(BT, 1) bidiag_kernel(const Args p) {
                 q = fma(c, c, q);
             }
             q = warp_sum(q);
-            if (lane == 0) slot_put(cnext + cta, q, kn + 1, mx > 0.0 ? ex : kEmptyExp);
+            if (lane == 0) slot_put(cnext + cta, q, kn + 1, mx > 0 ? ex : kEmptyExp);
         }
         // ---- pass 2: A - v w^T - x u^T stored, and its dots with the pivot column
         const bool powner = gl == kn;
@@ -382,7 +390,7 @@ __global__ void __launch_bounds__(BT, 1) bidiag_kernel(const Args p) {
                     const int l = b * RC + r;
                     vr[r] = s_v[l];
                     xr[r] = s_x[l];
-                    cr[r] = l * P + cta > kn ? s_c[l] * sc : 0.0;
+                    cr[r] = s_t[l] * sc;
                 }
 #pragma unroll
                 for (int i = 0; i < CB; ++i) {
