@@ -736,9 +736,11 @@ int qr_apply_wy(jlc_ctx* ctx, long long m, long long k0, long long cols, double*
     const double* v = q.v + i * q.ldv * kQrPanel + k0;
     const double* vt = q.vt + i * q.ldv * kQrPanel + k0;
     GemmDesc w{JLC_ROW_MAJOR, JLC_COL_MAJOR, kQrPanel, cols, rows, 1.0, 0.0, v, q.ldv, c + k0, ldc, q.w, q.ldw};
+    w.chained = true;
     int rc = run_device(ctx, w, precision, 0, nullptr);
     if (rc) return rc;
     GemmDesc u{JLC_COL_MAJOR, JLC_ROW_MAJOR, cols, rows, kQrPanel, -1.0, 1.0, q.w, q.ldw, vt, q.ldv, c + k0, ldc};
+    u.chained = true;
     return run_device(ctx, u, precision, 0, nullptr);
 }
 

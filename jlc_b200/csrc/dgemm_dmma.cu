@@ -90,6 +90,7 @@ struct Params {
     int* counters;      // ksplit > 1: arrivals per tile, zero between launches
     int* status;
     const int* gate;  // when non-null the kernel runs only if an Ozaki call's flags ask for FP64
+    int chained;      // launch attribute only: GemmDesc::chained
     int withhold;     // test hook: CTA 0 leaves its first stage unloaded, so a bounded wait runs out
 };
 
@@ -114,7 +115,6 @@ __global__ void __launch_bounds__(THREADS, 1)
     using C = Cfg<TBM, TBN>;
     constexpr int BM = C::BM, BN = C::BN, WARPS_N = C::WARPS_N, WM = C::WM, WN = C::WN, MT = C::MT, NT = C::NT;
     constexpr int A_STAGE = C::A_STAGE, STAGE_BYTES = C::STAGE_BYTES, STAGES = C::STAGES;
-    if (p.gate != nullptr && (p.gate[kFlagNonfiniteA] | p.gate[kFlagFallback] | p.gate[kFlagNonfiniteB]) == 0) return;
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     char* smem = reinterpret_cast<char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     uint64_t* full = reinterpret_cast<uint64_t*>(smem + STAGES * STAGE_BYTES);
@@ -131,6 +131,9 @@ __global__ void __launch_bounds__(THREADS, 1)
         fence_barrier_init();
     }
     __syncthreads();
+    grid_dep_wait();
+    grid_dep_launch();
+    if (p.gate != nullptr && (p.gate[kFlagNonfiniteA] | p.gate[kFlagFallback] | p.gate[kFlagNonfiniteB]) == 0) return;
 
     if (warp < PRODUCER_WARPS) {
         // ---------------- producer ----------------
@@ -416,8 +419,20 @@ static int launch_variant(const CUtensorMap& ma, const CUtensorMap& mb, const Pa
     constexpr int smem = Cfg<TBM, TBN>::SMEM_BYTES;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return JLC_E_LAUNCH;
-    kern<<<grid, THREADS, smem, st>>>(ma, mb, p);
-    return cudaGetLastError() == cudaSuccess ? JLC_OK : JLC_E_LAUNCH;
+    if (!p.chained) {
+        kern<<<grid, THREADS, smem, st>>>(ma, mb, p);
+        return cudaGetLastError() == cudaSuccess ? JLC_OK : JLC_E_LAUNCH;
+    }
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute at[1];
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(THREADS);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    at[0] = chained_launch();
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kern, ma, mb, p) == cudaSuccess ? JLC_OK : JLC_E_LAUNCH;
 }
 
 }  // namespace dmma
@@ -633,6 +648,7 @@ int launch_dgemm_dmma(const GemmDesc& g, cudaStream_t st, int sm_count, int* sta
     p.k_blocks = kbl;
     p.status = status;
     p.gate = gate;
+    p.chained = g.chained ? 1 : 0;
     p.withhold = g.withhold_stage ? 1 : 0;
     p.ksplit = 1;
     p.part = nullptr;

@@ -42,6 +42,9 @@ struct GemmDesc {
     const double* dot_mat = nullptr;
     long long dot_ld = 0;
     double* dot_partials = nullptr;
+    // The FP64 kernel may start while the kernel ahead of it in the stream ends
+    // (it waits for that one's end before it reads or writes global memory).
+    bool chained = false;
     // test hook (jlc_inject_fault, JLC_FAULT_WAIT): the FP64 kernel leaves one
     // stage unloaded so that a bounded wait runs out
     bool withhold_stage = false;

@@ -746,6 +746,8 @@ __global__ void __launch_bounds__(RG_THREADS, 1) qr_panel_rg_kernel(double* A, l
         mbar_arrive_expect_tx(&bar[0], bytes(0));
         mbar_arrive_expect_tx(&bar[1], bytes(1));
     }
+    grid_dep_wait();
+    grid_dep_launch();
     double a[RG_COLS][NR], x[NR];
 #pragma unroll
     for (int j = 0; j < RG_COLS; ++j)
@@ -1084,6 +1086,8 @@ __global__ void __launch_bounds__(VT_THREADS) qr_vt_kernel(const double* A, long
                                                            int shift, const double* tau, double* V, long long ldv,
                                                            double* T) {
     extern __shared__ double dyn[];
+    grid_dep_wait();
+    grid_dep_launch();
     double* part = dyn;                                                           // 64 x 64
     double(*t)[BT_LD] = reinterpret_cast<double(*)[BT_LD]>(dyn + 64 * 64);
     double(*sv)[VT_LD] = reinterpret_cast<double(*)[VT_LD]>(dyn + 64 * 64 + 64 * BT_LD);  // [row][column]
@@ -1163,6 +1167,8 @@ constexpr int VP_SMEM = 2 * 64 * VT_LD * 8;
 __global__ void __launch_bounds__(VT_THREADS) qr_vt_product_kernel(const double* V, long long ldv, int m, int p0,
                                                                    const double* T, int trans, double* VT) {
     extern __shared__ double dyn[];
+    grid_dep_wait();
+    grid_dep_launch();
     double(*sv)[VT_LD] = reinterpret_cast<double(*)[VT_LD]>(dyn);                // [column][row]
     double(*st)[VT_LD] = reinterpret_cast<double(*)[VT_LD]>(dyn + 64 * VT_LD);   // T: [row][column]
     const int pi = blockIdx.y, k0 = (p0 + pi) * 64, r0 = k0 + 64 * blockIdx.x;
@@ -1276,7 +1282,7 @@ int launch_qr_panel(double* a, long long lda, int m, int k0, int kb, double* tau
         if (cudaFuncSetAttribute((const void*)kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess)
             return JLC_E_LAUNCH;
         cudaLaunchConfig_t cfg = {};
-        cudaLaunchAttribute at[1];
+        cudaLaunchAttribute at[2];
         cfg.gridDim = dim3(cl);
         cfg.blockDim = dim3(qr::RG_THREADS);
         cfg.stream = st;
@@ -1284,8 +1290,9 @@ int launch_qr_panel(double* a, long long lda, int m, int k0, int kb, double* tau
         at[0].val.clusterDim.x = cl;
         at[0].val.clusterDim.y = 1;
         at[0].val.clusterDim.z = 1;
+        at[1] = chained_launch();
         cfg.attrs = at;
-        cfg.numAttrs = 1;
+        cfg.numAttrs = 2;
         return cudaLaunchKernelEx(&cfg, kern, a, lda, m, k0, kb, tau, status) == cudaSuccess ? JLC_OK : JLC_E_LAUNCH;
     }
     if ((size_t)((m - k0 + cl - 1) / cl) * kb * sizeof(double) <= (size_t)qr::CL_MAX_SLAB_BYTES) {
@@ -1355,7 +1362,7 @@ int launch_qr_vt(const double* a, long long lda, int m, int kmax, int p0, int pa
     const int rows = m - 64 * p0;  // of the tallest panel
     if (rows <= VT_MAX_ROWS) {
         cudaLaunchConfig_t cfg = {};
-        cudaLaunchAttribute at[1];
+        cudaLaunchAttribute at[2];
         const int cl = max(1, min((rows + 63) / 64, min(cluster_max, RG_MAX)));
         cfg.gridDim = dim3(cl * panels);
         cfg.blockDim = dim3(VT_THREADS);
@@ -1365,8 +1372,9 @@ int launch_qr_vt(const double* a, long long lda, int m, int kmax, int p0, int pa
         at[0].val.clusterDim.x = cl;
         at[0].val.clusterDim.y = 1;
         at[0].val.clusterDim.z = 1;
+        at[1] = chained_launch();
         cfg.attrs = at;
-        cfg.numAttrs = 1;
+        cfg.numAttrs = 2;
         const void* kern = (const void*)qr_vt_kernel;
         if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, VT_SMEM) != cudaSuccess ||
             cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
@@ -1393,9 +1401,19 @@ int launch_qr_vt(const double* a, long long lda, int m, int kmax, int p0, int pa
     if (cudaFuncSetAttribute((const void*)qr_vt_product_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, VP_SMEM) !=
         cudaSuccess)
         return JLC_E_LAUNCH;
-    qr_vt_product_kernel<<<dim3((unsigned)((rows + 63) / 64), (unsigned)panels), VT_THREADS, VP_SMEM, st>>>(
-        v, ldv, m, p0, t, trans ? 1 : 0, vt);
-    return cudaGetLastError() == cudaSuccess ? JLC_OK : JLC_E_LAUNCH;
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute at[1];
+    cfg.gridDim = dim3((unsigned)((rows + 63) / 64), (unsigned)panels);
+    cfg.blockDim = dim3(VT_THREADS);
+    cfg.dynamicSmemBytes = VP_SMEM;
+    cfg.stream = st;
+    at[0] = chained_launch();
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, qr_vt_product_kernel, (const double*)v, ldv, m, p0, (const double*)t, trans ? 1 : 0,
+                              vt) == cudaSuccess
+               ? JLC_OK
+               : JLC_E_LAUNCH;
 }
 
 }  // namespace jlc
