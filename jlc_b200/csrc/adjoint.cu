@@ -24,22 +24,50 @@ namespace {
 
 constexpr int RED_THREADS = 256;
 
-// partials[blockIdx.x] = sum over this block's rows of x(i,j) * y(i,j)
+// partials[blockIdx.x] = sum over this block's rows of x(i,j) * y(i,j); with
+// COPY also dst(i,j) = s * x(i,j), dst either apart from x and y or the same
+// matrix as one of them (a thread reads an element before it writes it).  Bound
+// by HBM, with two CTAs per SM by the loads in flight: eight of each operand.
+// 4096 x 4096, dot and copy: 62 us (402 MB, 6.5 TB/s) against 71 and 50 as two
+// kernels with one load in flight.
+template <bool COPY>
 __global__ void __launch_bounds__(RED_THREADS) dot2d_kernel(const double* x, long long ldx, const double* y,
                                                              long long ldy, long long rows, long long cols,
-                                                             double* partials) {
+                                                             double* partials, double* dst, long long ldd, double s) {
     __shared__ double red[RED_THREADS / 32];
+    constexpr int DEPTH = 8;
     double acc = 0.0;
-    for (long long i = blockIdx.x; i < rows; i += gridDim.x)
-        for (long long j = threadIdx.x; j < cols; j += RED_THREADS) acc = fma(x[i * ldx + j], y[i * ldy + j], acc);
+    for (long long i = blockIdx.x; i < rows; i += gridDim.x) {
+        const double *xi = x + i * ldx, *yi = y + i * ldy;
+        double* di = COPY ? dst + i * ldd : nullptr;
+        long long j = threadIdx.x;
+        for (; j + (DEPTH - 1) * RED_THREADS < cols; j += DEPTH * RED_THREADS) {
+            double a[DEPTH], b[DEPTH];
+#pragma unroll
+            for (int q = 0; q < DEPTH; ++q) {
+                a[q] = xi[j + q * RED_THREADS];
+                b[q] = yi[j + q * RED_THREADS];
+            }
+#pragma unroll
+            for (int q = 0; q < DEPTH; ++q) {
+                acc = fma(a[q], b[q], acc);
+                if (COPY) di[j + q * RED_THREADS] = s * a[q];
+            }
+        }
+        for (; j < cols; j += RED_THREADS) {
+            const double a = xi[j];
+            acc = fma(a, yi[j], acc);
+            if (COPY) di[j] = s * a;
+        }
+    }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
     if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = acc;
     __syncthreads();
     if (threadIdx.x == 0) {
-        double s = 0.0;
-        for (int w = 0; w < RED_THREADS / 32; ++w) s += red[w];
-        partials[blockIdx.x] = s;
+        double sum = 0.0;
+        for (int w = 0; w < RED_THREADS / 32; ++w) sum += red[w];
+        partials[blockIdx.x] = sum;
     }
 }
 
@@ -70,29 +98,35 @@ __global__ void scale_copy_kernel(double* dst, long long ldd, const double* src,
 
 }  // namespace
 
+// out = <x, y>, and dst = s * x when dst is given.  In one pass over the
+// operands unless dst lies across one of them.
 int launch_dot2d(const double* x, long long ldx, const double* y, long long ldy, long long rows, long long cols,
-                 double* partials, int nparts, double* out, cudaStream_t st) {
+                 double* partials, int nparts, double* out, double* dst, long long ldd, double s, cudaStream_t st) {
     if (rows <= 0 || cols <= 0) {
         return cudaMemsetAsync(out, 0, sizeof(double), st) == cudaSuccess ? JLC_OK : JLC_E_CUDA;
     }
     const int grid = (int)(rows < nparts ? rows : nparts);
-    dot2d_kernel<<<grid, RED_THREADS, 0, st>>>(x, ldx, y, ldy, rows, cols, partials);
+    auto apart_or_same = [&](const double* o, long long ldo) {
+        const double *oe = o + (rows - 1) * ldo + cols, *de = dst + (rows - 1) * ldd + cols;
+        return (o == dst && ldo == ldd) || oe <= dst || de <= o;
+    };
+    const bool fused = dst && apart_or_same(x, ldx) && apart_or_same(y, ldy);
+    if (fused)
+        dot2d_kernel<true><<<grid, RED_THREADS, 0, st>>>(x, ldx, y, ldy, rows, cols, partials, dst, ldd, s);
+    else
+        dot2d_kernel<false><<<grid, RED_THREADS, 0, st>>>(x, ldx, y, ldy, rows, cols, partials, nullptr, 0, 0.0);
     sum_kernel<<<1, RED_THREADS, 0, st>>>(partials, grid, out);
+    if (dst && !fused) {
+        long long blocks = (rows * cols + 255) / 256;
+        if (blocks > 148LL * 32) blocks = 148LL * 32;
+        scale_copy_kernel<<<(unsigned)blocks, 256, 0, st>>>(dst, ldd, x, ldx, rows, cols, s);
+    }
     return cudaGetLastError() == cudaSuccess ? JLC_OK : JLC_E_LAUNCH;
 }
 
 int launch_sum(const double* partials, int n, double* out, cudaStream_t st) {
     if (n <= 0) return cudaMemsetAsync(out, 0, sizeof(double), st) == cudaSuccess ? JLC_OK : JLC_E_CUDA;
     sum_kernel<<<1, RED_THREADS, 0, st>>>(partials, n, out);
-    return cudaGetLastError() == cudaSuccess ? JLC_OK : JLC_E_LAUNCH;
-}
-
-int launch_scale_copy(double* dst, long long ldd, const double* src, long long lds, long long rows, long long cols,
-                      double s, cudaStream_t st) {
-    if (rows <= 0 || cols <= 0) return JLC_OK;
-    long long blocks = (rows * cols + 255) / 256;
-    if (blocks > 148LL * 32) blocks = 148LL * 32;
-    scale_copy_kernel<<<(unsigned)blocks, 256, 0, st>>>(dst, ldd, src, lds, rows, cols, s);
     return cudaGetLastError() == cudaSuccess ? JLC_OK : JLC_E_LAUNCH;
 }
 

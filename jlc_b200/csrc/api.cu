@@ -1474,8 +1474,9 @@ int jlc_dgemm_adjoint_device(jlc_ctx* ctx, int64_t m, int64_t n, int64_t k, doub
         } else {
             rc = run_device(ctx, g, precision, 0, &sub);
             Phase ph(ctx, JLC_PHASE_REDUCE);
-            if (!rc) rc = launch_dot2d(a, lda, da, ldda, m, k, parts_a, 2 * np, dalpha, st);
-            if (!rc && alpha != 1.0) rc = launch_scale_copy(da, ldda, da, ldda, m, k, alpha, st);
+            if (!rc)
+                rc = launch_dot2d(da, ldda, a, lda, m, k, parts_a, 2 * np, dalpha, alpha != 1.0 ? da : nullptr, ldda,
+                                  alpha, st);
         }
         if (rc) return rc;
     } else {
@@ -1496,11 +1497,10 @@ int jlc_dgemm_adjoint_device(jlc_ctx* ctx, int64_t m, int64_t n, int64_t k, doub
     // 3) dbeta = <dC, C_in>;  4) dC_in = beta * dC
     {
         Phase ph(ctx, JLC_PHASE_REDUCE);
-        rc = launch_dot2d(dc, lddc, c_in, ldc_in, m, n, parts_b, 2 * np, dbeta, st);
-        if (!rc && dc_in) rc = launch_scale_copy(dc_in, lddc_in, dc, lddc, m, n, beta, st);
+        rc = launch_dot2d(dc, lddc, c_in, ldc_in, m, n, parts_b, 2 * np, dbeta, dc_in, lddc_in, beta, st);
     }
     if (rc) return set_err(ctx, rc, "adjoint reduction launch failed");
-    ctx->launches += 3;
+    ctx->launches += 2;
     return JLC_OK;
 }
 

@@ -227,10 +227,8 @@ int check_fp64_bound(const GemmDesc& g, const double* c_in, long long ldc_in, co
 // adjoint helpers (adjoint.cu): out[0] = <x, y> over a rows x cols window
 // (nparts block partials, fixed order); out[0] = sum of n partials; dst = s * src
 int launch_dot2d(const double* x, long long ldx, const double* y, long long ldy, long long rows, long long cols,
-                 double* partials, int nparts, double* out, cudaStream_t st);
+                 double* partials, int nparts, double* out, double* dst, long long ldd, double s, cudaStream_t st);
 int launch_sum(const double* partials, int n, double* out, cudaStream_t st);
-int launch_scale_copy(double* dst, long long ldd, const double* src, long long lds, long long rows, long long cols,
-                      double s, cudaStream_t st);
 
 // throughput probes (peaks.cu): out4 = {DMMA FP64, DFMA FP64, INT8 tcgen05, BF16 tcgen05} in T(FL)OP/s
 int measure_peaks(int sm_count, cudaStream_t st, int* status, double* out4, char* err, size_t errlen);

@@ -136,3 +136,30 @@ def test_adjoint_config_size(ctx, oracle, precision):
     ref_b = math.fsum((dC * Cin).ravel())
     assert abs(db - ref_b) <= 2 * (m * n) * U * float(np.sum(np.abs(dC) * np.abs(Cin)))
     np.testing.assert_array_equal(gC, dC)
+
+
+@pytest.mark.parametrize("place", ["apart", "over dC", "over C_in", "across C_in"])
+@pytest.mark.parametrize("n", [2048, 2300, 40])
+def test_adjoint_dc_in_placement(ctx, oracle, place, n):
+    """d(beta) and dC_in where dC_in is a matrix of its own, dC or C_in
+    themselves, or lies across C_in's rows (n: whole groups of eight columns a
+    thread, a remainder, fewer columns than threads).  dC_in = beta dC is one
+    rounding per entry, d(beta) a sum of m n products."""
+    import torch
+    m, k, beta = 37, 8, -1.25
+    A, B = oracle.normal((m, k), 31), oracle.normal((k, n), 32)
+    C, D = oracle.normal((m, n), 33), oracle.normal((m, n), 34)
+    t = lambda x: torch.from_numpy(x).cuda()
+    a, b, d, ga, gb = t(A), t(B), t(D), torch.empty(m, k).double().cuda(), torch.empty(k, n).double().cuda()
+    buf = torch.zeros(2 * m, n, dtype=torch.float64, device="cuda")   # C_in in its first rows
+    buf[:m] = t(C)
+    out = {"apart": buf[m:], "over dC": d, "over C_in": buf[:m], "across C_in": buf[m // 2:m // 2 + m]}[place]
+    s = torch.zeros(2, dtype=torch.float64, device="cuda")
+    torch.cuda.synchronize()
+    ctx.adjoint_device(m, n, k, 1.0, beta, a.data_ptr(), k, b.data_ptr(), n, buf.data_ptr(), n, d.data_ptr(), n,
+                       ga.data_ptr(), k, gb.data_ptr(), n, s.data_ptr(), s.data_ptr() + 8, out.data_ptr(), n,
+                       precision=0)
+    ctx.synchronize()
+    np.testing.assert_array_equal(out.cpu().numpy(), beta * D)
+    ref = math.fsum((D * C).ravel())
+    assert abs(float(s[1]) - ref) <= 2 * (m * n) * U * float(np.sum(np.abs(D) * np.abs(C)))
