@@ -712,7 +712,7 @@ def run_qr(args):
     device time of jlc_qr_factor_device per factorisation (the matrix is
     restored, untimed, before each), FLOPs 2mn^2 - 2n^3/3, and the share of the
     time in the panel kernels and the device time of every phase (phase
-    records: qr_panel, qr_vt, and dmma for the Gram and trailing-update GEMMs)."""
+    records: qr_panel, qr_vt, and dmma for the trailing-update GEMMs)."""
     import statistics
     import torch
     import jlc_b200
@@ -761,8 +761,8 @@ def run_qr(args):
                          "unit": "TFLOP/s", "frac": round(tflops / peaks["fp64_dmma_tflops"], 4), "traffic": None,
                          "peak_source": "FP64 DMMA probe (jlc_measure_peaks) in this run; MEASURED_PEAKS.json has "
                                         "no FP64 figure",
-                         "note": "the panel kernels, the largest share, are latency-bound (one barrier per "
-                                 "column), not tensor-bound"},
+                         "note": "the panel kernels, the largest share, are latency-bound (one cluster "
+                                 "exchange per column), not tensor-bound"},
             "cpu_baseline": cpu}
     print(json.dumps(line), flush=True)
     ctx.close()
@@ -827,8 +827,8 @@ def run_hessenberg(args):
             "value": round(flops / (ms * 1e-3) / 1e9, 1), "unit": "GFLOP/s", "n_gpus": 1, "steps": args.steps,
             "warmup": args.warmup, "ms_per_step": round(ms, 3), "higher_is_better": True, "dtype": "f64",
             "data": "synthetic uniform[-1,1) (torch Philox, seed 20260604), device resident",
-            "config": {"workload": f"Hessenberg {n}x{n} with Q, panels of 32, one GEMV per reflector, block "
-                                   "updates on the DMMA route"},
+            "config": {"workload": f"Hessenberg {n}x{n} with Q: one launch while the rows fit shared memory, "
+                                   "else panels of 32 with block updates on the DMMA route"},
             "phase_ms": {name: round(statistics.median(p.get(name, 0.0) for p in phases), 3)
                          for name in sorted({nm for p in phases for nm in p})},
             "cpu_baseline": cpu}

@@ -224,8 +224,8 @@ JLC_API int jlc_inject_fault(jlc_ctx* ctx, int kind, int after);
 #define JLC_PHASE_D2H 9         /* device -> host copy of C */
 #define JLC_PHASE_REDUCE 11     /* adjoint reductions: d(alpha) / d(beta) dots and sums, scaled copies */
 #define JLC_PHASE_QR_PANEL 12   /* blocked QR: one panel's factorisation kernel */
-#define JLC_PHASE_QR_VT 13      /* blocked QR: V packing and the T factor (the Gram GEMM is a dmma phase) */
-#define JLC_PHASE_HESS_PANEL 17     /* Hessenberg: one panel's reflectors (column, GEMV, Y updates) */
+#define JLC_PHASE_QR_VT 13      /* blocked QR: V, the T factor and V op(T) */
+#define JLC_PHASE_HESS_PANEL 17     /* Hessenberg: the one-launch reduction, or one panel's reflectors */
 #define JLC_PHASE_BIDIAG 18         /* bidiagonalisation: the reflectors' cooperative launch */
 #define JLC_PHASE_OZAKI_CERT 14     /* Ozaki accuracy certificate (magnitude product, route decision) */
 #define JLC_PHASE_OZAKI_SPLIT_HI 15 /* split at the higher count (runs only when the certificate picks it) */
@@ -377,12 +377,14 @@ JLC_API int jlc_bidiag_device(jlc_ctx* ctx, int64_t m, int64_t n, double* a, int
 /* Reduces the column-major n x n matrix A (lda >= n) on the device, in place,
  * to upper Hessenberg form H with A = Q H Q^T, as
  * BlockedHessenbergQR.decompose does (eigen/qr/BlockedHessenbergQR.java:99-146):
- * panels of 32 columns, the reference's reflectors (its 1e-12 skips
- * included), each panel's block reflector applied with W = V^T H, W = T^T W,
+ * the reference's reflectors (its 1e-12 skips included), entries below the
+ * first subdiagonal cleared.  Matrices whose rows fit the chip's shared memory
+ * (n up to 1744 on 148 SMs) are reduced in one launch; above, panels of 32
+ * columns, each one's block reflector applied with W = V^T H, W = T^T W,
  * H -= V W from the left and W = H V, W = W T, H -= W V^T from the right
- * (:277-345) on the GEMM route, entries below the first subdiagonal cleared.
- * q (column-major, ldq >= n), when not NULL, receives Q.  precision applies
- * to the block-update GEMMs.  New: the reference runs this on the CPU only. */
+ * (:277-345) on the GEMM route.  q (column-major, ldq >= n), when not NULL,
+ * receives Q, formed on the GEMM route.  precision applies to those GEMMs.
+ * New: the reference runs this on the CPU only. */
 JLC_API int jlc_hessenberg_device(jlc_ctx* ctx, int64_t n, double* a, int64_t lda, double* q, int64_t ldq,
                                   int precision, jlc_report* rep);
 

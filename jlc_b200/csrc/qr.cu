@@ -3,7 +3,7 @@
 // matrix (HouseholderQR.java:133-210, 215-343): panels of 64 columns are
 // factored column by column (max-normalised Householder vectors, each applied
 // to the panel's later columns), then the trailing columns are updated with
-// the compact-WY form Q^T C = C - V T^T V^T C as three GEMMs (api.cu).
+// the compact-WY form Q^T C = C - (V T^T) (V^T C) as two GEMMs (api.cu).
 //
 //   qr_panel_rg_kernel: the panel on one thread-block cluster (1..16 CTAs),
 //                      the rows held in registers; panels of up to 4096 rows;
