@@ -1150,9 +1150,9 @@ int jlc_qr_factor_device(jlc_ctx* ctx, int64_t m, int64_t n, double* a, int64_t 
     for (long long k0 = 0; k0 < kmax; k0 += kQrPanel) {
         const int kb = (int)(kmax - k0 < kQrPanel ? kmax - k0 : kQrPanel);
         {
-            // rows split over CTAs of >= 128 rows each: one cluster while
-            // the slabs fit its shared memory, else up to one CTA per SM in
-            // one cooperative launch
+            // one cluster of CTAs of >= 64 rows each while the rows fit its
+            // registers or shared memory, else up to one CTA per SM, of >= 128
+            // rows each, in one cooperative launch
             Phase ph(ctx, JLC_PHASE_QR_PANEL);
             ctx->launches += 1;
             long long ctas = (m - k0) / 128;

@@ -656,7 +656,7 @@ __global__ void __launch_bounds__(CL_THREADS, 1) qr_panel_cl_kernel(double* A, l
 // next pivot column (800), the dots (300); no pass touches shared memory but
 // for the pivot column.  The shared-memory cluster kernel walks its slab three
 // times per column between five CTA barriers and a cluster barrier, in 53 KB of
-// code.  us per column on B200: 2304 rows 5.7 -> 2.5, 1024 rows 5.1 -> 2.1.
+// code.  us per column on B200: 2304 rows 5.7 -> 2.3, 1024 rows 5.1 -> 1.9.
 constexpr int RG_THREADS = 512, RG_WARPS = RG_THREADS / 32;
 constexpr int RG_MAX = 16;              // CTAs of the cluster
 constexpr int RG_COLS = 64 / RG_WARPS;  // columns per warp
