@@ -647,8 +647,9 @@ __global__ void __launch_bounds__(CL_THREADS, 1) qr_panel_cl_kernel(double* A, l
 //     number of bytes per column; every warp waits for it, merges the CTAs'
 //     values for its own columns and forms the reflector (the same bits in
 //     every warp and CTA), and updates its registers.
-// Two buffers alternate by column parity: a CTA sends column k + 2 only after
-// it has every CTA's column k + 1, which each sends after merging column k.
+// What is received alternates between two buffers by column parity: a CTA sends
+// column k + 2 only after it has every CTA's column k + 1, which each sends
+// after merging column k.
 //
 // A column is a chain of latencies: the exchange (about 900 cycles from the
 // first send to the last arrival at 16 CTAs), the merge and the reflector
@@ -727,8 +728,8 @@ __global__ void __launch_bounds__(RG_THREADS, 1) qr_panel_rg_kernel(double* A, l
                                                                     double* tau, int* status) {
     __shared__ __align__(16) double part[2][RG_MAX][RG_PART];
     __shared__ __align__(16) double rrec[2][64];  // row k, by the dots' index
-    __shared__ double s_x[NR * 32];               // the pivot column below the pivot, times 2^-e
-    __shared__ int s_e;
+    __shared__ double s_x[2][NR * 32];            // the pivot column below the pivot, times 2^-e, by column parity
+    __shared__ int s_e[2];                        // its e
     __shared__ __align__(16) double s_row[64];
     __shared__ __align__(8) uint64_t bar[2];
     cg::cluster_group cluster = cg::this_cluster();
@@ -763,8 +764,11 @@ __global__ void __launch_bounds__(RG_THREADS, 1) qr_panel_rg_kernel(double* A, l
     const uint32_t to_part = cluster_addr(&part[0][cta][warp * 4 + 2 * half], dest < P ? dest : 0);
     const uint32_t to_rrec = cluster_addr(&rrec[0][warp * 4 + 2 * half], dest < P ? dest : 0);
     const uint32_t to_bar = cluster_addr(&bar[0], dest < P ? dest : 0);
-    // Column c of this warp (y), below the pivot and scaled by 2^-e, into shared memory
-    auto put_pivot = [&](double (&y)[NR], int k) {
+    // A column of this warp (y), below its pivot row k and scaled by 2^-e, into the buffer of its
+    // parity.  Two buffers, because nothing else keeps a warp from writing column k + 1 while another
+    // still reads column k: a warp past its last column sends nothing, so no one waits for it until
+    // the next step's CTA barrier, after which column k's buffer is written again.
+    auto put_pivot = [&](double (&y)[NR], int k, int par) {
         unsigned hi = 0;
 #pragma unroll
         for (int r = 0; r < NR; ++r) {
@@ -775,14 +779,14 @@ __global__ void __launch_bounds__(RG_THREADS, 1) qr_panel_rg_kernel(double* A, l
         const int e = hi == 0x7ff ? 0 : min(1000, max(-1000, (int)hi - 1023));
         const double sc = sp_pow2(-e);
 #pragma unroll
-        for (int r = 0; r < NR; ++r) s_x[lane + 32 * r] = r0 + lane + 32 * r > k ? y[r] * sc : 0.0;
-        if (lane == 0) s_e = hi == 0 ? kRgEmpty : e;  // (zeros and denormals: no reflector)
+        for (int r = 0; r < NR; ++r) s_x[par][lane + 32 * r] = r0 + lane + 32 * r > k ? y[r] * sc : 0.0;
+        if (lane == 0) s_e[par] = hi == 0 ? kRgEmpty : e;  // (zeros and denormals: no reflector)
     };
     if (warp == 0) {
         double y[NR];
 #pragma unroll
         for (int r = 0; r < NR; ++r) y[r] = a[0][r];
-        put_pivot(y, k0);
+        put_pivot(y, k0, 0);
     }
 #pragma unroll 1
     for (int kk = 0; kk < kb; ++kk) {
@@ -802,13 +806,13 @@ __global__ void __launch_bounds__(RG_THREADS, 1) qr_panel_rg_kernel(double* A, l
         }
         if (__syncthreads_or(fail)) break;  // the pivot column is in shared memory
         // ---- this CTA's dots with it
-        const int e_own = s_e;
+        const int e_own = s_e[par];
         double d[RG_COLS];
 #pragma unroll
         for (int j = 0; j < RG_COLS; ++j) d[j] = 0.0;
 #pragma unroll
         for (int r = 0; r < NR; ++r) {
-            x[r] = s_x[lane + 32 * r];
+            x[r] = s_x[par][lane + 32 * r];
 #pragma unroll
             for (int j = 0; j < RG_COLS; ++j) d[j] = fma(x[r], a[j][r], d[j]);
         }
@@ -876,7 +880,7 @@ __global__ void __launch_bounds__(RG_THREADS, 1) qr_panel_rg_kernel(double* A, l
 #pragma unroll
             for (int r = 0; r < NR; ++r)
                 y[r] = fma(-f, x[r], jn == 0 ? a[0][r] : jn == 1 ? a[1][r] : jn == 2 ? a[2][r] : a[3][r]);
-            put_pivot(y, k + 1);
+            put_pivot(y, k + 1, par ^ 1);
         }
 #pragma unroll
         for (int j = 0; j < RG_COLS; ++j) {

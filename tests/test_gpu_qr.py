@@ -234,3 +234,31 @@ def test_q_in_batches(ctx, m, n, qcols):
     r = torch.triu(f.T[:min(m, n)])
     rows = min(qcols, min(m, n))
     assert float((q[:rows] @ a.T - r[:rows]).norm() / a.norm()) < tol
+
+
+@pytest.mark.parametrize("m", [64, 100, 127, 200])
+def test_last_columns_of_a_panel(ctx, oracle, m):
+    """The last columns of a 64-column panel, where some warps have no column
+    left, on one CTA and on a small cluster: the same bits on 200 runs, with
+    columns whose scales differ by 2^1800, and every column as the restatement
+    of the unscaled matrix has it."""
+    import torch
+    n = 64
+    a = oracle.uniform((m, n), 90 + m)
+    s = np.array([2.0 ** (900 if j % 2 else -900) for j in range(n)])
+    at = torch.from_numpy(np.ascontiguousarray((a * s).T)).cuda()
+    work, first = torch.empty_like(at), None
+    tau = torch.zeros(n, dtype=torch.float64, device="cuda")
+    for _ in range(200):
+        work.copy_(at)
+        torch.cuda.synchronize()
+        ctx.qr_factor_device(m, n, work.data_ptr(), m, tau.data_ptr())
+        if first is None:
+            first = work.clone()
+        assert torch.equal(work, first)
+    f = first.cpu().numpy().T
+    f_ref, tau_ref = oracle.householder_qr_blocked(a)
+    np.testing.assert_allclose(tau.cpu().numpy(), tau_ref, rtol=0, atol=1e-12)
+    up = np.triu(np.ones((m, n), bool))
+    f = np.where(up, f / s, f)
+    np.testing.assert_allclose(f, f_ref, rtol=0, atol=1e-11 * max(1.0, np.abs(f_ref).max()))
