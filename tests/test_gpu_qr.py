@@ -262,3 +262,27 @@ def test_last_columns_of_a_panel(ctx, oracle, m):
     up = np.triu(np.ones((m, n), bool))
     f = np.where(up, f / s, f)
     np.testing.assert_allclose(f, f_ref, rtol=0, atol=1e-11 * max(1.0, np.abs(f_ref).max()))
+
+
+@pytest.mark.parametrize("m,n,i,j", [(60, 40, 5, 0), (60, 40, 5, 7), (60, 40, 7, 7), (300, 60, 200, 30), (300, 60, 0, 0)])
+@pytest.mark.parametrize("bad", [np.nan, np.inf, -np.inf])
+def test_non_finite_column_of_a_panel(ctx, oracle, m, n, i, j, bad):
+    """A NaN or an infinity in column j of a one-panel matrix.  The columns
+    before j are finished before it is reached: their reflectors and R's rows
+    above j keep the bits they have with the column zeroed.  A NaN norm gives
+    no reflector when the column's entry on the diagonal is a NaN too, and the
+    columns after j are then those of the matrix without it."""
+    a = oracle.uniform((m, n), 300 + m + j)
+    a[0] = np.abs(a[0])      # a NaN below a positive diagonal entry leaves the column without a reflector
+    zeroed, poisoned = a.copy(), a.copy()
+    zeroed[:, j], poisoned[i, j] = 0.0, bad
+    f, tau = (x.cpu().numpy() for x in _factor(ctx, poisoned))
+    f0, tau0 = (x.cpu().numpy() for x in _factor(ctx, zeroed))
+    f, f0 = f.T, f0.T
+    assert np.isfinite(f0).all()
+    np.testing.assert_array_equal(f[:, :j], f0[:, :j])          # finished columns
+    np.testing.assert_array_equal(tau[:j], tau0[:j])
+    np.testing.assert_array_equal(f[:j, j + 1:], f0[:j, j + 1:])  # finished rows
+    if np.isnan(bad) and (i, j) != (0, 0):
+        assert tau[j] == 0.0
+        np.testing.assert_array_equal(f[:, j + 1:], f0[:, j + 1:])
