@@ -664,7 +664,8 @@ constexpr int RG_MAX = 16;              // CTAs of the cluster
 constexpr int RG_COLS = 64 / RG_WARPS;  // columns per warp
 constexpr int RG_PART = 66;             // doubles from one CTA: 64 dots (4 w + j: column w + 16 j), sum of squares, exponent
 constexpr int RG_MAX_NR = 8;
-constexpr int kRgEmpty = -4096;
+constexpr int kRgEmpty = -4096;   // exponent sent for a zero column
+constexpr int kRgDenormal = -1001;  // and for one of denormals alone: below every normal one's (-1000 and up)
 
 __device__ __forceinline__ uint32_t cluster_addr(const void* p, int rank) {
     uint32_t a;
@@ -766,11 +767,17 @@ __global__ void __launch_bounds__(RG_THREADS, 1) qr_panel_rg_kernel(double* A, l
             hi = max(hi, (unsigned)__double2hiint(y[r]) & 0x7fffffffu);
         }
         hi = __reduce_max_sync(0xffffffffu, hi) >> 20;  // the maximum's biased exponent
-        const int e = hi == 0x7ff ? 0 : min(1000, max(-1000, (int)hi - 1023));
-        const double sc = sp_pow2(-e);
+        int e = hi == 0x7ff ? 0 : min(1000, max(-1000, (int)hi - 1023));
+        if (hi == 0) {
+            bool any = false;
+#pragma unroll
+            for (int r = 0; r < NR; ++r) any |= y[r] != 0.0;
+            e = __any_sync(0xffffffffu, any) ? kRgDenormal : kRgEmpty;
+        }
+        const double sc = sp_pow2(-max(e, kRgDenormal));
 #pragma unroll
         for (int r = 0; r < NR; ++r) s_x[par][lane + 32 * r] = r0 + lane + 32 * r > k ? y[r] * sc : 0.0;
-        if (lane == 0) s_e[par] = hi == 0 ? kRgEmpty : e;  // (zeros and denormals: no reflector)
+        if (lane == 0) s_e[par] = e;
     };
     if (warp == 0) {
         double y[NR];
@@ -851,7 +858,7 @@ __global__ void __launch_bounds__(RG_THREADS, 1) qr_panel_rg_kernel(double* A, l
         // ---- the reflector.  A zero tail leaves a sign flip or none, a NaN in it likewise; x is then
         // made finite, as the update multiplies it by 0 where it must change nothing
         RgReflector hh{0.0, x0, 0.0, 0};
-        if (m - k > 1 && E > kRgEmpty) {
+        if (m - k > 1 && E > kRgDenormal) {  // (a maximum below the normal range: no reflector)
             if (S > 0.0 && S <= DBL_MAX) {
                 hh = rg_reflector(x0, S, E);
             } else {

@@ -286,3 +286,23 @@ def test_non_finite_column_of_a_panel(ctx, oracle, m, n, i, j, bad):
     if np.isnan(bad) and (i, j) != (0, 0):
         assert tau[j] == 0.0
         np.testing.assert_array_equal(f[:, j + 1:], f0[:, j + 1:])
+
+
+def test_denormals_beside_normal_entries(ctx, oracle):
+    """A column whose maximum is a normal number on one CTA while the rows of
+    the others hold only denormals: they are part of the reflector.  A column
+    of denormals alone has none, as in the restatement."""
+    m, n = 300, 8
+    a = oracle.uniform((m, n), 77) * 2.0 ** -1030
+    a[3] = oracle.uniform((1, n), 78)[0] * 2.0 ** -1015
+    at, tau = _factor(ctx, a)
+    f = at[:, :m].cpu().numpy().T
+    f_ref, tau_ref = oracle.householder_qr_blocked(a)
+    # a denormal entry carries an absolute error of 2^-1075, 2^-60 of the columns' maxima
+    np.testing.assert_allclose(tau.cpu().numpy()[0], tau_ref[0], rtol=0, atol=1e-12)
+    np.testing.assert_allclose(f[1:, 0], f_ref[1:, 0], rtol=0, atol=1e-11)
+    assert np.abs(f[4:, 0]).max() > 1e-6
+    z = np.full((100, 1), 2.0 ** -1040)
+    at, tau = _factor(ctx, z)
+    assert tau.cpu().numpy()[0] == 0.0
+    np.testing.assert_array_equal(at.cpu().numpy().T, z)
