@@ -1242,8 +1242,9 @@ int qr_build_q_enqueue(jlc_ctx* ctx, long long m, long long kmax, long long qcol
         const long long first = last - nb;
         rc = qr_panels_vt(ctx, f, ldf, m, kmax, first, nb, shift, tau, false, q);
         for (int i = nb - 1; i >= 0 && !rc; --i) {
-            const long long k0 = (first + i) * kQrPanel;
-            rc = qr_apply_wy(ctx, m, k0, qcols - k0, q_out + k0 * ldq, ldq, q, i, precision);
+            // (the columns of Q up to k0 + shift are the identity's and have no entry in these rows)
+            const long long k0 = (first + i) * kQrPanel, c0 = k0 + shift;
+            rc = qr_apply_wy(ctx, m, k0, qcols - c0, q_out + c0 * ldq, ldq, q, i, precision);
         }
         if (rc) return rc;
         last = first;

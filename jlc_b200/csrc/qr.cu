@@ -923,9 +923,11 @@ __global__ void __launch_bounds__(RG_THREADS, 1) qr_panel_rg_kernel(double* A, l
 }
 
 // V (ldv x 64, column-major): column i < kb holds reflector k0+i (zeros above
-// row k0+i+shift, one on it, A's tail below); columns kb .. 63 are zero.
-__global__ void qr_pack_v_kernel(const double* A, long long lda, int m, int k0, int kb, int shift, double* V,
-                                 long long ldv) {
+// row k0+i+shift, one on it, A's tail below); columns kb .. 63 are zero.  A step
+// without a reflector (tau = 0) may have left anything below the diagonal, a NaN
+// for instance, which V^T V would spread over T: its tail is zero in V.
+__global__ void qr_pack_v_kernel(const double* A, long long lda, int m, int k0, int kb, int shift, const double* tau,
+                                 double* V, long long ldv) {
     const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= ldv * 64) return;
     const int i = (int)(e / ldv);
@@ -933,7 +935,7 @@ __global__ void qr_pack_v_kernel(const double* A, long long lda, int m, int k0, 
     double v = 0.0;
     if (i < kb && row < m) {
         const int k = k0 + i + shift;
-        v = row < k ? 0.0 : (row == k ? 1.0 : A[(long long)(k0 + i) * lda + row]);
+        v = row < k ? 0.0 : (row == k ? 1.0 : tau[i] != 0.0 ? A[(long long)(k0 + i) * lda + row] : 0.0);
     }
     V[e] = v;
 }
@@ -1119,6 +1121,9 @@ __global__ void __launch_bounds__(VT_THREADS) qr_vt_kernel(const double* A, long
     const int r0 = k0 + cta * R, r1 = min(m, r0 + R);
     double* Vp = V + (size_t)pi * ldv * 64;
     constexpr int CW = 64 / (VT_THREADS / 32);  // columns per warp
+    // this warp's columns with a reflector (the tails of the others are zero, as in qr_pack_v_kernel)
+    const int cl = warp * CW + (lane & (CW - 1));
+    const unsigned has = __ballot_sync(0xffffffffu, cl < kb && tau[min(k0 + cl, kmax - 1)] != 0.0);
     double v[CW];
     auto fetch = [&](int c0) {
         const int row = c0 + lane;
@@ -1141,8 +1146,9 @@ __global__ void __launch_bounds__(VT_THREADS) qr_vt_kernel(const double* A, long
     for (int c0 = r0; c0 < r1; c0 += VT_CHUNK) {
 #pragma unroll
         for (int i = 0; i < CW; ++i) {
-            sv[lane][warp * CW + i] = v[i];
-            if (c0 + lane < r1) Vp[(size_t)(warp * CW + i) * ldv + c0 + lane] = v[i];
+            const double x = (has >> i & 1) || c0 + lane == k0 + warp * CW + i + shift ? v[i] : 0.0;
+            sv[lane][warp * CW + i] = x;
+            if (c0 + lane < r1) Vp[(size_t)(warp * CW + i) * ldv + c0 + lane] = x;
         }
         __syncthreads();
         if (c0 + VT_CHUNK < r1) fetch(c0 + VT_CHUNK);
@@ -1407,7 +1413,8 @@ int launch_qr_vt(const double* a, long long lda, int m, int kmax, int p0, int pa
         for (int i = 0; i < panels; ++i) {
             const int k0 = 64 * (p0 + i), kb = min(64, kmax - k0);
             double* vi = v + (size_t)i * ldv * 64;
-            qr_pack_v_kernel<<<(unsigned)((ldv * 64 + 255) / 256), 256, 0, st>>>(a, lda, m, k0, kb, shift, vi, ldv);
+            qr_pack_v_kernel<<<(unsigned)((ldv * 64 + 255) / 256), 256, 0, st>>>(a, lda, m, k0, kb, shift, tau + k0, vi,
+                                                                                 ldv);
             int parts = (m - k0 + GR_CHUNK - 1) / GR_CHUNK;
             if (parts > sm_count) parts = sm_count;
             const int slab = (m - k0 + parts - 1) / parts;

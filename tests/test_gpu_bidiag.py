@@ -149,3 +149,22 @@ def test_range_of_the_input(ctx, s):
         outs.append((d.cpu().numpy() / scale, e.cpu().numpy() / scale, u.cpu().numpy(), v.cpu().numpy()))
     for x, y in zip(*outs):
         np.testing.assert_array_equal(x, y)
+
+
+@pytest.mark.parametrize("m,n", [(60, 40), (300, 150), (4200, 70)])   # the last: V^T V over the whole grid
+@pytest.mark.parametrize("bad", [np.nan, np.inf])
+def test_factors_of_a_matrix_with_a_non_finite_entry(ctx, m, n, bad):
+    """The steps whose norms are not finite have no reflector.  U and V, formed
+    from the others, are finite and orthogonal, V's first row and column the
+    identity's."""
+    import torch
+    a = O.uniform((n, m), 2600 + m)
+    a[7, 3] = bad
+    f = torch.from_numpy(a).cuda()
+    u, v = torch.empty(m, m, dtype=torch.float64).cuda(), torch.empty(n, n, dtype=torch.float64).cuda()
+    d, e = torch.empty(n, dtype=torch.float64).cuda(), torch.empty(n - 1, dtype=torch.float64).cuda()
+    ctx.bidiag_device(m, n, f.data_ptr(), m, d.data_ptr(), e.data_ptr(), u.data_ptr(), m, v.data_ptr(), n)
+    eye = torch.eye(n, dtype=torch.float64, device="cuda")
+    assert torch.equal(v[0], eye[0]) and torch.equal(v[:, 0], eye[:, 0])
+    assert float((v.T @ v - eye).abs().max()) < 1e-14 * n
+    assert float((u.T @ u - torch.eye(m, dtype=torch.float64, device="cuda")).abs().max()) < 1e-14 * m

@@ -161,3 +161,24 @@ def test_route_edges(ctx, n, with_q):
         q = q.T
         assert float((a.T - q @ h @ q.T).norm() / a.norm()) < tol
         assert float((q.T @ q - torch.eye(n, dtype=torch.float64, device="cuda")).norm()) < tol * n ** 0.5
+
+
+@pytest.mark.parametrize("n", [40, 200])
+@pytest.mark.parametrize("i,j,bad", [(0, 7, np.nan), (0, 7, np.inf), (5, 7, np.nan), (5, 0, np.nan), (39, 38, np.nan)])
+def test_q_of_a_matrix_with_a_non_finite_entry(ctx, oracle, n, i, j, bad):
+    """A column whose norm is a NaN has no reflector: Q is the product of the
+    others, finite and orthogonal.  (An infinity below the diagonal makes the
+    reflector itself NaN: only Q's first column is left.)"""
+    import torch
+    a = oracle.uniform((n, n), 1800 + n)
+    a[i, j] = bad
+    h = torch.from_numpy(np.ascontiguousarray(a.T)).cuda()
+    q = torch.zeros_like(h)
+    eye = torch.eye(n, dtype=torch.float64, device="cuda")
+    ctx.hessenberg_device(n, h.data_ptr(), n, q.data_ptr(), n)
+    assert float((q.T @ q - eye).abs().max()) < 1e-14 * n
+    a[i, j] = 0.5
+    a[5, 0] = np.inf
+    h = torch.from_numpy(np.ascontiguousarray(a.T)).cuda()
+    ctx.hessenberg_device(n, h.data_ptr(), n, q.data_ptr(), n)
+    assert torch.equal(q[0], eye[0])   # column-major: Q's first column
