@@ -27,7 +27,10 @@
 //
 // Layouts: H and Q column-major (ld), V and Y column-major m x 32 (ldv;
 // row r is global row k+1+r), T row-major 32 x 32.
+#include <cfloat>
 #include <cstdio>
+
+#include <math_constants.h>
 
 #include "jlc_device.cuh"
 #include "jlc_internal.h"
@@ -379,6 +382,14 @@ __device__ __noinline__ SlabReflector slab_reflector(double x0, double sigma, do
     return r;
 }
 
+template <int N>
+__device__ __forceinline__ bool any_non_finite(const double (&v)[N]) {
+    unsigned top = 0;  // the largest exponent, from bit 21
+#pragma unroll
+    for (int i = 0; i < N; ++i) top = max(top, (unsigned)__double2hiint(v[i]) << 1);
+    return top >= 0x7ffu << 21;
+}
+
 template <int CB>
 __global__ void __launch_bounds__(SLT, 1) hess_slab_kernel(const SlabArgs p) {
     extern __shared__ double slab[];  // [local row][column], then [warp][local row] sums
@@ -407,6 +418,9 @@ __global__ void __launch_bounds__(SLT, 1) hess_slab_kernel(const SlabArgs p) {
 #pragma unroll
     for (int i = 0; i < CB; ++i) w[i] = u[i] = 0.0;
     bool fail = false;
+    // Rows above a step's reflector take no part in its dots nor in v w^T.  With finite values a factor of
+    // 0 sees to that; where an infinity or a NaN turns up (in a dot, in w) the thread that has the column
+    // sets it right, so that the pass needs no conditions (with them n = 1744: 12.9 -> 14.0 ms, as it is 13.1).
     int gl = cta, lf = 0;  // the first of this CTA's rows past row k: global, local
     if (gl == 0) {
         gl += P;
@@ -462,6 +476,16 @@ __global__ void __launch_bounds__(SLT, 1) hess_slab_kernel(const SlabArgs p) {
                 }
             }
             if (!more) break;
+            if (any_non_finite(s)) {  // the rows above k + 2 may be the cause
+#pragma unroll
+                for (int i = 0; i < CB; ++i) {
+                    const int j = k + tid + i * SLT;
+                    s[i] = 0.0;
+                    if (j < n)
+#pragma unroll 1
+                        for (int l = lf + owner; l < rows; ++l) s[i] = fma(s_c[l], slab[(size_t)l * ld + j], s[i]);
+                }
+            }
 #pragma unroll
             for (int i = 0; i < CB; ++i) {
                 const int j = k + tid + i * SLT;
@@ -533,7 +557,7 @@ __global__ void __launch_bounds__(SLT, 1) hess_slab_kernel(const SlabArgs p) {
 #pragma unroll
         for (int i = 0; i < CB; ++i) {
             const int j = kn + tid + i * SLT;
-            u[i] = j < n ? (j == kn ? (tau != 0.0 ? 1.0 : 0.0) : u[i] * inv) : 0.0;
+            u[i] = j < n && tau != 0.0 ? (j == kn ? 1.0 : u[i] * inv) : 0.0;
         }
         // v on this CTA's rows; column k is finished: beta, and v's tail below it
         if (tid < rows) {
@@ -574,9 +598,20 @@ __global__ void __launch_bounds__(SLT, 1) hess_slab_kernel(const SlabArgs p) {
             }
             s = warp_sum(s);
             if (lane == 0) s_wv[warp] = s;
+            if (any_non_finite(w)) {
+#pragma unroll
+                for (int i = 0; i < CB; ++i) {
+                    if (fabs(w[i]) <= DBL_MAX) continue;
+                    // v w^T is not finite in this column, on the rows from k + 1 on
+#pragma unroll 1
+                    for (int l = lf; l < rows; ++l) slab[(size_t)l * ld + kn + tid + i * SLT] = CUDART_NAN;
+                    w[i] = 0.0;
+                }
+            }
             if (tid == 0) s_wk = w[0];
         }
         if (__syncthreads_or(fail)) return;
+        const int la = lf;
         if (owner) {
             gl += P;
             ++lf;
@@ -596,7 +631,7 @@ __global__ void __launch_bounds__(SLT, 1) hess_slab_kernel(const SlabArgs p) {
             y += shfl_xor(y, 2);
             wv += shfl_xor(wv, 2);
             if (part4 == 0) {
-                const double v = s_v[l], x = tau * fma(-v, wv, y);
+                const double v = s_v[l], wl = l >= la ? wv : 0.0, x = tau != 0.0 ? tau * fma(-v, wl, y) : 0.0;
                 s_x[l] = x;
                 s_c[l] = fma(-x, tau != 0.0 ? 1.0 : 0.0, fma(-v, s_wk, slab[(size_t)l * ld + kn]));
             }

@@ -182,3 +182,31 @@ def test_q_of_a_matrix_with_a_non_finite_entry(ctx, oracle, n, i, j, bad):
     h = torch.from_numpy(np.ascontiguousarray(a.T)).cuda()
     ctx.hessenberg_device(n, h.data_ptr(), n, q.data_ptr(), n)
     assert torch.equal(q[0], eye[0])   # column-major: Q's first column
+
+
+@pytest.mark.parametrize("n", [40, 200, 700])   # 8 rows per CTA; one and two columns per thread
+@pytest.mark.parametrize("bad", [np.nan, np.inf, -np.inf])
+def test_non_finite_entries_stay_where_a_reduction_leaves_them(ctx, oracle, n, bad):
+    """Row 0 takes part in no reflector's dots: an entry there that is not
+    finite changes row 0 alone, and Q not at all.  An entry below it reaches
+    the rows from 1 on, but not row 0.  A NaN in column 0, whose reflector is
+    then skipped, changes that column alone."""
+    import torch
+    clean = oracle.uniform((n, n), 1900 + n)
+
+    def reduce(i, j, value):
+        a = clean.copy()
+        a[i, j] = value
+        h, q = torch.from_numpy(np.ascontiguousarray(a.T)).cuda(), torch.empty(n, n, dtype=torch.float64).cuda()
+        ctx.hessenberg_device(n, h.data_ptr(), n, q.data_ptr(), n)
+        return h.cpu().numpy().T, q.cpu().numpy().T
+
+    h0, q0 = reduce(0, 7, 0.25)
+    h, q = reduce(0, 7, bad)
+    np.testing.assert_array_equal(h[1:], h0[1:])
+    np.testing.assert_array_equal(q, q0)
+    h, _ = reduce(n // 2, 7, np.nan)
+    assert np.isfinite(h[0]).all() and np.isnan(h[1:, 1:][np.triu_indices(n - 1, -1)]).all()
+    h0, q0 = reduce(5, 0, 0.0)
+    h, q = reduce(5, 0, np.nan)
+    assert np.isfinite(h[:, 1:]).all() and np.linalg.norm(q.T @ q - np.eye(n)) < 1e-14 * n
