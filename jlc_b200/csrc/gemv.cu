@@ -37,16 +37,16 @@ __device__ __forceinline__ void gemv_store(const GemvDesc& g, long long row, dou
 
 // Dot form: M(i,p) = mat[i*rs + p]; a warp takes R rows (x is loaded once for
 // them) of its share of the columns, lanes along the row.
-template <int R>
-__global__ void __launch_bounds__(GEMV_THREADS) gemv_dot_kernel(GemvDesc g, int wk, long long chunk, double* partial) {
+// U steps of 32 columns are in flight.
+template <int R, int U = GEMV_LOADS / R>
+__global__ void __launch_bounds__(GEMV_THREADS) gemv_dot_kernel(GemvDesc g, int lwk, long long chunk, double* partial) {
     __shared__ double red[GEMV_WARPS * R];
-    constexpr int U = GEMV_LOADS / R;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const long long row0 = ((long long)blockIdx.x * (GEMV_WARPS / wk) + warp / wk) * R;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, wk = 1 << lwk;  // (shifts: a 64-bit division is long)
+    const long long row0 = ((long long)blockIdx.x * (GEMV_WARPS >> lwk) + (warp >> lwk)) * R;
     const long long c0 = (long long)blockIdx.y * chunk, c1 = c0 + chunk < g.cols ? c0 + chunk : g.cols;
     // this warp's columns: its share of the chunk in whole trips
-    const long long trips = (c1 - c0 + 32 * U - 1) / (32 * U), per = (trips + wk - 1) / wk * (32 * U);
-    const long long p0 = c0 + (warp % wk) * per, p1 = p0 + per < c1 ? p0 + per : c1;
+    const long long trips = (c1 - c0 + 32 * U - 1) / (32 * U), per = ((trips + wk - 1) >> lwk) * (32 * U);
+    const long long p0 = c0 + (warp & (wk - 1)) * per, p1 = p0 + per < c1 ? p0 + per : c1;
     double acc[R];
     const double* rowp[R];
 #pragma unroll
@@ -94,7 +94,7 @@ __global__ void __launch_bounds__(GEMV_THREADS) gemv_dot_kernel(GemvDesc g, int 
     if (wk > 1) {
         if (lane < R) red[warp * R + lane] = mine;
         __syncthreads();
-        if (warp % wk != 0) return;
+        if ((warp & (wk - 1)) != 0) return;
         if (lane < R) {
             mine = 0.0;
             for (int w = 0; w < wk; ++w) mine += red[(warp + w) * R + lane];
@@ -108,8 +108,9 @@ __global__ void __launch_bounds__(GEMV_THREADS) gemv_dot_kernel(GemvDesc g, int 
 }
 
 // Axpy form: M(i,p) = mat[i + p*cs]; lanes own rows, the WK warps of a row group
-// split the chunk's columns, partial sums go to scratch[chunk][row].
-template <int WK>
+// split the chunk's columns, partial sums go to scratch[chunk][row] (one chunk:
+// no scratch, 10^6 x 2 in 8.3 us against 28.8 with a second kernel).
+template <int WK, bool DIRECT>
 __global__ void __launch_bounds__(GEMV_THREADS) gemv_axpy_partial_kernel(GemvDesc g, double* partial, long long chunk) {
     __shared__ double red[WK > 1 ? GEMV_THREADS : 1];
     const int lane = threadIdx.x & 31, part = (threadIdx.x >> 5) % WK;
@@ -139,7 +140,10 @@ __global__ void __launch_bounds__(GEMV_THREADS) gemv_axpy_partial_kernel(GemvDes
 #pragma unroll
         for (int w = 1; w < WK; ++w) s += red[threadIdx.x + 32 * w];
     }
-    if (WK == 1 || row < g.rows) partial[(long long)blockIdx.y * g.rows + row] = s;
+    if (WK == 1 || row < g.rows) {
+        if (DIRECT) gemv_store(g, row, s);
+        else partial[(long long)blockIdx.y * g.rows + row] = s;
+    }
 }
 
 // y from the chunks' partial sums: 32 rows per CTA, its warps split the chunks
@@ -208,11 +212,11 @@ GemvShape gemv_shape(const GemvDesc& g, int sm_count) {
 
 }  // namespace
 
-// partial sums: the axpy form's always, the dot form's when its columns are split over CTAs
+// partial sums, when the columns are split over CTAs
 size_t gemv_scratch_bytes(const GemvDesc& g, int sm_count) {
     if (g.rows <= 0 || g.cols <= 0) return 0;
     const GemvShape s = gemv_shape(g, sm_count);
-    return g.cs == 1 && s.chunks == 1 ? 0 : (size_t)s.chunks * (size_t)g.rows * sizeof(double);
+    return s.chunks == 1 ? 0 : (size_t)s.chunks * (size_t)g.rows * sizeof(double);
 }
 
 int launch_gemv(const GemvDesc& g, void* scratch, cudaStream_t st, int sm_count, char* err, size_t errlen) {
@@ -222,17 +226,22 @@ int launch_gemv(const GemvDesc& g, void* scratch, cudaStream_t st, int sm_count,
         return JLC_E_UNSUPPORTED;
     }
     const GemvShape s = gemv_shape(g, sm_count);
-    double* partial = g.cs == 1 && s.chunks == 1 ? nullptr : static_cast<double*>(scratch);
+    double* partial = s.chunks == 1 ? nullptr : static_cast<double*>(scratch);
     const long long groups = g.cs == 1 ? (g.rows + s.rows_per_warp - 1) / s.rows_per_warp : (g.rows + 31) / 32;
     const dim3 grid((unsigned)((groups * s.wk + GEMV_WARPS - 1) / GEMV_WARPS), (unsigned)s.chunks);
     if (g.cs == 1) {
-        auto kern = s.rows_per_warp == 4 ? gemv_dot_kernel<4> : s.rows_per_warp == 2 ? gemv_dot_kernel<2> : gemv_dot_kernel<1>;
-        kern<<<grid, GEMV_THREADS, 0, st>>>(g, s.wk, s.chunk, partial);
+        // (rows of at most 64 columns keep fewer loads than registers would be held for: 10^6 x 2
+        // 122 -> 86 us, 200000 x 16 27.8 -> 20.6)
+        auto kern = s.rows_per_warp == 4   ? g.cols <= 64 ? gemv_dot_kernel<4, 1> : gemv_dot_kernel<4>
+                    : s.rows_per_warp == 2 ? gemv_dot_kernel<2>
+                                           : gemv_dot_kernel<1>;
+        kern<<<grid, GEMV_THREADS, 0, st>>>(g, s.wk == 8 ? 3 : s.wk >> 1, s.chunk, partial);
     } else {
-        auto kern = s.wk == 1   ? gemv_axpy_partial_kernel<1>
-                    : s.wk == 2 ? gemv_axpy_partial_kernel<2>
-                    : s.wk == 4 ? gemv_axpy_partial_kernel<4>
-                                : gemv_axpy_partial_kernel<8>;
+        auto kern = s.wk == 1   ? partial ? gemv_axpy_partial_kernel<1, false> : gemv_axpy_partial_kernel<1, true>
+                    : s.wk == 2 ? partial ? gemv_axpy_partial_kernel<2, false> : gemv_axpy_partial_kernel<2, true>
+                    : s.wk == 4 ? partial ? gemv_axpy_partial_kernel<4, false> : gemv_axpy_partial_kernel<4, true>
+                    : partial   ? gemv_axpy_partial_kernel<8, false>
+                                : gemv_axpy_partial_kernel<8, true>;
         kern<<<grid, GEMV_THREADS, 0, st>>>(g, partial, s.chunk);
     }
     if (partial)

@@ -140,7 +140,7 @@ void tune_store(const std::string& key, int value);
 size_t dmma_splitk_bytes(long long m, long long n, long long k, int ksplit, int sm_count);
 
 // y[i*incy] = alpha * sum_p M(i,p) x[p*incx] + beta * y[i*incy], M(i,p) = mat[i*rs + p*cs]
-// with rs == 1 or cs == 1.  scratch: ceil-split partial sums for the rs == 1 form.
+// with rs == 1 or cs == 1.  scratch: partial sums where the columns are split over CTAs.
 struct GemvDesc {
     long long rows, cols;
     double alpha, beta;

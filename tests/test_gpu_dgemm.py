@@ -506,3 +506,17 @@ def test_matvec_shapes(ctx, oracle, la, m, k):
     assert (y[:, 1] == 7.0).all()
     assert_fp64_bound(f"matvec {m}x{k}", y[:, :1], a, x, c, 1.5, -0.5)
     assert_fp64_bound(f"vecmat {m}x{k}", row.cpu().numpy(), x.T, a.T, c.T, 1.5, -0.5)
+
+
+@pytest.mark.parametrize("la", [0, 1])
+@pytest.mark.parametrize("m,k", [(20001, 2), (9000, 31), (5000, 64), (5000, 65), (300, 700), (50, 50), (12345, 1)])
+def test_gemv_of_few_columns(ctx, oracle, la, m, k):
+    """Tall matrices of few columns: the row form's short tail (up to two steps
+    of 32 columns) and the column form that needs no partial sums."""
+    import torch
+    A, B, C = oracle.uniform((m, k), 61 + k), oracle.uniform((k, 1), 62 + k), oracle.uniform((m, 1), 63 + k)
+    dA = torch.from_numpy(np.ascontiguousarray(A if la == 0 else A.T)).cuda()
+    dB, dC = torch.from_numpy(B).cuda(), torch.from_numpy(C.copy()).cuda()
+    ctx.dgemm_device(la, 0, m, 1, k, 1.5, dA.data_ptr(), dA.shape[1], dB.data_ptr(), 1, 0.5, dC.data_ptr(), 1)
+    ctx.synchronize()
+    assert_fp64_bound(f"gemv {m}x{k} la={la}", dC.cpu().numpy(), A, B, C, 1.5, 0.5)
