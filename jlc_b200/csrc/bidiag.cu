@@ -154,12 +154,20 @@ __global__ void __launch_bounds__(BT, 1) bidiag_kernel(const Args p) {
     double* slab = SMEM ? dyn : p.slab + (size_t)cta * rows * ld;  // [local row][column]
     double* red = SMEM ? dyn + (size_t)rows * ld : dyn;            // [warp][local row]
     Slot* part = p.part + (size_t)cta * ld;
-    // this CTA's rows into its slab (rows past m are zero)
-    for (int l = 0; l < rows; ++l) {
-        const int g = l * P + cta;
+    // f(local row, global row, column) over the slab.  A matrix of few columns takes several rows at a
+    // time, a power of two of threads each (37000 x 2: 197 us row by row, 95 so)
+    auto over_slab = [&](auto f) {
+        int span = BT;
+        while (span >= 2 * ld) span >>= 1;
+        for (int l = tid / span; l < rows; l += BT / span) {
 #pragma unroll 1
-        for (int j = tid; j < ld; j += BT) slab[(size_t)l * ld + j] = g < m && j < n ? p.a[g + (long long)j * p.lda] : 0.0;
-    }
+            for (int j = tid & (span - 1); j < ld; j += span) f(l, l * P + cta, j);
+        }
+    };
+    // this CTA's rows into its slab (rows past m are zero)
+    over_slab([&](int l, int g, int j) {
+        slab[(size_t)l * ld + j] = g < m && j < n ? p.a[g + (long long)j * p.lda] : 0.0;
+    });
     for (int l = tid; l < rows; l += BT) {
         s_v[l] = 0.0;
         s_x[l] = 0.0;
@@ -516,12 +524,9 @@ __global__ void __launch_bounds__(BT, 1) bidiag_kernel(const Args p) {
         }
     }
     __syncthreads();
-    for (int l = 0; l < rows; ++l) {
-        const int g = l * P + cta;
-        if (g < m)
-#pragma unroll 1
-            for (int j = tid; j < n; j += BT) p.a[g + (long long)j * p.lda] = slab[(size_t)l * ld + j];
-    }
+    over_slab([&](int l, int g, int j) {
+        if (g < m && j < n) p.a[g + (long long)j * p.lda] = slab[(size_t)l * ld + j];
+    });
 }
 
 // Right reflectors, stored in the rows of A beyond the superdiagonal, as the
