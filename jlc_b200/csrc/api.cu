@@ -64,6 +64,17 @@ int ws_reserve(jlc_ctx* ctx, size_t bytes) {
     return workspace_reserve(ctx->ws, bytes, ctx->err, sizeof(ctx->err));
 }
 
+// The counters of a split product about to be launched.  Each launch has a number
+// of its own, so that nothing an earlier one left in them matters, whichever
+// stream it ran on and however it ended.  A captured launch keeps its number
+// from replay to replay: its counters are cleared in the graph.
+SplitCounters split_counters(jlc_ctx* ctx) {
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(ctx->stream, &cs) == cudaSuccess && cs == cudaStreamCaptureStatusActive)
+        cudaMemsetAsync(ctx->d_counters, 0, kSplitTiles * sizeof(*ctx->d_counters), ctx->stream);
+    return {ctx->d_counters, ++ctx->split_launches << kSplitShift};
+}
+
 // a failed copy of the single-shot host entry: the stream is drained so the
 // context is idle when the error returns
 int copy_failed(jlc_ctx* ctx, cudaError_t e, const char* what) {
@@ -314,7 +325,7 @@ int run_device(jlc_ctx* ctx, const GemmDesc& g0, int precision, int slices, jlc_
     return launch_dgemm_dmma(g, ctx->stream, ctx->sm_count, ctx->d_status, ozaki ? ctx->d_flags : nullptr,
                              ctx->dmma_k, ctx->err, sizeof(ctx->err), ksplit,
                              splitk_bytes ? static_cast<char*>(ctx->ws.ptr) + splitk_off : nullptr, splitk_bytes,
-                             ctx->d_counters);
+                             splitk_bytes ? split_counters(ctx) : SplitCounters{});
 }
 
 int finish_sync(jlc_ctx* ctx) {
@@ -324,9 +335,10 @@ int finish_sync(jlc_ctx* ctx) {
     e = cudaMemcpy(&st, ctx->d_status, sizeof(int), cudaMemcpyDeviceToHost);
     if (e != cudaSuccess) return cuda_err(ctx, e, "status read");
     if (st != 0) {
-        cudaMemset(ctx->d_status, 0, sizeof(int));
-        // a kernel that gave up may have left split-K arrivals behind
-        cudaMemset(ctx->d_counters, 0, kSplitTiles * sizeof(int));
+        // (on the context's stream, which the legacy stream is not ordered with)
+        e = cudaMemsetAsync(ctx->d_status, 0, sizeof(int), ctx->stream);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
+        if (e != cudaSuccess) return cuda_err(ctx, e, "status reset");
         if (st & JLC_DEV_TIMEOUT) return set_err(ctx, JLC_E_TIMEOUT, "a device wait timed out (status 0x%x)", st);
         return set_err(ctx, JLC_E_CUDA, "device status 0x%x", st);
     }
@@ -792,11 +804,13 @@ int jlc_init(int device, jlc_ctx** out) {
     bool ok = cudaStreamCreateWithFlags(&ctx->own_stream, cudaStreamNonBlocking) == cudaSuccess &&
               cudaMalloc(&ctx->d_status, 4 * sizeof(int)) == cudaSuccess &&
               cudaMalloc(&ctx->d_flags, 4 * sizeof(int)) == cudaSuccess &&
-              cudaMalloc(&ctx->d_counters, kSplitTiles * sizeof(int)) == cudaSuccess &&
+              cudaMalloc(&ctx->d_counters, kSplitTiles * sizeof(*ctx->d_counters)) == cudaSuccess &&
               cudaEventCreate(&ctx->ev0) == cudaSuccess && cudaEventCreate(&ctx->ev1) == cudaSuccess;
-    if (ok) ok = cudaMemset(ctx->d_status, 0, 4 * sizeof(int)) == cudaSuccess &&
-                 cudaMemset(ctx->d_flags, 0, 4 * sizeof(int)) == cudaSuccess &&
-                 cudaMemset(ctx->d_counters, 0, kSplitTiles * sizeof(int)) == cudaSuccess;
+    if (ok) ok = cudaMemsetAsync(ctx->d_status, 0, 4 * sizeof(int), ctx->own_stream) == cudaSuccess &&
+                 cudaMemsetAsync(ctx->d_flags, 0, 4 * sizeof(int), ctx->own_stream) == cudaSuccess &&
+                 cudaMemsetAsync(ctx->d_counters, 0, kSplitTiles * sizeof(*ctx->d_counters), ctx->own_stream) ==
+                     cudaSuccess &&
+                 cudaStreamSynchronize(ctx->own_stream) == cudaSuccess;
     if (!ok) {
         cudaGetLastError();
         jlc_destroy(ctx);
@@ -861,7 +875,8 @@ int jlc_autotune_splitk(jlc_ctx* ctx, int64_t m, int64_t n, int64_t k, int* spli
         for (int rep = 0; rep < 4; ++rep) {  // one warm-up, three timed
             cudaEventRecord(ctx->ev0, ctx->stream);
             rc = launch_dgemm_dmma(g, ctx->stream, ctx->sm_count, ctx->d_status, nullptr, ctx->dmma_k, ctx->err,
-                                   sizeof(ctx->err), s, wsb ? ctx->ws.ptr : nullptr, wsb, ctx->d_counters);
+                                   sizeof(ctx->err), s, wsb ? ctx->ws.ptr : nullptr, wsb,
+                                   wsb ? split_counters(ctx) : SplitCounters{});
             if (rc) return rc;
             cudaEventRecord(ctx->ev1, ctx->stream);
             cudaError_t e = cudaEventSynchronize(ctx->ev1);

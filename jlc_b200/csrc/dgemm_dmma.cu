@@ -25,8 +25,10 @@
 // Split-K (products whose tiles would leave SMs idle): the k-blocks of a tile
 // are cut into ksplit contiguous parts, one work unit each.  A unit's partial
 // tile goes to workspace; the CTA whose unit arrives last at the tile's counter
-// sums the parts in index order (deterministic whatever the arrival order),
-// clears the counter and runs the normal epilogue.  No CTA waits for another.
+// sums the parts in index order (deterministic whatever the arrival order) and
+// runs the normal epilogue.  No CTA waits for another.  A counter carries the
+// number of the launch that it counts for: arrivals that an abandoned launch
+// left behind are older and count for nothing.
 // The tile shape does not enter the sums: an element is the same chain of MMAs
 // over k in every shape, so only the split decides a result's bits.
 //
@@ -87,7 +89,8 @@ struct Params {
     int tiles_m, tiles_n, num_tiles, k_blocks;
     int ksplit;         // k parts per tile (1: no split)
     double* part;       // ksplit > 1: BM*BN partial sums per (tile, part)
-    int* counters;      // ksplit > 1: arrivals per tile, zero between launches
+    unsigned long long* counters;  // ksplit > 1: arrivals per tile, below the number of their launch
+    unsigned long long launch;     // this launch's number << kSplitShift, above that of any before it
     int* status;
     const int* gate;  // when non-null the kernel runs only if an Ozaki call's flags ask for FP64
     int chained;      // launch attribute only: GemmDesc::chained
@@ -317,9 +320,9 @@ __global__ void __launch_bounds__(THREADS, 1)
             int* last_flag = reinterpret_cast<int*>(empty + STAGES);
             asm volatile("bar.sync 2, %0;" ::"n"(MMA_WARPS * 32) : "memory");
             if (ct == 0) {
-                const bool last = atomicAdd(&p.counters[tile], 1) == p.ksplit - 1;
-                if (last) p.counters[tile] = 0;  // as the next launch expects it
-                *last_flag = last;
+                atomicMax(&p.counters[tile], p.launch);  // (older arrivals are forgotten)
+                const unsigned long long before = atomicAdd(&p.counters[tile], 1ull);
+                *last_flag = before - p.launch == (unsigned long long)(p.ksplit - 1);
             }
             asm volatile("bar.sync 2, %0;" ::"n"(MMA_WARPS * 32) : "memory");
             // (the next unit's write of the flag comes after its first barrier,
@@ -598,7 +601,8 @@ size_t dmma_splitk_bytes(long long m, long long n, long long k, int ksplit, int 
 }
 
 int launch_dgemm_dmma(const GemmDesc& g, cudaStream_t st, int sm_count, int* status, const int* gate,
-                      int mma_k, char* err, size_t errlen, int ksplit, void* splitk_ws, size_t splitk_ws_bytes, int* splitk_counters) {
+                      int mma_k, char* err, size_t errlen, int ksplit, void* splitk_ws, size_t splitk_ws_bytes,
+                      SplitCounters split_counters) {
     using namespace dmma;
     if (!dmma_operand_ok(g.a, g.lda) || !dmma_operand_ok(g.b, g.ldb)) {
         snprintf(err, errlen, "DMMA kernel needs 16-byte aligned A/B and even leading dimensions");
@@ -609,7 +613,7 @@ int launch_dgemm_dmma(const GemmDesc& g, cudaStream_t st, int sm_count, int* sta
     // split-K needs the caller's workspace; the adjoint's fused dot keeps one
     // unit per tile (its per-CTA partial dots must not depend on arrival order)
     const int kbl = (int)((g.k + BK - 1) / BK);
-    int split = ksplit > 1 && splitk_ws && splitk_counters && !g.dot_mat ? (ksplit < kbl ? ksplit : kbl) : 1;
+    int split = ksplit > 1 && splitk_ws && split_counters.word && !g.dot_mat ? (ksplit < kbl ? ksplit : kbl) : 1;
     if (split > 1 && dmma_splitk_bytes(g.m, g.n, g.k, split, sm_count) > splitk_ws_bytes) split = 1;
     const Tile tile = dmma_tile(g.m, g.n, g.k, split, sm_count);
     const int bm = tile.bm, bn = tile.bn;
@@ -653,10 +657,12 @@ int launch_dgemm_dmma(const GemmDesc& g, cudaStream_t st, int sm_count, int* sta
     p.ksplit = 1;
     p.part = nullptr;
     p.counters = nullptr;
+    p.launch = 0;
     if (split > 1) {
         p.ksplit = split;
         p.part = static_cast<double*>(splitk_ws);
-        p.counters = splitk_counters;
+        p.counters = split_counters.word;
+        p.launch = split_counters.launch;
     }
     const int units = p.num_tiles * p.ksplit;
     const int grid = units < sm_count ? units : sm_count;

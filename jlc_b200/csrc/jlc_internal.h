@@ -84,7 +84,7 @@ bool dmma_operand_ok(const void* ptr, long long ld);
 // dimensions.  gate != nullptr: the kernel only runs if one of the Ozaki
 // call's flags gate[kFlagNonfiniteA], gate[kFlagFallback],
 // gate[kFlagNonfiniteB] is set.
-// ksplit > 1 with splitk_counters and splitk_ws of at least dmma_splitk_bytes(m, n, k, ksplit, sm_count):
+// ksplit > 1 with split_counters and splitk_ws of at least dmma_splitk_bytes(m, n, k, ksplit, sm_count):
 // split-K over ksplit parts; otherwise every tile is one work unit.
 // blocked Householder QR kernels (qr.cu)
 size_t qr_panel_mp_scratch_bytes(int P);
@@ -119,12 +119,17 @@ size_t hess_panel_scratch_bytes(int sm_count);
 int launch_hess_panel(const double* h, long long ldh, int n, int k, int pw, double* V, long long ldv, double* Y,
                       double* T, double* tau, double* wbuf, void* scratch, int sm_count, int* status,
                       cudaStream_t st);
+// Arrivals per tile of split products (kSplitTiles words) and the number of the
+// launch, above that of every launch before it that used the words.
+constexpr int kSplitTiles = 4096;  // tiles a split product may have
+constexpr int kSplitShift = 8;     // a word is launch number << 8 | arrivals (8 at most)
+struct SplitCounters {
+    unsigned long long* word = nullptr;
+    unsigned long long launch = 0;  // << kSplitShift
+};
 int launch_dgemm_dmma(const GemmDesc& g, cudaStream_t st, int sm_count, int* status, const int* gate, int mma_k,
                       char* err, size_t errlen, int ksplit = 1, void* splitk_ws = nullptr,
-                      size_t splitk_ws_bytes = 0, int* splitk_counters = nullptr);
-// tiles a split product may have (the length of splitk_counters, all zero
-// between launches: the unit that finishes a tile clears its counter)
-constexpr int kSplitTiles = 4096;
+                      size_t splitk_ws_bytes = 0, SplitCounters split_counters = {});
 int dmma_splitk(long long m, long long n, long long k, int sm_count);
 // split-K tuning (dgemm_dmma.cu): legal factors, the shape class, and the
 // tuned factor of a class (0: none cached); remember() records a new choice
@@ -272,7 +277,8 @@ struct jlc_ctx {
     cudaStream_t stream = nullptr;
     int* d_status = nullptr;  // status block: JLC_DEV_* bits written by kernels, wait limit at byte 8
     int* d_flags = nullptr;   // control words of an Ozaki call (kFlag*)
-    int* d_counters = nullptr;  // split-K arrivals per tile (kSplitTiles, zero between launches)
+    unsigned long long* d_counters = nullptr;  // split-K arrivals per tile (kSplitTiles words)
+    unsigned long long split_launches = 0;     // split products launched, in the counters' upper bits
     DevBuf bufA, bufB, bufC;
     DevBuf bufR;  // reduction partials (adjoint)
     DevBuf bufQ;  // blocked QR: V, G, T and the two W panels

@@ -520,3 +520,49 @@ def test_gemv_of_few_columns(ctx, oracle, la, m, k):
     ctx.dgemm_device(la, 0, m, 1, k, 1.5, dA.data_ptr(), dA.shape[1], dB.data_ptr(), 1, 0.5, dC.data_ptr(), 1)
     ctx.synchronize()
     assert_fp64_bound(f"gemv {m}x{k} la={la}", dC.cpu().numpy(), A, B, C, 1.5, 0.5)
+
+
+def test_captured_split_products_among_others(oracle):
+    """A captured split product, replayed between eager split products of the
+    same context: every result has the bits of the first."""
+    import jlc_b200
+    import torch
+    ctx, st = jlc_b200.Context(0), torch.cuda.Stream()
+    try:
+        ctx.set_stream(st.cuda_stream)
+        shapes = [(640, 512, 2048), (256, 256, 4096)]
+        ops = [(torch.from_numpy(oracle.uniform((m, k), 71 + i)).cuda(),
+                torch.from_numpy(oracle.uniform((k, n), 81 + i)).cuda(),
+                torch.zeros(m, n, dtype=torch.float64, device="cuda")) for i, (m, n, k) in enumerate(shapes)]
+        torch.cuda.synchronize()
+
+        def product(i):
+            (m, n, k), (a, b, c) = shapes[i], ops[i]
+            assert ctx.splitk_choice(m, n, k) > 1
+            ctx.dgemm_device(0, 0, m, n, k, 1.0, a.data_ptr(), k, b.data_ptr(), n, 0.0, c.data_ptr(), n, report=False)
+
+        def result(i):
+            ctx.synchronize()
+            c = ops[i][2].clone()
+            ops[i][2].zero_()
+            torch.cuda.synchronize()
+            return c
+
+        first = []
+        for i in (0, 1):
+            product(i)
+            first.append(result(i))
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=st):
+            product(0)
+        for step in (0, 0, 1, 0, "eager 0", 0, 1, 1, 0):
+            if step == 1 or step == "eager 0":
+                i = 1 if step == 1 else 0
+                product(i)
+            else:
+                i = 0
+                with torch.cuda.stream(st):
+                    graph.replay()
+            assert torch.equal(result(i), first[i]), step
+    finally:
+        ctx.close()

@@ -136,6 +136,42 @@ def test_grouped_wait_runs_out_and_plan_recovers(ctx, oracle):
         plan.close()
 
 
+def test_split_product_recovers(ctx, oracle):
+    """A wait of a split product runs out: units of the abandoned launch have
+    counted themselves at their tiles, and one has not.  The next products,
+    split in the same and in other ways, have the bits they had before it."""
+    import torch
+    from jlc_b200 import JlcError
+    shapes = [(256, 256, 4096), (640, 512, 2048), (64, 2048, 2304)]
+    ops = []
+    for i, (m, n, k) in enumerate(shapes):
+        assert ctx.splitk_choice(m, n, k) > 1
+        ops.append((torch.from_numpy(oracle.uniform((m, k), 1571 + i)).cuda(),
+                    torch.from_numpy(oracle.uniform((k, n), 1581 + i)).cuda()))
+
+    def product(i):
+        (m, n, k), (a, b) = shapes[i], ops[i]
+        c = torch.zeros((m, n), dtype=torch.float64, device="cuda")
+        torch.cuda.synchronize()
+        ctx.dgemm_device(0, 0, m, n, k, 1.0, a.data_ptr(), k, b.data_ptr(), n, 0.0, c.data_ptr(), n, precision=0,
+                         report=False)
+        ctx.synchronize()
+        return c
+
+    before = [product(i) for i in range(3)]
+    ctx.set_wait_limit(0.05)
+    try:
+        for i in range(3):
+            ctx.inject_fault(WAIT, 0)
+            with pytest.raises(JlcError) as exc:
+                product(i)
+            assert exc.value.code == E_TIMEOUT, exc.value
+            for j in (i, 0, 1, 2):
+                assert torch.equal(product(j), before[j]), (i, j)
+    finally:
+        ctx.set_wait_limit(0.0)
+
+
 def test_timeout_through_the_host_entry_returns_false(oracle):
     import jlc_b200
     from jlc_b200 import CudaGemm
