@@ -37,11 +37,12 @@ __device__ __forceinline__ void gemv_store(const GemvDesc& g, long long row, dou
 
 // Dot form: M(i,p) = mat[i*rs + p]; a warp takes R rows (x is loaded once for
 // them) of its share of the columns, lanes along the row.
-// U steps of 32 columns are in flight.
+// U steps of 32 columns are in flight (U = 1, matrices of at most 64 columns: wk = 1).
+// Four CTAs of the <4> form fit an SM at 64 registers (8192 x 16384: 159 us; 167 with three).
 template <int R, int U = GEMV_LOADS / R>
-__global__ void __launch_bounds__(GEMV_THREADS) gemv_dot_kernel(GemvDesc g, int lwk, long long chunk, double* partial) {
+__global__ void __launch_bounds__(GEMV_THREADS, R == 4 ? 4 : 1) gemv_dot_kernel(GemvDesc g, int lwk0, long long chunk, double* partial) {
     __shared__ double red[GEMV_WARPS * R];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, wk = 1 << lwk;  // (shifts: a 64-bit division is long)
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, lwk = U == 1 ? 0 : lwk0, wk = 1 << lwk;  // (shifts: a 64-bit division is long)
     const long long row0 = ((long long)blockIdx.x * (GEMV_WARPS >> lwk) + (warp >> lwk)) * R;
     const long long c0 = (long long)blockIdx.y * chunk, c1 = c0 + chunk < g.cols ? c0 + chunk : g.cols;
     // this warp's columns: its share of the chunk in whole trips
@@ -231,7 +232,7 @@ int launch_gemv(const GemvDesc& g, void* scratch, cudaStream_t st, int sm_count,
     const dim3 grid((unsigned)((groups * s.wk + GEMV_WARPS - 1) / GEMV_WARPS), (unsigned)s.chunks);
     if (g.cs == 1) {
         // (rows of at most 64 columns keep fewer loads than registers would be held for: 10^6 x 2
-        // 122 -> 86 us, 200000 x 16 27.8 -> 20.6)
+        // 122 -> 80 us, 200000 x 16 27.8 -> 18.8)
         auto kern = s.rows_per_warp == 4   ? g.cols <= 64 ? gemv_dot_kernel<4, 1> : gemv_dot_kernel<4>
                     : s.rows_per_warp == 2 ? gemv_dot_kernel<2>
                                            : gemv_dot_kernel<1>;
