@@ -4,11 +4,15 @@
 // (PackingUtils.scaleCPanel, PackingUtils.java:159-183).
 #include <cstdio>
 
+#include <cooperative_groups.h>
+
 #include "jlc_device.cuh"
 #include "jlc_internal.h"
 
 namespace jlc {
 namespace {
+
+namespace cg = cooperative_groups;
 
 constexpr int GEMV_THREADS = 256, GEMV_WARPS = GEMV_THREADS / 32;
 constexpr int GEMV_LOADS = 16;     // matrix loads a lane keeps in flight (dot form)
@@ -26,7 +30,7 @@ constexpr int GEMV_AXPY_CTAS = 8;  // resident CTAs per SM (axpy form)
 struct GemvShape {
     int rows_per_warp;  // dot form: 4, 2 or 1
     int wk;             // warps that share a row group and split its columns (1, 2, 4, 8)
-    int chunks;         // column chunks over CTAs (partial sums in scratch when > 1)
+    int chunks;         // column chunks over CTAs (dot form: of a cluster; else partial sums in scratch when > 1)
     long long chunk;    // columns per chunk
 };
 
@@ -39,8 +43,10 @@ __device__ __forceinline__ void gemv_store(const GemvDesc& g, long long row, dou
 // them) of its share of the columns, lanes along the row.
 // U steps of 32 columns are in flight (U = 1, matrices of at most 64 columns: wk = 1).
 // Four CTAs of the <4> form fit an SM at 64 registers (8192 x 16384: 159 us; 167 with three).
-template <int R, int U = GEMV_LOADS / R>
-__global__ void __launch_bounds__(GEMV_THREADS, R == 4 ? 4 : 1) gemv_dot_kernel(GemvDesc g, int lwk0, long long chunk, double* partial) {
+// CLUSTER: the chunks of the same rows are the CTAs of a cluster, the first of which adds their sums
+// in order, so that a few long rows need neither scratch nor a second kernel.
+template <int R, int U = GEMV_LOADS / R, bool CLUSTER = false>
+__global__ void __launch_bounds__(GEMV_THREADS, R == 4 ? 4 : 1) gemv_dot_kernel(GemvDesc g, int lwk0, long long chunk) {
     __shared__ double red[GEMV_WARPS * R];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, lwk = U == 1 ? 0 : lwk0, wk = 1 << lwk;  // (shifts: a 64-bit division is long)
     const long long row0 = ((long long)blockIdx.x * (GEMV_WARPS >> lwk) + (warp >> lwk)) * R;
@@ -92,20 +98,30 @@ __global__ void __launch_bounds__(GEMV_THREADS, R == 4 ? 4 : 1) gemv_dot_kernel(
 #pragma unroll
     for (int r = 1; r < R; ++r)
         if (lane == r) mine = acc[r];
+    const bool lead = (warp & (wk - 1)) == 0;
     if (wk > 1) {
         if (lane < R) red[warp * R + lane] = mine;
         __syncthreads();
-        if ((warp & (wk - 1)) != 0) return;
-        if (lane < R) {
+        if (!CLUSTER && !lead) return;
+        if (lead && lane < R) {
             mine = 0.0;
             for (int w = 0; w < wk; ++w) mine += red[(warp + w) * R + lane];
         }
     }
-    const long long row = row0 + lane;
-    if (lane < R && row < g.rows) {
-        if (partial) partial[(long long)blockIdx.y * g.rows + row] = mine;
-        else gemv_store(g, row, mine);
+    if (CLUSTER) {
+        __shared__ double sum[GEMV_WARPS * R];
+        cg::cluster_group cluster = cg::this_cluster();
+        double* slot = &sum[(warp >> lwk) * R + lane % R];
+        if (lead && lane < R) *slot = mine;
+        cluster.sync();
+        const bool first = cluster.block_rank() == 0;
+        if (first && lead && lane < R)
+            for (unsigned q = 1; q < cluster.num_blocks(); ++q) mine += *cluster.map_shared_rank(slot, q);
+        cluster.sync();  // (no CTA leaves while its sums are read)
+        if (!first || !lead) return;
     }
+    const long long row = row0 + lane;
+    if (lane < R && row < g.rows) gemv_store(g, row, mine);
 }
 
 // Axpy form: M(i,p) = mat[i + p*cs]; lanes own rows, the WK warps of a row group
@@ -187,7 +203,7 @@ GemvShape gemv_shape(const GemvDesc& g, int sm_count) {
         if (ctas() < target / 2 && most > 1) {
             long long want = (target + ctas() - 1) / ctas();
             if (want > most) want = most;
-            if (want > 64) want = 64;
+            if (want > 8) want = 8;  // CTAs of a cluster
             s.chunk = (g.cols + want - 1) / want;
         }
     } else {
@@ -213,11 +229,11 @@ GemvShape gemv_shape(const GemvDesc& g, int sm_count) {
 
 }  // namespace
 
-// partial sums, when the columns are split over CTAs
+// partial sums of the axpy form, when the columns are split over CTAs
 size_t gemv_scratch_bytes(const GemvDesc& g, int sm_count) {
     if (g.rows <= 0 || g.cols <= 0) return 0;
     const GemvShape s = gemv_shape(g, sm_count);
-    return s.chunks == 1 ? 0 : (size_t)s.chunks * (size_t)g.rows * sizeof(double);
+    return g.cs == 1 || s.chunks == 1 ? 0 : (size_t)s.chunks * (size_t)g.rows * sizeof(double);
 }
 
 int launch_gemv(const GemvDesc& g, void* scratch, cudaStream_t st, int sm_count, char* err, size_t errlen) {
@@ -227,16 +243,32 @@ int launch_gemv(const GemvDesc& g, void* scratch, cudaStream_t st, int sm_count,
         return JLC_E_UNSUPPORTED;
     }
     const GemvShape s = gemv_shape(g, sm_count);
-    double* partial = s.chunks == 1 ? nullptr : static_cast<double*>(scratch);
+    double* partial = g.cs == 1 || s.chunks == 1 ? nullptr : static_cast<double*>(scratch);
     const long long groups = g.cs == 1 ? (g.rows + s.rows_per_warp - 1) / s.rows_per_warp : (g.rows + 31) / 32;
     const dim3 grid((unsigned)((groups * s.wk + GEMV_WARPS - 1) / GEMV_WARPS), (unsigned)s.chunks);
     if (g.cs == 1) {
-        // (rows of at most 64 columns keep fewer loads than registers would be held for: 10^6 x 2
-        // 122 -> 80 us, 200000 x 16 27.8 -> 18.8)
-        auto kern = s.rows_per_warp == 4   ? g.cols <= 64 ? gemv_dot_kernel<4, 1> : gemv_dot_kernel<4>
-                    : s.rows_per_warp == 2 ? gemv_dot_kernel<2>
-                                           : gemv_dot_kernel<1>;
-        kern<<<grid, GEMV_THREADS, 0, st>>>(g, s.wk == 8 ? 3 : s.wk >> 1, s.chunk, partial);
+        const int lwk = s.wk == 8 ? 3 : s.wk >> 1;
+        if (s.chunks > 1) {  // (few rows: one per warp)
+            cudaLaunchConfig_t cfg = {};
+            cudaLaunchAttribute at[1];
+            cfg.gridDim = grid;
+            cfg.blockDim = dim3(GEMV_THREADS);
+            cfg.stream = st;
+            at[0].id = cudaLaunchAttributeClusterDimension;
+            at[0].val.clusterDim.x = 1;
+            at[0].val.clusterDim.y = (unsigned)s.chunks;
+            at[0].val.clusterDim.z = 1;
+            cfg.attrs = at;
+            cfg.numAttrs = 1;
+            cudaLaunchKernelEx(&cfg, gemv_dot_kernel<1, GEMV_LOADS, true>, g, lwk, s.chunk);
+        } else {
+            // (rows of at most 64 columns keep fewer loads than registers would be held for: 10^6 x 2
+            // 122 -> 80 us, 200000 x 16 27.8 -> 18.8)
+            auto kern = s.rows_per_warp == 4   ? g.cols <= 64 ? gemv_dot_kernel<4, 1> : gemv_dot_kernel<4>
+                        : s.rows_per_warp == 2 ? gemv_dot_kernel<2>
+                                               : gemv_dot_kernel<1>;
+            kern<<<grid, GEMV_THREADS, 0, st>>>(g, lwk, s.chunk);
+        }
     } else {
         auto kern = s.wk == 1   ? partial ? gemv_axpy_partial_kernel<1, false> : gemv_axpy_partial_kernel<1, true>
                     : s.wk == 2 ? partial ? gemv_axpy_partial_kernel<2, false> : gemv_axpy_partial_kernel<2, true>

@@ -566,3 +566,34 @@ def test_captured_split_products_among_others(oracle):
             assert torch.equal(result(i), first[i]), step
     finally:
         ctx.close()
+
+
+@pytest.mark.parametrize("m,k", [(1, 100001), (7, 40000), (100, 16384), (443, 9000), (33, 4097)])
+def test_few_long_rows_captured_by_a_new_context(oracle, m, k):
+    """A matrix-vector product of few rows, whose columns are split over the
+    CTAs of a cluster, takes no device memory: the first call of a context can
+    be captured.  The replay and an eager call give the same bits."""
+    import jlc_b200
+    import torch
+    ctx, st = jlc_b200.Context(0), torch.cuda.Stream()
+    try:
+        ctx.set_stream(st.cuda_stream)
+        A, B, C = oracle.uniform((m, k), 91), oracle.uniform((k, 1), 92), oracle.uniform((m, 1), 93)
+        dA, dB = torch.from_numpy(A).cuda(), torch.from_numpy(B).cuda()
+        dC = [torch.from_numpy(C.copy()).cuda() for _ in range(2)]
+
+        def product(c):
+            ctx.dgemm_device(0, 0, m, 1, k, 1.5, dA.data_ptr(), k, dB.data_ptr(), 1, 0.5, c.data_ptr(), 1, report=False)
+
+        torch.cuda.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=st):
+            product(dC[0])
+        with torch.cuda.stream(st):
+            graph.replay()
+        product(dC[1])
+        ctx.synchronize()
+        assert torch.equal(dC[0], dC[1])
+        assert_fp64_bound(f"gemv {m}x{k}", dC[0].cpu().numpy(), A, B, C, 1.5, 0.5)
+    finally:
+        ctx.close()
