@@ -167,11 +167,11 @@ JLC_API int jlc_dgemm_ozaki_crt_device(jlc_ctx* ctx, int layout_a, int layout_b,
  * GemmDispatch.java:118-149, picks CPU blocking; this picks how many k parts
  * a product's tiles are split into).  jlc_autotune_splitk times every legal
  * factor (1..8, at least 256 k per part, at most 8 waves of work) for the
- * class of an m x n x k product -- its tile count and k to a power of two --
+ * class of an m x n x k product -- m and n in units of 32, k to a power of two --
  * on this context's device, stores the fastest in the tuning cache
  * ($JLCGPU_TUNE_CACHE, default ~/.cache/jlcgpu/grouped_tune.txt, shared with
  * the grouped tuner) and returns it; later products of the class use it (the
- * wave-balance rule otherwise).  jlc_splitk_choice reports the factor a
+ * cheapest by the kernel's cost rule otherwise).  jlc_splitk_choice reports the factor a
  * product would use now.  A different factor sums k in different groups:
  * results stay inside the FP64 bound but may change in the last bits. */
 JLC_API int jlc_autotune_splitk(jlc_ctx* ctx, int64_t m, int64_t n, int64_t k, int* split);

@@ -853,8 +853,6 @@ int jlc_autotune_splitk(jlc_ctx* ctx, int64_t m, int64_t n, int64_t k, int* spli
     if (!ctx || !split || m < 2 || n < 2 || k < 1 || m > (1 << 20) || n > (1 << 20) || k > (1 << 20))
         return set_err(ctx, JLC_E_ARG, "autotune_splitk: bad arguments");
     cudaSetDevice(ctx->device);
-    const long long bm = dmma_bm(m);
-    const long long tiles = ((m + bm - 1) / bm) * ((n + 127) / 128), kbl = (k + 15) / 16;
     const long long lda = round_up(k, 8), ldb = round_up(n, 8), ldc = n;
     int rc = reserve(ctx, ctx->bufA, (size_t)(m * lda) * 8, "autotune A");
     if (!rc) rc = reserve(ctx, ctx->bufB, (size_t)(k * ldb) * 8, "autotune B");
@@ -868,7 +866,7 @@ int jlc_autotune_splitk(jlc_ctx* ctx, int64_t m, int64_t n, int64_t k, int* spli
     int best = 1;
     float best_ms = 0.f;
     for (int s = 1; s <= 8; ++s) {
-        if (!dmma_splitk_legal(tiles, kbl, s, ctx->sm_count)) continue;
+        if (!dmma_splitk_legal(m, n, k, s, ctx->sm_count)) continue;
         const size_t wsb = dmma_splitk_bytes(m, n, k, s, ctx->sm_count);
         if (wsb && (rc = ws_reserve(ctx, wsb))) return rc;
         float ms_min = 0.f;
@@ -893,7 +891,7 @@ int jlc_autotune_splitk(jlc_ctx* ctx, int64_t m, int64_t n, int64_t k, int* spli
     }
     rc = finish_sync(ctx);
     if (rc) return rc;
-    const std::string cls = dmma_splitk_class(ctx->sm_count, tiles, kbl);
+    const std::string cls = dmma_splitk_class(ctx->sm_count, m, n, k);
     grp::tune_store(cls, best);
     dmma_splitk_remember(cls, best);
     *split = best;

@@ -441,7 +441,7 @@ static int launch_variant(const CUtensorMap& ma, const CUtensorMap& mb, const Pa
 }  // namespace dmma
 
 // tile height of the split-K classes: 32 or 64 rows for thin products, else 128
-int dmma_bm(long long m) { return m <= 32 ? 32 : (m <= 64 ? 64 : 128); }
+static int dmma_bm(long long m) { return m <= 32 ? 32 : (m <= 64 ? 64 : 128); }
 
 namespace {
 struct Tile {
@@ -535,19 +535,29 @@ bool dmma_operand_ok(const void* ptr, long long ld) {
     return (reinterpret_cast<uintptr_t>(ptr) % 16 == 0) && ((ld * 8) % 16 == 0) && ld > 0;
 }
 
+// Tiles of the split-K classes' height and 128 columns, and k-blocks
+static long long class_tiles(long long m, long long n) {
+    const long long bm = dmma_bm(m);
+    return ((m + bm - 1) / bm) * ((n + 127) / 128);
+}
+static long long k_blocks(long long k) { return (k + dmma::BK - 1) / dmma::BK; }
+
 // Split factors a product may use: at least 16 k-blocks (256 k) per part and
 // at most 8 waves of work units over the persistent grid.
-bool dmma_splitk_legal(long long tiles, long long kbl, int s, int sm_count) {
-    return s == 1 || (s >= 2 && s <= 8 && kbl / s >= 16 && tiles * s <= 8LL * sm_count);
+bool dmma_splitk_legal(long long m, long long n, long long k, int s, int sm_count) {
+    return s == 1 || (s >= 2 && s <= 8 && k_blocks(k) / s >= 16 && class_tiles(m, n) * s <= 8LL * sm_count);
 }
 
-// Shape class of the split-K tuner: the exact tile count (what the wave
-// balance depends on) and the k-block count to a power of two.
-std::string dmma_splitk_class(int sm_count, long long tiles, long long kbl) {
+// Shape class of the split-K tuner: m and n in units of 32, which fix the number
+// of tiles of every shape the kernel may take (what the wave balance depends
+// on), and the k-block count to a power of two.  Entries without those units
+// are of kernels whose tiles were 128 columns wide: no key matches them.
+std::string dmma_splitk_class(int sm_count, long long m, long long n, long long k) {
     int lg = 0;
-    while ((2LL << lg) <= kbl) ++lg;
+    while ((2LL << lg) <= k_blocks(k)) ++lg;
     return "sm" + std::to_string(sm_count) + "|v" + std::to_string(JLCGPU_VERSION) + "|dmma-splitk|t" +
-           std::to_string(tiles) + "|kb" + std::to_string(lg);
+           std::to_string(class_tiles(m, n)) + "|kb" + std::to_string(lg) + "|r" + std::to_string((m + 31) / 32) + "x" +
+           std::to_string((n + 31) / 32);
 }
 
 namespace {
@@ -561,8 +571,8 @@ void dmma_splitk_remember(const std::string& cls, int s) {
     g_split_table[cls] = s;
 }
 
-int dmma_splitk_tuned(int sm_count, long long tiles, long long kbl) {
-    const std::string cls = dmma_splitk_class(sm_count, tiles, kbl);
+static int dmma_splitk_tuned(int sm_count, long long m, long long n, long long k) {
+    const std::string cls = dmma_splitk_class(sm_count, m, n, k);
     std::lock_guard<std::mutex> lock(g_split_mu);
     auto it = g_split_table.find(cls);
     if (it == g_split_table.end()) it = g_split_table.emplace(cls, grp::tune_lookup(cls)).first;
@@ -570,20 +580,16 @@ int dmma_splitk_tuned(int sm_count, long long tiles, long long kbl) {
 }
 
 // k parts per tile for an m x n x k product (1: no split): the tuner's choice
-// for the shape class when one is cached, else the wave-balance rule.  A row
+// for the shape class when one is cached, else the cheapest by tile_cost.  A row
 // block of a pipelined product passes the whole product's m, so that every
 // block sums in the same order as the single-shot call.
 int dmma_splitk(long long m, long long n, long long k, int sm_count) {
-    using namespace dmma;
-    const long long bm = dmma_bm(m);
-    const long long tiles = ((m + bm - 1) / bm) * ((n + 127) / 128);
-    const long long kbl = (k + BK - 1) / BK;
-    const int tuned = dmma_splitk_tuned(sm_count, tiles, kbl);
-    if (tuned > 0 && dmma_splitk_legal(tiles, kbl, tuned, sm_count)) return tuned;
+    const int tuned = dmma_splitk_tuned(sm_count, m, n, k);
+    if (tuned > 0 && dmma_splitk_legal(m, n, k, tuned, sm_count)) return tuned;
     int best = 1;
     double cost = 0.0;
     for (int s = 1; s <= 8; ++s) {
-        if (!dmma_splitk_legal(tiles, kbl, s, sm_count)) break;
+        if (!dmma_splitk_legal(m, n, k, s, sm_count)) break;
         const double c = tile_cost(dmma_tile(m, n, k, s, sm_count), m, n, k, s, sm_count);
         if (s == 1 || c < cost) {
             best = s;

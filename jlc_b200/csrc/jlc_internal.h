@@ -58,8 +58,6 @@ struct RepackDesc {
     long long ld_dst = 0, rows = 0, cols = 0;
 };
 int launch_repack(const RepackDesc& d0, const RepackDesc& d1, const int* gate, cudaStream_t st);
-// tile height of an m-row product's split-K class (32, 64 or 128)
-int dmma_bm(long long m);
 // number of CTAs the Ozaki GEMM kernel launches for this shape
 int ozaki_grid(long long m, long long n, int sm_count);
 
@@ -131,11 +129,10 @@ int launch_dgemm_dmma(const GemmDesc& g, cudaStream_t st, int sm_count, int* sta
                       char* err, size_t errlen, int ksplit = 1, void* splitk_ws = nullptr,
                       size_t splitk_ws_bytes = 0, SplitCounters split_counters = {});
 int dmma_splitk(long long m, long long n, long long k, int sm_count);
-// split-K tuning (dgemm_dmma.cu): legal factors, the shape class, and the
-// tuned factor of a class (0: none cached); remember() records a new choice
-bool dmma_splitk_legal(long long tiles, long long kbl, int s, int sm_count);
-std::string dmma_splitk_class(int sm_count, long long tiles, long long kbl);
-int dmma_splitk_tuned(int sm_count, long long tiles, long long kbl);
+// split-K tuning (dgemm_dmma.cu): legal factors and the shape class;
+// remember() records a tuned factor
+bool dmma_splitk_legal(long long m, long long n, long long k, int s, int sm_count);
+std::string dmma_splitk_class(int sm_count, long long m, long long n, long long k);
 void dmma_splitk_remember(const std::string& cls, int s);
 // the tuning cache file shared by the tuners ($JLCGPU_TUNE_CACHE)
 namespace grp {

@@ -597,3 +597,18 @@ def test_few_long_rows_captured_by_a_new_context(oracle, m, k):
         assert_fp64_bound(f"gemv {m}x{k}", dC[0].cpu().numpy(), A, B, C, 1.5, 0.5)
     finally:
         ctx.close()
+
+
+def test_tuned_splits_are_those_of_the_shape(ctx, tmp_path, monkeypatch):
+    """65 x 300 and 128 x 384 products have as many 128-column tiles, but the
+    kernel cuts them into different numbers of smaller ones: an entry tuned for
+    one is not the other's.  An entry that names 128-column tiles alone, as an
+    earlier kernel stored it, is nobody's."""
+    cache = tmp_path / "tune.txt"
+    monkeypatch.setenv("JLCGPU_TUNE_CACHE", str(cache))
+    ctx.autotune_splitk(96, 100, 1024)
+    prefix = cache.read_text().split("dmma-splitk")[0] + "dmma-splitk"
+    cache.write_text(f"{prefix}|t3|kb8 5\n{prefix}|t3|kb8|r4x12 5\n")
+    assert ctx.splitk_choice(128, 384, 4096) == 5
+    assert ctx.splitk_choice(65, 300, 4096) != 5
+    assert ctx.splitk_choice(100, 300, 4096) != 5   # r4x10
