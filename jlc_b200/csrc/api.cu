@@ -227,8 +227,8 @@ int run_device(jlc_ctx* ctx, const GemmDesc& g0, int precision, int slices, jlc_
     // Small products split k across CTAs, partials in the workspace (after
     // the Ozaki split data when the FP64 kernel is the gated fallback, so
     // that its split choice, and with it its sums, match the native route).
-    const int ksplit = g.dot_mat ? 1 : dmma_splitk(whole_m, g.n, g.k, ctx->sm_count);
-    const size_t splitk_bytes = dmma_splitk_bytes(g.m, g.n, g.k, ksplit, ctx->sm_count);
+    const int ksplit = g.dot_mat ? 1 : dmma_splitk(whole_m, g.n, g.k, ctx->sm_count, ctx->dmma_k);
+    const size_t splitk_bytes = dmma_splitk_bytes(g.m, whole_m, g.n, g.k, ksplit, ctx->sm_count, ctx->dmma_k);
     size_t splitk_off = 0;
     int rc = JLC_OK;
     if (ozaki) {
@@ -845,7 +845,7 @@ int jlc_set_wait_limit(jlc_ctx* ctx, double seconds) {
 
 int jlc_splitk_choice(jlc_ctx* ctx, int64_t m, int64_t n, int64_t k, int* split) {
     if (!ctx || !split || m < 1 || n < 1 || k < 1) return set_err(ctx, JLC_E_ARG, "splitk_choice: bad arguments");
-    *split = dmma_splitk(m, n, k, ctx->sm_count);
+    *split = dmma_splitk(m, n, k, ctx->sm_count, ctx->dmma_k);
     return JLC_OK;
 }
 
@@ -867,7 +867,7 @@ int jlc_autotune_splitk(jlc_ctx* ctx, int64_t m, int64_t n, int64_t k, int* spli
     float best_ms = 0.f;
     for (int s = 1; s <= 8; ++s) {
         if (!dmma_splitk_legal(m, n, k, s, ctx->sm_count)) continue;
-        const size_t wsb = dmma_splitk_bytes(m, n, k, s, ctx->sm_count);
+        const size_t wsb = dmma_splitk_bytes(m, m, n, k, s, ctx->sm_count, ctx->dmma_k);
         if (wsb && (rc = ws_reserve(ctx, wsb))) return rc;
         float ms_min = 0.f;
         for (int rep = 0; rep < 4; ++rep) {  // one warm-up, three timed
@@ -891,7 +891,7 @@ int jlc_autotune_splitk(jlc_ctx* ctx, int64_t m, int64_t n, int64_t k, int* spli
     }
     rc = finish_sync(ctx);
     if (rc) return rc;
-    const std::string cls = dmma_splitk_class(ctx->sm_count, m, n, k);
+    const std::string cls = dmma_splitk_class(ctx->sm_count, m, n, k, ctx->dmma_k);
     grp::tune_store(cls, best);
     dmma_splitk_remember(cls, best);
     *split = best;

@@ -30,7 +30,9 @@
 // number of the launch that it counts for: arrivals that an abandoned launch
 // left behind are older and count for nothing.
 // The tile shape does not enter the sums: an element is the same chain of MMAs
-// over k in every shape, so only the split decides a result's bits.
+// over k in every shape, so only the split decides a result's bits.  (With a k
+// step other than 8, which the 128 x 128 tile alone is built for, products of
+// more than 64 rows run on that tile; the whole product's rows decide.)
 //
 // K permutation: inside each k-step the logical k index of the mma fragment
 // layout is remapped to a physical column of the shared tile so that the four
@@ -469,8 +471,9 @@ double tile_cost(const Tile& t, long long m, long long n, long long k, int s, in
     return waves * unit + (s > 1 ? 4000.0 : 0.0);
 }
 
-// the tile for an m x n x k product whose k is cut into s parts
-Tile dmma_tile(long long m, long long n, long long k, int s, int sm_count) {
+// the tile for an m x n x k product, rows of one of whole_m rows, whose k is cut into s parts
+Tile dmma_tile(long long m, long long whole_m, long long n, long long k, int s, int sm_count, int mma_k) {
+    if (mma_k != 8) return {dmma_bm(whole_m), 128};
     Tile best = kTiles[0];
     double cost = tile_cost(best, m, n, k, s, sm_count);
     for (const Tile& t : kTiles) {
@@ -552,12 +555,12 @@ bool dmma_splitk_legal(long long m, long long n, long long k, int s, int sm_coun
 // of tiles of every shape the kernel may take (what the wave balance depends
 // on), and the k-block count to a power of two.  Entries without those units
 // are of kernels whose tiles were 128 columns wide: no key matches them.
-std::string dmma_splitk_class(int sm_count, long long m, long long n, long long k) {
+std::string dmma_splitk_class(int sm_count, long long m, long long n, long long k, int mma_k) {
     int lg = 0;
     while ((2LL << lg) <= k_blocks(k)) ++lg;
     return "sm" + std::to_string(sm_count) + "|v" + std::to_string(JLCGPU_VERSION) + "|dmma-splitk|t" +
            std::to_string(class_tiles(m, n)) + "|kb" + std::to_string(lg) + "|r" + std::to_string((m + 31) / 32) + "x" +
-           std::to_string((n + 31) / 32);
+           std::to_string((n + 31) / 32) + (mma_k == 8 ? "" : "|mk" + std::to_string(mma_k));
 }
 
 namespace {
@@ -571,8 +574,8 @@ void dmma_splitk_remember(const std::string& cls, int s) {
     g_split_table[cls] = s;
 }
 
-static int dmma_splitk_tuned(int sm_count, long long m, long long n, long long k) {
-    const std::string cls = dmma_splitk_class(sm_count, m, n, k);
+static int dmma_splitk_tuned(int sm_count, long long m, long long n, long long k, int mma_k) {
+    const std::string cls = dmma_splitk_class(sm_count, m, n, k, mma_k);
     std::lock_guard<std::mutex> lock(g_split_mu);
     auto it = g_split_table.find(cls);
     if (it == g_split_table.end()) it = g_split_table.emplace(cls, grp::tune_lookup(cls)).first;
@@ -583,14 +586,14 @@ static int dmma_splitk_tuned(int sm_count, long long m, long long n, long long k
 // for the shape class when one is cached, else the cheapest by tile_cost.  A row
 // block of a pipelined product passes the whole product's m, so that every
 // block sums in the same order as the single-shot call.
-int dmma_splitk(long long m, long long n, long long k, int sm_count) {
-    const int tuned = dmma_splitk_tuned(sm_count, m, n, k);
+int dmma_splitk(long long m, long long n, long long k, int sm_count, int mma_k) {
+    const int tuned = dmma_splitk_tuned(sm_count, m, n, k, mma_k);
     if (tuned > 0 && dmma_splitk_legal(m, n, k, tuned, sm_count)) return tuned;
     int best = 1;
     double cost = 0.0;
     for (int s = 1; s <= 8; ++s) {
         if (!dmma_splitk_legal(m, n, k, s, sm_count)) break;
-        const double c = tile_cost(dmma_tile(m, n, k, s, sm_count), m, n, k, s, sm_count);
+        const double c = tile_cost(dmma_tile(m, m, n, k, s, sm_count, mma_k), m, n, k, s, sm_count);
         if (s == 1 || c < cost) {
             best = s;
             cost = c;
@@ -599,9 +602,9 @@ int dmma_splitk(long long m, long long n, long long k, int sm_count) {
     return best;
 }
 
-size_t dmma_splitk_bytes(long long m, long long n, long long k, int ksplit, int sm_count) {
+size_t dmma_splitk_bytes(long long m, long long whole_m, long long n, long long k, int ksplit, int sm_count, int mma_k) {
     if (ksplit < 2) return 0;
-    const Tile t = dmma_tile(m, n, k, ksplit, sm_count);
+    const Tile t = dmma_tile(m, whole_m, n, k, ksplit, sm_count, mma_k);
     const long long tiles = ((m + t.bm - 1) / t.bm) * ((n + t.bn - 1) / t.bn);
     return (size_t)(tiles * ksplit) * t.bm * t.bn * sizeof(double);
 }
@@ -620,8 +623,9 @@ int launch_dgemm_dmma(const GemmDesc& g, cudaStream_t st, int sm_count, int* sta
     // unit per tile (its per-CTA partial dots must not depend on arrival order)
     const int kbl = (int)((g.k + BK - 1) / BK);
     int split = ksplit > 1 && splitk_ws && split_counters.word && !g.dot_mat ? (ksplit < kbl ? ksplit : kbl) : 1;
-    if (split > 1 && dmma_splitk_bytes(g.m, g.n, g.k, split, sm_count) > splitk_ws_bytes) split = 1;
-    const Tile tile = dmma_tile(g.m, g.n, g.k, split, sm_count);
+    const long long whole_m = g.ws_m > g.m ? g.ws_m : g.m;
+    if (split > 1 && dmma_splitk_bytes(g.m, whole_m, g.n, g.k, split, sm_count, mma_k) > splitk_ws_bytes) split = 1;
+    const Tile tile = dmma_tile(g.m, whole_m, g.n, g.k, split, sm_count, mma_k);
     const int bm = tile.bm, bn = tile.bn;
     CUtensorMap ma, mb;
     int rc;

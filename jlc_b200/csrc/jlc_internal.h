@@ -82,7 +82,7 @@ bool dmma_operand_ok(const void* ptr, long long ld);
 // dimensions.  gate != nullptr: the kernel only runs if one of the Ozaki
 // call's flags gate[kFlagNonfiniteA], gate[kFlagFallback],
 // gate[kFlagNonfiniteB] is set.
-// ksplit > 1 with split_counters and splitk_ws of at least dmma_splitk_bytes(m, n, k, ksplit, sm_count):
+// ksplit > 1 with split_counters and splitk_ws of at least dmma_splitk_bytes():
 // split-K over ksplit parts; otherwise every tile is one work unit.
 // blocked Householder QR kernels (qr.cu)
 size_t qr_panel_mp_scratch_bytes(int P);
@@ -128,18 +128,19 @@ struct SplitCounters {
 int launch_dgemm_dmma(const GemmDesc& g, cudaStream_t st, int sm_count, int* status, const int* gate, int mma_k,
                       char* err, size_t errlen, int ksplit = 1, void* splitk_ws = nullptr,
                       size_t splitk_ws_bytes = 0, SplitCounters split_counters = {});
-int dmma_splitk(long long m, long long n, long long k, int sm_count);
+// (mma_k: the k step of the MMAs, 8 unless the context is set otherwise)
+int dmma_splitk(long long m, long long n, long long k, int sm_count, int mma_k);
 // split-K tuning (dgemm_dmma.cu): legal factors and the shape class;
 // remember() records a tuned factor
 bool dmma_splitk_legal(long long m, long long n, long long k, int s, int sm_count);
-std::string dmma_splitk_class(int sm_count, long long m, long long n, long long k);
+std::string dmma_splitk_class(int sm_count, long long m, long long n, long long k, int mma_k);
 void dmma_splitk_remember(const std::string& cls, int s);
 // the tuning cache file shared by the tuners ($JLCGPU_TUNE_CACHE)
 namespace grp {
 int tune_lookup(const std::string& key);
 void tune_store(const std::string& key, int value);
 }  // namespace grp
-size_t dmma_splitk_bytes(long long m, long long n, long long k, int ksplit, int sm_count);
+size_t dmma_splitk_bytes(long long m, long long whole_m, long long n, long long k, int ksplit, int sm_count, int mma_k);
 
 // y[i*incy] = alpha * sum_p M(i,p) x[p*incx] + beta * y[i*incy], M(i,p) = mat[i*rs + p*cs]
 // with rs == 1 or cs == 1.  scratch: partial sums where the columns are split over CTAs.

@@ -612,3 +612,28 @@ def test_tuned_splits_are_those_of_the_shape(ctx, tmp_path, monkeypatch):
     assert ctx.splitk_choice(128, 384, 4096) == 5
     assert ctx.splitk_choice(65, 300, 4096) != 5
     assert ctx.splitk_choice(100, 300, 4096) != 5   # r4x10
+
+
+@pytest.mark.parametrize("k_step", [4, 16])
+@pytest.mark.parametrize("m,n,k", [(2048, 1024, 512), (1064, 1024, 512), (1536, 1100, 300)])
+def test_k_step_setting_in_row_blocks(oracle, monkeypatch, k_step, m, n, k):
+    """JLCGPU_DMMA_K: the row blocks of a pipelined host product, the last one
+    of 40 rows too, sum in the same steps of k as the device entry's product."""
+    import jlc_b200
+    import torch
+    monkeypatch.setenv("JLCGPU_DMMA_K", str(k_step))
+    ctx = jlc_b200.Context(0)
+    monkeypatch.delenv("JLCGPU_DMMA_K")
+    try:
+        A, B = oracle.uniform((m, k), 95), oracle.uniform((k, n), 96)
+        dA, dB = torch.from_numpy(A).cuda(), torch.from_numpy(B).cuda()
+        dC = torch.zeros((m, n), dtype=torch.float64, device="cuda")
+        torch.cuda.synchronize()
+        ctx.dgemm_device(0, 0, m, n, k, 1.0, dA.data_ptr(), k, dB.data_ptr(), n, 0.0, dC.data_ptr(), n, report=False)
+        ctx.synchronize()
+        host = np.zeros((m, n))
+        ctx.dgemm(0, 0, m, n, k, 1.0, A, k, B, n, 0.0, host, n, precision=0)
+        np.testing.assert_array_equal(host, dC.cpu().numpy())
+        assert_fp64_bound(f"k step {k_step}", host, A, B, None, 1.0, 0.0)
+    finally:
+        ctx.close()
