@@ -64,14 +64,17 @@ int ws_reserve(jlc_ctx* ctx, size_t bytes) {
     return workspace_reserve(ctx->ws, bytes, ctx->err, sizeof(ctx->err));
 }
 
+bool capturing(jlc_ctx* ctx) {
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    return cudaStreamIsCapturing(ctx->stream, &cs) == cudaSuccess && cs == cudaStreamCaptureStatusActive;
+}
+
 // The counters of a split product about to be launched.  Each launch has a number
 // of its own, so that nothing an earlier one left in them matters, whichever
 // stream it ran on and however it ended.  A captured launch keeps its number
 // from replay to replay: its counters are cleared in the graph.
 SplitCounters split_counters(jlc_ctx* ctx) {
-    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(ctx->stream, &cs) == cudaSuccess && cs == cudaStreamCaptureStatusActive)
-        cudaMemsetAsync(ctx->d_counters, 0, kSplitTiles * sizeof(*ctx->d_counters), ctx->stream);
+    if (capturing(ctx)) cudaMemsetAsync(ctx->d_counters, 0, kSplitTiles * sizeof(*ctx->d_counters), ctx->stream);
     return {ctx->d_counters, ++ctx->split_launches << kSplitShift};
 }
 
@@ -227,8 +230,8 @@ int run_device(jlc_ctx* ctx, const GemmDesc& g0, int precision, int slices, jlc_
     // Small products split k across CTAs, partials in the workspace (after
     // the Ozaki split data when the FP64 kernel is the gated fallback, so
     // that its split choice, and with it its sums, match the native route).
-    const int ksplit = g.dot_mat ? 1 : dmma_splitk(whole_m, g.n, g.k, ctx->sm_count, ctx->dmma_k);
-    const size_t splitk_bytes = dmma_splitk_bytes(g.m, whole_m, g.n, g.k, ksplit, ctx->sm_count, ctx->dmma_k);
+    int ksplit = g.dot_mat ? 1 : dmma_splitk(whole_m, g.n, g.k, ctx->sm_count, ctx->dmma_k);
+    size_t splitk_bytes = dmma_splitk_bytes(g.m, whole_m, g.n, g.k, ksplit, ctx->sm_count, ctx->dmma_k);
     size_t splitk_off = 0;
     int rc = JLC_OK;
     if (ozaki) {
@@ -315,8 +318,13 @@ int run_device(jlc_ctx* ctx, const GemmDesc& g0, int precision, int slices, jlc_
     if (!ozaki && rep) rep->kernel = JLC_KERNEL_DMMA;
     if (!ozaki && fault_hit(ctx, JLC_FAULT_WAIT)) g.withhold_stage = true;
     if (!ozaki && splitk_bytes > 0) {
-        rc = ws_reserve(ctx, splitk_bytes);
-        if (rc) return rc;
+        // Without room for the partials -- a capture cannot allocate -- the product runs unsplit.
+        const bool grow = splitk_bytes > ctx->ws.bytes;
+        if ((grow && capturing(ctx)) || ws_reserve(ctx, splitk_bytes) != JLC_OK) {
+            ctx->err[0] = 0;
+            ksplit = 1;
+            splitk_bytes = 0;
+        }
     }
     // After an Ozaki launch the FP64 kernel is gated on the split's
     // non-finite flag: it only runs when Inf/NaN made slicing impossible.

@@ -637,3 +637,39 @@ def test_k_step_setting_in_row_blocks(oracle, monkeypatch, k_step, m, n, k):
         assert_fp64_bound(f"k step {k_step}", host, A, B, None, 1.0, 0.0)
     finally:
         ctx.close()
+
+
+@pytest.mark.parametrize("m,n,k", [(301, 6144, 1614), (256, 256, 4096)])
+def test_split_product_without_a_workspace(oracle, m, n, k):
+    """A product that would be split along k runs unsplit where the partial
+    sums find no room: as the first call of a context, captured into a graph,
+    and where the allocation fails."""
+    import jlc_b200
+    import torch
+    ctx, st = jlc_b200.Context(0), torch.cuda.Stream()
+    try:
+        ctx.set_stream(st.cuda_stream)
+        assert ctx.splitk_choice(m, n, k) > 1
+        A, B = oracle.uniform((m, k), 97), oracle.uniform((k, n), 98)
+        dA, dB = torch.from_numpy(A).cuda(), torch.from_numpy(B).cuda()
+        dC = [torch.zeros((m, n), dtype=torch.float64, device="cuda") for _ in range(3)]
+
+        def product(c):
+            ctx.dgemm_device(0, 0, m, n, k, 1.0, dA.data_ptr(), k, dB.data_ptr(), n, 0.0, c.data_ptr(), n, report=False)
+
+        torch.cuda.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=st):
+            product(dC[0])
+        with torch.cuda.stream(st):
+            graph.replay()
+        ctx.inject_fault(1)   # the next allocation
+        product(dC[1])
+        product(dC[2])        # with a workspace: split
+        ctx.synchronize()
+        assert torch.equal(dC[0], dC[1])
+        rows, cols = oracle.sample_entries(m, n, 2000, 3)
+        for c in (dC[0], dC[2]):
+            assert_fp64_bound(f"{m}x{n}x{k}", c.cpu().numpy(), A, B, None, 1.0, 0.0, rows=rows, cols=cols)
+    finally:
+        ctx.close()
