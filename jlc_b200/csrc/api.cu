@@ -712,18 +712,23 @@ struct QrWork {
 };
 
 // Workspace for an m-row factor applied to `cols` columns, with V, T and V op(T)
-// of up to `panels` panels at a time, within 256 MB (one panel at least).
+// of up to `panels` panels at a time, within 256 MB (one panel at least, and no
+// more than the device has room for).
 int qr_work(jlc_ctx* ctx, long long m, long long cols, long long panels, QrWork& q) {
     q.ldv = round_up(m > 0 ? m : 1, 8);
     q.ldw = round_up(cols > 0 ? cols : 1, 8);
     const long long per = 2 * q.ldv * kQrPanel + kQrPanel * kQrPanel;  // doubles per panel
     const long long most = (256LL << 20) / (per * (long long)sizeof(double));
     q.batch = (int)(panels < 1 ? 1 : (most < 1 ? 1 : (panels < most ? panels : most)));
-    const size_t doubles = (size_t)(per * q.batch + kQrPanel * q.ldw);
     const size_t scratch = round_up(qr_panel_mp_scratch_bytes(ctx->sm_count > 0 ? ctx->sm_count : 1), 256);
     const size_t gram = qr_gram_scratch_bytes(ctx->sm_count);
-    int rc = reserve(ctx, ctx->bufQ, doubles * sizeof(double) + scratch + gram, "QR workspace");
-    if (rc) return rc;
+    for (int rc;; q.batch = (q.batch + 1) / 2) {
+        const size_t doubles = (size_t)(per * q.batch + kQrPanel * q.ldw);
+        rc = reserve(ctx, ctx->bufQ, doubles * sizeof(double) + scratch + gram, "QR workspace");
+        if (rc == JLC_OK) break;
+        if (rc != JLC_E_OOM || q.batch == 1) return rc;
+    }
+    ctx->err[0] = 0;
     if (ctx->qr_cluster_max == 0) ctx->qr_cluster_max = qr_panel_cluster_max();
     q.v = static_cast<double*>(ctx->bufQ.ptr);
     q.vt = q.v + q.ldv * kQrPanel * q.batch;

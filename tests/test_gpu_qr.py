@@ -306,3 +306,28 @@ def test_denormals_beside_normal_entries(ctx, oracle):
     at, tau = _factor(ctx, z)
     assert tau.cpu().numpy()[0] == 0.0
     np.testing.assert_array_equal(at.cpu().numpy().T, z)
+
+
+def test_q_with_little_room(ctx, oracle):
+    """Where the workspace for all panels finds no room, Q is formed in smaller
+    batches (the sums of V^T V may be cut differently: equal to rounding, a
+    small multiple of m u); a factorisation, one panel at a time, reports the
+    failure."""
+    from jlc_b200 import JlcError
+    import jlc_b200
+    c2 = jlc_b200.Context(0)
+    try:
+        m, n = 700, 500
+        a = oracle.uniform((m, n), 41)
+        at, tau = _factor(ctx, a)
+        q = _q(ctx, at, tau, m, n, m, n)
+        c2.inject_fault(1)   # the next allocation
+        assert np.abs(_q(c2, at, tau, m, n, m, n) - q).max() < 1e-14 * m
+        c3 = jlc_b200.Context(0)
+        c3.inject_fault(1)
+        with pytest.raises(JlcError) as exc:
+            _factor(c3, a)
+        assert exc.value.code == -3
+        c3.close()
+    finally:
+        c2.close()
