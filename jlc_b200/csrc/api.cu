@@ -1405,22 +1405,31 @@ int jlc_bidiag_device(jlc_ctx* ctx, int64_t m, int64_t n, double* a, int64_t lda
     cudaEventRecord(ctx->ev0, st);
     int rc = JLC_OK;
     if (m > 0 && n > 0) {
-        // workspace: tau of the column and row reflectors, the kernel's
-        // partials, and the row reflectors rearranged as a QR factor
+        // workspace: tau of the column and row reflectors, the kernel's slots,
+        // and a region for its copy of the rows (past shared memory), which the
+        // row reflectors rearranged as a QR factor take over.  Without room for
+        // the copy the reduction runs in place.
         const long long ldw = round_up(n, 8);
         const long long ldt = round_up(n, 8);
-        const size_t kdoubles = bidiag_work_doubles((int)m, (int)n, ctx->sm_count);
-        const size_t wdoubles = v ? (size_t)ldw * (size_t)n : 0;
-        if ((rc = reserve(ctx, ctx->bufH, (2 * (size_t)ldt + kdoubles + wdoubles) * sizeof(double),
-                          "bidiagonalisation workspace")))
-            return rc;
+        size_t sdoubles = 0;
+        const size_t kdoubles = bidiag_work_doubles((int)m, (int)n, ctx->sm_count, &sdoubles);
+        const size_t wdoubles = v ? (size_t)ldw * (size_t)n : 0, base = 2 * (size_t)ldt + kdoubles;
+        bool in_place = false;
+        rc = reserve(ctx, ctx->bufH, (base + (sdoubles > wdoubles ? sdoubles : wdoubles)) * sizeof(double),
+                     "bidiagonalisation workspace");
+        if (rc == JLC_E_OOM && sdoubles > 0) {
+            in_place = true;
+            rc = reserve(ctx, ctx->bufH, (base + wdoubles) * sizeof(double), "bidiagonalisation workspace");
+        }
+        if (rc) return rc;
+        ctx->err[0] = 0;
         double* tauq = static_cast<double*>(ctx->bufH.ptr);
         double* taup = tauq + ldt;
         double* kwork = taup + ldt;
         double* wr = kwork + kdoubles;
         {
             Phase ph(ctx, JLC_PHASE_BIDIAG);
-            rc = launch_bidiag(a, lda, (int)m, (int)n, d, e, tauq, taup, kwork, ctx->sm_count, ctx->d_status, st);
+            rc = launch_bidiag(a, lda, (int)m, (int)n, d, e, tauq, taup, kwork, in_place, ctx->sm_count, ctx->d_status, st);
             if (rc) return set_err(ctx, rc, "bidiagonalisation: launch failed");
             ctx->launches += 1;
         }

@@ -15,7 +15,10 @@
 // g % P (at most one CTA per SM), so that every CTA keeps rows in play as the
 // trailing matrix shrinks, and a CTA's rows -- its slab -- sit in shared
 // memory for the whole reduction (row-major, a thread per column) while they
-// fit, else in a global work array laid out the same way.
+// fit, else in a global work array laid out the same way; where the device has
+// no room for that array, they stay in the matrix (IN_PLACE: its columns are lda
+// apart, so a thread per column reads 32 bytes for 8: 4096 x 4096 747 ms, 168
+// with the array).
 //
 // A step needs two sums over all CTAs and no more, because everything else is
 // formed redundantly from their results:
@@ -133,7 +136,7 @@ __device__ __noinline__ Reflector reflector(int E, double S, double x0) {
     return h;
 }
 
-template <bool SMEM, int CB>
+template <bool SMEM, int CB, bool IN_PLACE = false>
 __global__ void __launch_bounds__(BT, 1) bidiag_kernel(const Args p) {
     extern __shared__ double dyn[];
     // (aligned for vector loads: the passes read 8 rows of each)
@@ -152,6 +155,10 @@ __global__ void __launch_bounds__(BT, 1) bidiag_kernel(const Args p) {
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int m = p.m, n = p.n, rows = p.rows, ld = p.ld;
     double* slab = SMEM ? dyn : p.slab + (size_t)cta * rows * ld;  // [local row][column]
+    const int live = (m - cta + P - 1) / P;                        // IN_PLACE: the matrix has no rows past these
+    auto at = [&](int l, int j) -> double& {
+        return IN_PLACE ? p.a[(long long)l * P + cta + j * p.lda] : slab[(size_t)l * ld + j];
+    };
     double* red = SMEM ? dyn + (size_t)rows * ld : dyn;            // [warp][local row]
     Slot* part = p.part + (size_t)cta * ld;
     // f(local row, global row, column) over the slab.  A matrix of few columns takes several rows at a
@@ -165,9 +172,10 @@ __global__ void __launch_bounds__(BT, 1) bidiag_kernel(const Args p) {
         }
     };
     // this CTA's rows into its slab (rows past m are zero)
-    over_slab([&](int l, int g, int j) {
-        slab[(size_t)l * ld + j] = g < m && j < n ? p.a[g + (long long)j * p.lda] : 0.0;
-    });
+    if constexpr (!IN_PLACE)
+        over_slab([&](int l, int g, int j) {
+            slab[(size_t)l * ld + j] = g < m && j < n ? p.a[g + (long long)j * p.lda] : 0.0;
+        });
     for (int l = tid; l < rows; l += BT) {
         s_v[l] = 0.0;
         s_x[l] = 0.0;
@@ -196,7 +204,7 @@ __global__ void __launch_bounds__(BT, 1) bidiag_kernel(const Args p) {
         for (int b = b0 + warp; b < rows / RC; b += WARPS) {
             if (b >= b0 + WARPS) s = row_sum(b, f);
             const int l = b * RC + (lane >> 2), g = l * P + cta;
-            const double v = s_v[l], t = fma(-v, wk, slab[(size_t)l * ld + kn]);
+            const double v = s_v[l], t = IN_PLACE && g >= m ? 0.0 : fma(-v, wk, at(l, kn));
             const bool in = g >= kn && g < m;
             const double x = in && tau != 0.0 ? tau * fma(hinv, fma(-v, wy, s), t) : 0.0;
             const double c = in ? t - x : 0.0;
@@ -265,7 +273,7 @@ __global__ void __launch_bounds__(BT, 1) bidiag_kernel(const Args p) {
                 }
             }
             const bool owner = gl == k;
-            double* krow = slab + (size_t)l0 * ld;
+            const int lk = l0;  // row k
             if (owner) {
                 ++l0;
                 gl += P;
@@ -303,7 +311,11 @@ __global__ void __launch_bounds__(BT, 1) bidiag_kernel(const Args p) {
                     for (int i = 0; i < CB; ++i) {
                         const int j = j0 + tid + i * BT;
                         const double yi = SMEM ? y[i] : u[i];
-                        if (j < n) {
+                        if (IN_PLACE && j < n) {
+#pragma unroll
+                            for (int r = 0; r < RC; ++r)
+                                if (b * RC + r < live) acc[r] = fma(at(b * RC + r, j), yi, acc[r]);
+                        } else if (j < n) {
                             const double* q = slab + (size_t)b * RC * ld + j;
 #pragma unroll
                             for (int r = 0; r < RC; ++r) acc[r] = fma(q[(size_t)r * ld], yi, acc[r]);
@@ -352,12 +364,12 @@ __global__ void __launch_bounds__(BT, 1) bidiag_kernel(const Args p) {
                     const int j = c0 + tid + i * BT;
                     const double rj = u[i];
                     u[i] = j == kn ? u0 : u0 != 0.0 ? rj * ir : 0.0;
-                    if (owner && j < n) krow[j] = u0 != 0.0 && j > kn ? u[i] : rj;
+                    if (owner && j < n) at(lk, j) = u0 != 0.0 && j > kn ? u[i] : rj;
                 }
             } else if (owner) {
                 for (int j = c0 + tid; j < n; j += BT) {
                     const double rj = slot_value(prow + j) - slot_value(p.w + j);
-                    krow[j] = u0 != 0.0 && j > kn ? rj * ir : rj;
+                    at(lk, j) = u0 != 0.0 && j > kn ? rj * ir : rj;
                 }
             }
         }
@@ -407,7 +419,8 @@ __global__ void __launch_bounds__(BT, 1) bidiag_kernel(const Args p) {
                         double* q = slab + (size_t)b * RC * ld + j;
                         double x[RC];
 #pragma unroll
-                        for (int r = 0; r < RC; ++r) x[r] = q[(size_t)r * ld];
+                        for (int r = 0; r < RC; ++r)
+                            x[r] = !IN_PLACE ? q[(size_t)r * ld] : b * RC + r < live ? at(b * RC + r, j) : 0.0;
 #pragma unroll
                         for (int r = 0; r < RC; ++r) {
                             x[r] = fma(-xr[r], u[i], fma(-vr[r], w[i], x[r]));
@@ -415,7 +428,8 @@ __global__ void __launch_bounds__(BT, 1) bidiag_kernel(const Args p) {
                         }
 #pragma unroll
                         for (int r = 0; r < RC; ++r)
-                            if (b * RC + r >= l0) q[(size_t)r * ld] = x[r];
+                            if (b * RC + r >= l0 && (!IN_PLACE || b * RC + r < live))
+                                (IN_PLACE ? at(b * RC + r, j) : q[(size_t)r * ld]) = x[r];
                     }
                 }
             }
@@ -424,7 +438,7 @@ __global__ void __launch_bounds__(BT, 1) bidiag_kernel(const Args p) {
                 const int j = j0 + tid + i * BT;
                 if (j < n) {
                     slot_put(part + j, s[i], kn + 1, 0);
-                    if (powner) slot_put(pnext + j, slab[(size_t)l0 * ld + j], kn + 1, 0);
+                    if (powner) slot_put(pnext + j, at(l0, j), kn + 1, 0);
                 }
             }
         }
@@ -506,7 +520,7 @@ __global__ void __launch_bounds__(BT, 1) bidiag_kernel(const Args p) {
             double v = 0.0;
             if (tau != 0.0 && g >= kn && g < m) {
                 v = g == kn ? 1.0 : (s_c[l] * pow2(-s_E)) * vinv;
-                if (g > kn) slab[(size_t)l * ld + kn] = v;
+                if (g > kn) at(l, kn) = v;
             }
             s_v[l] = v;
         }
@@ -524,7 +538,7 @@ __global__ void __launch_bounds__(BT, 1) bidiag_kernel(const Args p) {
         }
     }
     __syncthreads();
-    over_slab([&](int l, int g, int j) {
+    if constexpr (!IN_PLACE) over_slab([&](int l, int g, int j) {
         if (g < m && j < n) p.a[g + (long long)j * p.lda] = slab[(size_t)l * ld + j];
     });
 }
@@ -566,15 +580,17 @@ static bool slab_in_smem(int rows, int n, int ld) {
 // Slots of the exchange: part, cpair, pivot and w.
 static size_t bidiag_slots(int P, int ld) { return (size_t)P * ld + 2 * (size_t)P + 3 * (size_t)ld; }
 
-size_t bidiag_work_doubles(int m, int n, int sm_count) {
+// Work array: the slots, then (slab_doubles) the global slabs.
+size_t bidiag_work_doubles(int m, int n, int sm_count, size_t* slab_doubles) {
     using namespace bidiag;
     int rows = 0;
     const int P = bidiag_grid(m, n, sm_count, &rows), ld = (n + 3) / 4 * 4;
-    return 2 * bidiag_slots(P, ld) + (slab_in_smem(rows, n, ld) ? 0 : (size_t)P * rows * ld);
+    *slab_doubles = slab_in_smem(rows, n, ld) ? 0 : (size_t)P * rows * ld;
+    return 2 * bidiag_slots(P, ld);
 }
 
 int launch_bidiag(double* a, long long lda, int m, int n, double* d, double* e, double* tauq, double* taup,
-                  double* work, int sm_count, int* status, cudaStream_t st) {
+                  double* work, bool in_place, int sm_count, int* status, cudaStream_t st) {
     using namespace bidiag;
     Args p;
     int rows = 0;
@@ -596,10 +612,10 @@ int launch_bidiag(double* a, long long lda, int m, int n, double* d, double* e, 
     p.pivot = p.cpair + 2 * P;
     p.w = p.pivot + 2 * (size_t)p.ld;
     const bool smem = slab_in_smem(rows, n, p.ld);
-    p.slab = smem ? nullptr : work + 2 * slots;
+    p.slab = smem || in_place ? nullptr : work + 2 * slots;
     p.status = status;
     // (1400^2: 9.0 ms with 3 columns per thread, 11.4 with 4; up to 512 columns 1 gains nothing on 2)
-    const void* kern = !smem        ? (const void*)bidiag_kernel<false, 4>
+    const void* kern = !smem        ? in_place ? (const void*)bidiag_kernel<false, 4, true> : (const void*)bidiag_kernel<false, 4>
                        : n > 3 * BT ? (const void*)bidiag_kernel<true, 4>
                        : n > 2 * BT ? (const void*)bidiag_kernel<true, 3>
                                     : (const void*)bidiag_kernel<true, 2>;

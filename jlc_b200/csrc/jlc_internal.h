@@ -98,12 +98,13 @@ int launch_set_identity(double* q, long long ldq, long long m, long long cols, c
 // blocked Hessenberg reduction kernels (hess.cu)
 size_t hess_work_doubles(long long n);
 // Golub-Kahan bidiagonalisation (bidiag.cu): rows per CTA and CTA count (0:
-// too many rows), the kernel's workspace in doubles, the cooperative launch,
-// and the row reflectors rearranged as the columns of a QR factor.
+// too many rows), the kernel's workspace in doubles (and what it wants on top
+// for its rows, unless they stay in place), the cooperative launch, and the row
+// reflectors rearranged as the columns of a QR factor.
 int bidiag_grid(int m, int n, int sm_count, int* rows_per_cta);
-size_t bidiag_work_doubles(int m, int n, int sm_count);
+size_t bidiag_work_doubles(int m, int n, int sm_count, size_t* slab_doubles);
 int launch_bidiag(double* a, long long lda, int m, int n, double* d, double* e, double* tauq, double* taup,
-                  double* work, int sm_count, int* status, cudaStream_t st);
+                  double* work, bool in_place, int sm_count, int* status, cudaStream_t st);
 int launch_bidiag_right_factor(const double* a, long long lda, int n, double* w, long long ldw, cudaStream_t st);
 int launch_hess_clear(double* h, long long ldh, int n, cudaStream_t st);
 // the whole reduction in one launch, for matrices that fit in the chip's shared memory

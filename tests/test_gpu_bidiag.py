@@ -168,3 +168,27 @@ def test_factors_of_a_matrix_with_a_non_finite_entry(ctx, m, n, bad):
     assert torch.equal(v[0], eye[0]) and torch.equal(v[:, 0], eye[:, 0])
     assert float((v.T @ v - eye).abs().max()) < 1e-14 * n
     assert float((u.T @ u - torch.eye(m, dtype=torch.float64, device="cuda")).abs().max()) < 1e-14 * m
+
+
+@pytest.mark.parametrize("m,n", [(6000, 700), (2300, 2100), (20001, 301)])   # past shared memory
+def test_in_place_where_the_copy_finds_no_room(m, n):
+    """The reduction keeps its rows in a work array past shared memory.  Where
+    that cannot be allocated they stay in the matrix: the same bits."""
+    import jlc_b200
+    import torch
+    g = torch.Generator(device="cuda").manual_seed(m)
+    a = torch.rand(n, m + 2, dtype=torch.float64, device="cuda", generator=g) * 2 - 1
+    outs = []
+    for full in (False, True):
+        ctx = jlc_b200.Context(0)
+        f, d, e = a.clone(), torch.zeros(n, dtype=torch.float64).cuda(), torch.zeros(n, dtype=torch.float64).cuda()
+        v = torch.zeros(n, n, dtype=torch.float64, device="cuda")
+        torch.cuda.synchronize()
+        if full:
+            ctx.inject_fault(1)   # the next allocation
+        ctx.bidiag_device(m, n, f.data_ptr(), m + 2, d.data_ptr(), e.data_ptr(), None, m, v.data_ptr(), n)
+        outs.append((f, d, e, v))
+        ctx.close()
+    for x, y in zip(*outs):
+        assert torch.equal(x, y)
+    assert torch.equal(outs[0][0][:, m:], a[:, m:])   # the padding rows are untouched
