@@ -1184,8 +1184,10 @@ int jlc_qr_factor_device(jlc_ctx* ctx, int64_t m, int64_t n, double* a, int64_t 
             long long ctas = (m - k0) / 128;
             if (ctas > ctx->sm_count) ctas = ctx->sm_count;
             if (ctas < 1) ctas = 1;
+            const bool withhold =
+                qr_panel_waits((int)m, (int)k0, ctx->qr_cluster_max) && fault_hit(ctx, JLC_FAULT_WAIT);
             rc = launch_qr_panel(a, lda, (int)m, (int)k0, kb, tau, (int)ctas, ctx->qr_cluster_max, q.panel_scratch,
-                                 ctx->d_status, ctx->stream);
+                                 ctx->d_status, withhold, ctx->stream);
             if (rc) return set_err(ctx, rc, "QR: panel launch failed");
         }
         const long long trail = n - (k0 + kb);
@@ -1305,7 +1307,8 @@ int jlc_hessenberg_device(jlc_ctx* ctx, int64_t n, double* a, int64_t lda, doubl
         double* tau = static_cast<double*>(ctx->bufH.ptr);
         {
             Phase ph(ctx, JLC_PHASE_HESS_PANEL);
-            rc = launch_hess_slab(a, lda, (int)n, tau, tau + ldt, ctx->sm_count, ctx->d_status, st);
+            rc = launch_hess_slab(a, lda, (int)n, tau, tau + ldt, ctx->sm_count, ctx->d_status,
+                                  fault_hit(ctx, JLC_FAULT_WAIT), st);
             if (rc) return set_err(ctx, rc, "Hessenberg: launch failed");
             ctx->launches += 1;
         }
@@ -1429,7 +1432,8 @@ int jlc_bidiag_device(jlc_ctx* ctx, int64_t m, int64_t n, double* a, int64_t lda
         double* wr = kwork + kdoubles;
         {
             Phase ph(ctx, JLC_PHASE_BIDIAG);
-            rc = launch_bidiag(a, lda, (int)m, (int)n, d, e, tauq, taup, kwork, in_place, ctx->sm_count, ctx->d_status, st);
+            rc = launch_bidiag(a, lda, (int)m, (int)n, d, e, tauq, taup, kwork, in_place, ctx->sm_count, ctx->d_status,
+                               fault_hit(ctx, JLC_FAULT_WAIT), st);
             if (rc) return set_err(ctx, rc, "bidiagonalisation: launch failed");
             ctx->launches += 1;
         }

@@ -362,6 +362,7 @@ struct SlabArgs {
     Slot* w;          // [ld]
     int* status;
     double eps;
+    int withhold;     // test hook: CTA 0 leaves its first sum out, so the others' waits run out
 };
 
 struct SlabReflector {
@@ -439,7 +440,7 @@ __global__ void __launch_bounds__(SLT, 1) hess_slab_kernel(const SlabArgs p) {
             if (warp == SLW - 1) {
                 const double c = lane < rows && lane >= lf + owner ? s_c[lane] : 0.0;
                 const double q = warp_sum(c * c);
-                if (lane == 0) slot_put(sig + cta, q, kn, 0);
+                if (lane == 0 && !(p.withhold && cta == 0 && k == 0)) slot_put(sig + cta, q, kn, 0);
             }
         }
         // ---- H - v w^T - x v^T stored, and its dots with the column's tail
@@ -680,7 +681,7 @@ size_t hess_slab_work_doubles(int n, int sm_count) {
 // form, with the reflectors' tails below its subdiagonal and their scales in
 // tau (n - 2); a skipped reflector has tau 0 and leaves its column's tail.
 int launch_hess_slab(double* h, long long ldh, int n, double* tau, double* work, int sm_count, int* status,
-                     cudaStream_t st) {
+                     bool withhold, cudaStream_t st) {
     using namespace hess;
     SlabArgs a;
     a.h = h;
@@ -697,6 +698,7 @@ int launch_hess_slab(double* h, long long ldh, int n, double* tau, double* work,
     a.w = a.prow + 2 * (size_t)a.ld;
     a.status = status;
     a.eps = 1e-12;
+    a.withhold = withhold ? 1 : 0;
     // the fewest columns per thread, as empty ones cost a step their issue slots (n = 512: 3.9 us with 1
     // against 4.1 with 2; n = 1400: 5.5 with 3 against 6.0 with 4)
     const void* kern = n > 3 * SLT   ? (const void*)hess_slab_kernel<4>

@@ -88,7 +88,8 @@ bool dmma_operand_ok(const void* ptr, long long ld);
 size_t qr_panel_mp_scratch_bytes(int P);
 int qr_panel_cluster_max();
 int launch_qr_panel(double* a, long long lda, int m, int k0, int kb, double* tau, int P, int cluster_max,
-                    void* scratch, int* status, cudaStream_t st);
+                    void* scratch, int* status, bool withhold, cudaStream_t st);
+bool qr_panel_waits(int m, int k0, int cluster_max);  // whether launch_qr_panel takes the kernel that has the test hook
 // V, T and V op(T) of consecutive panels; gram holds qr_gram_scratch_bytes(sm_count)
 size_t qr_gram_scratch_bytes(int sm_count);
 int launch_qr_vt(const double* a, long long lda, int m, int kmax, int p0, int panels, int shift, const double* tau,
@@ -104,14 +105,14 @@ size_t hess_work_doubles(long long n);
 int bidiag_grid(int m, int n, int sm_count, int* rows_per_cta);
 size_t bidiag_work_doubles(int m, int n, int sm_count, size_t* slab_doubles);
 int launch_bidiag(double* a, long long lda, int m, int n, double* d, double* e, double* tauq, double* taup,
-                  double* work, bool in_place, int sm_count, int* status, cudaStream_t st);
+                  double* work, bool in_place, int sm_count, int* status, bool withhold, cudaStream_t st);
 int launch_bidiag_right_factor(const double* a, long long lda, int n, double* w, long long ldw, cudaStream_t st);
 int launch_hess_clear(double* h, long long ldh, int n, cudaStream_t st);
 // the whole reduction in one launch, for matrices that fit in the chip's shared memory
 bool hess_slab_fits(int n, int sm_count);
 size_t hess_slab_work_doubles(int n, int sm_count);
 int launch_hess_slab(double* h, long long ldh, int n, double* tau, double* work, int sm_count, int* status,
-                     cudaStream_t st);
+                     bool withhold, cudaStream_t st);
 // all reflectors of one panel in one cooperative launch (rows in slabs over
 // up to sm_count CTAs); scratch of hess_panel_scratch_bytes
 size_t hess_panel_scratch_bytes(int sm_count);

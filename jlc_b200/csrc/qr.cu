@@ -716,7 +716,7 @@ __device__ __forceinline__ int rg_live_pairs(int kk) { return 32 - min(16, max(0
 
 template <int NR>
 __global__ void __launch_bounds__(RG_THREADS, 1) qr_panel_rg_kernel(double* A, long long lda, int m, int k0, int kb,
-                                                                    double* tau, int* status) {
+                                                                    double* tau, int* status, int withhold) {
     __shared__ __align__(16) double part[2][RG_MAX][RG_PART];
     __shared__ __align__(16) double rrec[2][64];  // row k, by the dots' index
     __shared__ double s_x[2][NR * 32];            // the pivot column below the pivot, times 2^-e, by column parity
@@ -832,11 +832,18 @@ __global__ void __launch_bounds__(RG_THREADS, 1) qr_panel_rg_kernel(double* A, l
 #pragma unroll
             for (int r = 0; r < NR; ++r) q = fma(x[r], x[r], q);
             q = warp_sum(q);
-            if (lane < P) send2(cluster_addr(&part[par][cta][64], lane), q, (double)e_own, cluster_addr(&bar[par], lane));
+            // (withhold, a test hook: CTA 0 leaves the first column's scalars out, so the waits run out)
+            if (lane < P && !(withhold && cta == 0 && kk == 0))
+                send2(cluster_addr(&part[par][cta][64], lane), q, (double)e_own, cluster_addr(&bar[par], lane));
         }
         // ---- merge: lane q (and q + 16) takes CTA q's dots of columns 0, 1 (2, 3) of this warp
-        fail |= !wait_sent(&bar[par], (kk >> 1) & 1, status);
-        __syncwarp();
+        if (__any_sync(0xffffffffu, !wait_sent(&bar[par], (kk >> 1) & 1, status))) {
+            // Given up: the CTA leaves at the next barrier.  Nothing else of the step, least of all the arming
+            // below: this phase is still open, and a second arrival in it takes its count below zero, which
+            // ends the kernel with an error.
+            fail = true;
+            continue;
+        }
         const int q = lane & 15, h = lane >> 4;
         const double* pq = part[par][q < P ? q : 0];
         const double2 se = *reinterpret_cast<const double2*>(pq + 64);
@@ -870,7 +877,8 @@ __global__ void __launch_bounds__(RG_THREADS, 1) qr_panel_rg_kernel(double* A, l
             }
         }
         if (cta == 0 && tid == 0) tau[k] = hh.tau;
-        if (tid == 0) mbar_arrive_expect_tx(&bar[par], bytes(kk + 2));  // armed for column kk + 2
+        // armed for column kk + 2
+        if (tid == 0) mbar_arrive_expect_tx(&bar[par], bytes(kk + 2));
         // ---- update: f_t = tau (a_kt + dot v0s), columns right of the pivot (f = 0 elsewhere), rows from k
         // on (v = 0 above, but a NaN f would take those with it; with both guards the factorisation of
         // 2304 x 2048 takes 5.93 ms, 5.85 without)
@@ -912,7 +920,14 @@ __global__ void __launch_bounds__(RG_THREADS, 1) qr_panel_rg_kernel(double* A, l
             }
         }
     }
-    cluster.sync();  // no CTA leaves while another may still send to it
+    // No CTA leaves while another may still send to it.  What a CTA waited for has arrived; one that gave
+    // up lets its own sends land first (they take a microsecond).
+    if (__syncthreads_or(fail)) {
+        const uint64_t t0 = globaltimer_ns();
+        while (globaltimer_ns() - t0 < 100000) {
+        }
+    }
+    cluster.sync();
 #pragma unroll
     for (int j = 0; j < RG_COLS; ++j)
 #pragma unroll
@@ -1283,24 +1298,32 @@ int qr_panel_cluster_max() {
     return 1;
 }
 
+namespace qr {
+// one CTA per 64 rows, up to the largest cluster (measured against 128 rows per
+// CTA: 13.8 vs 14.2 ms at 2048^2, 32.6 vs 33.0 at 4096^2)
+static int panel_ctas(int m, int k0, int cluster_max) { return max(1, min((m - k0) / 64, min(cluster_max, CL_MAX))); }
+}  // namespace qr
+
+bool qr_panel_waits(int m, int k0, int cluster_max) {
+    const int cl = qr::panel_ctas(m, k0, cluster_max);
+    return (m - k0 + cl - 1) / cl <= 32 * qr::RG_MAX_NR;
+}
+
 // Factors columns k0 .. k0+kb-1 of the column-major m x n matrix A (rows from
 // the diagonal down), writing tau[k0 ..]; A's entries below the diagonal of
 // those columns become the reflectors' tails (v0 = 1 implied), the diagonal
 // the new R entries (computeHouseholder / applyHouseholderToColumn,
-// HouseholderQR.java:219-384).  One cluster of CTAs with >= 128 rows each (a
-// single CTA below 256 rows) when their slabs fit in shared memory, else a
-// cooperative grid of P CTAs.
+// HouseholderQR.java:219-384).  One cluster of CTAs with >= 64 rows each (a
+// single CTA below 128 rows) when their rows fit in registers or shared memory,
+// else a cooperative grid of P CTAs.
 int launch_qr_panel(double* a, long long lda, int m, int k0, int kb, double* tau, int P, int cluster_max,
-                    void* scratch, int* status, cudaStream_t st) {
-    // one CTA per 64 rows, up to the largest cluster (measured against 128
-    // rows per CTA: 13.8 vs 14.2 ms at 2048^2, 32.6 vs 33.0 at 4096^2)
-    const int cl = max(1, min((m - k0) / 64, min(cluster_max, qr::CL_MAX)));
-    const int rows = (m - k0 + cl - 1) / cl;
+                    void* scratch, int* status, bool withhold, cudaStream_t st) {
+    const int cl = qr::panel_ctas(m, k0, cluster_max), rows = (m - k0 + cl - 1) / cl;
     // rows in registers while every CTA has at most 256 (3.2 us per column at 4000 rows, against 6.8
     // with the slab in shared memory and 9.4 on the grid)
-    if (rows <= 32 * qr::RG_MAX_NR) {
+    if (qr_panel_waits(m, k0, cluster_max)) {
         using namespace qr;
-        static void (*const kerns[RG_MAX_NR + 1])(double*, long long, int, int, int, double*, int*) = {
+        static void (*const kerns[RG_MAX_NR + 1])(double*, long long, int, int, int, double*, int*, int) = {
             nullptr,
             qr_panel_rg_kernel<1>, qr_panel_rg_kernel<2>, qr_panel_rg_kernel<3>, qr_panel_rg_kernel<4>,
             qr_panel_rg_kernel<5>, qr_panel_rg_kernel<6>, qr_panel_rg_kernel<7>, qr_panel_rg_kernel<8>};
@@ -1319,7 +1342,9 @@ int launch_qr_panel(double* a, long long lda, int m, int k0, int kb, double* tau
         at[1] = chained_launch();
         cfg.attrs = at;
         cfg.numAttrs = 2;
-        return cudaLaunchKernelEx(&cfg, kern, a, lda, m, k0, kb, tau, status) == cudaSuccess ? JLC_OK : JLC_E_LAUNCH;
+        return cudaLaunchKernelEx(&cfg, kern, a, lda, m, k0, kb, tau, status, withhold ? 1 : 0) == cudaSuccess
+                   ? JLC_OK
+                   : JLC_E_LAUNCH;
     }
     if ((size_t)((m - k0 + cl - 1) / cl) * kb * sizeof(double) <= (size_t)qr::CL_MAX_SLAB_BYTES) {
         const void* kern = (const void*)qr::qr_panel_cl_kernel;

@@ -15,6 +15,8 @@ the caller falls back; the next call works.  Here:
   * the same hook on a grouped plan: CTA 0 of the 64 x 64 tile kernel leaves
     one slot's copies unreported, every warp's bounded wait ends, the run
     reports JLC_E_TIMEOUT, and the plan runs correctly afterwards;
+  * and on the factorisations' kernels: one sum is not sent, and every CTA that
+    waits for it ends;
   * JLCGPU_FAULT arms the same hook when a context is created.
 """
 import os
@@ -170,6 +172,48 @@ def test_split_product_recovers(ctx, oracle):
                 assert torch.equal(product(j), before[j]), (i, j)
     finally:
         ctx.set_wait_limit(0.0)
+
+
+@pytest.mark.parametrize("kind,m,n", [
+    ("qr", 64, 64), ("qr", 2304, 200),         # one CTA; a cluster of 16
+    ("hessenberg", 8, 8), ("hessenberg", 600, 600),
+    ("bidiag", 8, 5), ("bidiag", 300, 200),    # one CTA; rows in shared memory
+    ("bidiag", 2300, 2100),                    # and in the work array
+])
+def test_factorisation_wait_runs_out(ctx, oracle, kind, m, n):
+    """One sum of the first step is not sent: every CTA that waits for it gives
+    up at the limit, the call reports JLC_E_TIMEOUT, and the next one returns
+    the bits it returned before."""
+    import torch
+    from jlc_b200 import JlcError
+    a = torch.from_numpy(oracle.uniform((n, m), 1591 + m)).cuda()
+    new = lambda *shape: torch.zeros(*shape, dtype=torch.float64, device="cuda")  # noqa: E731
+
+    def run():
+        f, x, y, q = a.clone(), new(n), new(n), new(n, n)
+        torch.cuda.synchronize()
+        if kind == "qr":
+            ctx.qr_factor_device(m, n, f.data_ptr(), m, x.data_ptr())
+        elif kind == "hessenberg":
+            ctx.hessenberg_device(n, f.data_ptr(), n, q.data_ptr(), n)
+        else:
+            ctx.bidiag_device(m, n, f.data_ptr(), m, x.data_ptr(), y.data_ptr(), None, m, q.data_ptr(), n)
+        return f, x, y, q
+
+    first = run()
+    ctx.set_wait_limit(0.05)
+    try:
+        ctx.inject_fault(WAIT, 0)
+        t0 = time.perf_counter()
+        with pytest.raises(JlcError) as exc:
+            run()
+        elapsed = time.perf_counter() - t0
+        assert exc.value.code == E_TIMEOUT, exc.value
+        assert elapsed < 2.0, f"the wait ran {elapsed:.2f} s: the 50 ms limit was not applied"
+    finally:
+        ctx.set_wait_limit(0.0)
+    for x, y in zip(run(), first):
+        assert torch.equal(x, y)
 
 
 def test_timeout_through_the_host_entry_returns_false(oracle):
