@@ -1297,8 +1297,11 @@ int jlc_hessenberg_device(jlc_ctx* ctx, int64_t n, double* a, int64_t lda, doubl
     cudaStream_t st = ctx->stream;
     cudaEventRecord(ctx->ev0, st);
     int rc = JLC_OK;
-    if (q && (rc = launch_set_identity(q, ldq, n, n, st))) return set_err(ctx, rc, "Hessenberg: identity launch failed");
-    if (n > 2 && hess_slab_fits((int)n, ctx->sm_count)) {
+    const bool slab = n > 2 && hess_slab_fits((int)n, ctx->sm_count);
+    // (the Q builder behind the one-launch reduction starts from an identity of its own)
+    if (q && !slab && (rc = launch_set_identity(q, ldq, n, n, st)))
+        return set_err(ctx, rc, "Hessenberg: identity launch failed");
+    if (slab) {
         // the whole reduction in one launch, then Q from the reflectors below the subdiagonal
         const long long ldt = round_up(n, 8);
         if ((rc = reserve(ctx, ctx->bufH, (ldt + hess_slab_work_doubles((int)n, ctx->sm_count)) * sizeof(double),
