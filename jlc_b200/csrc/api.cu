@@ -744,9 +744,10 @@ int qr_work(jlc_ctx* ctx, long long m, long long cols, long long panels, QrWork&
 int qr_panels_vt(jlc_ctx* ctx, const double* f, long long ldf, long long m, long long kmax, long long p0, int panels,
                  int shift, const double* tau, bool trans, const QrWork& q) {
     Phase ph(ctx, JLC_PHASE_QR_VT);
-    ctx->launches += 2;
+    int nl = 0;
     const int rc = launch_qr_vt(f, ldf, (int)m, (int)kmax, (int)p0, panels, shift, tau, q.v, q.ldv, q.t, q.vt, trans,
-                                q.gram, ctx->qr_cluster_max, ctx->sm_count, ctx->stream);
+                                q.gram, ctx->qr_cluster_max, ctx->sm_count, ctx->stream, &nl);
+    ctx->launches += nl;
     return rc ? set_err(ctx, rc, "QR: V / T launch failed") : JLC_OK;
 }
 

@@ -90,11 +90,11 @@ int qr_panel_cluster_max();
 int launch_qr_panel(double* a, long long lda, int m, int k0, int kb, double* tau, int P, int cluster_max,
                     void* scratch, int* status, bool withhold, cudaStream_t st);
 bool qr_panel_waits(int m, int k0, int cluster_max);  // whether launch_qr_panel takes the kernel that has the test hook
-// V, T and V op(T) of consecutive panels; gram holds qr_gram_scratch_bytes(sm_count)
+// V, T and V op(T) of consecutive panels (*launches: kernels launched); gram holds qr_gram_scratch_bytes(sm_count)
 size_t qr_gram_scratch_bytes(int sm_count);
 int launch_qr_vt(const double* a, long long lda, int m, int kmax, int p0, int panels, int shift, const double* tau,
                  double* v, long long ldv, double* t, double* vt, bool trans, double* gram, int cluster_max,
-                 int sm_count, cudaStream_t st);
+                 int sm_count, cudaStream_t st, int* launches);
 int launch_set_identity(double* q, long long ldq, long long m, long long cols, cudaStream_t st);
 // blocked Hessenberg reduction kernels (hess.cu)
 size_t hess_work_doubles(long long n);

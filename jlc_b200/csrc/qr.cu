@@ -1408,9 +1408,10 @@ size_t qr_gram_scratch_bytes(int sm_count) {
 // panel p0 + i's at v + i 64 ldv, t + i 64^2 and vt + i 64 ldv.
 int launch_qr_vt(const double* a, long long lda, int m, int kmax, int p0, int panels, int shift, const double* tau,
                  double* v, long long ldv, double* t, double* vt, bool trans, double* gram, int cluster_max,
-                 int sm_count, cudaStream_t st) {
+                 int sm_count, cudaStream_t st, int* launches) {
     using namespace qr;
     const int rows = m - 64 * p0;  // of the tallest panel
+    *launches = rows <= VT_MAX_ROWS ? 2 : 4 * panels + 1;
     if (rows <= VT_MAX_ROWS) {
         cudaLaunchConfig_t cfg = {};
         cudaLaunchAttribute at[2];

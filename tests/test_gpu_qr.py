@@ -331,3 +331,18 @@ def test_q_with_little_room(ctx, oracle):
         c3.close()
     finally:
         c2.close()
+
+
+def test_launch_count_of_tall_panels(ctx):
+    """One panel of Q takes two launches for V, T and V T, and five above 4096
+    rows, beside the same two GEMMs."""
+    import torch
+    counts = []
+    for m in (4000, 4200):
+        f, tau = torch.full((64, m), 0.01, dtype=torch.float64, device="cuda"), torch.ones(64, dtype=torch.float64).cuda()
+        q = torch.zeros(64, m, dtype=torch.float64, device="cuda")
+        torch.cuda.synchronize()
+        before = ctx.launch_count()
+        ctx.qr_build_q_device(m, 64, 64, f.data_ptr(), m, tau.data_ptr(), q.data_ptr(), m)
+        counts.append(ctx.launch_count() - before)
+    assert counts[1] - counts[0] == 3
