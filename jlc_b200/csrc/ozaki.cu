@@ -111,18 +111,18 @@ constexpr int kModeCert = 2;    // accuracy certificate: one product of the magn
 // 2600 (one tile per pair) 232 -> 201, 3000 x 2304 x 2600 400 -> 350, 4096 x 4096 x
 // 2048 664 -> 565, 4096^3 852 -> 823; certificate 3000 x 2304 x 2600 64 -> 45, 8192^3
 // 379 -> 338.  Where the MMAs of many long tiles hide the epilogue the GEMM runs at
-// the power cap and 8 warps are as fast or faster (6144 x 6144 x 8192 2887 against
-// 2893, 8192^3 5053 against 5095).  The slice epilogue holds FP64 sums in 166
-// registers and keeps 8.
-template <int EW>
+// the power cap, and 8 and 16 are equal to within what runs differ by (three runs
+// each, in turn: 6144 x 6144 x 7000 3244-3411 and 3215-3425, 8192^3 6859-7181 and
+// 6703-7191, 8192 x 8192 x 4096 3713-3989 and 3575-3594).  The slice epilogue holds
+// FP64 sums in 166 registers and keeps 8.
+template <int MODE>
 struct Epi {
-    static constexpr int PARTS = EW / 4;    // warps that share a lane quarter split the columns
+    static constexpr int WARPS = MODE == kModeSlices ? 8 : 16;
+    static constexpr int PARTS = WARPS / 4;    // warps that share a lane quarter split the columns
     static constexpr int COLS = BN / PARTS;  // columns per warp
-    static constexpr int THREADS = 64 + 32 * EW;
+    static constexpr int THREADS = 64 + 32 * WARPS;
     static constexpr int RECON_GROUPS = COLS / 4;  // groups of 4 columns per thread and tile
 };
-// epilogue warps of the residue GEMM
-static int crt_epi_warps(long long tiles, int pairs, long long k) { return k > 6144 && tiles > 4LL * pairs ? 8 : 16; }
 
 // Route decision of the certificate (kModeCert), made by the CTA that
 // finishes last.  For a level (slice or modulus count) the certified ratio is
@@ -221,13 +221,13 @@ __device__ __forceinline__ void cert_decide(const Params& p) {
     __threadfence();
 }
 
-template <int MODE, int EPI_WARPS>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(Epi<EPI_WARPS>::THREADS, 1)
+template <int MODE>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(Epi<MODE>::THREADS, 1)
     ozaki_gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB,
                       const Params p) {
     constexpr bool CRT = MODE == kModeCrt;
     constexpr bool CERT = MODE == kModeCert;
-    constexpr int COLS = Epi<EPI_WARPS>::COLS, RECON_GROUPS = Epi<EPI_WARPS>::RECON_GROUPS;
+    constexpr int EPI_WARPS = Epi<MODE>::WARPS, COLS = Epi<MODE>::COLS, RECON_GROUPS = Epi<MODE>::RECON_GROUPS;
     // both CTAs of a pair read the same flags, so both leave here or neither
     if ((p.flags[kFlagNonfiniteA] | p.flags[kFlagNonfiniteB]) != 0) return;
     if (p.route_want >= 0 && p.flags[kFlagRoute] != p.route_want) return;
@@ -1245,18 +1245,15 @@ static int launch_mode(int mode, const GemmDesc& g, const OzakiBufs& b, int coun
         p.dot_partials = g.dot_partials;
     }
     if (mode == kModeCrt) crt_constants(count, g.k, p.crt);
-    const int ew = mode == kModeSlices ? 8 : mode == kModeCert ? 16 : crt_epi_warps(b.tiles_m * b.tiles_n, b.grid / 2, g.k);
-    auto kern = mode == kModeSlices ? ozaki_gemm_kernel<kModeSlices, 8>
-                : mode == kModeCert ? ozaki_gemm_kernel<kModeCert, 16>
-                : ew == 16          ? ozaki_gemm_kernel<kModeCrt, 16>
-                                    : ozaki_gemm_kernel<kModeCrt, 8>;
+    auto kern = mode == kModeSlices ? ozaki_gemm_kernel<kModeSlices>
+                : mode == kModeCert ? ozaki_gemm_kernel<kModeCert>
+                                    : ozaki_gemm_kernel<kModeCrt>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
     if (e != cudaSuccess) {
         snprintf(err, errlen, "Ozaki smem attribute: %s", cudaGetErrorString(e));
         return JLC_E_LAUNCH;
     }
-    const int threads = ew == 16 ? Epi<16>::THREADS : Epi<8>::THREADS;
-    kern<<<b.grid, threads, SMEM_BYTES, st>>>(ma, mb, p);
+    kern<<<b.grid, mode == kModeSlices ? Epi<kModeSlices>::THREADS : Epi<kModeCrt>::THREADS, SMEM_BYTES, st>>>(ma, mb, p);
     e = cudaGetLastError();
     if (e != cudaSuccess) {
         snprintf(err, errlen, "Ozaki GEMM launch failed: %s", cudaGetErrorString(e));
