@@ -93,7 +93,9 @@ JLC_API void jlc_destroy(jlc_ctx* ctx);
 /* message of the last failing call on this context ("" if none) */
 JLC_API const char* jlc_last_error(const jlc_ctx* ctx);
 /* run this context's device work on a caller-supplied cudaStream_t (NULL:
- * back to the context's own stream) */
+ * back to the context's own stream).  It neither waits for the work on the
+ * stream before nor orders the new one behind it: the context's workspace and
+ * buffers serve one call at a time, so the caller orders the two streams. */
 JLC_API int jlc_set_stream(jlc_ctx* ctx, void* cuda_stream);
 JLC_API int jlc_synchronize(jlc_ctx* ctx);
 /* page-lock caller memory (e.g. an OffHeapMatrix segment) so host entries

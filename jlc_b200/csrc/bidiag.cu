@@ -53,7 +53,7 @@
 //   slots instead of barriers                    5.4     11.4       -     227
 //   the same in 43 KB of code                    3.1      7.1      13.4   191
 //   one pass for A r and its norm, few polls,
-//   3 columns per thread (this kernel)           2.4      5.3       8.8   183
+//   3 columns per thread (this kernel)           2.4      5.3       8.8   166
 // U and V are formed afterwards from the stored reflectors by the blocked
 // compact-WY Q builder of the QR route (GEMM kernels).
 //

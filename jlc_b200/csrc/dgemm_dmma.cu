@@ -456,11 +456,12 @@ constexpr Tile kTiles[] = {{128, 128}, {128, 64}, {64, 128}, {64, 64}, {32, 128}
 // parts: waves of the persistent grid, each of a unit's k-blocks (an area's
 // worth of MMAs at 0.88 of the DMMA rate and the ring's hand-over), its
 // epilogue, and with a split the partial tile's trip through L2.  Fitted to a
-// sweep of all tiles and splits over products from 32 x 32 x 4096 to 4096 x
-// 4096 x 256 on B200; the shape it picks is within 3 % of the best of the sweep,
-// in us (128 x 128 tiles with their best split -> this rule): 96 x 80 x 112
-// 23.6 -> 8.9, 256^3 47 -> 10, 512^3 54 -> 17, 700^3 70 -> 33, 1024^3 93 -> 84,
-// 2048^3 597 -> 569, 32 x 32 x 4096 93 -> 15, 64 x 2048 x 2304 63 -> 33.
+// sweep of all tiles and splits on B200.  Over 16 products from 96 x 80 x 112 to
+// 8192 x 256 x 8192 (profiles/dgemm_tiles.txt) its pick is within 3.5 % of the
+// best and but for one at it, in us (128 x 128 tiles with their best split ->
+// this rule): 96 x 80 x 112 23.4 -> 6.3, 256^3 48 -> 10, 512^3 53 -> 17, 700^3
+// 68 -> 33, 1024^3 93 -> 85, 2048^3 596 -> 567, 32 x 32 x 4096 93 -> 15, 64 x
+// 2048 x 2304 62 -> 33.
 double tile_cost(const Tile& t, long long m, long long n, long long k, int s, int sm_count) {
     const long long tiles = ((m + t.bm - 1) / t.bm) * ((n + t.bn - 1) / t.bn);
     const long long kbl = (k + dmma::BK - 1) / dmma::BK, part = (kbl + s - 1) / s;

@@ -27,6 +27,7 @@ constexpr int GEMV_AXPY_CTAS = 8;  // resident CTAs per SM (axpy form)
 // at last the columns are split over CTAs.  us before -> after, A row-major:
 // 16384^2 371 -> 335 (6.4 TB/s), 4096 x 8192 145 -> 44, 512 x 16384 293 -> 16;
 // column-major: 16384^2 457 -> 316, 2000 x 16000 67 -> 49, 512 x 16384 60 -> 26.
+// (16384^2 by rows is 1024 CTAs, 6.9 per SM and four of them resident.)
 struct GemvShape {
     int rows_per_warp;  // dot form: 4, 2 or 1
     int wk;             // warps that share a row group and split its columns (1, 2, 4, 8)
@@ -196,7 +197,8 @@ GemvShape gemv_shape(const GemvDesc& g, int sm_count) {
     GemvShape s{4, 1, 1, g.cols};
     if (g.cs == 1) {
         auto ctas = [&] { return (g.rows * s.wk + (long long)GEMV_WARPS * s.rows_per_warp - 1) / (GEMV_WARPS * s.rows_per_warp); };
-        // a warp keeps at least one trip (512 / rows_per_warp columns) of its rows
+        // A warp keeps at least 128 columns, a trip at four rows.  With fewer rows a trip is 256 or 512
+        // columns, and the last warps of a short row have none (512 x 1024: two of eight have).
         while (ctas() < target && s.wk < GEMV_WARPS && g.cols >= 2 * s.wk * 128) s.wk *= 2;
         while (ctas() < target && s.rows_per_warp > 1) s.rows_per_warp /= 2;
         const long long most = g.cols / (512 * s.wk);  // chunks of at least 512 columns per warp

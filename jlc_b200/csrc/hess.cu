@@ -339,7 +339,7 @@ __global__ void __launch_bounds__(PT, 1) hess_panel_kernel(const PanelArgs p) {
 // takes 4.0 us at n = 1024 and 3.2 us at n = 128.  The panel route pays two
 // grid barriers and a GEMV from L2 per reflector (15 us at n = 1024), six GEMMs
 // per panel, and 107 KB of straight-line code per reflector against 34 KB
-// here.  Measured on B200, H and Q, ms: n = 1024 20.9 -> 4.6.
+// here.  Measured on B200, H and Q, ms: n = 1024 20.9 -> 4.5.
 constexpr int SLT = 512;  // threads per CTA
 constexpr int SLW = SLT / 32;
 constexpr int RC = 8;     // rows per register block: a CTA holds a multiple of RC rows
@@ -664,7 +664,8 @@ static size_t slab_slots(int n, int P) {
 
 // Whether an n x n reduction runs in the one-launch kernel: its rows fit in the
 // shared memory of the chip (n up to 1 744 on 148 SMs).  It is the faster route
-// wherever it fits (n = 1744: 14.9 ms with Q against 38.9 ms on the panel route; n = 64: 0.33 against 1.02).
+// wherever it fits (n = 1744: 13.3 ms with Q against
+// 38.9 ms on the panel route; n = 64: 0.33 against 1.02).
 bool hess_slab_fits(int n, int sm_count) {
     using namespace hess;
     const int rows = slab_rows(n, sm_count);

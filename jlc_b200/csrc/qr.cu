@@ -658,7 +658,7 @@ __global__ void __launch_bounds__(CL_THREADS, 1) qr_panel_cl_kernel(double* A, l
 // next pivot column (800), the dots (300); no pass touches shared memory but
 // for the pivot column.  The shared-memory cluster kernel walks its slab three
 // times per column between five CTA barriers and a cluster barrier, in 53 KB of
-// code.  us per column on B200: 2304 rows 5.7 -> 2.3, 1024 rows 5.1 -> 1.9.
+// code.  us per column on B200: 2304 rows 5.7 -> 2.3, 1024 rows 5.1 -> 2.0.
 constexpr int RG_THREADS = 512, RG_WARPS = RG_THREADS / 32;
 constexpr int RG_MAX = 16;              // CTAs of the cluster
 constexpr int RG_COLS = 64 / RG_WARPS;  // columns per warp
@@ -1319,7 +1319,7 @@ bool qr_panel_waits(int m, int k0, int cluster_max) {
 int launch_qr_panel(double* a, long long lda, int m, int k0, int kb, double* tau, int P, int cluster_max,
                     void* scratch, int* status, bool withhold, cudaStream_t st) {
     const int cl = qr::panel_ctas(m, k0, cluster_max), rows = (m - k0 + cl - 1) / cl;
-    // rows in registers while every CTA has at most 256 (3.2 us per column at 4000 rows, against 6.8
+    // rows in registers while every CTA has at most 256 (3.0 us per column at 4000 rows, against 6.8
     // with the slab in shared memory and 9.4 on the grid)
     if (qr_panel_waits(m, k0, cluster_max)) {
         using namespace qr;
